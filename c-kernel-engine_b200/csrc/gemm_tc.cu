@@ -16,25 +16,31 @@
 //
 // Two kernels:
 //  * gemm_x_tiles_kernel expands the Q8_K activations once into fp16 operand tiles in the exact shared-memory
-//    layout of the MMA (K-major, no swizzle, 8 x 16-byte core matrices), one contiguous blob per (128-token tile,
+//    layout of the MMA (K-major, no swizzle, 8 x 16-byte core matrices), one contiguous blob per (token tile,
 //    superblock), so the GEMM fetches them with plain 1-D bulk copies.
-//  * gemm_kq_tc_kernel<WF>: one CTA owns 128 weight rows (the M = 128 operand, one TMEM lane each) and one 128-token
-//    tile (the N = 128 operand, TMEM columns; fewer tokens are zero-padded).  Warp-specialised, 20 warps:
-//        warp 0       loader: bulk copies of activation k-stages (and of the bsum tile / block scales of each superblock)
+//  * gemm_kq_tc_kernel<WF, NT>: one CTA owns 128 weight rows (the M = 128 operand, one TMEM lane each) and one tile of NT tokens
+//    (the N operand, TMEM columns; fewer tokens are zero-padded).  Warp-specialised:
+//        warp 0       loader of activations: bulk copies of 128-deep stages, of the bsum tile and of the block scales of each superblock
 //        warp 1       issuer: tcgen05.mma from one elected lane; tcgen05.commit frees stages and publishes accumulators
-//        warps 4-11   two expander warpgroups: weights -> fp16 operand tiles, alternate k-stages (Q4_K) or halves (Q6_K)
-//        warps 12-19  drain: tcgen05.ld of T|T2 (two TMEM buffers, 512 columns), fp32 sums in registers
-//    One ring of 6 stages carries both operands of a 64-deep k-stage.  A stage has ONE "full" barrier (4 expander
-//    warps + the loader's expect_tx arrival + the copy's bytes) and ONE "empty" barrier (a tcgen05.commit) that the
-//    loader and the expanders both wait on: the issuer's timeline is a chain of barrier waits, MMA issues and commits
-//    of roughly 100-180 cycles each, so every stage costs it one wait and one commit, not two of each.
-// Every wait is bounded; a timeout sets the device error word, the CTA drains, frees TMEM and returns.
+//        warp 2       Q4_K: the 16-deep tile of mins and the (d, dmin) pairs of a superblock
+//        warp 3       loader of weights: the raw superblocks of all 128 rows, one tiled bulk copy each (Q6_K: one per plane)
+//        warps 4-11   two expander sets, thread = row: raw bytes -> fp16 operand, alternate 64-deep k-stages
+//        warps 12-    drain: tcgen05.ld of T and T2, fp32 sums in registers
+//    Every wait is bounded; a timeout sets the device error word, the CTA drains, frees TMEM and returns.
 //
-// Measured and not kept (each correct, each 3-8 % slower than this form): 128-deep ring stages (eight MMAs per barrier round), weight
-// bytes loaded a superblock ahead into two register sets with an L2 prefetch (the expanders no longer wait for loads), two issuer
-// warps on alternate superblocks (one accumulator buffer each).  The roles are co-limited: issuer chain, expanders, drain and the
-// shared-memory data pipe (63 % busy: operand reads by the tensor core, tile writes, bulk copies) each need about a thousand cycles
-// per 128-deep step, and they share four schedulers, so relieving one of them moves the wait to the next.
+// What bounds it, and why it is split like this.  The MMAs of a superblock take 17 x 64 cycles at NT = 128.  With the expanded weights in
+// shared memory the data pipe alone would need about 3700 (uncoalesced weight loads 1536 tag cycles, operand tile written 512 and read
+// 512, activations written 512 and read 512), and the kernel took 5100.  So the expanded weights never touch shared memory: an expander
+// thread owns a row, a row is a TMEM lane, and tcgen05.st puts its 64 halves where the MMA reads its A operand.  Nor is a proxy
+// fence needed between the two.  The raw weights come as 144-byte rows by tiled copies (coalesced, and conflict-free to read at that pitch).
+// A nibble becomes a half with one AND-OR (0x6400 | n = 1024 + n, or 1024 + 16 n for the upper one) and one fused multiply-add; the halves of a
+// register are then elements 0, 2 and 1, 3 of a 4-byte word, and the activation tiles are written in that order: k is a summation index.
+// The 512 TMEM columns at NT = 128: two T buffers (256), one T2 (128), four weight stages (128).
+// A superblock now takes about 1960 cycles: issuer, expanders and drain are each busy for 1500 of them and share four schedulers.
+// Measured (28672 x 4096 Q4_K at 512 / 2048 tokens): 142 / 512 us = 847 / 940 TFLOP/s, with the operand through shared memory 268 / 1055 us; 4096 x 14336 Q6_K
+// at 512 tokens 110 us (181 before); 333 tokens of 28672 x 4096: 126 us against 205 with activations quantised.
+#include <cuda.h>
+
 #include "quant_units.cuh"
 #include "launch.h"
 #include "pdl.cuh"
@@ -43,44 +49,53 @@
 
 namespace ckb {
 
-constexpr int TC_ROWS = 128;                          // rows of either operand per MMA
-constexpr int TC_CHUNK = TC_ROWS * 16;                // one 8-element k-chunk of 128 rows: 2048 B
-constexpr int TC_STAGE = 8 * TC_CHUNK;                // 64-deep k-stage of 128 rows: 16 KB
-constexpr int TC_AUX = 2 * TC_CHUNK;                  // 16-deep tile (mins / bsums): 4 KB
+constexpr int TC_ROWS = 128;                          // rows of the weight operand per MMA
+constexpr int TC_AUX = TC_ROWS * 32;                  // 16-deep tile of the mins: 4 KB
+constexpr int TC_ASLOTS = 4, TC_BSLOTS = 4, TC_RSLOTS = 3, TC_XSLOTS = 4;   // rings: 64-deep weight stages in TMEM, 128-deep activation stages, raw
+                                                                          // superblocks, per-superblock extras (mins, bsums, scales)
+enum { TC_W_Q4K = 0, TC_W_Q6K_PLANAR = 1 };           // weight operand formats
 
-// Everything that depends on the width NT of the token tile (the N operand of the MMA).  NT = 128 is the prefill
-// shape: one CTA of 640 threads per SM.  NT = 32 is the batched-decode shape (up to 64 tokens): the activation tiles,
-// the drain and the accumulators shrink so far that two CTAs of 512 threads share an SM, and every latency of the
-// per-stage chain (weight loads, barrier waits, MMA issue, commit) is overlapped by the neighbour.
+// Activation blob of one (tile of NT tokens, superblock): four 64-deep k-stages, the 16-deep bsum tile, NT block scales.
 template <int NT>
-struct TcCfg {
-    static constexpr int STAGES = NT == 128 ? 6 : 5;          // ring depth (a stage = weight tile + activation tile)
-    static constexpr int B_CHUNK = NT * 16;                   // one 8-element k-chunk of NT tokens
-    static constexpr int B_STAGE = 8 * B_CHUNK;               // 64-deep k-stage of NT tokens
-    static constexpr int B_AUX = 2 * B_CHUNK;                 // 16-deep bsum tile
-    // activation blob of one (token tile, superblock): 4 k-stages, the bsum tile, NT block scales
-    static constexpr int XBLOB_B2 = 4 * B_STAGE, XBLOB_DX = XBLOB_B2 + B_AUX, XBLOB = XBLOB_DX + NT * 4;   // a multiple of 16
-    static constexpr int OFF_A = 0;                                      // weight tiles   [STAGES][16 KB]
-    static constexpr int OFF_B = OFF_A + STAGES * TC_STAGE;              // activation tiles
-    static constexpr int OFF_A2 = OFF_B + STAGES * B_STAGE;              // mins tiles     [2][4 KB]
-    static constexpr int OFF_B2 = OFF_A2 + 2 * TC_AUX;                   // bsum tiles     [2]
-    static constexpr int OFF_DX = OFF_B2 + 2 * B_AUX;                    // block scales   [2][NT] fp32
-    static constexpr int OFF_BAR = OFF_DX + 2 * NT * 4;
-    static constexpr int BAR_FULL = 0, BAR_EMPTY = STAGES, BAR_A2_EMPTY = 2 * STAGES, BAR_B2_EMPTY = BAR_A2_EMPTY + 2, BAR_DX_FULL = BAR_B2_EMPTY + 2,
-                         BAR_T_FULL = BAR_DX_FULL + 2, BAR_T_EMPTY = BAR_T_FULL + 2, BAR_COUNT = BAR_T_EMPTY + 2;
-    static constexpr int SMEM = OFF_BAR + BAR_COUNT * 8 + 16;
-    static constexpr int DRAIN_WARPS = NT == 128 ? 8 : 4;     // 4 TMEM lane quarters x column halves
+struct TcTile {
+    static constexpr int CHUNK = NT * 16;                     // one 8-element k-chunk of NT tokens
+    static constexpr int STAGE = 8 * CHUNK;                   // 64-deep
+    static constexpr int AUX = 2 * CHUNK;
+    static constexpr int XBLOB_B2 = 4 * STAGE, XBLOB_DX = XBLOB_B2 + AUX, XBLOB = XBLOB_DX + NT * 4;   // a multiple of 16
+};
+
+// Everything that depends on the width NT of the token tile and on the weight format.  NT = 32: the accumulators and the staging shrink so far that
+// two CTAs share an SM and each covers the other's latencies.
+template <int WF, int NT>
+struct TcCfg : TcTile<NT> {
+    static constexpr bool Q4 = WF == TC_W_Q4K;
+    // raw superblocks of 128 rows: 144-byte rows, or the planes ql | qh | scales (1024-byte aligned: they are written swizzled)
+    static constexpr int RAW_QH = TC_ROWS * 128, RAW_SC = RAW_QH + TC_ROWS * 64, RAW = Q4 ? TC_ROWS * Q4K_BYTES : RAW_SC + TC_ROWS * 16;
+    static constexpr int OFF_RAW = 0;
+    static constexpr int OFF_B = OFF_RAW + TC_RSLOTS * RAW;
+    static constexpr int OFF_A2 = OFF_B + TC_BSLOTS * 2 * TcTile<NT>::STAGE;
+    static constexpr int OFF_B2 = OFF_A2 + (Q4 ? TC_XSLOTS * TC_AUX : 0);
+    static constexpr int OFF_DX = OFF_B2 + (Q4 ? TC_XSLOTS * TcTile<NT>::AUX : 0);
+    static constexpr int OFF_DD = OFF_DX + TC_XSLOTS * NT * 4;                     // fp16 d | dmin of the rows
+    static constexpr int OFF_BAR = OFF_DD + (Q4 ? TC_XSLOTS * TC_ROWS * 4 : 0);
+    static constexpr int A_FULL = 0, A_EMPTY = A_FULL + TC_ASLOTS, B_FULL = A_EMPTY + TC_ASLOTS, B_EMPTY = B_FULL + TC_BSLOTS, R_FULL = B_EMPTY + TC_BSLOTS,
+                         R_EMPTY = R_FULL + TC_RSLOTS, X_FULL = R_EMPTY + TC_RSLOTS, X_EMPTY = X_FULL + TC_XSLOTS, T_FULL = X_EMPTY + TC_XSLOTS, T_EMPTY = T_FULL + 2,
+                         T2_EMPTY = T_EMPTY + 2, DONE = T2_EMPTY + 1, BARS = DONE + 1;
+    static constexpr int SMEM = OFF_BAR + BARS * 8 + 16;
+    static constexpr int DRAIN_WARPS = NT > 32 ? 8 : 4;       // 4 TMEM lane quarters x column halves
     static constexpr int DRAIN_COLS = NT / (DRAIN_WARPS / 4); // token columns per drain thread
-    static constexpr int THREADS = (12 + DRAIN_WARPS) * 32, CTAS_PER_SM = NT == 128 ? 1 : 2;
+    static constexpr int THREADS = (12 + DRAIN_WARPS) * 32, CTAS_PER_SM = NT > 32 ? 1 : 2;
     // Register counts per role after setmaxnreg.  setmaxnreg.inc blocks until the CTA's own pool (threads x registers
     // at launch) can supply the registers, so 128 * CTL + 256 * EXP + 32 * DRAIN_WARPS * DRAIN must not exceed
     // THREADS * LAUNCH; the launcher checks the compiled register count against LAUNCH before the first launch.
-    static constexpr int REGS_LAUNCH = NT == 128 ? 96 : 64, REGS_CTL = 32, REGS_EXP = 72, REGS_DRAIN = NT == 128 ? 152 : 80;
+    static constexpr int REGS_LAUNCH = NT > 32 ? 96 : 64, REGS_CTL = 48, REGS_EXP = 72, REGS_DRAIN = NT > 32 ? 144 : 64;
     static_assert(128 * REGS_CTL + 256 * REGS_EXP + 32 * DRAIN_WARPS * REGS_DRAIN <= THREADS * REGS_LAUNCH, "setmaxnreg targets exceed the CTA's register pool");
     static_assert(THREADS * REGS_LAUNCH * CTAS_PER_SM <= 65536, "register plan");
-    static constexpr uint32_t TMEM_COLS = NT == 128 ? 512 : 128, T_BUF = TMEM_COLS / 2, T2_OFF = NT;   // buffer u & 1 at column T_BUF * (u & 1): T at +0, T2 at +NT
+    static constexpr uint32_t TM_T2 = 2 * NT, TM_A = 3 * NT, TMEM_COLS = NT > 32 ? 512 : 256;      // T buffer u at column u * NT
+    static_assert(TM_A + 32 * TC_ASLOTS <= TMEM_COLS && CTAS_PER_SM * TMEM_COLS <= 512, "tensor memory plan");
     // instruction descriptor: f16 x f16 -> f32, both operands K-major, M = 128, N = NT
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
+    static_assert(NT % 32 == 0 && NT <= 128 && RAW % (Q4 ? 16 : 1024) == 0 && OFF_BAR % 8 == 0 && OFF_B % 128 == 0, "layout");
     static_assert(CTAS_PER_SM * (SMEM + 1024) <= 228 * 1024 && SMEM <= 227 * 1024, "shared memory plan");
 };
 
@@ -96,50 +111,109 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t chunk_b
     return d;
 }
 
-// four unsigned bytes (each < 64) -> two half2 holding 1024 + byte: 0x6400 | b is the fp16 bit pattern of 1024 + b
-__device__ __forceinline__ void bytes_to_half2_biased(uint32_t v, uint32_t &h01, uint32_t &h23)
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
+// (a & mask) | bits in one instruction
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits)
 {
-    h01 = __byte_perm(v, 0x64646464u, 0x5140);
-    h23 = __byte_perm(v, 0x64646464u, 0x7362);
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
+    return r;
 }
 
-// eight 4-bit values (two words of nibbles already masked to 0x0F0F0F0F) times an integer scale -> 8 fp16, exact:
-// (1024 + q) * sc - 1024 * sc in one fused multiply-add per pair (only the result, at most 945, is rounded)
-__device__ __forceinline__ uint4 q4_chunk_to_half(uint32_t w0, uint32_t w1, __half2 sc2, __half2 bias2)
-{
-    uint32_t h[4];
-    bytes_to_half2_biased(w0, h[0], h[1]);
-    bytes_to_half2_biased(w1, h[2], h[3]);
-    uint4 out;
-    uint32_t *o = reinterpret_cast<uint32_t *>(&out);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 r = __hfma2(*reinterpret_cast<__half2 *>(&h[i]), sc2, bias2);
-        o[i] = *reinterpret_cast<const uint32_t *>(&r);
-    }
-    return out;
-}
-
-// eight int8 -> 8 fp16, exact: (x ^ 0x80) is x + 128 as an unsigned byte; 0x6400 | that is 1152 + x
+// eight int8 -> 8 fp16, exact, in the order 0 2 1 3 4 6 5 7: (x ^ 0x80) is x + 128 as an unsigned byte; 0x6400 | that is 1152 + x
 __device__ __forceinline__ uint4 s8_chunk_to_half(uint32_t w0, uint32_t w1)
 {
-    uint32_t h[4];
-    bytes_to_half2_biased(w0 ^ 0x80808080u, h[0], h[1]);
-    bytes_to_half2_biased(w1 ^ 0x80808080u, h[2], h[3]);
     const __half2 off = __floats2half2_rn(1152.0f, 1152.0f);
-    uint4 out;
-    uint32_t *o = reinterpret_cast<uint32_t *>(&out);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&h[i]), off);
-        o[i] = *reinterpret_cast<const uint32_t *>(&r);
-    }
-    return out;
+    const uint32_t u0 = w0 ^ 0x80808080u, u1 = w1 ^ 0x80808080u;
+    return make_uint4(h2_bits(__hsub2(bits_h2(and_or(u0, 0x00FF00FFu, 0x64006400u)), off)), h2_bits(__hsub2(bits_h2(and_or(u0 >> 8, 0x00FF00FFu, 0x64006400u)), off)),
+                      h2_bits(__hsub2(bits_h2(and_or(u1, 0x00FF00FFu, 0x64006400u)), off)), h2_bits(__hsub2(bits_h2(and_or(u1 >> 8, 0x00FF00FFu, 0x64006400u)), off)));
 }
 
-__device__ __forceinline__ uint32_t tc_tile_offset(int row, int kchunk) { return (uint32_t)(kchunk * TC_CHUNK + (row >> 3) * 128 + (row & 7) * 16); }
 template <int NT>
-__device__ __forceinline__ uint32_t tc_xtile_offset(int tok, int kchunk) { return (uint32_t)(kchunk * TcCfg<NT>::B_CHUNK + (tok >> 3) * 128 + (tok & 7) * 16); }
+__device__ __forceinline__ uint32_t tc_xtile_offset(int tok, int kchunk) { return (uint32_t)(kchunk * TcTile<NT>::CHUNK + (tok >> 3) * 128 + (tok & 7) * 16); }
+
+// A operand in tensor memory (one lane per row, two k per column)
+__device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u));
+}
+// 32 columns of this warp's 32 lanes
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tc_tma(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+
+// two fp32 at a time (Blackwell's packed fp32 instructions: half the issue slots)
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi)); return r; }
+__device__ __forceinline__ uint64_t pack2f(float lo, float hi) { return pack2(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
+// The 64 weights of one row in k-stage s of a Q4_K superblock (sub-blocks 2s and 2s + 1: 32 nibble bytes) times their 6-bit scales:
+// (1024 + n) * sc - 1024 * sc and (1024 + 16 n) * sc / 16 - 64 * sc, exact: only the result (at most 945) is rounded
+__device__ __forceinline__ void q4k_expand(const uint4 &hdr, const uint4 &qa, const uint4 &qb, int s, uint32_t (&o)[32])
+{
+    uint32_t sc2, m2;
+    q4k_scales(hdr.y, hdr.z, hdr.w, s, sc2, m2);
+    const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f);
+    const __half2 s_lo = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4040)), k1024), s_hi = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4141)), k1024);
+    const __half2 b_lo = __hmul2(s_lo, __floats2half2_rn(-1024.0f, -1024.0f)), b_hi = __hmul2(s_hi, __floats2half2_rn(-64.0f, -64.0f));
+    const __half2 s_hi16 = __hmul2(s_hi, __floats2half2_rn(0.0625f, 0.0625f));
+    const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t v = w[i], v8 = v >> 8;
+        o[2 * i] = h2_bits(__hfma2(bits_h2(and_or(v, 0x000F000Fu, 0x64006400u)), s_lo, b_lo));
+        o[2 * i + 1] = h2_bits(__hfma2(bits_h2(and_or(v8, 0x000F000Fu, 0x64006400u)), s_lo, b_lo));
+        o[16 + 2 * i] = h2_bits(__hfma2(bits_h2(and_or(v, 0x00F000F0u, 0x64006400u)), s_hi16, b_hi));
+        o[16 + 2 * i + 1] = h2_bits(__hfma2(bits_h2(and_or(v8, 0x00F000F0u, 0x64006400u)), s_hi16, b_hi));
+    }
+}
+
+// The same for Q6_K: k-stage 2 n + hi holds weights 128 n + 64 hi .. + 63: nibbles `hi` of the 64 ql bytes of half n, 2-bit planes 2 hi and
+// 2 hi + 1 of its 32 qh bytes, scales 8 n + 4 hi .. + 3.  raw: the row's planes as the swizzled copies left them.
+__device__ __forceinline__ void q6k_expand(const uint8_t *raw_ql, const uint8_t *raw_qh, uint32_t scw, int row, int n, int hi, uint32_t (&o)[32])
+{
+    const __half2 c66 = __floats2half2_rn(66.0f, 66.0f);
+    uint32_t qhw[8];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {            // 64-byte swizzle: 16-byte pieces permuted by bits 1-2 of the row
+        const uint4 v = *reinterpret_cast<const uint4 *>(raw_qh + row * 64 + (((2 * n + j) ^ ((row >> 1) & 3)) << 4));
+        qhw[4 * j] = v.x >> (4 * hi); qhw[4 * j + 1] = v.y >> (4 * hi); qhw[4 * j + 2] = v.z >> (4 * hi); qhw[4 * j + 3] = v.w >> (4 * hi);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {            // 128-byte swizzle: 16-byte pieces permuted by the row's low three bits
+        const uint4 v = *reinterpret_cast<const uint4 *>(raw_ql + row * 128 + (((4 * n + j) ^ (row & 7)) << 4));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        const float scf = 16.0f * (float)(int)(int8_t)((scw >> (8 * j)) & 255u);      // 16 weights per scale = one 16-byte piece
+        const __half2 sc2 = __floats2half2_rn(scf, scf);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t nib = (w[i] >> (4 * hi)) & 0x0F0F0F0Fu, h = qhw[4 * (j & 1) + i];
+            const uint32_t q = nib | ((j < 2 ? h << 4 : h << 2) & 0x30303030u);
+            // 0x5400 | q is the fp16 bit pattern of 64 + q / 16: (q - 32) / 16 * 16 sc
+            o[8 * j + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(and_or(q, 0x00FF00FFu, 0x54005400u)), c66), sc2));
+            o[8 * j + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(and_or(q >> 8, 0x00FF00FFu, 0x54005400u)), c66), sc2));
+        }
+    }
+}
 
 // ---------------------------------------------------------------- activation tiles
 
@@ -150,10 +224,12 @@ __device__ __forceinline__ uint32_t tc_xtile_offset(int tok, int kchunk) { retur
 template <int NT>
 __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__restrict__ A_q8, uint8_t *__restrict__ xt, int M, int nb)
 {
-    using Cfg = TcCfg<NT>;
+    using Cfg = TcTile<NT>;
     constexpr int PITCH = 66;                                  // words per token in shared memory: 64 + 2, 8-byte reads two-way at worst
     __shared__ __align__(8) uint32_t q[NT * PITCH];
     const int b = blockIdx.x, mt = blockIdx.y;
+    pdl_trigger();
+    pdl_wait();
     const int kcz = 32 / (int)gridDim.z, kc0 = (int)blockIdx.z * kcz;     // this CTA's k-chunks [kc0, kc0 + kcz)
     uint8_t *blob = xt + ((size_t)mt * nb + b) * Cfg::XBLOB;
     for (int it = threadIdx.x; it < NT * kcz * 2; it += 256) {
@@ -166,7 +242,7 @@ __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__rest
     for (int it = threadIdx.x; it < NT * kcz; it += 256) {
         const int t = it % NT, kl = it / NT, kc = kc0 + kl;
         const uint2 w = *reinterpret_cast<const uint2 *>(&q[t * PITCH + 2 * kl]);
-        *reinterpret_cast<uint4 *>(blob + (kc >> 3) * Cfg::B_STAGE + tc_xtile_offset<NT>(t, kc & 7)) = s8_chunk_to_half(w.x, w.y);
+        *reinterpret_cast<uint4 *>(blob + (kc >> 3) * Cfg::STAGE + tc_xtile_offset<NT>(t, kc & 7)) = s8_chunk_to_half(w.x, w.y);
     }
     if (blockIdx.z != 0) return;
     if (threadIdx.x < 2 * NT) {
@@ -190,51 +266,52 @@ __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__rest
 
 // ---------------------------------------------------------------- GEMM
 
-// Timeline of CTA (0,0), a tuning aid compiled out by default: TC_TRACE(role, slot) stores the SM clock.
-#ifdef CKB_TC_TRACE
-__device__ long long g_tc_trace[4][1024];
-#define TC_TRACE(role, slot) do { if (blockIdx.x == 0 && blockIdx.y == 0 && (slot) < 1024) g_tc_trace[role][slot] = clock64(); } while (0)
-#else
-#define TC_TRACE(role, slot) do { } while (0)
-#endif
+template <uint32_t V> struct TcConst { static constexpr uint32_t value = V; };
+struct TcMaps { CUtensorMap w[3]; };                  // Q4_K: rows; Q6_K: planes ql, qh, scales
 
-enum { TC_W_Q4K = 0, TC_W_Q6K_PLANAR = 1 };       // weight operand formats
+// Work of a launch: units of (K slice, row tile, token tile), token tiles innermost, dealt round-robin to persistent CTAs.  A slice z takes the superblocks
+// [z * nbz, z * nbz + nbz) and writes its partial sums to C + z * cz (the launcher adds the slices up in a fixed order); a single slice writes C
+// itself, bias included.  Only the loaders and the drain know where a unit ends; the other roles see one run of superblocks, so that the next unit's
+// weights are expanded and multiplied while the last one's sums are stored (a CTA per unit spent 6 us of 23 starting and storing).
+struct TcWork {
+    int units, mtiles, ntiles, nb_row, nbz;
+    __device__ __forceinline__ int mt(int u) const { return u % mtiles; }
+    __device__ __forceinline__ int nt(int u) const { return u / mtiles % ntiles; }
+    __device__ __forceinline__ int z(int u) const { return u / mtiles / ntiles; }
+    __device__ __forceinline__ int kb0(int u) const { return z(u) * nbz; }
+    __device__ __forceinline__ int nb(int u) const { return min(nbz, nb_row - kb0(u)); }
+};
 
-// Split K: blockIdx.z takes the superblocks [z * nbz, z * nbz + nbz) and writes its partial sums to C + z * cz
-// (the launcher adds the slices up in a fixed order); a single slice writes C itself, bias included.
 template <int WF, int NT>
-__global__ void __launch_bounds__(TcCfg<NT>::THREADS, TcCfg<NT>::CTAS_PER_SM)
-gemm_kq_tc_kernel(const uint8_t *__restrict__ xt, const uint8_t *__restrict__ B, const float *__restrict__ bias, float *__restrict__ C, int ldc, size_t cz,
-                  int M, int N, int nb_row, int nbz, int *__restrict__ dev_err)
+__global__ void __launch_bounds__(TcCfg<WF, NT>::THREADS, TcCfg<WF, NT>::CTAS_PER_SM)
+gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const uint8_t *__restrict__ xt, const uint8_t *__restrict__ B, const float *__restrict__ bias,
+                  float *__restrict__ C, int ldc, size_t cz, int M, int N, int *__restrict__ dev_err)
 {
-    using Cfg = TcCfg<NT>;
-    constexpr int TC_STAGES = Cfg::STAGES, BAR_FULL = Cfg::BAR_FULL, BAR_EMPTY = Cfg::BAR_EMPTY, BAR_A2_EMPTY = Cfg::BAR_A2_EMPTY, BAR_B2_EMPTY = Cfg::BAR_B2_EMPTY,
-                  BAR_DX_FULL = Cfg::BAR_DX_FULL, BAR_T_FULL = Cfg::BAR_T_FULL, BAR_T_EMPTY = Cfg::BAR_T_EMPTY;
-    constexpr int TC_OFF_A = Cfg::OFF_A, TC_OFF_A2 = Cfg::OFF_A2, TC_OFF_DX = Cfg::OFF_DX;
-    const int kb0 = blockIdx.z * nbz, nb = min(nbz, nb_row - kb0);         // this slice: superblocks kb0 .. kb0 + nb of rows that hold nb_row
-    extern __shared__ __align__(128) uint8_t smem[];
-    const uint32_t s_base = smem_u32(smem);
-    const uint32_t sA = s_base + Cfg::OFF_A, sB = s_base + Cfg::OFF_B, sA2 = s_base + Cfg::OFF_A2, sB2 = s_base + Cfg::OFF_B2, sDX = s_base + Cfg::OFF_DX;
-    const uint32_t sBar = s_base + Cfg::OFF_BAR;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Cfg::OFF_BAR + Cfg::BAR_COUNT * 8);
-#define BAR(i) (sBar + 8u * (uint32_t)(i))
+    using Cfg = TcCfg<WF, NT>;
+    constexpr bool Q4 = Cfg::Q4;
+    uint32_t total = 0;                               // superblocks of all this CTA's units
+    for (int u = blockIdx.x; u < work.units; u += gridDim.x) total += (uint32_t)work.nb(u);
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t s_base = smem_u32(smem), s_bar = s_base + Cfg::OFF_BAR;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Cfg::OFF_BAR + Cfg::BARS * 8);
+#define BAR(i) (s_bar + 8u * (uint32_t)(i))
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n0 = blockIdx.x * TC_ROWS, mt = blockIdx.y, m0 = mt * NT;
-    const uint32_t stages = (uint32_t)nb * 4u;
 
     if (tid == 0) {
-        for (int i = 0; i < TC_STAGES; ++i) { mbar_init(BAR(BAR_FULL + i), 5); mbar_init(BAR(BAR_EMPTY + i), 1); }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(BAR(BAR_A2_EMPTY + i), 1);
-            mbar_init(BAR(BAR_B2_EMPTY + i), 1 + Cfg::DRAIN_WARPS);   // the T2 MMA (or, for Q6_K, the unit's last commit) and the drain warps
-            mbar_init(BAR(BAR_DX_FULL + i), 1);
-            mbar_init(BAR(BAR_T_FULL + i), 1);
-            mbar_init(BAR(BAR_T_EMPTY + i), Cfg::DRAIN_WARPS);
+        for (int i = 0; i < TC_ASLOTS; ++i) { mbar_init(BAR(Cfg::A_FULL + i), 4); mbar_init(BAR(Cfg::A_EMPTY + i), 1); }
+        for (int i = 0; i < TC_BSLOTS; ++i) { mbar_init(BAR(Cfg::B_FULL + i), 1); mbar_init(BAR(Cfg::B_EMPTY + i), 1); }
+        for (int i = 0; i < TC_RSLOTS; ++i) { mbar_init(BAR(Cfg::R_FULL + i), 1); mbar_init(BAR(Cfg::R_EMPTY + i), Q4 ? 9 : 8); }     // expander warps and warp 2
+        for (int i = 0; i < TC_XSLOTS; ++i) {
+            mbar_init(BAR(Cfg::X_FULL + i), Q4 ? 2 : 1);                            // loader (and its bytes), warp 2
+            mbar_init(BAR(Cfg::X_EMPTY + i), Cfg::DRAIN_WARPS + (Q4 ? 1 : 0));      // drain, T2's MMA
         }
+        for (int i = 0; i < 2; ++i) { mbar_init(BAR(Cfg::T_FULL + i), 1); mbar_init(BAR(Cfg::T_EMPTY + i), Cfg::DRAIN_WARPS); }
+        mbar_init(BAR(Cfg::T2_EMPTY), Cfg::DRAIN_WARPS);
+        mbar_init(BAR(Cfg::DONE), 1);
         mbar_fence_init();
     }
-    if (warp == 0) {
+    if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(Cfg::TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -242,6 +319,7 @@ gemm_kq_tc_kernel(const uint8_t *__restrict__ xt, const uint8_t *__restrict__ B,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_trigger();
 
 #define TC_SETMAXNREG(op, n) asm volatile("setmaxnreg." op ".sync.aligned.u32 %0;" ::"n"(n))
 #define TC_WAIT(bar, parity, code)                                        \
@@ -250,255 +328,263 @@ gemm_kq_tc_kernel(const uint8_t *__restrict__ xt, const uint8_t *__restrict__ B,
     if (warp < 4) {
         TC_SETMAXNREG("dec", Cfg::REGS_CTL);
         if (warp == 0) {
-            // ------------------------------------------------------------ loader
-            uint32_t issued = 0;
-            for (uint32_t it = 0; it < stages; ++it) {
-                const uint32_t b = it >> 2, s = it & 3u, i = it % TC_STAGES, x = b & 1u;
-                const uint8_t *blob = xt + ((size_t)mt * nb_row + kb0 + b) * Cfg::XBLOB;
-                TC_WAIT(BAR(BAR_EMPTY + i), ((it / TC_STAGES) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT);
-                if (s == 3) { TC_WAIT(BAR(BAR_B2_EMPTY + x), ((b >> 1) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT); }
-                if (tc_elect_one()) {
-                    // the bsum tile of the superblock rides on the barrier of its last k-stage (the issuer needs it for the T2 MMA
-                    // right after that stage); the block scales have their own barrier, for the drain warps
-                    const bool with_bsums = s == 3 && WF == TC_W_Q4K;
-                    mbar_arrive_expect_tx(BAR(BAR_FULL + i), Cfg::B_STAGE + (with_bsums ? Cfg::B_AUX : 0));
-                    bulk_g2s(sB + i * Cfg::B_STAGE, blob + s * Cfg::B_STAGE, Cfg::B_STAGE, BAR(BAR_FULL + i));
-                    if (with_bsums) bulk_g2s(sB2 + x * Cfg::B_AUX, blob + Cfg::XBLOB_B2, Cfg::B_AUX, BAR(BAR_FULL + i));
-                    if (s == 3) {
-                        mbar_arrive_expect_tx(BAR(BAR_DX_FULL + x), NT * 4);
-                        bulk_g2s(sDX + x * NT * 4, blob + Cfg::XBLOB_DX, NT * 4, BAR(BAR_DX_FULL + x));
-                    }
-                }
-                issued = it + 1;
-            }
-            if (issued < stages) {                     // gave up: copies still in flight must land before the CTA's shared memory goes away
-                for (uint32_t c = issued > TC_STAGES ? issued - TC_STAGES : 0; c < issued; ++c)
-                    mbar_wait_spin(BAR(BAR_FULL + c % TC_STAGES), (c / TC_STAGES) & 1u);
-            }
-        } else if (warp == 1) {
-            // ------------------------------------------------------------ issuer: the warp runs the loop and the waits uniformly
-            // (descriptors and addresses stay in uniform registers), one elected lane issues
-            const uint64_t dA = tc_smem_desc(sA, TC_CHUNK), dB = tc_smem_desc(sB, Cfg::B_CHUNK), dA2 = tc_smem_desc(sA2, TC_CHUNK), dB2 = tc_smem_desc(sB2, Cfg::B_CHUNK);
-            for (uint32_t it = 0; it < stages; ++it) {
-                const uint32_t b = it >> 2, s = it & 3u, i = it % TC_STAGES, buf = b & 1u, tacc = tmem + Cfg::T_BUF * buf;
-                if (s == 0) {
-                    TC_WAIT(BAR(BAR_T_EMPTY + buf), ((b >> 1) & 1u) ^ 1u, DEV_ERR_MMA_WAIT);
-                    tc_fence_after();                  // orders the drain's tcgen05.ld of this buffer before the MMAs that overwrite it
-                }
-                if (lane == 0) TC_TRACE(0, 3 * it + 0);
-                TC_WAIT(BAR(BAR_FULL + i), (it / TC_STAGES) & 1u, DEV_ERR_FULL_WAIT);
-                if (lane == 0) TC_TRACE(0, 3 * it + 1);
-                const uint64_t da = dA + (uint64_t)(i * (TC_STAGE >> 4)), db = dB + (uint64_t)(i * (Cfg::B_STAGE >> 4));
-                if (tc_elect_one()) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma(tacc, da + (uint64_t)(k * (2 * TC_CHUNK >> 4)), db + (uint64_t)(k * (2 * Cfg::B_CHUNK >> 4)), Cfg::IDESC, (s | (uint32_t)k) ? 1u : 0u);
-                    tc_commit(BAR(BAR_EMPTY + i));
-                    if (s == 3) {
-                        if constexpr (WF == TC_W_Q4K) {
-                            tc_mma(tacc + Cfg::T2_OFF, dA2 + (uint64_t)(buf * (TC_AUX >> 4)), dB2 + (uint64_t)(buf * (Cfg::B_AUX >> 4)), Cfg::IDESC, 0u);
-                            tc_commit(BAR(BAR_A2_EMPTY + buf));
-                        }
-                        tc_commit(BAR(BAR_B2_EMPTY + buf));
-                        tc_commit(BAR(BAR_T_FULL + buf));
-                    }
-                    TC_TRACE(0, 3 * it + 2);
-                }
-            }
-        }
-    } else if (warp < 12) {
-        // ------------------------------------------------------------ weight expanders: thread = row
-        if constexpr (Cfg::REGS_EXP < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", Cfg::REGS_EXP);
-        else TC_SETMAXNREG("inc", Cfg::REGS_EXP);
-        const int set = (warp - 4) >> 2, row = tid & 127;
-        if constexpr (WF == TC_W_Q6K_PLANAR) {
-            // set e takes half n = e of every superblock: its 64 ql bytes and 32 qh bytes feed two k-stages
-            const size_t rb = ((size_t)nb_row * Q6K_BYTES + 15) & ~(size_t)15;
-            const uint8_t *wrow = B + (size_t)min(n0 + row, N - 1) * rb;
-            const size_t off_qh = (size_t)nb_row * 128, off_sc = (size_t)nb_row * 192;
-            const __half2 c66 = __floats2half2_rn(66.0f, 66.0f);
+            // ------------------------------------------------------------ activations
+            pdl_wait();                                // the tiles are what the kernel before this one writes; weights are nobody's output
+            uint32_t g = 0, issued = 0, extras = 0;
             bool go = true;
-            for (uint32_t b = 0; b < (uint32_t)nb && go; ++b) {
-                const uint32_t n = (uint32_t)set;
-                uint4 ql[4], qh[2];
+            for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+                const uint8_t *blob = xt + ((size_t)work.mt(u) * work.nb_row + work.kb0(u)) * Cfg::XBLOB;
+                for (int nb = work.nb(u); nb > 0 && go; --nb, ++g, blob += Cfg::XBLOB) {
+                    const uint32_t x = g % TC_XSLOTS;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) ql[j] = __ldg(reinterpret_cast<const uint4 *>(wrow + (size_t)(kb0 + b) * 128 + 64 * n + 16 * j));
-#pragma unroll
-                for (int j = 0; j < 2; ++j) qh[j] = __ldg(reinterpret_cast<const uint4 *>(wrow + off_qh + (size_t)(kb0 + b) * 64 + 32 * n + 16 * j));
-                const uint2 sc8 = __ldg(reinterpret_cast<const uint2 *>(wrow + off_sc + (size_t)(kb0 + b) * 16 + 8 * n));
-                const uint32_t qlw[16] = {ql[0].x, ql[0].y, ql[0].z, ql[0].w, ql[1].x, ql[1].y, ql[1].z, ql[1].w,
-                                          ql[2].x, ql[2].y, ql[2].z, ql[2].w, ql[3].x, ql[3].y, ql[3].z, ql[3].w};
-                const uint32_t qhw[8] = {qh[0].x, qh[0].y, qh[0].z, qh[0].w, qh[1].x, qh[1].y, qh[1].z, qh[1].w};
-#pragma unroll 1
-                for (uint32_t hi = 0; hi < 2; ++hi) {
-                    const uint32_t it = 4u * b + 2u * n + hi, i = it % TC_STAGES;
-                    const uint32_t scw = hi ? sc8.y : sc8.x;       // scale groups 8n + 4hi + {0, 1, 2, 3}
-                    if (!mbar_wait_spin(BAR(BAR_EMPTY + i), ((it / TC_STAGES) & 1u) ^ 1u)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
-                    uint8_t *dst = smem + TC_OFF_A + i * TC_STAGE;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {                  // chunk c: weights (c < 4 ? ql[l] : ql[32 + l]) with l = 8 (c & 3) .. + 7
-                        const int sb = 2 * (c >> 2) + ((c & 3) >> 1);
-                        const float scf = 16.0f * (float)(int)(int8_t)((scw >> (8 * sb)) & 255u);
-                        const __half2 sc2 = __floats2half2_rn(scf, scf);
-                        uint32_t o[4];
-#pragma unroll
-                        for (int w2 = 0; w2 < 2; ++w2) {
-                            const uint32_t lw = qlw[8 * (c >> 2) + 2 * (c & 3) + w2], hw = qhw[2 * (c & 3) + w2];
-                            const uint32_t nib = (lw >> (4u * hi)) & 0x0F0F0F0Fu;
-                            const uint32_t two = ((hw >> (4u * hi + 2u * (uint32_t)(c >> 2))) << 4) & 0x30303030u;
-                            // 0x5400 | q is the fp16 bit pattern of 64 + q / 16
-                            uint32_t h01 = __byte_perm(nib | two, 0x54545454u, 0x5140), h23 = __byte_perm(nib | two, 0x54545454u, 0x7362);
-                            const __half2 r0 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h01), c66), sc2);   // (q - 32) / 16 * 16 sc
-                            const __half2 r1 = __hmul2(__hsub2(*reinterpret_cast<__half2 *>(&h23), c66), sc2);
-                            o[2 * w2] = *reinterpret_cast<const uint32_t *>(&r0);
-                            o[2 * w2 + 1] = *reinterpret_cast<const uint32_t *>(&r1);
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        const uint32_t i = 2 * (g & 1u) + h;
+                        if (!mbar_wait_spin(BAR(Cfg::B_EMPTY + i), ((g >> 1) & 1u) ^ 1u)) { go = false; break; }
+                        if (tc_elect_one()) {
+                            mbar_arrive_expect_tx(BAR(Cfg::B_FULL + i), 2 * Cfg::STAGE);
+                            bulk_g2s(s_base + Cfg::OFF_B + i * 2 * Cfg::STAGE, blob + h * 2 * Cfg::STAGE, 2 * Cfg::STAGE, BAR(Cfg::B_FULL + i));
                         }
-                        *reinterpret_cast<uint4 *>(dst + tc_tile_offset(row, c)) = make_uint4(o[0], o[1], o[2], o[3]);
+                        ++issued;
+                    }
+                    if (!go || !mbar_wait_spin(BAR(Cfg::X_EMPTY + x), ((g / TC_XSLOTS) & 1u) ^ 1u)) { go = false; break; }
+                    if (tc_elect_one()) {
+                        mbar_arrive_expect_tx(BAR(Cfg::X_FULL + x), NT * 4 + (Q4 ? Cfg::AUX : 0));
+                        bulk_g2s(s_base + Cfg::OFF_DX + x * NT * 4, blob + Cfg::XBLOB_DX, NT * 4, BAR(Cfg::X_FULL + x));
+                        if (Q4) bulk_g2s(s_base + Cfg::OFF_B2 + x * Cfg::AUX, blob + Cfg::XBLOB_B2, Cfg::AUX, BAR(Cfg::X_FULL + x));
+                    }
+                    ++extras;
+                }
+            }
+            if (!go) atomicExch(dev_err, DEV_ERR_EMPTY_WAIT);
+            // copies still in flight land before the CTA's shared memory goes away, whatever became of the roles that wait for them
+            for (uint32_t j = issued > TC_BSLOTS ? issued - TC_BSLOTS : 0; j < issued; ++j) mbar_wait_spin(BAR(Cfg::B_FULL + j % TC_BSLOTS), (j / TC_BSLOTS) & 1u);
+            for (uint32_t b = extras > TC_XSLOTS ? extras - TC_XSLOTS : 0; b < extras; ++b) mbar_wait_spin(BAR(Cfg::X_FULL + b % TC_XSLOTS), (b / TC_XSLOTS) & 1u);
+        } else if (warp == 1) {
+            // ------------------------------------------------------------ issuer: the warp runs the loop and the waits uniformly, one lane issues.  This
+            // warp is a chain of short dependent steps, and the MMAs of a 64-deep stage take 256 cycles: two superblocks are unrolled so that
+            // slots, descriptors and most parities are constants (with them computed in a loop of stages the chain took 900 cycles a stage).
+            const uint64_t dB = tc_smem_desc(s_base + Cfg::OFF_B, Cfg::CHUNK), dA2 = tc_smem_desc(s_base + Cfg::OFF_A2, TC_ROWS * 16), dB2 = tc_smem_desc(s_base + Cfg::OFF_B2, Cfg::CHUNK);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const bool leader = tc_elect_one();
+            auto superblock = [&](auto odd, uint32_t b) -> bool {
+                constexpr uint32_t u = decltype(odd)::value;
+                const uint32_t p = (b >> 1) & 1u, x [[maybe_unused]] = b % TC_XSLOTS;
+                if (!mbar_wait_spin(BAR(Cfg::T_EMPTY + u), p ^ 1u)) return false;
+#pragma unroll
+                for (uint32_t s = 0; s < 4; ++s) {
+                    constexpr uint32_t half = Cfg::STAGE >> 4;
+                    const uint32_t i = 2 * u + (s >> 1);
+                    if (!(s & 1u) && !mbar_wait_spin(BAR(Cfg::B_FULL + i), p)) return false;
+                    if (!mbar_wait_spin(BAR(Cfg::A_FULL + s), u)) return false;
+                    tc_fence_after();                  // the expanders' stores, and (s = 0) the drain's loads of this accumulator, come before these MMAs
+                    if (leader) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k)
+                            tc_mma_ta(tm + NT * u, tm + Cfg::TM_A + 32 * s + 8 * k, dB + (uint64_t)(half * (2 * i + (s & 1u)) + k * (2 * Cfg::CHUNK >> 4)), Cfg::IDESC, (s | k) ? 1u : 0u);
+                        tc_commit(BAR(Cfg::A_EMPTY + s));
+                        if (s & 1u) tc_commit(BAR(Cfg::B_EMPTY + i));
+                    }
+                    __syncwarp();
+                }
+                if constexpr (Q4) {
+                    if (!mbar_wait_spin(BAR(Cfg::T2_EMPTY), u ^ 1u) || !mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) return false;
+                    tc_fence_after();
+                }
+                if (leader) {
+                    if constexpr (Q4) {
+                        tc_mma(tm + Cfg::TM_T2, dA2 + (uint64_t)(x * (TC_AUX >> 4)), dB2 + (uint64_t)(x * (Cfg::AUX >> 4)), Cfg::IDESC, 0u);
+                        tc_commit(BAR(Cfg::X_EMPTY + x));
+                    }
+                    tc_commit(BAR(Cfg::T_FULL + u));
+                }
+                __syncwarp();
+                return true;
+            };
+            for (uint32_t b = 0; b < total; b += 2)
+                if (!superblock(TcConst<0>(), b) || (b + 1 < total && !superblock(TcConst<1>(), b + 1))) {
+                    atomicExch(dev_err, DEV_ERR_MMA_WAIT);
+                    break;
+                }
+            if (leader) tc_commit(BAR(Cfg::DONE));          // MMAs in flight finish before the tensor memory is freed
+            mbar_wait_spin(BAR(Cfg::DONE), 0);
+        } else if (warp == 2) {
+            // ------------------------------------------------------------ Q4_K: mins (each doubled: bsums come per 16 elements) and block scales
+            if constexpr (Q4) {
+                for (uint32_t b = 0; b < total; ++b) {
+                    const uint32_t r = b % TC_RSLOTS, x = b % TC_XSLOTS;
+                    TC_WAIT(BAR(Cfg::X_EMPTY + x), ((b / TC_XSLOTS) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT);
+                    TC_WAIT(BAR(Cfg::R_FULL + r), (b / TC_RSLOTS) & 1u, DEV_ERR_FULL_WAIT);
+#pragma unroll 1
+                    for (int row = lane; row < TC_ROWS; row += 32) {
+                        const uint4 hdr = *reinterpret_cast<const uint4 *>(smem + Cfg::OFF_RAW + r * Cfg::RAW + row * Q4K_BYTES);
+                        const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f);
+                        uint32_t o[8];
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) {
+                            uint32_t sc2, m2;
+                            q4k_scales(hdr.y, hdr.z, hdr.w, s, sc2, m2);
+                            o[2 * s] = h2_bits(__hsub2(bits_h2(__byte_perm(m2, 0x64646464u, 0x4040)), k1024));
+                            o[2 * s + 1] = h2_bits(__hsub2(bits_h2(__byte_perm(m2, 0x64646464u, 0x4141)), k1024));
+                        }
+                        uint8_t *a2 = smem + Cfg::OFF_A2 + x * TC_AUX + (row >> 3) * 128 + (row & 7) * 16;
+                        *reinterpret_cast<uint4 *>(a2) = make_uint4(o[0], o[1], o[2], o[3]);
+                        *reinterpret_cast<uint4 *>(a2 + TC_ROWS * 16) = make_uint4(o[4], o[5], o[6], o[7]);
+                        *reinterpret_cast<uint32_t *>(smem + Cfg::OFF_DD + (x * TC_ROWS + row) * 4) = hdr.x;
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
+                    __threadfence_block();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(BAR(BAR_FULL + i));
+                    if (lane == 0) { mbar_arrive(BAR(Cfg::X_FULL + x)); mbar_arrive(BAR(Cfg::R_EMPTY + r)); }
                 }
             }
         } else {
-            // set e takes the k-stages (quarters of a superblock) it = e, e + 2, ...
-            const uint8_t *wrow = B + ((size_t)min(n0 + row, N - 1) * nb_row + kb0) * Q4K_BYTES;
-            uint4 cur_a, cur_b, hdr;
-            {
-                const uint8_t *p0 = wrow + 16 + 32 * set;
-                cur_a = __ldg(reinterpret_cast<const uint4 *>(p0));
-                cur_b = __ldg(reinterpret_cast<const uint4 *>(p0 + 16));
-                hdr = __ldg(reinterpret_cast<const uint4 *>(wrow));
+            // ------------------------------------------------------------ raw weights
+            uint32_t issued = 0, r = 0, ph = 1;
+            bool go = true;
+            for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+                const int n0 = work.nt(u) * TC_ROWS, kb0 = work.kb0(u), end = kb0 + work.nb(u);
+                for (int kb = kb0; kb < end; ++kb) {
+                    if (!mbar_wait_spin(BAR(Cfg::R_EMPTY + r), ph)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
+                    if (tc_elect_one()) {
+                        const uint32_t dst = s_base + Cfg::OFF_RAW + r * Cfg::RAW;
+                        mbar_arrive_expect_tx(BAR(Cfg::R_FULL + r), Cfg::RAW);
+                        if constexpr (Q4) {
+                            tc_tma(dst, &maps.w[0], kb * Q4K_BYTES, n0, BAR(Cfg::R_FULL + r));
+                        } else {
+                            tc_tma(dst, &maps.w[0], kb * 128, n0, BAR(Cfg::R_FULL + r));
+                            tc_tma(dst + Cfg::RAW_QH, &maps.w[1], kb * 64, n0, BAR(Cfg::R_FULL + r));
+                            tc_tma(dst + Cfg::RAW_SC, &maps.w[2], kb * 16, n0, BAR(Cfg::R_FULL + r));
+                        }
+                    }
+                    ++issued;
+                    if (++r == TC_RSLOTS) { r = 0; ph ^= 1u; }
+                }
             }
-            for (uint32_t it = (uint32_t)set; it < stages; it += 2) {
-                const uint32_t b = it >> 2, s = it & 3u, i = it % TC_STAGES, x2 = b & 1u;
-                uint4 nxt_a = cur_a, nxt_b = cur_b, hdr_next = hdr;
-                if (it + 2 < stages) {                    // this thread's next quarter, possibly of the next superblock
-                    const uint8_t *pn = wrow + (size_t)((it + 2) >> 2) * Q4K_BYTES;
-                    nxt_a = __ldg(reinterpret_cast<const uint4 *>(pn + 16 + 32 * ((it + 2) & 3u)));
-                    nxt_b = __ldg(reinterpret_cast<const uint4 *>(pn + 32 + 32 * ((it + 2) & 3u)));
-                    if (((it + 2) >> 2) != b) hdr_next = __ldg(reinterpret_cast<const uint4 *>(pn));
+            for (uint32_t b = issued > TC_RSLOTS ? issued - TC_RSLOTS : 0; b < issued; ++b) mbar_wait_spin(BAR(Cfg::R_FULL + b % TC_RSLOTS), (b / TC_RSLOTS) & 1u);
+        }
+    } else if (warp < 12) {
+        // ------------------------------------------------------------ weight expanders: thread = row = TMEM lane; set e takes the k-stages e and e + 2
+        if constexpr (Cfg::REGS_EXP < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", Cfg::REGS_EXP);
+        else TC_SETMAXNREG("inc", Cfg::REGS_EXP);
+        const int set = (warp - 4) >> 2, row = tid & 127;
+        const uint32_t ta = tmem + Cfg::TM_A + ((uint32_t)(row & 96) << 16);
+        bool go = true;
+        for (uint32_t b = 0; b < total && go; ++b) {
+            const uint32_t r = b % TC_RSLOTS;
+            const uint8_t *raw = smem + Cfg::OFF_RAW + r * Cfg::RAW;
+            TC_WAIT(BAR(Cfg::R_FULL + r), (b / TC_RSLOTS) & 1u, DEV_ERR_FULL_WAIT);
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int s = 2 * h + set;
+                uint32_t o[32];
+                if constexpr (Q4) {
+                    const uint8_t *p = raw + row * Q4K_BYTES;
+                    q4k_expand(*reinterpret_cast<const uint4 *>(p), *reinterpret_cast<const uint4 *>(p + 16 + 32 * s), *reinterpret_cast<const uint4 *>(p + 32 + 32 * s), s, o);
+                } else {
+                    const uint2 sc8 = *reinterpret_cast<const uint2 *>(raw + Cfg::RAW_SC + row * 16 + 8 * h);
+                    q6k_expand(raw, raw + Cfg::RAW_QH, set ? sc8.y : sc8.x, row, h, set, o);
                 }
-                uint32_t sc2, m2;
-                q4k_scales(hdr.y, hdr.z, hdr.w, (int)s, sc2, m2);
-                const float sclo = (float)(sc2 & 255u), schi = (float)(sc2 >> 8);
-                const __half2 s_lo = __floats2half2_rn(sclo, sclo), s_hi = __floats2half2_rn(schi, schi);
-                const __half2 b_lo = __floats2half2_rn(-1024.0f * sclo, -1024.0f * sclo), b_hi = __floats2half2_rn(-1024.0f * schi, -1024.0f * schi);
-                const float mlo = (float)(m2 & 255u), mhi = (float)(m2 >> 8);
-                const __half2 mm_lo = __floats2half2_rn(mlo, mlo), mm_hi = __floats2half2_rn(mhi, mhi);
-                if (tid == 128) TC_TRACE(1, 3 * (it >> 1) + 0);
-                TC_WAIT(BAR(BAR_EMPTY + i), ((it / TC_STAGES) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT);
-                if (s < 2) { TC_WAIT(BAR(BAR_A2_EMPTY + x2), ((b >> 1) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT); }   // this set's first write of the superblock's mins
-                if (tid == 128) TC_TRACE(1, 3 * (it >> 1) + 1);
-                const uint32_t ml = 0x0F0F0F0Fu;
-                const uint32_t w[8] = {cur_a.x, cur_a.y, cur_a.z, cur_a.w, cur_b.x, cur_b.y, cur_b.z, cur_b.w};
-                uint8_t *dst = smem + TC_OFF_A + i * TC_STAGE;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {     // low nibbles = sub-block 2s: k-chunks 0-3 of the stage; high nibbles = sub-block 2s+1: k-chunks 4-7
-                    *reinterpret_cast<uint4 *>(dst + tc_tile_offset(row, c)) = q4_chunk_to_half(w[2 * c] & ml, w[2 * c + 1] & ml, s_lo, b_lo);
-                    *reinterpret_cast<uint4 *>(dst + tc_tile_offset(row, 4 + c)) = q4_chunk_to_half((w[2 * c] >> 4) & ml, (w[2 * c + 1] >> 4) & ml, s_hi, b_hi);
-                }
-                // the two mins of this quarter, each doubled (bsums come per 16 elements): positions 4s .. 4s+3 of the 16-deep tile.  They
-                // are written before this stage's arrival, and the T2 MMA is issued after the superblock's last stage: no barrier of their own.
-                uint32_t *d2 = reinterpret_cast<uint32_t *>(smem + TC_OFF_A2 + x2 * TC_AUX + tc_tile_offset(row, (int)(s >> 1))) + 2 * (s & 1u);
-                d2[0] = *reinterpret_cast<const uint32_t *>(&mm_lo);
-                d2[1] = *reinterpret_cast<const uint32_t *>(&mm_hi);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
+                if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + s), (b & 1u) ^ 1u)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
+                tc_fence_after();
+                tc_st32(ta + 32 * s, o);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(BAR_FULL + i));
-                cur_a = nxt_a;
-                cur_b = nxt_b;
-                hdr = hdr_next;
-                if (tid == 128) TC_TRACE(1, 3 * (it >> 1) + 2);
+                if (lane == 0) {
+                    mbar_arrive(BAR(Cfg::A_FULL + s));
+                    if (h) mbar_arrive(BAR(Cfg::R_EMPTY + r));       // every lane's reads of the superblock have gone into what it stored
+                }
             }
         }
     } else {
-        // ------------------------------------------------------------ accumulator drain: thread = TMEM lane (weight row), 64 token columns
-        TC_SETMAXNREG("inc", Cfg::REGS_DRAIN);
-        constexpr int COLS = Cfg::DRAIN_COLS;         // token columns of this thread
+        // ------------------------------------------------------------ accumulator drain: thread = TMEM lane (weight row), DRAIN_COLS token columns
+        if constexpr (Cfg::REGS_DRAIN < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", Cfg::REGS_DRAIN);
+        else TC_SETMAXNREG("inc", Cfg::REGS_DRAIN);
+        constexpr int COLS = Cfg::DRAIN_COLS;
         const int dw = warp - 12;
         const int q = dw & 3, ch = dw >> 2;           // warp % 4 is the TMEM lane quarter this warp may read (12 % 4 == 0)
-        const int row = 32 * q + lane, n = n0 + row;
-        constexpr size_t DSTRIDE = WF == TC_W_Q4K ? Q4K_BYTES : 2;        // bytes between the block scales of consecutive superblocks
-        const uint8_t *wrow = WF == TC_W_Q4K ? B + ((size_t)min(n, N - 1) * nb_row + kb0) * Q4K_BYTES
-                                             : B + (size_t)min(n, N - 1) * (((size_t)nb_row * Q6K_BYTES + 15) & ~(size_t)15) + (size_t)nb_row * 208 + (size_t)kb0 * 2;
-        float acc[COLS];
+        const int row = 32 * q + lane;
+        const size_t rb6 = ((size_t)work.nb_row * Q6K_BYTES + 15) & ~(size_t)15;
+        uint32_t b = 0;
+        bool go = true;
+        for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+            const int n = work.nt(u) * TC_ROWS + row, m0 = work.mt(u) * NT, nb = work.nb(u);
+            const uint8_t *d_plane = Q4 ? nullptr : B + (size_t)min(n, N - 1) * rb6 + (size_t)work.nb_row * 208 + (size_t)work.kb0(u) * 2;
+            uint64_t acc[COLS / 2];
 #pragma unroll
-        for (int i = 0; i < COLS; ++i) acc[i] = 0.0f;
-        auto load_dd = [&](int b) -> uint32_t {       // Q4_K: fp16 d | dmin of the superblock; Q6_K: fp16 d
-            if constexpr (WF == TC_W_Q4K) return __ldg(reinterpret_cast<const uint32_t *>(wrow + (size_t)b * DSTRIDE));
-            else return ldg_nc_u16(wrow + (size_t)b * DSTRIDE);
-        };
-        uint32_t dd_next = load_dd(0);
-        int b = 0;
-        for (; b < nb; ++b) {
-            const uint32_t dd_bits = dd_next;
-            if (b + 1 < nb) dd_next = load_dd(b + 1);
-            const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&dd_bits));
-            const uint32_t buf = (uint32_t)b & 1u;
-            const float4 *dxp = reinterpret_cast<const float4 *>(smem + TC_OFF_DX + buf * NT * 4) + ch * (COLS / 4);
-            if (lane == 0 && dw == 0) TC_TRACE(2, 3 * b + 0);
-            TC_WAIT(BAR(BAR_DX_FULL + buf), ((uint32_t)b >> 1) & 1u, DEV_ERR_FULL_WAIT);
-            TC_WAIT(BAR(BAR_T_FULL + buf), ((uint32_t)b >> 1) & 1u, DEV_ERR_MMA_WAIT);
-            if (lane == 0 && dw == 0) TC_TRACE(2, 3 * b + 1);
-            tc_fence_after();
-            const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + Cfg::T_BUF * buf + (uint32_t)(COLS * ch);
-            constexpr int RJ = NT == 128 ? 2 : 1;     // 16-column loads in flight per round (registers: 16 or 32 per accumulator)
+            for (int i = 0; i < COLS / 2; ++i) acc[i] = 0;
+            uint32_t d_next = 0;
+            if constexpr (!Q4) d_next = ldg_nc_u16(d_plane);
+            for (int kb = 0; kb < nb; ++kb, ++b) {
+                const uint32_t buf = b & 1u, x = b % TC_XSLOTS;
+                uint32_t dd_bits = d_next;
+                if constexpr (!Q4) { if (kb + 1 < nb) d_next = ldg_nc_u16(d_plane + 2 * (size_t)(kb + 1)); }
+                if (!mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
+                if constexpr (Q4) dd_bits = *reinterpret_cast<const uint32_t *>(smem + Cfg::OFF_DD + (x * TC_ROWS + row) * 4);
+                const float2 dd = __half22float2(bits_h2(dd_bits));
+                const uint64_t d2 = pack2f(dd.x, dd.x), m2 = pack2f(-dd.y, -dd.y);
+                const uint32_t dx = s_base + Cfg::OFF_DX + (x * NT + COLS * ch) * 4;
+                if (!mbar_wait_spin(BAR(Cfg::T_FULL + buf), (b >> 1) & 1u)) { go = false; break; }
+                tc_fence_after();
+                const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(COLS * ch);
 #pragma unroll
-            for (int c = 0; c < COLS / (16 * RJ); ++c) {
-                uint32_t t1[RJ][16], t2[RJ][16];
-#pragma unroll
-                for (int j = 0; j < RJ; ++j) {
-                    tc_ld16(taddr + (uint32_t)(16 * (RJ * c + j)), t1[j]);
-                    if constexpr (WF == TC_W_Q4K) tc_ld16(taddr + Cfg::T2_OFF + (uint32_t)(16 * (RJ * c + j)), t2[j]);
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < RJ; ++j)
-#pragma unroll
-                    for (int i4 = 0; i4 < 4; ++i4) {
-                        const float4 dx = dxp[4 * (RJ * c + j) + i4];
-                        const float dxf[4] = {dx.x, dx.y, dx.z, dx.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if constexpr (WF == TC_W_Q4K)
-                                acc[16 * (RJ * c + j) + 4 * i4 + i] +=
-                                    dxf[i] * (dd.x * __uint_as_float(t1[j][4 * i4 + i]) - dd.y * __uint_as_float(t2[j][4 * i4 + i]));
-                            else
-                                acc[16 * (RJ * c + j) + 4 * i4 + i] += (dxf[i] * dd.x) * __uint_as_float(t1[j][4 * i4 + i]);
+                for (int c = 0; c < COLS / 16; ++c) {
+                    uint32_t t1[16], t2[16];
+                    tc_ld16(taddr + NT * buf + 16 * c, t1);
+                    if constexpr (Q4) tc_ld16(taddr + Cfg::TM_T2 + 16 * c, t2);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c == COLS / 16 - 1) {             // the accumulators are in registers: the next superblocks may overwrite them
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(BAR(Cfg::T_EMPTY + buf));
+                            if (Q4) mbar_arrive(BAR(Cfg::T2_EMPTY));
                         }
                     }
-            }
-            // Every lane has read block scales from shared memory with plain loads, and lane 0's arrival below tells the loader that
-            // the buffer may be overwritten (by a bulk copy, which neither the compiler nor the warp barrier knows about).  The fence
-            // makes each lane's loads complete before the warp barrier, so that none of them can still be in flight when the copy
-            // lands.  Without it a pipeline that is not starved elsewhere corrupts a few 4-token groups of a 32-row quarter per call.
-            __threadfence_block();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(BAR(BAR_T_EMPTY + buf));
-                mbar_arrive(BAR(BAR_B2_EMPTY + buf));
-            }
-            if (lane == 0 && dw == 0) TC_TRACE(2, 3 * b + 2);
-        }
-        if (b == nb && n < N) {
-            const float bv = bias && gridDim.z == 1 ? bias[n] : 0.0f;
-            float *Cz = C + (size_t)blockIdx.z * cz;
 #pragma unroll
-            for (int i = 0; i < COLS; ++i) {
-                const int m = m0 + COLS * ch + i;
-                if (m < M) Cz[(size_t)m * ldc + n] = acc[i] + bv;
+                    for (int i4 = 0; i4 < 4; ++i4) {
+                        uint64_t dxp[2];
+                        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(dxp[0]), "=l"(dxp[1]) : "r"(dx + 64 * c + 16 * i4));
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint64_t t = pack2(t1[4 * i4 + 2 * i], t1[4 * i4 + 2 * i + 1]);
+                            uint64_t &a = acc[8 * c + 2 * i4 + i];
+                            if constexpr (Q4) a = fma2(dxp[i], fma2(d2, t, mul2(m2, pack2(t2[4 * i4 + 2 * i], t2[4 * i4 + 2 * i + 1]))), a);
+                            else a = fma2(mul2(dxp[i], d2), t, a);
+                        }
+                    }
+                }
+                // Every lane has read block scales from shared memory with plain loads, and lane 0's arrival below tells the loader that
+                // the buffer may be overwritten (by a bulk copy, which neither the compiler nor the warp barrier knows about).  The fence
+                // makes each lane's loads complete before the warp barrier, so that none of them can still be in flight when the copy
+                // lands.  Without it a pipeline that is not starved elsewhere corrupts a few 4-token groups of a 32-row quarter per call.
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(Cfg::X_EMPTY + x));
+            }
+            if (go && n < N) {
+                const float bv = bias && work.nbz == work.nb_row ? bias[n] : 0.0f;
+                float *Cz = C + (size_t)work.z(u) * cz;
+#pragma unroll
+                for (int i = 0; i < COLS / 2; ++i) {
+                    const int m = m0 + COLS * ch + 2 * i;
+                    float lo, hi;
+                    unpack2(acc[i], lo, hi);
+                    if (m < M) Cz[(size_t)m * ldc + n] = lo + bv;
+                    if (m + 1 < M) Cz[(size_t)(m + 1) * ldc + n] = hi + bv;
+                }
             }
         }
+        if (!go) atomicExch(dev_err, DEV_ERR_MMA_WAIT);
     }
 #undef TC_WAIT
 #undef TC_SETMAXNREG
-#undef BAR
     __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::TMEM_COLS));
+    tc_fence_after();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::TMEM_COLS));
+#undef BAR
 }
 
 // sum of the split-K slices in slice order, plus bias: C[m * ldc + n] = sum_z part[z][m][n] + bias[n]
@@ -551,15 +637,84 @@ static int tc_pick_slices(int tiles, int nb, int slots)
     return best;
 }
 
+// How a product is cut: K slices of nbz superblocks, and row tiles that go to a second launch with K split.
+struct TcPlan { int mtiles, ntiles, Z, nbz, tail_nt, Zt, nbzt; double us; };
+static TcPlan tc_plan(int wf, int width, int M, int N, int nb, int ctas_per_sm, bool may_tail)
+{
+    TcPlan p = {(M + width - 1) / width, (N + TC_ROWS - 1) / TC_ROWS, 1, nb, 0, 1, nb, 0.0};
+    const int slots = ckb_sm_count() * ctas_per_sm, tiles = p.ntiles * p.mtiles;
+    // K is split for a handful of tokens, and for any product whose tiles leave more than half of the SMs without a CTA (the k and
+    // v projections of a prompt: 8 x 4 tiles)
+    const int splitk = ckb_tune_get("gemm_tc_splitk", 1);
+    if (splitk && (M <= 128 || (splitk != 2 && 2 * tiles <= slots))) p.Z = tc_pick_slices(tiles, nb, slots);
+    const int forced = ckb_tune_get("gemm_tc_slices", 0);
+    if (forced > 0 && forced <= nb) p.Z = forced;
+    p.nbz = (nb + p.Z - 1) / p.Z;
+    p.Z = (nb + p.nbz - 1) / p.nbz;                    // no empty slice
+    // A grid of whole waves plus a few units pays a full wave for those few (28672 x 4096 at 512 tokens: 896 tiles = 6 waves of 148
+    // and 8 tiles).  The row tiles behind that remainder then go to a second launch with K split, which fills the SMs for a
+    // fraction of a wave; its partial sums are added as for any split.  The two extra launches cost about 10 us, so not where a unit takes
+    // less (9728 x 1024 at 129 tokens: 25.7 us with the second launch, 19 without).  Library workspace only (a caller's workspace is sized for one launch).
+    if (p.Z == 1 && may_tail && nb >= 8 && ckb_tune_get("gemm_tc_tail", 1)) {
+        const int rem = tiles % slots;
+        if (tiles > slots && rem > 0 && 4 * rem <= slots && rem % p.mtiles == 0 && rem / p.mtiles < p.ntiles && N % TC_ROWS == 0) {
+            p.Zt = tc_pick_slices(rem, nb, slots);
+            if (p.Zt > 1) p.tail_nt = rem / p.mtiles;
+        }
+    }
+    p.nbzt = (nb + p.Zt - 1) / p.Zt;
+    if (p.tail_nt) p.Zt = (nb + p.nbzt - 1) / p.nbzt;
+    // time: rounds of units, a superblock of a unit at the measured rate (us, by width and format), its stores, and the launches of a split
+    const double per_sb = wf == TC_W_Q4K ? (width == 128 ? 1.06 : (width == 96 ? 0.98 : 0.78)) : (width == 128 ? 1.32 : (width == 96 ? 1.26 : 1.13));
+    const int units = (p.ntiles - p.tail_nt) * p.mtiles * p.Z, rounds = (units + slots - 1) / slots;
+    p.us = rounds * (p.nbz * per_sb + 1.5 * width / 128) + (p.Z > 1 ? 4.0 : 0.0) + (p.tail_nt ? 10.0 + p.nbzt * per_sb : 0.0);
+    return p;
+}
+
 // The operand tiles that the last launch made, and the caller's promise that the activations behind them have not changed.
 static struct { const void *a; int M, nb, nt; const uint8_t *xt; cudaStream_t st; } g_tc_tiles = {nullptr, 0, 0, 0, nullptr, nullptr};
 static int g_tc_same_activations = 0;
 extern "C" void ckb_gemm_tc_hint_same_activations(int on) { g_tc_same_activations = on; }
 
+typedef CUresult (*tc_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// `rows` rows of row_bytes bytes (a multiple of 16), boxes of box_bytes x 128 rows; rows past the end read as zeros
+static bool tc_make_map(CUtensorMap *map, const void *base, size_t row_bytes, size_t rows, unsigned box_bytes, CUtensorMapSwizzle swizzle)
+{
+    static tc_encode_fn fn = nullptr;
+    if (!fn) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        fn = (tc_encode_fn)p;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {box_bytes, TC_ROWS}, estr[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// weights of a launch over rows [0, N); Q6_K: the planes lie behind one another in every row
+template <int WF>
+static bool tc_maps(TcMaps *maps, const uint8_t *B, int N, int nb)
+{
+    if (WF == TC_W_Q4K) {
+        if (!tc_make_map(&maps->w[0], B, (size_t)nb * Q4K_BYTES, (size_t)N, Q4K_BYTES, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+        maps->w[1] = maps->w[2] = maps->w[0];
+        return true;
+    }
+    const size_t rb = ((size_t)nb * Q6K_BYTES + 15) & ~(size_t)15;
+    return tc_make_map(&maps->w[0], B, rb, (size_t)N, 128, CU_TENSOR_MAP_SWIZZLE_128B) &&
+           tc_make_map(&maps->w[1], B + (size_t)nb * 128, rb, (size_t)N, 64, CU_TENSOR_MAP_SWIZZLE_64B) &&
+           tc_make_map(&maps->w[2], B + (size_t)nb * 192, rb, (size_t)N, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 template <int WF, int NT>
 static int launch_tc(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, uint8_t *ws, size_t ws_bytes, cudaStream_t st)
 {
-    using Cfg = TcCfg<NT>;
+    using Cfg = TcCfg<WF, NT>;
     auto kernel = gemm_kq_tc_kernel<WF, NT>;
     static int attr_set = 0;
     if (!attr_set) {
@@ -570,30 +725,11 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
         if (ckb_check_cuda((int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM), "smem attr")) return CKB_ERR_CUDA;
         attr_set = 1;
     }
-    const int mtiles = (M + NT - 1) / NT, ntiles = (N + TC_ROWS - 1) / TC_ROWS;
-    // K is split for a handful of tokens, and for any product whose tiles leave more than half of the SMs without a CTA (the k and
-    // v projections of a prompt: 8 x 4 tiles)
+    TcMaps maps;
+    if (!tc_maps<WF>(&maps, (const uint8_t *)B, N, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", N, nb);
     const int slots = ckb_sm_count() * Cfg::CTAS_PER_SM;
-    const int splitk = ckb_tune_get("gemm_tc_splitk", 1);
-    int Z = splitk && (M <= 128 || (splitk != 2 && 2 * ntiles * mtiles <= slots)) ? tc_pick_slices(ntiles * mtiles, nb, slots) : 1;
-    const int forced = ckb_tune_get("gemm_tc_slices", 0);
-    if (forced > 0 && forced <= nb) Z = forced;
-    const int nbz = (nb + Z - 1) / Z;
-    Z = (nb + nbz - 1) / nbz;                          // no empty slice
-    // A grid of whole waves plus a few CTAs pays a full wave for those few (28672 x 4096 at 512 tokens: 896 tiles = 6 waves of 148
-    // and 8 tiles).  The row tiles behind that remainder then go to a second launch with K split, which fills the SMs for a
-    // fraction of a wave; its partial sums are added as for any split.  Library workspace only (a caller's workspace is sized
-    // for one launch).
-    int tail_nt = 0, Zt = 1;
-    if (Z == 1 && !ws && ckb_tune_get("gemm_tc_tail", 1)) {
-        const int tiles = ntiles * mtiles, rem = tiles % slots;
-        if (tiles > slots && rem > 0 && 4 * rem <= slots && rem % mtiles == 0 && rem / mtiles < ntiles && N % TC_ROWS == 0) {
-            Zt = tc_pick_slices(rem, nb, slots);
-            if (Zt > 1) tail_nt = rem / mtiles;
-        }
-    }
-    const int nbzt = (nb + Zt - 1) / Zt;
-    if (tail_nt) Zt = (nb + nbzt - 1) / nbzt;
+    const TcPlan plan = tc_plan(WF, NT, M, N, nb, Cfg::CTAS_PER_SM, ws == nullptr);
+    const int mtiles = plan.mtiles, ntiles = plan.ntiles, Z = plan.Z, nbz = plan.nbz, tail_nt = plan.tail_nt, Zt = plan.Zt, nbzt = plan.nbzt;
     const int Nt = tail_nt * TC_ROWS;                  // rows (output columns) of the tail launch
     const size_t xt_bytes = ((size_t)mtiles * nb * Cfg::XBLOB + 255) & ~(size_t)255;
     const size_t part_bytes = Z > 1 ? (size_t)Z * M * N * sizeof(float) : (tail_nt ? (size_t)Zt * M * Nt * sizeof(float) : 0);
@@ -610,20 +746,25 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
                        g_tc_tiles.xt == xt && g_tc_tiles.st == st;
     if (!reuse) {
         const int xz = nb * mtiles >= 2 * ckb_sm_count() ? 1 : (nb * mtiles >= ckb_sm_count() ? 2 : 4);      // enough CTAs for every SM
-        gemm_x_tiles_kernel<NT><<<dim3(nb, mtiles, xz), 256, 0, st>>>((const uint8_t *)A_q8, xt, M, nb);
-        if (int rc = ckb_check_launch("gemm_x_tiles")) return rc;
+        if (int rc = launch_pdl("gemm_x_tiles", gemm_x_tiles_kernel<NT>, dim3(nb, mtiles, xz), dim3(256), (size_t)0, st, (const uint8_t *)A_q8, xt, M, nb)) return rc;
         g_tc_tiles.a = A_q8; g_tc_tiles.M = M; g_tc_tiles.nb = nb; g_tc_tiles.nt = NT; g_tc_tiles.xt = xt; g_tc_tiles.st = st;
     }
-    const dim3 grid(ntiles - tail_nt, mtiles, Z);
+    TcWork work = {(ntiles - tail_nt) * mtiles * Z, mtiles, ntiles - tail_nt, nb, nbz};
+    dim3 grid((unsigned)(work.units < slots ? work.units : slots));
     if (Z == 1) {
-        kernel<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(xt, (const uint8_t *)B, bias, C, ldc, (size_t)0, M, N - Nt, nb, nbz, ckb_device_error_word());
-        if (int rc = ckb_check_launch("gemm_kq_tc")) return rc;
+        if (int rc = launch_pdl("gemm_kq_tc", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, (const uint8_t *)B, bias, C, ldc, (size_t)0, M, N - Nt,
+                                ckb_device_error_word()))
+            return rc;
         if (!tail_nt) return 0;
         const int n0 = N - Nt;
         const size_t rb = WF == TC_W_Q4K ? (size_t)nb * Q4K_BYTES : (((size_t)nb * Q6K_BYTES + 15) & ~(size_t)15);
-        kernel<<<dim3(tail_nt, mtiles, Zt), Cfg::THREADS, Cfg::SMEM, st>>>(xt, (const uint8_t *)B + (size_t)n0 * rb, nullptr, part, Nt, (size_t)M * Nt, M, Nt, nb, nbzt,
-                                                                         ckb_device_error_word());
-        if (int rc = ckb_check_launch("gemm_kq_tc tail")) return rc;
+        const uint8_t *Bt = (const uint8_t *)B + (size_t)n0 * rb;
+        if (!tc_maps<WF>(&maps, Bt, Nt, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", Nt, nb);
+        work = {tail_nt * mtiles * Zt, mtiles, tail_nt, nb, nbzt};
+        grid = dim3((unsigned)(work.units < slots ? work.units : slots));
+        if (int rc = launch_pdl("gemm_kq_tc tail", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, Bt, nullptr, part, Nt, (size_t)M * Nt, M, Nt,
+                                ckb_device_error_word()))
+            return rc;
         const size_t mnt = (size_t)M * Nt;
         const unsigned tb = (unsigned)((mnt + 1023) / 1024 < 1184 ? (mnt + 1023) / 1024 : 1184);
         const float *bt = bias ? bias + n0 : nullptr;
@@ -631,8 +772,9 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
         else gemm_splitk_sum_kernel<false><<<tb, 256, 0, st>>>(part, Zt, bt, C + n0, ldc, M, Nt);
         return ckb_check_launch("gemm_splitk_sum");
     }
-    kernel<<<grid, Cfg::THREADS, Cfg::SMEM, st>>>(xt, (const uint8_t *)B, nullptr, part, N, (size_t)M * N, M, N, nb, nbz, ckb_device_error_word());
-    if (int rc = ckb_check_launch("gemm_kq_tc")) return rc;
+    if (int rc = launch_pdl("gemm_kq_tc", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, (const uint8_t *)B, nullptr, part, N, (size_t)M * N, M, N,
+                            ckb_device_error_word()))
+        return rc;
     const size_t mn = (size_t)M * N;
     const unsigned blocks = (unsigned)((mn + 1023) / 1024 < 1184 ? (mn + 1023) / 1024 : 1184);
     if (N % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)C | (uintptr_t)bias) & 15) == 0) gemm_splitk_sum_kernel<true><<<blocks, 256, 0, st>>>(part, Z, bias, C, ldc, M, N);
@@ -640,13 +782,16 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
     return ckb_check_launch("gemm_splitk_sum");
 }
 
-#ifdef CKB_TC_TRACE
-extern "C" int ckb200_tc_trace(long long *out4096) { return (int)cudaMemcpyFromSymbol(out4096, g_tc_trace, sizeof(long long) * 4096); }
-#endif
+template <int NT>
+static int tc_launch_wf(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, uint8_t *ws, size_t ws_bytes, cudaStream_t st)
+{
+    return wf == TC_W_Q6K_PLANAR ? launch_tc<TC_W_Q6K_PLANAR, NT>(A_q8, B, bias, C, ldc, M, N, nb, ws, ws_bytes, st)
+                                 : launch_tc<TC_W_Q4K, NT>(A_q8, B, bias, C, ldc, M, N, nb, ws, ws_bytes, st);
+}
 
 // C[m * ldc + n] = A_q8[m] . W[n] (+ bias[n]).  wf: TC_W_Q4K (the reference's block_q4_K rows) or TC_W_Q6K_PLANAR.
 // Returns -1 when the shape is not handled here (caller falls back to the per-token path).  min_tokens: smallest M
-// worth the tensor-core path (the token tile is 128 wide; fewer tokens are padded with zeros).
+// worth the tensor-core path (tokens past M are zeros).
 extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,
                                      void *ws, size_t ws_bytes, void *stream)
 {
@@ -655,10 +800,25 @@ extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, co
     cudaStream_t st = ckb_stream(stream);
     uint8_t *w8 = (uint8_t *)ws;
     if (M <= ckb_tune_get("gemm_tc_small_max", 64))     // batched decode: 32-token tiles, two CTAs per SM
-        return wf == TC_W_Q6K_PLANAR ? launch_tc<TC_W_Q6K_PLANAR, 32>(A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st)
-                                     : launch_tc<TC_W_Q4K, 32>(A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
-    return wf == TC_W_Q6K_PLANAR ? launch_tc<TC_W_Q6K_PLANAR, 128>(A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st)
-                                 : launch_tc<TC_W_Q4K, 128>(A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
+        return tc_launch_wf<32>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
+    // the width whose plan takes least; a product that may reuse the tiles of the one before it keeps their width
+    int width = ckb_tune_get("gemm_tc_nt", 0);
+    if (width != 64 && width != 96 && width != 128) {
+        width = 128;
+        if (g_tc_same_activations && g_tc_tiles.a == A_q8 && g_tc_tiles.M == M && g_tc_tiles.nb == nb && g_tc_tiles.nt != 32) {
+            width = g_tc_tiles.nt;
+        } else {
+            const TcPlan wide = tc_plan(wf, 128, M, N, nb, 1, ws == nullptr);
+            double best = wide.us;
+            for (int w = 96; w >= 64 && !wide.tail_nt; w -= 32) {
+                const double us = tc_plan(wf, w, M, N, nb, 1, ws == nullptr).us;
+                if (us < 0.97 * best) { best = us; width = w; }
+            }
+        }
+    }
+    if (width == 64) return tc_launch_wf<64>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
+    if (width == 96) return tc_launch_wf<96>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
+    return tc_launch_wf<128>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
 }
 
 extern "C" int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,
@@ -673,12 +833,16 @@ extern "C" size_t ckb_gemm_tc_workspace_bytes(int M, int N, int K)
 {
     if (M <= 0 || N <= 0 || K <= 0 || K % QK_K) return 0;
     const int nb = K / QK_K;
-    const size_t blob = TcCfg<32>::XBLOB > TcCfg<128>::XBLOB ? TcCfg<32>::XBLOB : TcCfg<128>::XBLOB;
+    const size_t blob = TcTile<128>::XBLOB;
     const size_t mtiles = (size_t)(M + 31) / 32;
     const size_t xt = (mtiles * nb * blob + 255) & ~(size_t)255;
     int zmax = nb / 4 < 1 ? 1 : (nb / 4 > 16 ? 16 : nb / 4);
-    if (M > 128) zmax = 1;
-    return xt + (zmax > 1 ? (size_t)zmax * M * N * sizeof(float) : 0) + 256;
+    size_t part = zmax > 1 ? (size_t)zmax * M * N * sizeof(float) : 0;
+    if (M > 128) {                                     // split only while the tiles leave half of the SMs idle
+        const size_t most = (size_t)zmax * (ckb_sm_count() / 2) * TC_ROWS * 128 * sizeof(float);
+        if (part > most) part = most;
+    }
+    return xt + part + 256;
 }
 
 extern "C" int ckb_launch_gemm_q4k_tc(const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)
