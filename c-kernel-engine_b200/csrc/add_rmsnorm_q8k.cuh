@@ -37,9 +37,11 @@ __device__ __forceinline__ ArqGamma arq_prefetch_gamma(const float *__restrict__
     return g;
 }
 
-// block-wide sum of squares -> rstd; one warp per 256-element block scales by gamma and quantises (row t of the output)
+// block-wide sum of squares -> rstd; one warp per 256-element block scales by gamma and quantises (row t of the output; TILES: out_q8 holds operand
+// tiles of tile_nt tokens)
+template <bool TILES = false>
 __device__ __forceinline__ void arq_norm_quant(float ss, const float *row, float *red, const float *__restrict__ gamma, uint8_t *__restrict__ out_q8,
-                                               float *__restrict__ norm_out, int t, int d_model, int aligned, float eps, const ArqGamma *pre = nullptr)
+                                               float *__restrict__ norm_out, int t, int d_model, int aligned, float eps, const ArqGamma *pre = nullptr, int tile_nt = 0)
 {
     ss = group_sum<32>(ss);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -67,13 +69,25 @@ __device__ __forceinline__ void arq_norm_quant(float ss, const float *row, float
             v[j] = i < d_model ? __fmul_rn(__fmul_rn(row[i], rstd), gv[j]) : 0.0f;
             if (norm_out) norm_out[(size_t)t * aligned + i] = v[j];
         }
-        quantize_block_q8k(v, out_q8 + ((size_t)t * nb + b) * Q8K_BYTES, lane);
+        if (TILES) quantize_block_q8k_tile(v, out_q8 + ((size_t)(t / tile_nt) * nb + b) * q8k_tile_bytes(tile_nt), tile_nt, t % tile_nt, lane);
+        else quantize_block_q8k(v, out_q8 + ((size_t)t * nb + b) * Q8K_BYTES, lane);
     }
 }
 
 // The same tail for a consumer with 32-element blocks (Q8_0 / Q5_0 weights): the first `cols` elements of the normalised row
 // (a multiple of 32) go to Q8_0 blocks with the arithmetic of quantize_row_q8_0 (src/kernels/gemm_kernels_q8_0.c:70-175;
-// quantize.cu): one warp per block, amax over the 32 lanes, d = amax / 127 as fp16, q = rint(x * (127 / amax)).
+// quantize.cu): one warp per block, amax over the 32 lanes, d = amax / 127 as fp16, q = rint(x * (127 / amax)).  PLANAR: rows of all quants, then
+// all d, padded to 16 bytes (gemv_q80_planar.cu), what the batched product reads.
+__device__ __forceinline__ void store_block_q80_planar(float v, uint8_t *row, int nb, int b, int lane)
+{
+    float amax = fabsf(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+    row[(size_t)b * 32 + lane] = (uint8_t)__float2int_rn(__fmul_rn(v, id));
+    if (lane == 0) reinterpret_cast<__half *>(row + (size_t)nb * 32)[b] = __float2half_rn(__fdiv_rn(amax, 127.0f));
+}
+template <bool PLANAR = false>
 __device__ __forceinline__ void arq_norm_quant_q80(float ss, const float *row, float *red, const float *__restrict__ gamma, uint8_t *__restrict__ out_q80,
                                                    int t, int d_model, int cols, float eps)
 {
@@ -89,6 +103,10 @@ __device__ __forceinline__ void arq_norm_quant_q80(float ss, const float *row, f
     for (int b = warp; b < nb; b += nw) {
         const int i = b * 32 + lane;
         const float v = i < d_model ? __fmul_rn(__fmul_rn(row[i], rstd), gamma[i]) : 0.0f;
+        if (PLANAR) {
+            store_block_q80_planar(v, out_q80 + (size_t)t * (((size_t)nb * Q80_BYTES + 15) & ~(size_t)15), nb, b, lane);
+            continue;
+        }
         float amax = fabsf(v);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));

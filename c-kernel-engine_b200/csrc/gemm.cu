@@ -63,7 +63,7 @@ extern "C" int ckb200_dev_gemm_nt_q6_k_q8_k(const void *A_q8, const void *B, con
 // already has a planar copy) and the integer tensor-core kernel of gemm_q80_mma.cu reads every weight tile once per 128 tokens.
 extern "C" size_t ckb200_q8_0_planar_bytes(int rows, int cols);
 extern "C" int ckb200_dev_q8_0_to_planar(void *dst, const void *src, int rows, int cols, void *stream);
-extern "C" int ckb_launch_gemm_q80_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int M, int N, int K, void *stream);
+extern "C" int ckb_launch_gemm_q80_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream);
 
 // B_planar may be NULL (then B_raw is converted into the library's scratch).  Returns -1 when the tensor-core path does not apply.
 extern "C" int ckb_gemm_nt_q80_tc(const void *A_raw, const void *B_raw, const void *B_planar, const float *bias, float *C, int M, int N, int K, void *stream)
@@ -73,13 +73,14 @@ extern "C" int ckb_gemm_nt_q80_tc(const void *A_raw, const void *B_raw, const vo
     const size_t a_bytes = (ckb200_q8_0_planar_bytes(M, K) + 255) & ~(size_t)255, b_bytes = B_planar ? 0 : ckb200_q8_0_planar_bytes(N, K);
     uint8_t *ws = (uint8_t *)ckb_scratch(CKB_SLOT_P, a_bytes + b_bytes);
     if (!ws) return CKB_ERR_CUDA;
+    const int resident = B_planar != nullptr;
     int rc = ckb200_dev_q8_0_to_planar(ws, A_raw, M, K, stream);
     if (!rc && !B_planar) {
         rc = ckb200_dev_q8_0_to_planar(ws + a_bytes, B_raw, N, K, stream);
         B_planar = ws + a_bytes;
     }
     if (rc) return rc;
-    return ckb_launch_gemm_q80_mma(ws, B_planar, bias, C, M, N, K, stream);
+    return ckb_launch_gemm_q80_mma(ws, B_planar, bias, C, N, M, N, K, resident, stream);
 }
 
 extern "C" int ckb200_dev_gemm_nt_q8_0_q8_0(const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)

@@ -41,6 +41,7 @@
 // at 512 tokens 110 us (181 before); 333 tokens of 28672 x 4096: 126 us against 205 with activations quantised.
 #include <cuda.h>
 
+#include "q8k_block.cuh"
 #include "quant_units.cuh"
 #include "launch.h"
 #include "pdl.cuh"
@@ -62,6 +63,7 @@ struct TcTile {
     static constexpr int STAGE = 8 * CHUNK;                   // 64-deep
     static constexpr int AUX = 2 * CHUNK;
     static constexpr int XBLOB_B2 = 4 * STAGE, XBLOB_DX = XBLOB_B2 + AUX, XBLOB = XBLOB_DX + NT * 4;   // a multiple of 16
+    static_assert(XBLOB == q8k_tile_bytes(NT), "the layout that quantize_block_q8k_tile writes");
 };
 
 // Everything that depends on the width NT of the token tile and on the weight format.  NT = 32: the accumulators and the staging shrink so far that
@@ -228,8 +230,8 @@ __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__rest
     constexpr int PITCH = 66;                                  // words per token in shared memory: 64 + 2, 8-byte reads two-way at worst
     __shared__ __align__(8) uint32_t q[NT * PITCH];
     const int b = blockIdx.x, mt = blockIdx.y;
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();                                             // the product reads weights ahead of its own wait: whatever re-laid them is complete by now
     const int kcz = 32 / (int)gridDim.z, kc0 = (int)blockIdx.z * kcz;     // this CTA's k-chunks [kc0, kc0 + kcz)
     uint8_t *blob = xt + ((size_t)mt * nb + b) * Cfg::XBLOB;
     for (int it = threadIdx.x; it < NT * kcz * 2; it += 256) {
@@ -671,10 +673,10 @@ static TcPlan tc_plan(int wf, int width, int M, int N, int nb, int ctas_per_sm, 
     return p;
 }
 
-// The operand tiles that the last launch made, and the caller's promise that the activations behind them have not changed.
-static struct { const void *a; int M, nb, nt; const uint8_t *xt; cudaStream_t st; } g_tc_tiles = {nullptr, 0, 0, 0, nullptr, nullptr};
-static int g_tc_same_activations = 0;
-extern "C" void ckb_gemm_tc_hint_same_activations(int on) { g_tc_same_activations = on; }
+static size_t tc_part_bytes(const TcPlan &p, int M, int N)
+{
+    return p.Z > 1 ? (size_t)p.Z * M * N * sizeof(float) : (p.tail_nt ? (size_t)p.Zt * M * p.tail_nt * TC_ROWS * sizeof(float) : 0);
+}
 
 typedef CUresult (*tc_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -711,8 +713,9 @@ static bool tc_maps(TcMaps *maps, const uint8_t *B, int N, int nb)
            tc_make_map(&maps->w[2], B + (size_t)nb * 192, rb, (size_t)N, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
+// The product over operand tiles: xt holds them (tiles of NT tokens), part the partial sums of a K split (part_bytes at hand).
 template <int WF, int NT>
-static int launch_tc(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, uint8_t *ws, size_t ws_bytes, cudaStream_t st)
+static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part, size_t part_bytes, cudaStream_t st)
 {
     using Cfg = TcCfg<WF, NT>;
     auto kernel = gemm_kq_tc_kernel<WF, NT>;
@@ -727,28 +730,11 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
     }
     TcMaps maps;
     if (!tc_maps<WF>(&maps, (const uint8_t *)B, N, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", N, nb);
+    if (tc_part_bytes(plan, M, N) > part_bytes)
+        return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the workspace holds %zu bytes of partial sums, this call needs %zu", part_bytes, tc_part_bytes(plan, M, N));
     const int slots = ckb_sm_count() * Cfg::CTAS_PER_SM;
-    const TcPlan plan = tc_plan(WF, NT, M, N, nb, Cfg::CTAS_PER_SM, ws == nullptr);
     const int mtiles = plan.mtiles, ntiles = plan.ntiles, Z = plan.Z, nbz = plan.nbz, tail_nt = plan.tail_nt, Zt = plan.Zt, nbzt = plan.nbzt;
     const int Nt = tail_nt * TC_ROWS;                  // rows (output columns) of the tail launch
-    const size_t xt_bytes = ((size_t)mtiles * nb * Cfg::XBLOB + 255) & ~(size_t)255;
-    const size_t part_bytes = Z > 1 ? (size_t)Z * M * N * sizeof(float) : (tail_nt ? (size_t)Zt * M * Nt * sizeof(float) : 0);
-    // A caller that records the launch in a CUDA graph brings its own workspace: the library's pool may be freed and
-    // regrown by any later call that needs more, which would leave a captured pointer dangling.
-    if (ws && xt_bytes + part_bytes > ws_bytes)
-        return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the caller's workspace holds %zu bytes, this call needs %zu", ws_bytes, xt_bytes + part_bytes);
-    uint8_t *xt = ws ? ws : (uint8_t *)ckb_scratch(CKB_SLOT_G, xt_bytes + part_bytes);
-    if (!xt) return CKB_ERR_CUDA;
-    float *part = reinterpret_cast<float *>(xt + xt_bytes);
-    // q, k and v of a prompt read the same activation rows: a caller that says so between its calls gets the operand tiles of
-    // the previous product again, provided they still lie where this call would put them.
-    const bool reuse = g_tc_same_activations && g_tc_tiles.a == A_q8 && g_tc_tiles.M == M && g_tc_tiles.nb == nb && g_tc_tiles.nt == NT &&
-                       g_tc_tiles.xt == xt && g_tc_tiles.st == st;
-    if (!reuse) {
-        const int xz = nb * mtiles >= 2 * ckb_sm_count() ? 1 : (nb * mtiles >= ckb_sm_count() ? 2 : 4);      // enough CTAs for every SM
-        if (int rc = launch_pdl("gemm_x_tiles", gemm_x_tiles_kernel<NT>, dim3(nb, mtiles, xz), dim3(256), (size_t)0, st, (const uint8_t *)A_q8, xt, M, nb)) return rc;
-        g_tc_tiles.a = A_q8; g_tc_tiles.M = M; g_tc_tiles.nb = nb; g_tc_tiles.nt = NT; g_tc_tiles.xt = xt; g_tc_tiles.st = st;
-    }
     TcWork work = {(ntiles - tail_nt) * mtiles * Z, mtiles, ntiles - tail_nt, nb, nbz};
     dim3 grid((unsigned)(work.units < slots ? work.units : slots));
     if (Z == 1) {
@@ -782,11 +768,47 @@ static int launch_tc(const void *A_q8, const void *B, const float *bias, float *
     return ckb_check_launch("gemm_splitk_sum");
 }
 
-template <int NT>
-static int tc_launch_wf(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, uint8_t *ws, size_t ws_bytes, cudaStream_t st)
+static int tc_launch(int wf, int nt, const uint8_t *xt, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part,
+                     size_t part_bytes, cudaStream_t st)
 {
-    return wf == TC_W_Q6K_PLANAR ? launch_tc<TC_W_Q6K_PLANAR, NT>(A_q8, B, bias, C, ldc, M, N, nb, ws, ws_bytes, st)
-                                 : launch_tc<TC_W_Q4K, NT>(A_q8, B, bias, C, ldc, M, N, nb, ws, ws_bytes, st);
+#define TC_GO(WF, NT) return launch_tc<WF, NT>(xt, B, bias, C, ldc, M, N, nb, plan, part, part_bytes, st)
+    if (wf == TC_W_Q6K_PLANAR) switch (nt) { case 32: TC_GO(TC_W_Q6K_PLANAR, 32); case 64: TC_GO(TC_W_Q6K_PLANAR, 64); case 96: TC_GO(TC_W_Q6K_PLANAR, 96); default: TC_GO(TC_W_Q6K_PLANAR, 128); }
+    switch (nt) { case 32: TC_GO(TC_W_Q4K, 32); case 64: TC_GO(TC_W_Q4K, 64); case 96: TC_GO(TC_W_Q4K, 96); default: TC_GO(TC_W_Q4K, 128); }
+#undef TC_GO
+}
+static int tc_make_tiles(const void *A_q8, uint8_t *xt, int nt, int M, int nb, cudaStream_t st)
+{
+    const int mtiles = (M + nt - 1) / nt, xz = nb * mtiles >= 2 * ckb_sm_count() ? 1 : (nb * mtiles >= ckb_sm_count() ? 2 : 4);      // enough CTAs for every SM
+    auto kernel = nt == 32 ? gemm_x_tiles_kernel<32> : (nt == 64 ? gemm_x_tiles_kernel<64> : (nt == 96 ? gemm_x_tiles_kernel<96> : gemm_x_tiles_kernel<128>));
+    return launch_pdl("gemm_x_tiles", kernel, dim3(nb, mtiles, xz), dim3(256), (size_t)0, st, (const uint8_t *)A_q8, xt, M, nb);
+}
+
+// Token tile: 32 for batched decode (up to 64 tokens: two CTAs per SM), else the width whose plan takes least.
+static int tc_width(int wf, int M, int N, int nb, bool may_tail)
+{
+    if (M <= ckb_tune_get("gemm_tc_small_max", 64)) return 32;
+    const int forced = ckb_tune_get("gemm_tc_nt", 0);
+    if (forced == 64 || forced == 96 || forced == 128) return forced;
+    const TcPlan wide = tc_plan(wf, 128, M, N, nb, 1, may_tail);
+    double best = wide.us;
+    int width = 128;
+    for (int w = 96; w >= 64 && !wide.tail_nt; w -= 32) {
+        const double us = tc_plan(wf, w, M, N, nb, 1, may_tail).us;
+        if (us < 0.97 * best) { best = us; width = w; }
+    }
+    return width;
+}
+
+// A caller that quantises rows straight into operand tiles (quantize_block_q8k_tile: one blob per tile of nt tokens and superblock) asks for the width
+// and the sizes first.  Products over the same rows share one width: the one that suits the largest of them.
+extern "C" int ckb_gemm_tc_width(int wf, int M, int N, int K) { return tc_width(wf, M, N, K / QK_K, true); }
+extern "C" size_t ckb_gemm_tc_tile_bytes(int nt, int M, int K) { return (size_t)((M + nt - 1) / nt) * (K / QK_K) * q8k_tile_bytes(nt); }
+extern "C" size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K) { return tc_part_bytes(tc_plan(wf, nt, M, N, K / QK_K, nt == 32 ? 2 : 1, true), M, N); }
+extern "C" int ckb_launch_gemm_tc_tiles(int wf, const void *tiles, int nt, const void *B, float *C, int ldc, int M, int N, int K, void *part, size_t part_bytes, void *stream)
+{
+    if (K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)tiles & 15)) return -1;
+    return tc_launch(wf, nt, (const uint8_t *)tiles, B, nullptr, C, ldc, M, N, K / QK_K, tc_plan(wf, nt, M, N, K / QK_K, nt == 32 ? 2 : 1, true), (float *)part, part_bytes,
+                     ckb_stream(stream));
 }
 
 // C[m * ldc + n] = A_q8[m] . W[n] (+ bias[n]).  wf: TC_W_Q4K (the reference's block_q4_K rows) or TC_W_Q6K_PLANAR.
@@ -796,29 +818,18 @@ extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, co
                                      void *ws, size_t ws_bytes, void *stream)
 {
     if (M < min_tokens || K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3) || ((uintptr_t)ws & 255) || ckb_tune_get("gemm_tc", 1) == 0) return -1;
-    const int nb = K / QK_K;
+    const int nb = K / QK_K, nt = tc_width(wf, M, N, nb, ws == nullptr);
+    const TcPlan plan = tc_plan(wf, nt, M, N, nb, nt == 32 ? 2 : 1, ws == nullptr);
+    const size_t xt_bytes = (ckb_gemm_tc_tile_bytes(nt, M, K) + 255) & ~(size_t)255, part_bytes = tc_part_bytes(plan, M, N);
+    // A caller that records the launch in a CUDA graph brings its own workspace: the library's pool may be freed and
+    // regrown by any later call that needs more, which would leave a captured pointer dangling.
+    if (ws && xt_bytes + part_bytes > ws_bytes)
+        return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the caller's workspace holds %zu bytes, this call needs %zu", ws_bytes, xt_bytes + part_bytes);
+    uint8_t *xt = ws ? (uint8_t *)ws : (uint8_t *)ckb_scratch(CKB_SLOT_G, xt_bytes + part_bytes);
+    if (!xt) return CKB_ERR_CUDA;
     cudaStream_t st = ckb_stream(stream);
-    uint8_t *w8 = (uint8_t *)ws;
-    if (M <= ckb_tune_get("gemm_tc_small_max", 64))     // batched decode: 32-token tiles, two CTAs per SM
-        return tc_launch_wf<32>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
-    // the width whose plan takes least; a product that may reuse the tiles of the one before it keeps their width
-    int width = ckb_tune_get("gemm_tc_nt", 0);
-    if (width != 64 && width != 96 && width != 128) {
-        width = 128;
-        if (g_tc_same_activations && g_tc_tiles.a == A_q8 && g_tc_tiles.M == M && g_tc_tiles.nb == nb && g_tc_tiles.nt != 32) {
-            width = g_tc_tiles.nt;
-        } else {
-            const TcPlan wide = tc_plan(wf, 128, M, N, nb, 1, ws == nullptr);
-            double best = wide.us;
-            for (int w = 96; w >= 64 && !wide.tail_nt; w -= 32) {
-                const double us = tc_plan(wf, w, M, N, nb, 1, ws == nullptr).us;
-                if (us < 0.97 * best) { best = us; width = w; }
-            }
-        }
-    }
-    if (width == 64) return tc_launch_wf<64>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
-    if (width == 96) return tc_launch_wf<96>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
-    return tc_launch_wf<128>(wf, A_q8, B, bias, C, ldc, M, N, nb, w8, ws_bytes, st);
+    if (int rc = tc_make_tiles(A_q8, xt, nt, M, nb, st)) return rc;
+    return tc_launch(wf, nt, xt, B, bias, C, ldc, M, N, nb, plan, reinterpret_cast<float *>(xt + xt_bytes), part_bytes, st);
 }
 
 extern "C" int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,

@@ -70,6 +70,8 @@ typedef struct {
     Tensor t[CKB_T_PER_LAYER];
 } Layer;
 
+enum { PF_X, PF_DELTA, PF_O, PF_Q, PF_K, PF_V, PF_QH, PF_OH, PF_GU, PF_ROWS, PF_PART0, PF_PART1, PF_PART2, PF_IDS, PF_BUFFERS };
+
 typedef struct {
     struct CKB200Model;     /* shared fields (model_internal.h) */
     int D, Da;              /* embed dim and its 256-aligned width */
@@ -94,10 +96,13 @@ typedef struct {
     float *x2;              /* second residual row of the fused step (each fused launch reads one and writes the other) */
     float *mf;              /* fp32 SwiGLU output of the fused step, round256(Il) wide, tail zero */
     int *attn_counters;     /* arrival counters of the attention kernel's in-launch split merge */
-    /* batched prefill (grown on demand to the longest prompt seen): token-major rows and head-major attention tensors */
-    int pf_tokens;
+    /* batched prefill, grown on demand to the longest prompt seen: token-major rows, head-major attention tensors, quantised rows (Q8_K blocks, operand tiles of the
+     * tensor-core product, or row-planar Q8_0), partial sums of the three products that run side by side, prompt ids */
     float *pf_x, *pf_delta, *pf_o, *pf_q, *pf_k, *pf_v, *pf_qh, *pf_oh, *pf_gu;
-    uint8_t *pf_hq, *pf_aq, *pf_mq;
+    uint8_t *pf_rows, *pf_part[3];
+    int32_t *pf_ids;
+    uint8_t *pf_arena;      /* all of them */
+    size_t pf_cap[PF_BUFFERS];
     uint8_t *hq, *aq, *mq;
     uint8_t *gemm_ws;       /* workspace of the tensor-core GEMM of batched decode: the step's graph keeps this pointer */
     size_t gemm_ws_bytes;
@@ -321,7 +326,7 @@ static void kq_destroy(CKB200Model *model)
     KqModel *m = (KqModel *)model;
     void *ptrs[] = { m->arena, m->planar_arena, m->kv, m->rope_cos, m->rope_sin, m->x, m->prev, m->o, m->q, m->k, m->v, m->att, m->gu,
                      m->hq, m->aq, m->mq, m->attn_scratch, m->gemm_ws, m->x2, m->mf, m->attn_counters,
-                     m->pf_x, m->pf_delta, m->pf_o, m->pf_q, m->pf_k, m->pf_v, m->pf_qh, m->pf_oh, m->pf_gu, m->pf_hq, m->pf_aq, m->pf_mq };
+                     m->pf_arena };
     for (size_t i = 0; i < sizeof ptrs / sizeof ptrs[0]; ++i) if (ptrs[i]) cudaFree(ptrs[i]);
     for (int i = 0; i < 2; ++i) {
         if (m->side[i]) cudaStreamDestroy(m->side[i]);
@@ -862,85 +867,200 @@ static int issue_step(KqModel *m, void *st)
  * A prompt of T tokens as ONE pass (the reference's generated ck_prefill, version/v7/scripts/codegen_prefill_v7.py:194-208): per
  * layer the T rows are normalised and quantised together, every projection is one quantised GEMM on the tensor cores (the
  * weights are read once for all tokens), RoPE and the KV-cache fill run over all tokens, attention is the causal prefill
- * kernel.  Only the last token's logits are produced.  Used from an empty cache (position 0) by one sequence on one GPU with
- * K-quant projections; every other case (and prompts shorter than 16 tokens) falls back to T decode steps. */
+ * kernel over the T new keys and the ones already in the cache.  Only the last token's logits are produced.  Used by one sequence on one GPU with
+ * fp32 caches; prompts shorter than 16 tokens and other cases fall back to T decode steps.
+ *
+ * How a product is done depends on the format and on T:
+ *   K-quants, T <= 64   Q8_K rows, integer-MMA kernels (48 x 4096 x 4096: 12 us; the tcgen05 kernel with 32-token tiles 17)
+ *   K-quants, T > 64    the producer of the rows quantises them straight into operand tiles, tcgen05 kernel
+ *   Q5_0, Q8_0          row-planar Q8_0 rows, gemm_q80_mma.cu
+ * q, k and v run on three streams: one of them alone leaves SMs idle (512 x 1024 x 4096 is 32 tiles) or ends in a part of a wave. */
 
 int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens, void *stream);
+int ckb_gemm_tc_width(int wf, int M, int N, int K);                                                                    /* gemm_tc.cu */
+size_t ckb_gemm_tc_tile_bytes(int nt, int M, int K);
+size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K);
+int ckb_launch_gemm_tc_tiles(int wf, const void *tiles, int nt, const void *B, float *C, int ldc, int M, int N, int K, void *part, size_t part_bytes, void *stream);
+int ckb_add_rmsnorm_tiles(float *x, const float *delta, const float *gamma, void *tiles, int tile_nt, int tokens, int d_model, int aligned, float eps, void *stream);   /* step_kernels.cu */
+int ckb_add_rmsnorm_q80_planar(float *x, const float *delta, const float *gamma, void *out_planar, int tokens, int d_model, int aligned, int cols, float eps, void *stream);
+int ckb_swiglu_tiles(const float *gate_up, void *tiles, int tile_nt, int tokens, int dim, void *stream);
+int ckb_prefill_gather_tiles(const float *out_hm, void *tiles, int tile_nt, int tokens, int num_heads, int head_dim, int cols, void *stream);      /* prefill_kernels.cu */
+int ckb_prefill_gather_q80_planar(const float *out_hm, void *planar, int tokens, int num_heads, int head_dim, int cols, void *stream);
+int ckb_launch_gemm_q80_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream);   /* gemm_q80_mma.cu */
+int ckb_launch_gemm_q50_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream);
+int ckb_launch_attn_prefill_mma(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, int aligned_head_dim,
+                                int kv_stride_tokens, int before, int causal, void *stream);                          /* attention_prefill_mma.cu */
 
-void ckb_gemm_tc_hint_same_activations(int on);              /* gemm_tc.cu */
+#define PF_SMALL 64            /* most tokens of the integer-MMA kernels */
+
+static int tc_format(const Tensor *w) { return w->fmt == FMT_Q6K; }
+static const void *tc_weights(const Tensor *w) { return w->fmt == FMT_Q6K ? w->planar : w->w; }
+/* Whether T tokens go through operand tiles for this consumer (0: no), and how wide those are.  Layers mostly repeat the same shapes: `memo` holds the
+ * last answer for this kind of consumer during one pass. */
+typedef struct { int fmt, rows, cols, nt; } WidthMemo;
+static int tile_width(const Tensor *w, int T, WidthMemo *memo)
+{
+    if (fmt_block32(w->fmt) || T <= PF_SMALL) return 0;
+    if (memo->fmt != w->fmt || memo->rows != w->rows || memo->cols != w->cols) {
+        const WidthMemo now = { w->fmt, w->rows, w->cols, ckb_gemm_tc_width(tc_format(w), T, w->rows, w->cols) };
+        *memo = now;
+    }
+    return memo->nt;
+}
+
+static int prefill_takes(const Tensor *w)
+{
+    if (w->fmt == FMT_Q50) return w->planar != NULL && w->cols % 128 == 0;
+    return w->fmt == FMT_Q4K || (w->fmt == FMT_Q6K && w->planar);
+}
 
 static int prefill_ok(const KqModel *m, int T)
 {
-    if (m->c.batch != 1 || m->c.tp_size != 1 || m->kv_eb != 4 || T < 16 || m->host_pos != 0 || T > m->c.max_seq_len || !ckb_tune_get("model_prefill", 1)) return 0;
+    if (m->c.batch != 1 || m->c.tp_size != 1 || m->kv_eb != 4 || T < 16 || m->host_pos + T > m->c.max_seq_len || !ckb_tune_get("model_prefill", 1)) return 0;
+    if (m->host_pos && !ckb_tune_get("attn_prefill_mma", 1)) return 0;        /* the only prompt kernel that sees keys before its own */
     for (int l = 0; l < m->c.num_layers; ++l) {
+        const Tensor *t = m->layers[l].t;
         static const int which[6] = { CKB_T_WQ, CKB_T_WK, CKB_T_WV, CKB_T_WO, CKB_T_W1, CKB_T_W2 };
-        for (int i = 0; i < 6; ++i) {
-            const Tensor *t = &m->layers[l].t[which[i]];
-            if (!(t->fmt == FMT_Q4K || (t->fmt == FMT_Q6K && t->planar))) return 0;
-        }
+        for (int i = 0; i < 6; ++i)
+            if (!prefill_takes(&t[which[i]])) return 0;
+        if (fmt_block32(t[CKB_T_WK].fmt) != fmt_block32(t[CKB_T_WQ].fmt) || fmt_block32(t[CKB_T_WV].fmt) != fmt_block32(t[CKB_T_WQ].fmt) || fmt_block32(t[CKB_T_W2].fmt)) return 0;
     }
     const int group = m->Hl / m->Hkvl;
     return m->Il % 256 == 0 && m->d % 8 == 0 && (m->d == 64 || m->d == 128) && group <= 8 && m->Hl % m->Hkvl == 0;
 }
 
+/* Buffers of a prompt of T tokens.  Layers agree on nothing but their shapes, so the partial sums are sized over all of them. */
 static int prefill_buffers(KqModel *m, int T)
 {
-    if (T <= m->pf_tokens) return 0;
+    const size_t t = (size_t)T, kvw = (size_t)m->Hkvl * m->d, widest = (size_t)(m->Da > m->Ala ? m->Da : m->Ala) > (size_t)m->Il ? (size_t)(m->Da > m->Ala ? m->Da : m->Ala) : (size_t)m->Il;
+    size_t need[PF_BUFFERS] = { t * m->Da * 4, t * m->Da * 4, t * m->Da * 4, t * m->Al * 4, t * kvw * 4, t * kvw * 4, t * m->Al * 4, t * m->Al * 4, t * 2 * m->Il * 4 };
+    need[PF_ROWS] = (t + 127) * (widest / 256) * 548;          /* operand tiles of any width up to 128: 548 bytes per token and superblock, more than the other forms */
+    need[PF_IDS] = t * sizeof(int32_t);
+    WidthMemo memo[CKB_T_PER_LAYER] = { { 0 } };
+    if (T > PF_SMALL)
+        for (int l = 0; l < m->c.num_layers; ++l) {
+            const Tensor *w = m->layers[l].t;
+            static const int which[6][3] = { { CKB_T_WQ, CKB_T_WQ, PF_PART0 }, { CKB_T_WK, CKB_T_WQ, PF_PART1 }, { CKB_T_WV, CKB_T_WQ, PF_PART2 },
+                                             { CKB_T_WO, CKB_T_WO, PF_PART0 }, { CKB_T_W1, CKB_T_W1, PF_PART0 }, { CKB_T_W2, CKB_T_W2, PF_PART0 } };
+            for (int i = 0; i < 6; ++i) {
+                const Tensor *p = &w[which[i][0]];
+                const int nt = tile_width(&w[which[i][1]], T, &memo[which[i][1]]);
+                const size_t b = nt ? ckb_gemm_tc_part_bytes(tc_format(p), nt, T, p->rows, p->cols) : 0;
+                if (b > need[which[i][2]]) need[which[i][2]] = b;
+            }
+        }
+    int grow = 0;
+    size_t total = 0;
+    for (int i = 0; i < PF_BUFFERS; ++i) {
+        if (need[i] <= m->pf_cap[i]) need[i] = m->pf_cap[i];
+        else grow = 1;
+        total += align_up(need[i] + 256, 256);
+    }
+    if (!grow) return 0;
+    /* one allocation for all of them: each costs tens of microseconds, which a first prompt pays */
     cudaStreamSynchronize(ckb_stream(NULL));
-    void **ptrs[] = { (void **)&m->pf_x, (void **)&m->pf_delta, (void **)&m->pf_o, (void **)&m->pf_q, (void **)&m->pf_k, (void **)&m->pf_v, (void **)&m->pf_qh,
-                      (void **)&m->pf_oh, (void **)&m->pf_gu, (void **)&m->pf_hq, (void **)&m->pf_aq, (void **)&m->pf_mq };
-    for (unsigned i = 0; i < sizeof ptrs / sizeof ptrs[0]; ++i) { if (*ptrs[i]) cudaFree(*ptrs[i]); *ptrs[i] = NULL; }
-    m->pf_tokens = 0;
-    const size_t t = (size_t)T, kvw = (size_t)m->Hkvl * m->d;
-    const size_t sizes[] = { t * m->Da * 4, t * m->Da * 4, t * m->Da * 4, t * m->Al * 4, t * kvw * 4, t * kvw * 4, t * m->Al * 4, t * m->Al * 4, t * 2 * m->Il * 4,
-                             t * (m->Da / 256) * 292, t * (m->Ala / 256) * 292, t * (m->Il / 256) * 292 };
-    for (unsigned i = 0; i < sizeof ptrs / sizeof ptrs[0]; ++i)
-        if (ckb_check_cuda((int)cudaMalloc(ptrs[i], sizes[i] + 256), "cudaMalloc(prefill)")) return CKB_ERR_CUDA;
+    if (m->pf_arena) cudaFree(m->pf_arena);
+    m->pf_arena = NULL;
+    memset(m->pf_cap, 0, sizeof m->pf_cap);
+    if (ckb_check_cuda((int)cudaMalloc((void **)&m->pf_arena, total), "cudaMalloc(prefill)")) return CKB_ERR_CUDA;
+    void **ptrs[PF_BUFFERS] = { (void **)&m->pf_x, (void **)&m->pf_delta, (void **)&m->pf_o, (void **)&m->pf_q, (void **)&m->pf_k, (void **)&m->pf_v, (void **)&m->pf_qh,
+                                (void **)&m->pf_oh, (void **)&m->pf_gu, (void **)&m->pf_rows, (void **)&m->pf_part[0], (void **)&m->pf_part[1], (void **)&m->pf_part[2], (void **)&m->pf_ids };
+    size_t at = 0;
+    for (int i = 0; i < PF_BUFFERS; ++i) {
+        *ptrs[i] = m->pf_arena + at;
+        m->pf_cap[i] = need[i];
+        at += align_up(need[i] + 256, 256);
+    }
     /* rows wider than the data (Da > D) keep a zero tail: the GEMMs write only the first D columns */
-    cudaMemsetAsync(m->pf_delta, 0, sizes[1], ckb_stream(NULL));
-    cudaMemsetAsync(m->pf_o, 0, sizes[2], ckb_stream(NULL));
-    m->pf_tokens = T;
+    cudaMemsetAsync(m->pf_delta, 0, need[PF_DELTA], ckb_stream(NULL));
+    cudaMemsetAsync(m->pf_o, 0, need[PF_O], ckb_stream(NULL));
     return 0;
 }
 
-static int prefill_gemm(const Tensor *w, const uint8_t *xq, float *y, int ldc, int T, void *st)
+/* y = W . rows, the rows (m->pf_rows) in the form that `nt` and the format say; `lane`: which partial-sum buffer */
+static int prefill_gemm(KqModel *m, const Tensor *w, int nt, float *y, int ldc, int T, int lane, void *st)
 {
-    const int rc = ckb_launch_gemm_tc(w->fmt == FMT_Q6K, xq, w->fmt == FMT_Q6K ? w->planar : w->w, NULL, y, ldc, T, w->rows, w->cols, 16, st);
-    return rc == -1 ? ckb_fail(CKB_ERR_SHAPE, "prefill: projection %d x %d not handled by the tensor-core GEMM", w->rows, w->cols) : rc;
+    int rc = -1;
+    if (w->fmt == FMT_Q50) rc = ckb_launch_gemm_q50_mma(m->pf_rows, w->planar, NULL, y, ldc, T, w->rows, w->cols, 1, st);
+    else if (nt) rc = ckb_launch_gemm_tc_tiles(tc_format(w), m->pf_rows, nt, tc_weights(w), y, ldc, T, w->rows, w->cols, m->pf_part[lane], m->pf_cap[PF_PART0 + lane], st);
+    else {
+        rc = w->fmt == FMT_Q4K ? ckb_launch_gemm_q4k_mma(m->pf_rows, w->w, NULL, y, ldc, T, w->rows, w->cols, st)
+                               : ckb_launch_gemm_q6k_mma(m->pf_rows, w->planar, NULL, y, ldc, T, w->rows, w->cols, st);
+        if (rc == -1) rc = ckb_launch_gemm_tc(tc_format(w), m->pf_rows, tc_weights(w), NULL, y, ldc, T, w->rows, w->cols, 16, st);
+    }
+    return rc == -1 ? ckb_fail(CKB_ERR_SHAPE, "prefill: projection %d x %d not handled by the batched products", w->rows, w->cols) : rc;
+}
+
+/* x += delta, normalised rows for `consumer` */
+static int prefill_norm(KqModel *m, const float *delta, const Tensor *gamma, const Tensor *consumer, int nt, int T, void *st)
+{
+    const float *g = (const float *)gamma->w;
+    if (fmt_block32(consumer->fmt)) return ckb_add_rmsnorm_q80_planar(m->pf_x, delta, g, m->pf_rows, T, m->D, m->Da, consumer->cols, m->c.rms_eps, st);
+    if (nt) return ckb_add_rmsnorm_tiles(m->pf_x, delta, g, m->pf_rows, nt, T, m->D, m->Da, m->c.rms_eps, st);
+    return ckb200_dev_add_rmsnorm_q8k(m->pf_x, delta, g, m->pf_rows, NULL, T, m->D, m->Da, m->c.rms_eps, st);
+}
+
+/* the three products over one set of rows, side by side; the 32-token form of the tcgen05 kernel shares the library's scratch and stays on one stream */
+static int prefill_qkv(KqModel *m, const Tensor *t, int nt, int T, void *st)
+{
+    const Tensor *w[3] = { &t[CKB_T_WQ], &t[CKB_T_WK], &t[CKB_T_WV] };
+    float *out[3] = { m->pf_q, m->pf_k, m->pf_v };
+    const int ld[3] = { m->Al, m->Hkvl * m->d, m->Hkvl * m->d };
+    int apart = ckb_tune_get("model_qkv_streams", 1);
+    for (int i = 0; i < 3 && apart && !nt && !fmt_block32(w[0]->fmt); ++i)
+        apart = w[i]->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_takes(m->pf_rows, w[i]->w, T, w[i]->rows, w[i]->cols) : ckb_gemm_q6k_mma_takes(m->pf_rows, w[i]->planar, T, w[i]->rows, w[i]->cols);
+    cudaStream_t main_st = (cudaStream_t)st;
+    int rc;
+    if (apart && ckb_check_cuda((int)cudaEventRecord(m->ev_fork, main_st), "fork")) return CKB_ERR_CUDA;
+    if ((rc = prefill_gemm(m, w[0], nt, out[0], ld[0], T, 0, st))) return rc;
+    for (int i = 1; i < 3; ++i) {
+        cudaStream_t s = apart ? m->side[i - 1] : main_st;
+        if (apart && ckb_check_cuda((int)cudaStreamWaitEvent(s, m->ev_fork, 0), "fork wait")) return CKB_ERR_CUDA;
+        if ((rc = prefill_gemm(m, w[i], nt, out[i], ld[i], T, i, s))) return rc;
+        if (apart && (ckb_check_cuda((int)cudaEventRecord(m->ev_join[i - 1], s), "join") || ckb_check_cuda((int)cudaStreamWaitEvent(main_st, m->ev_join[i - 1], 0), "join wait"))) return CKB_ERR_CUDA;
+    }
+    return 0;
 }
 
 static int issue_prefill(KqModel *m, int T, void *st)
 {
     const CKB200ModelConfig *c = &m->c;
-    const int L = c->num_layers, kvw = m->Hkvl * m->d;
+    const int L = c->num_layers, before = m->host_pos;
     int rc;
-    rc = ckb200_dev_embedding_rows(m->tokens_dev, T, c->vocab_size, m->emb.w, m->emb.fmt, m->emb.cols, m->pf_x, m->Da, m->D, st);
+    rc = ckb200_dev_embedding_rows(m->pf_ids, T, c->vocab_size, m->emb.w, m->emb.fmt, m->emb.cols, m->pf_x, m->Da, m->D, st);
     if (rc) return rc;
     const float *delta = NULL;
+    WidthMemo memo[4] = { { 0 } };
     for (int l = 0; l < L; ++l) {
         Tensor *t = m->layers[l].t;
         float *kc = (float *)kv_at(m, l, 0), *vc = (float *)kv_at(m, l, 1);
-        if ((rc = ckb200_dev_add_rmsnorm_q8k(m->pf_x, delta, (const float *)t[CKB_T_LN1].w, m->pf_hq, NULL, T, m->D, m->Da, c->rms_eps, st))) return rc;
-        if ((rc = prefill_gemm(&t[CKB_T_WQ], m->pf_hq, m->pf_q, m->Al, T, st))) return rc;
-        ckb_gemm_tc_hint_same_activations(1);                  /* k and v read the rows q read: one set of operand tiles */
-        rc = prefill_gemm(&t[CKB_T_WK], m->pf_hq, m->pf_k, kvw, T, st);
-        if (!rc) rc = prefill_gemm(&t[CKB_T_WV], m->pf_hq, m->pf_v, kvw, T, st);
-        ckb_gemm_tc_hint_same_activations(0);
+        const int nt_q = tile_width(&t[CKB_T_WQ], T, &memo[0]), nt_o = tile_width(&t[CKB_T_WO], T, &memo[1]), nt_1 = tile_width(&t[CKB_T_W1], T, &memo[2]),
+                  nt_2 = tile_width(&t[CKB_T_W2], T, &memo[3]);
+        if ((rc = prefill_norm(m, delta, &t[CKB_T_LN1], &t[CKB_T_WQ], nt_q, T, st))) return rc;
+        if ((rc = prefill_qkv(m, t, nt_q, T, st))) return rc;
+        if ((rc = ckb200_dev_prefill_rope_scatter(m->pf_q, m->pf_k, m->pf_v, m->pf_qh, kc, vc, m->rope_cos, m->rope_sin, T, m->Hl, m->Hkvl, m->d, c->max_seq_len, before, st))) return rc;
+        if (before) {
+            rc = ckb_launch_attn_prefill_mma(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, before, 1, st);
+            if (rc == -1) rc = ckb_fail(CKB_ERR_SHAPE, "prefill: attention over earlier keys not handled");
+        } else rc = ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st);
         if (rc) return rc;
-        if ((rc = ckb200_dev_prefill_rope_scatter(m->pf_q, m->pf_k, m->pf_v, m->pf_qh, kc, vc, m->rope_cos, m->rope_sin, T, m->Hl, m->Hkvl, m->d, c->max_seq_len, 0, st))) return rc;
-        if ((rc = ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st))) return rc;
-        if ((rc = ckb200_dev_prefill_gather_q8k(m->pf_oh, m->pf_aq, T, m->Hl, m->d, m->Ala, st))) return rc;
-        if ((rc = prefill_gemm(&t[CKB_T_WO], m->pf_aq, m->pf_o, m->Da, T, st))) return rc;
-        if ((rc = ckb200_dev_add_rmsnorm_q8k(m->pf_x, m->pf_o, (const float *)t[CKB_T_LN2].w, m->pf_hq, NULL, T, m->D, m->Da, c->rms_eps, st))) return rc;
-        if ((rc = prefill_gemm(&t[CKB_T_W1], m->pf_hq, m->pf_gu, 2 * m->Il, T, st))) return rc;
-        if ((rc = ckb200_dev_swiglu_q8k(m->pf_gu, m->pf_mq, T, m->Il, st))) return rc;
-        if ((rc = prefill_gemm(&t[CKB_T_W2], m->pf_mq, m->pf_delta, m->Da, T, st))) return rc;
+        if (fmt_block32(t[CKB_T_WO].fmt)) rc = ckb_prefill_gather_q80_planar(m->pf_oh, m->pf_rows, T, m->Hl, m->d, t[CKB_T_WO].cols, st);
+        else if (nt_o) rc = ckb_prefill_gather_tiles(m->pf_oh, m->pf_rows, nt_o, T, m->Hl, m->d, m->Ala, st);
+        else rc = ckb200_dev_prefill_gather_q8k(m->pf_oh, m->pf_rows, T, m->Hl, m->d, m->Ala, st);
+        if (rc) return rc;
+        if ((rc = prefill_gemm(m, &t[CKB_T_WO], nt_o, m->pf_o, m->Da, T, 0, st))) return rc;
+        if ((rc = prefill_norm(m, m->pf_o, &t[CKB_T_LN2], &t[CKB_T_W1], nt_1, T, st))) return rc;
+        if ((rc = prefill_gemm(m, &t[CKB_T_W1], nt_1, m->pf_gu, 2 * m->Il, T, 0, st))) return rc;
+        if ((rc = nt_2 ? ckb_swiglu_tiles(m->pf_gu, m->pf_rows, nt_2, T, m->Il, st) : ckb200_dev_swiglu_q8k(m->pf_gu, m->pf_rows, T, m->Il, st))) return rc;
+        if ((rc = prefill_gemm(m, &t[CKB_T_W2], nt_2, m->pf_delta, m->Da, T, 0, st))) return rc;
         delta = m->pf_delta;
     }
     /* logits of the last token only: its residual row, final norm, LM head as a GEMV */
     const size_t last = (size_t)(T - 1) * m->Da;
-    if ((rc = ckb200_dev_add_rmsnorm_q8k(m->pf_x + last, delta ? delta + last : NULL, (const float *)m->final_gamma.w, m->hq, NULL, 1, m->D, m->Da, c->rms_eps, st))) return rc;
-    return matvec(m, &m->lm_head, m->hq, m->logits, m->Vl, st);
+    const float *gamma = (const float *)m->final_gamma.w;
+    if (fmt_block32(m->lm_head.fmt)) rc = ckb200_dev_add_rmsnorm_q8_0(m->pf_x + last, delta ? delta + last : NULL, gamma, m->hq, 1, m->D, m->Da, m->lm_head.cols, c->rms_eps, st);
+    else rc = ckb200_dev_add_rmsnorm_q8k(m->pf_x + last, delta ? delta + last : NULL, gamma, m->hq, NULL, 1, m->D, m->Da, c->rms_eps, st);
+    return rc ? rc : matvec(m, &m->lm_head, m->hq, m->logits, m->Vl, st);
 }
 
 static int kq_extend(CKB200Model *model, const int32_t *tokens, int count, const int32_t *want, int n_want, float *logits_host)
@@ -949,21 +1069,13 @@ static int kq_extend(CKB200Model *model, const int32_t *tokens, int count, const
     if (n_want > 1 || (n_want == 1 && want[0] != count - 1) || !prefill_ok(m, count)) return -1;
     cudaStream_t st = ckb_stream(NULL);
     if (prefill_buffers(m, count)) return CKB_ERR_CUDA;
-    int32_t *ids = NULL;
-    if (ckb_check_cuda((int)cudaMalloc((void **)&ids, (size_t)count * sizeof(int32_t)), "cudaMalloc(prompt ids)")) return CKB_ERR_CUDA;
-    int rc = ckb_check_cuda((int)cudaMemcpyAsync(ids, tokens, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, st), "prompt ids H2D");
-    int32_t *saved = m->tokens_dev;
-    m->tokens_dev = ids;
+    const int32_t end = m->host_pos + count;
+    int rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pf_ids, tokens, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, st), "prompt ids H2D");
     if (!rc) rc = issue_prefill(m, count, st);
-    m->tokens_dev = saved;
-    if (!rc) {
-        const int32_t p = count;
-        rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pos_dev, &p, sizeof p, cudaMemcpyHostToDevice, st), "prefill pos");
-    }
+    if (!rc) rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pos_dev, &end, sizeof end, cudaMemcpyHostToDevice, st), "prefill pos");
     if (!rc && n_want) rc = ckb_check_cuda((int)cudaMemcpyAsync(logits_host, m->logits, (size_t)m->Vl * sizeof(float), cudaMemcpyDeviceToHost, st), "logits D2H");
     if (!rc) rc = ckb_sync_check(st, "model_prefill");
-    cudaFree(ids);
-    if (!rc) m->host_pos = count;
+    if (!rc) m->host_pos = end;
     return rc;
 }
 

@@ -7,7 +7,9 @@
 //   prefill_rope_scatter   rope_forward_qk (rotate-half, src/kernels/rope_kernels.c:320-417) on q and k of every token,
 //                          q -> [H][T][d], k and v -> cache rows pos0 .. pos0 + T - 1 (kv_cache_store per token)
 //   prefill_gather_q8k     attention output [H][T][d] -> token rows, quantised to Q8_K for the o projection (quantize_row_q8_k)
+#include "add_rmsnorm_q8k.cuh"
 #include "launch.h"
+#include "pdl.cuh"
 #include "q8k_block.cuh"
 #include "runtime.h"
 
@@ -54,6 +56,8 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const floa
                                                                       const float *__restrict__ cos_cache, const float *__restrict__ sin_cache, int T, int H,
                                                                       int Hkv, int d, int max_seq, int pos0)
 {
+    pdl_wait();
+    pdl_trigger();
     const int half = d / 2, q4 = half / 4;
     const long long per_tok = (long long)(H + 2 * Hkv) * q4, n = (long long)T * per_tok;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -72,7 +76,7 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const floa
             src = v_tm + ((size_t)t * Hkv + (h - H - Hkv)) * d;
             dst = vc + ((size_t)(h - H - Hkv) * max_seq + pos) * d;
         }
-        const float4 a = *reinterpret_cast<const float4 *>(src + j), b = *reinterpret_cast<const float4 *>(src + j + half);
+        const float4 a = __ldcg(reinterpret_cast<const float4 *>(src + j)), b = __ldcg(reinterpret_cast<const float4 *>(src + j + half));
         if (h >= H + Hkv) {
             *reinterpret_cast<float4 *>(dst + j) = a;
             *reinterpret_cast<float4 *>(dst + j + half) = b;
@@ -89,9 +93,13 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const floa
     }
 }
 
-// one warp per (token, 256-element block): lane l takes elements 8l .. 8l+7 of the block (d is a multiple of 8, so they lie in one head)
-__global__ void __launch_bounds__(256) prefill_gather_q8k_kernel(const float *__restrict__ out_hm, uint8_t *__restrict__ aq, int T, int H, int d, int cols)
+// one warp per (token, 256-element block): lane l takes elements 8l .. 8l+7 of the block (d is a multiple of 8, so they lie in one head); TILES: into
+// operand tiles of tile_nt tokens
+template <bool TILES>
+__global__ void __launch_bounds__(256) prefill_gather_q8k_kernel(const float *__restrict__ out_hm, uint8_t *__restrict__ aq, int T, int H, int d, int cols, int tile_nt)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, nb = cols / QK_K;
     const long long blk = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (blk >= (long long)T * nb) return;
@@ -100,13 +108,28 @@ __global__ void __launch_bounds__(256) prefill_gather_q8k_kernel(const float *__
     float v[8];
     if (e0 < H * d) {
         const int h = e0 / d, e = e0 - h * d;
-        const float4 lo = *reinterpret_cast<const float4 *>(out_hm + ((size_t)h * T + t) * d + e), hi = *reinterpret_cast<const float4 *>(out_hm + ((size_t)h * T + t) * d + e + 4);
+        const float4 *src = reinterpret_cast<const float4 *>(out_hm + ((size_t)h * T + t) * d + e);
+        const float4 lo = __ldcg(src), hi = __ldcg(src + 1);
         v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = 0.0f;             // the zero tail of a row narrower than its 256-aligned width
     }
-    quantize_block_q8k(v, aq + (size_t)blk * Q8K_BYTES, lane);
+    if (TILES) quantize_block_q8k_tile(v, aq + ((size_t)(t / tile_nt) * nb + b) * q8k_tile_bytes(tile_nt), tile_nt, t % tile_nt, lane);
+    else quantize_block_q8k(v, aq + (size_t)blk * Q8K_BYTES, lane);
+}
+
+// the same for a consumer with 32-element blocks: one warp per (token, block), row-planar Q8_0 rows of cols = H * d elements
+__global__ void __launch_bounds__(256) prefill_gather_q80_kernel(const float *__restrict__ out_hm, uint8_t *__restrict__ planar, int T, int H, int d, int cols)
+{
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, nb = cols / 32;
+    const long long blk = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (blk >= (long long)T * nb) return;
+    const int t = (int)(blk / nb), b = (int)(blk - (long long)t * nb), e0 = 32 * b + lane, h = e0 / d;
+    const float v = h < H ? __ldcg(out_hm + ((size_t)h * T + t) * d + (e0 - h * d)) : 0.0f;
+    store_block_q80_planar(v, planar + (size_t)t * (((size_t)nb * Q80_BYTES + 15) & ~(size_t)15), nb, b, lane);
 }
 
 }  // namespace ckb
@@ -126,9 +149,8 @@ extern "C" int ckb200_dev_prefill_rope_scatter(const float *q_tm, const float *k
     if (head_dim % 8 == 0 && (all & 15) == 0) {
         const long long n4 = n / 4;
         const unsigned g4 = (unsigned)((n4 + 255) / 256 < 4736 ? (n4 + 255) / 256 : 4736);
-        prefill_rope_scatter_v4_kernel<<<g4, 256, 0, ckb_stream(stream)>>>(q_tm, k_tm, v_tm, q_hm, k_cache, v_cache, cos_cache, sin_cache, tokens, num_heads,
-                                                                           num_kv_heads, head_dim, max_seq_len, pos0);
-        return ckb_check_launch("prefill_rope_scatter");
+        return launch_pdl("prefill_rope_scatter", prefill_rope_scatter_v4_kernel, dim3(g4), dim3(256), (size_t)0, ckb_stream(stream), q_tm, k_tm, v_tm, q_hm, k_cache, v_cache,
+                          cos_cache, sin_cache, tokens, num_heads, num_kv_heads, head_dim, max_seq_len, pos0);
     }
     const unsigned grid = (unsigned)((n + 255) / 256 < 4736 ? (n + 255) / 256 : 4736);
     prefill_rope_scatter_kernel<<<grid, 256, 0, ckb_stream(stream)>>>(q_tm, k_tm, v_tm, q_hm, k_cache, v_cache, cos_cache, sin_cache, tokens, num_heads, num_kv_heads,
@@ -136,13 +158,31 @@ extern "C" int ckb200_dev_prefill_rope_scatter(const float *q_tm, const float *k
     return ckb_check_launch("prefill_rope_scatter");
 }
 
-extern "C" int ckb200_dev_prefill_gather_q8k(const float *out_hm, void *out_q8, int tokens, int num_heads, int head_dim, int cols, void *stream)
+template <bool TILES>
+static int gather_launch(const float *out_hm, void *out_q8, int tokens, int num_heads, int head_dim, int cols, int tile_nt, void *stream)
 {
     if (!out_hm || !out_q8 || tokens <= 0 || num_heads <= 0) return 0;
     if (head_dim % 8 || cols % QK_K || cols < num_heads * head_dim || ((uintptr_t)out_hm & 15))
         return ckb_fail(CKB_ERR_SHAPE, "prefill_gather_q8k: head_dim %d, cols %d", head_dim, cols);
     if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
     const long long blocks = (long long)tokens * (cols / QK_K);
-    prefill_gather_q8k_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, ckb_stream(stream)>>>(out_hm, (uint8_t *)out_q8, tokens, num_heads, head_dim, cols);
-    return ckb_check_launch("prefill_gather_q8k");
+    return launch_pdl("prefill_gather_q8k", prefill_gather_q8k_kernel<TILES>, dim3((unsigned)((blocks + 7) / 8)), dim3(256), (size_t)0, ckb_stream(stream), out_hm, (uint8_t *)out_q8,
+                      tokens, num_heads, head_dim, cols, tile_nt);
+}
+extern "C" int ckb200_dev_prefill_gather_q8k(const float *out_hm, void *out_q8, int tokens, int num_heads, int head_dim, int cols, void *stream)
+{
+    return gather_launch<false>(out_hm, out_q8, tokens, num_heads, head_dim, cols, 0, stream);
+}
+extern "C" int ckb_prefill_gather_tiles(const float *out_hm, void *tiles, int tile_nt, int tokens, int num_heads, int head_dim, int cols, void *stream)
+{
+    return gather_launch<true>(out_hm, tiles, tokens, num_heads, head_dim, cols, tile_nt, stream);
+}
+extern "C" int ckb_prefill_gather_q80_planar(const float *out_hm, void *planar, int tokens, int num_heads, int head_dim, int cols, void *stream)
+{
+    if (!out_hm || !planar || tokens <= 0 || num_heads <= 0) return 0;
+    if (cols % 32 || cols < num_heads * head_dim) return ckb_fail(CKB_ERR_SHAPE, "prefill_gather_q80: head_dim %d, cols %d", head_dim, cols);
+    if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
+    const long long blocks = (long long)tokens * (cols / 32);
+    return launch_pdl("prefill_gather_q80", prefill_gather_q80_kernel, dim3((unsigned)((blocks + 7) / 8)), dim3(256), (size_t)0, ckb_stream(stream), out_hm, (uint8_t *)planar, tokens,
+                      num_heads, head_dim, cols);
 }

@@ -20,16 +20,19 @@ namespace ckb {
 // grid = tokens, block = aligned / 4 threads rounded up to a warp multiple, at most 1024.
 // x[t] += delta[t] (when delta != NULL; x is updated in place), then h = rmsnorm(x[t]) * gamma, zero beyond
 // d_model, quantised to Q8_K blocks of `aligned` elements.  Optionally also writes the fp32 normalised row.
-// Every thread issues all of its 16-byte loads before it uses any of them (one L2 round trip per row).
+// Every thread issues all of its 16-byte loads before it uses any of them (one L2 round trip per row).  TILES (prompts): straight into the operand
+// tiles of the tensor-core product, which saves it a pass over the quantised rows (5 us and a launch at 512 tokens of 4096).
+template <bool TILES>
 __global__ void __launch_bounds__(1024) add_rmsnorm_q8k_kernel(float *__restrict__ x, const float *__restrict__ delta,
                                                                const float *__restrict__ gamma, uint8_t *__restrict__ out_q8,
-                                                               float *__restrict__ norm_out, int d_model, int aligned, float eps)
+                                                               float *__restrict__ norm_out, int d_model, int aligned, float eps, int tile_nt)
 {
     extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
-    pdl_trigger();
+    if (!TILES) pdl_trigger();
     const ArqGamma pre = arq_prefetch_gamma(gamma, d_model);
     pdl_wait();
+    if (TILES) pdl_trigger();           // the product that follows reads weights ahead of its own wait: by then everything before this kernel is complete
     const int t = blockIdx.x;
     float *xr = x + (size_t)t * aligned;
     const float *dr = delta ? delta + (size_t)t * aligned : nullptr;
@@ -58,11 +61,12 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_q8k_kernel(float *__restrict
             arq_keep_piece(v, i, d_model, row, ss);
         }
     }
-    arq_norm_quant(ss, row, red, gamma, out_q8, norm_out, t, d_model, aligned, eps, &pre);
+    arq_norm_quant<TILES>(ss, row, red, gamma, out_q8, norm_out, t, d_model, aligned, eps, &pre, tile_nt);
 }
 
 // add_rmsnorm_q8k for a consumer that takes Q8_0 activations (Q8_0 / Q5_0 weights): the same row kernel, Q8_0 blocks of the
 // first `cols` elements out
+template <bool PLANAR>
 __global__ void __launch_bounds__(1024) add_rmsnorm_q80_kernel(float *__restrict__ x, const float *__restrict__ delta, const float *__restrict__ gamma,
                                                                uint8_t *__restrict__ out_q80, int d_model, int aligned, int cols, float eps)
 {
@@ -84,15 +88,16 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_q80_kernel(float *__restrict
         }
         arq_keep_piece(v, i, d_model, row, ss);
     }
-    arq_norm_quant_q80(ss, row, red, gamma, out_q80, t, d_model, cols, eps);
+    arq_norm_quant_q80<PLANAR>(ss, row, red, gamma, out_q80, t, d_model, cols, eps);
 }
 
 // one warp per 256-element block of the output: out = silu(gate) * up, quantised to Q8_K (VEC: gate_up is 16-byte aligned)
-template <bool VEC>
-__global__ void __launch_bounds__(128) swiglu_q8k_kernel(const float *__restrict__ gate_up, uint8_t *__restrict__ out_q8, int tokens, int dim)
+template <bool VEC, bool TILES>
+__global__ void __launch_bounds__(128) swiglu_q8k_kernel(const float *__restrict__ gate_up, uint8_t *__restrict__ out_q8, int tokens, int dim, int tile_nt)
 {
-    pdl_trigger();
+    if (!TILES) pdl_trigger();
     pdl_wait();
+    if (TILES) pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int nb = dim / QK_K;
     const long long blk = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -118,7 +123,8 @@ __global__ void __launch_bounds__(128) swiglu_q8k_kernel(const float *__restrict
         const float sg = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-gs[j])));
         v[j] = __fmul_rn(__fmul_rn(gs[j], sg), us[j]);
     }
-    quantize_block_q8k(v, out_q8 + blk * Q8K_BYTES, lane);
+    if (TILES) quantize_block_q8k_tile(v, out_q8 + ((size_t)(t / tile_nt) * nb + b) * q8k_tile_bytes(tile_nt), tile_nt, t % tile_nt, lane);
+    else quantize_block_q8k(v, out_q8 + blk * Q8K_BYTES, lane);
 }
 
 // One token per sequence.  q [B][H][d] is rotated in place; k [B][Hkv][d] is rotated and written, v copied,
@@ -244,8 +250,9 @@ static inline unsigned grid_for(long long n, int block, int cap) { long long g =
 
 using namespace ckb;
 
-extern "C" int ckb200_dev_add_rmsnorm_q8k(float *x, const float *delta, const float *gamma, void *out_q8, float *norm_out, int tokens,
-                                          int d_model, int aligned_embed_dim, float eps, void *stream)
+template <bool TILES>
+static int add_rmsnorm_launch(float *x, const float *delta, const float *gamma, void *out_q8, float *norm_out, int tokens, int d_model, int aligned_embed_dim, float eps,
+                              int tile_nt, void *stream)
 {
     if (!x || !gamma || !out_q8 || tokens <= 0 || d_model <= 0) return 0;
     if (aligned_embed_dim % QK_K || aligned_embed_dim < d_model) return ckb_fail(CKB_ERR_SHAPE, "add_rmsnorm_q8k: aligned width %d must be a multiple of 256 and >= d_model", aligned_embed_dim);
@@ -260,16 +267,27 @@ extern "C" int ckb200_dev_add_rmsnorm_q8k(float *x, const float *delta, const fl
     if (smem > 48 * 1024) {
         static size_t set = 0;
         if (smem > set) {
-            if (ckb_check_cuda((int)cudaFuncSetAttribute(add_rmsnorm_q8k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr")) return CKB_ERR_CUDA;
+            if (ckb_check_cuda((int)cudaFuncSetAttribute(add_rmsnorm_q8k_kernel<TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr")) return CKB_ERR_CUDA;
             set = smem;
         }
     }
-    return launch_pdl("add_rmsnorm_q8k", add_rmsnorm_q8k_kernel, dim3(tokens), dim3(threads), smem, ckb_stream(stream), x, delta, gamma,
-                      (uint8_t *)out_q8, norm_out, d_model, aligned_embed_dim, eps);
+    return launch_pdl("add_rmsnorm_q8k", add_rmsnorm_q8k_kernel<TILES>, dim3(tokens), dim3(threads), smem, ckb_stream(stream), x, delta, gamma,
+                      (uint8_t *)out_q8, norm_out, d_model, aligned_embed_dim, eps, tile_nt);
 }
 
-extern "C" int ckb200_dev_add_rmsnorm_q8_0(float *x, const float *delta, const float *gamma, void *out_q80, int tokens, int d_model,
-                                           int aligned_embed_dim, int cols, float eps, void *stream)
+extern "C" int ckb200_dev_add_rmsnorm_q8k(float *x, const float *delta, const float *gamma, void *out_q8, float *norm_out, int tokens,
+                                          int d_model, int aligned_embed_dim, float eps, void *stream)
+{
+    return add_rmsnorm_launch<false>(x, delta, gamma, out_q8, norm_out, tokens, d_model, aligned_embed_dim, eps, 0, stream);
+}
+// the same into operand tiles of tile_nt tokens (ckb_gemm_tc_tile_bytes)
+extern "C" int ckb_add_rmsnorm_tiles(float *x, const float *delta, const float *gamma, void *tiles, int tile_nt, int tokens, int d_model, int aligned_embed_dim, float eps, void *stream)
+{
+    return add_rmsnorm_launch<true>(x, delta, gamma, tiles, nullptr, tokens, d_model, aligned_embed_dim, eps, tile_nt, stream);
+}
+
+template <bool PLANAR>
+static int add_rmsnorm_q80_launch(float *x, const float *delta, const float *gamma, void *out_q80, int tokens, int d_model, int aligned_embed_dim, int cols, float eps, void *stream)
 {
     if (!x || !gamma || !out_q80 || tokens <= 0 || d_model <= 0) return 0;
     if (aligned_embed_dim % 4 || aligned_embed_dim < d_model || cols % 32 || cols > aligned_embed_dim || cols <= 0)
@@ -283,26 +301,41 @@ extern "C" int ckb200_dev_add_rmsnorm_q8_0(float *x, const float *delta, const f
     if (smem > 48 * 1024) {
         static size_t set = 0;
         if (smem > set) {
-            if (ckb_check_cuda((int)cudaFuncSetAttribute(add_rmsnorm_q80_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr")) return CKB_ERR_CUDA;
+            if (ckb_check_cuda((int)cudaFuncSetAttribute(add_rmsnorm_q80_kernel<PLANAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr")) return CKB_ERR_CUDA;
             set = smem;
         }
     }
-    return launch_pdl("add_rmsnorm_q80", add_rmsnorm_q80_kernel, dim3(tokens), dim3(threads), smem, ckb_stream(stream), x, delta, gamma, (uint8_t *)out_q80,
+    return launch_pdl("add_rmsnorm_q80", add_rmsnorm_q80_kernel<PLANAR>, dim3(tokens), dim3(threads), smem, ckb_stream(stream), x, delta, gamma, (uint8_t *)out_q80,
                       d_model, aligned_embed_dim, cols, eps);
 }
 
-extern "C" int ckb200_dev_swiglu_q8k(const float *gate_up, void *out_q8, int tokens, int dim, void *stream)
+extern "C" int ckb200_dev_add_rmsnorm_q8_0(float *x, const float *delta, const float *gamma, void *out_q80, int tokens, int d_model,
+                                           int aligned_embed_dim, int cols, float eps, void *stream)
+{
+    return add_rmsnorm_q80_launch<false>(x, delta, gamma, out_q80, tokens, d_model, aligned_embed_dim, cols, eps, stream);
+}
+// the same into the row-planar layout of the batched product
+extern "C" int ckb_add_rmsnorm_q80_planar(float *x, const float *delta, const float *gamma, void *out_planar, int tokens, int d_model, int aligned_embed_dim, int cols, float eps,
+                                          void *stream)
+{
+    return add_rmsnorm_q80_launch<true>(x, delta, gamma, out_planar, tokens, d_model, aligned_embed_dim, cols, eps, stream);
+}
+
+template <bool TILES>
+static int swiglu_launch(const float *gate_up, void *out_q8, int tokens, int dim, int tile_nt, void *stream)
 {
     if (!gate_up || !out_q8 || tokens <= 0 || dim <= 0) return 0;
     if (dim % QK_K) return ckb_fail(CKB_ERR_SHAPE, "swiglu_q8k: dim %d is not a multiple of 256", dim);
     if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
     const long long nblocks = (long long)tokens * (dim / QK_K);
     if (((uintptr_t)gate_up & 15) == 0)
-        return launch_pdl("swiglu_q8k", swiglu_q8k_kernel<true>, dim3((unsigned)((nblocks + 3) / 4)), dim3(128), 0, ckb_stream(stream), gate_up,
-                          (uint8_t *)out_q8, tokens, dim);
-    return launch_pdl("swiglu_q8k", swiglu_q8k_kernel<false>, dim3((unsigned)((nblocks + 3) / 4)), dim3(128), 0, ckb_stream(stream), gate_up,
-                      (uint8_t *)out_q8, tokens, dim);
+        return launch_pdl("swiglu_q8k", swiglu_q8k_kernel<true, TILES>, dim3((unsigned)((nblocks + 3) / 4)), dim3(128), 0, ckb_stream(stream), gate_up,
+                          (uint8_t *)out_q8, tokens, dim, tile_nt);
+    return launch_pdl("swiglu_q8k", swiglu_q8k_kernel<false, TILES>, dim3((unsigned)((nblocks + 3) / 4)), dim3(128), 0, ckb_stream(stream), gate_up,
+                      (uint8_t *)out_q8, tokens, dim, tile_nt);
 }
+extern "C" int ckb200_dev_swiglu_q8k(const float *gate_up, void *out_q8, int tokens, int dim, void *stream) { return swiglu_launch<false>(gate_up, out_q8, tokens, dim, 0, stream); }
+extern "C" int ckb_swiglu_tiles(const float *gate_up, void *tiles, int tile_nt, int tokens, int dim, void *stream) { return swiglu_launch<true>(gate_up, tiles, tokens, dim, tile_nt, stream); }
 
 extern "C" int ckb200_dev_rope_kv_store(float *q, const float *k, const float *v, float *k_cache, float *v_cache, const float *cos_cache,
                                         const float *sin_cache, const int *pos_dev, int batch, int num_heads, int num_kv_heads,

@@ -1,0 +1,94 @@
+"""Batched prompt passes behind keys that are already in the cache, over 32-element formats, and at the token counts where a pass changes its kernels:
+logits and every layer's new cache rows against the same tokens fed one by one through the decode step (itself checked against the CPU step)."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import cases
+import step_oracle as so
+
+pytestmark = pytest.mark.gpu
+
+QWEN = dict(embed_dim=384, num_heads=6, num_kv_heads=2, head_dim=64, intermediate_size=768, num_layers=2, vocab_size=500, max_seq_len=400, rms_eps=1e-6, rope_theta=1.0e6,
+            fmt_q=0, fmt_k=0, fmt_v=1, fmt_o=0, fmt_gate_up=0, fmt_down=1, fmt_lm_head=1)
+LLAMA = dict(QWEN, embed_dim=512, num_heads=8, num_kv_heads=2, head_dim=128, intermediate_size=1024, rms_eps=1e-5, rope_theta=5.0e5)
+Q5_0 = dict(QWEN, fmt_q=3, fmt_k=3, fmt_v=3, fmt_o=3, fmt_gate_up=3)
+
+
+def cosine(a, b):
+    a, b = a.astype(np.float64).reshape(-1), b.astype(np.float64).reshape(-1)
+    return float(a @ b / (np.linalg.norm(a) * np.linalg.norm(b)))
+
+
+@pytest.mark.parametrize("cfg", [QWEN, LLAMA, Q5_0], ids=["qwen", "llama", "q5_0"])
+@pytest.mark.parametrize("before,T", [(0, 16), (1, 17), (63, 64), (64, 65), (100, 129), (7, 300)])
+def test_portion_matches_decode_steps(ck, cfg, before, T):
+    so.bind_model_api(ck)
+    model = so.CpuModel(cfg, seed=11)
+    ids = np.random.default_rng(before + T).integers(0, cfg["vocab_size"], size=before + T).astype(np.int32)
+    Hkv, S, d = cfg["num_kv_heads"], cfg["max_seq_len"], cfg["head_dim"]
+    results = []
+    for batched in (1, 0):
+        handle = ck.ckb200_model_create(C.byref(so.make_cfg(cfg, batch=1)))
+        assert handle, ck.ckb200_last_error_message()
+        try:
+            so.upload_whole_model(ck, handle, model, 1)
+            ck.ckb200_tune_set(b"model_prefill", 0)
+            if before:
+                assert ck.ckb200_model_prefill(handle, cases.vptr(ids), before, None) == 0
+            ck.ckb200_tune_set(b"model_prefill", batched)
+            ck.ckb200_launch_count.restype = C.c_longlong
+            n0 = ck.ckb200_launch_count()
+            logits = np.full((1, cfg["vocab_size"]), np.nan, np.float32)
+            assert ck.ckb200_model_prefill(handle, cases.vptr(ids[before:]), T, cases.vptr(logits)) == 0, ck.ckb200_last_error_message()
+            if batched:
+                assert ck.ckb200_launch_count() - n0 < 45 * cfg["num_layers"], "the portion ran token by token"
+            assert ck.ckb200_model_get_pos(handle) == before + T
+            kv = np.zeros((cfg["num_layers"], 2, Hkv, S, d), np.float32)
+            assert ck.ckb200_copy_to_host(cases.vptr(kv), C.c_void_p(ck.ckb200_model_kv_device(handle, 0, 0)), kv.nbytes) == 0
+            results.append((logits, kv))
+        finally:
+            ck.ckb200_tune_set(b"model_prefill", 1)
+            ck.ckb200_model_free(handle)
+    (got, kv), (want, ref) = results
+    assert not kv[:, :, :, before + T:].any()
+    assert np.array_equal(kv[:, :, :, :before], ref[:, :, :, :before])
+    new, old = kv[:, :, :, before:before + T], ref[:, :, :, before:before + T]
+    for is_v in (0, 1):                                   # layer 0 sees the same rows: fp32 summation order only
+        assert float(np.max(np.abs(new[0, is_v] - old[0, is_v]))) <= 1e-4 * float(np.max(np.abs(old[0, is_v])))
+    # deeper layers: the bar that the repository sets for whole steps (values that round to the other side of an 8-bit step)
+    assert cosine(new, old) >= 0.9999
+    assert cosine(got, want) >= 0.9999
+
+
+@pytest.mark.parametrize("tile", [64, 128])
+@pytest.mark.parametrize("m,n,k", [(16, 40, 128), (65, 130, 384), (200, 300, 896)])
+def test_q5_0_product_is_bit_identical(ck, orc, tile, m, n, k):
+    """Q5_0 x Q8_0 over the planes: exact int32 block sums, fp32 in the reference's block order."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    w = cases.synth.make_weights("q5_0", n, k, seed=m)
+    aq = cases.quantize_act(orc, "oracle_", "q5_0", cases.synth.make_x(k, seed=n, rows=m), rows=m)
+    want = cases.gemm_nt(orc, "oracle_", "q5_0", aq, w, None, m, n, k)
+    raw, taq = torch.from_numpy(w).to(dev), torch.from_numpy(aq).to(dev)
+    ck.ckb200_q5_0_planar_bytes.restype = ck.ckb200_q8_0_planar_bytes.restype = C.c_size_t
+    wp = torch.empty(ck.ckb200_q5_0_planar_bytes(n, k) + 256, dtype=torch.uint8, device=dev)
+    ap = torch.empty(ck.ckb200_q8_0_planar_bytes(m, k) + 256, dtype=torch.uint8, device=dev)
+    c = torch.full((m, n + 3), float("nan"), device=dev)
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    assert ck.ckb200_dev_q5_0_to_planar(p(wp), p(raw), n, k, None) == 0
+    assert ck.ckb200_dev_q8_0_to_planar(p(ap), p(taq), m, k, None) == 0
+    try:
+        ck.ckb200_tune_set(b"gemm_q80_tile", tile)
+        assert ck.ckb_launch_gemm_q50_mma(p(ap), p(wp), None, p(c), n + 3, m, n, k, 0, None) == 0
+    finally:
+        ck.ckb200_tune_set(b"gemm_q80_tile", 0)
+    assert ck.ckb200_synchronize() == 0
+    got = c.cpu().numpy()
+    assert np.array_equal(got[:, :n], want)
+    assert np.isnan(got[:, n:]).all()
