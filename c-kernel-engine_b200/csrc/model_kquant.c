@@ -34,7 +34,7 @@
 #include "launch.h"
 #include "model_internal.h"
 #include "runtime.h"
-#include "step_fused.h"
+#include "step_persistent.h"
 
 /* tensor-core GEMM of gemm_tc.cu: wf 0 = Q4_K rows, 1 = Q6_K row-planar; -1 when the shape is not handled.  The workspace
  * (activation tiles + split-K partial sums) is the model's own: a pointer recorded in the step's graph must not come from
@@ -93,8 +93,12 @@ typedef struct {
     float *rope_cos, *rope_sin;
     /* activations */
     float *x, *prev, *q, *k, *v, *att, *o, *gu, *attn_scratch;
-    float *x2;              /* second residual row of the fused step (each fused launch reads one and writes the other) */
-    float *mf;              /* fp32 SwiGLU output of the fused step, round256(Il) wide, tail zero */
+    float *mf;              /* fp32 SwiGLU output of the one-launch step, round256(Il) wide, tail zero */
+    PsParams ps;            /* the one-launch step: arguments, table of layers, partial attention results, counters */
+    void *ps_table;
+    float *ps_part;
+    unsigned *ps_sync;
+    int ps_ready;
     int *attn_counters;     /* arrival counters of the attention kernel's in-launch split merge */
     /* batched prefill, grown on demand to the longest prompt seen: token-major rows, head-major attention tensors, quantised rows (Q8_K blocks, operand tiles of the
      * tensor-core product, or row-planar Q8_0), partial sums of the three products that run side by side, prompt ids */
@@ -128,6 +132,7 @@ static void *kv_at(const KqModel *m, int layer, int is_v)
 {
     return m->kv + ((size_t)layer * (size_t)m->kv_layer_stride + (is_v ? (size_t)m->c.batch * (size_t)m->kv_batch_stride : 0)) * (size_t)m->kv_eb;
 }
+static int ps_build(KqModel *m, cudaStream_t st);
 static int round256(int v) { return (v + 255) / 256 * 256; }
 
 static size_t fmt_row_bytes(int fmt, int cols)
@@ -267,7 +272,6 @@ CKB200Model *ckb200_model_create(const CKB200ModelConfig *cfg)
     DEV_ALLOC(m->hq, (size_t)B * (m->Da / 32) * 34 + (size_t)B * (m->Da / 256) * 292 + 256);
     DEV_ALLOC(m->aq, (size_t)B * (m->Ala / 32) * 34 + (size_t)B * (m->Ala / 256) * 292 + 256);
     DEV_ALLOC(m->mq, (size_t)B * ((m->Il + 255) / 256) * 292 * 2 + 256);
-    DEV_ALLOC(m->x2, (size_t)B * m->Da * sizeof(float));
     DEV_ALLOC(m->mf, (size_t)B * round256(m->Il) * sizeof(float));
     DEV_ALLOC(m->attn_counters, ckb200_attention_decode_counter_bytes(B, m->Hkvl) + 256);
     if (B >= MODEL_GEMM_MIN_BATCH) {
@@ -313,11 +317,10 @@ CKB200Model *ckb200_model_create(const CKB200ModelConfig *cfg)
     cudaMemsetAsync(m->x, 0, (size_t)B * m->Da * sizeof(float), st);
     cudaMemsetAsync(m->prev, 0, (size_t)B * m->Da * sizeof(float), st);
     cudaMemsetAsync(m->o, 0, (size_t)B * m->Da * sizeof(float), st);
-    cudaMemsetAsync(m->x2, 0, (size_t)B * m->Da * sizeof(float), st);
     cudaMemsetAsync(m->mf, 0, (size_t)B * round256(m->Il) * sizeof(float), st);
     cudaMemsetAsync(m->attn_counters, 0, ckb200_attention_decode_counter_bytes(B, m->Hkvl) + 256, st);
     ckb200_dev_rope_precompute_cache_split(m->rope_cos, m->rope_sin, S, m->d, cfg->rope_theta, NULL);
-    if (ckb_check_cuda((int)cudaStreamSynchronize(st), "model init")) { ckb200_model_free((CKB200Model *)m); return NULL; }
+    if (ps_build(m, st) || ckb_check_cuda((int)cudaStreamSynchronize(st), "model init")) { ckb200_model_free((CKB200Model *)m); return NULL; }
     return (CKB200Model *)m;
 }
 
@@ -325,8 +328,8 @@ static void kq_destroy(CKB200Model *model)
 {
     KqModel *m = (KqModel *)model;
     void *ptrs[] = { m->arena, m->planar_arena, m->kv, m->rope_cos, m->rope_sin, m->x, m->prev, m->o, m->q, m->k, m->v, m->att, m->gu,
-                     m->hq, m->aq, m->mq, m->attn_scratch, m->gemm_ws, m->x2, m->mf, m->attn_counters,
-                     m->pf_arena };
+                     m->hq, m->aq, m->mq, m->attn_scratch, m->gemm_ws, m->mf, m->attn_counters,
+                     m->pf_arena, m->ps_table, m->ps_part, m->ps_sync };
     for (size_t i = 0; i < sizeof ptrs / sizeof ptrs[0]; ++i) if (ptrs[i]) cudaFree(ptrs[i]);
     for (int i = 0; i < 2; ++i) {
         if (m->side[i]) cudaStreamDestroy(m->side[i]);
@@ -588,207 +591,102 @@ static int ensure_planar(KqModel *m, void *st)
     return 0;
 }
 
-/* ------------------------------------------------------------------ the fused step (one sequence, one GPU)
+/* ------------------------------------------------------------------ the one-launch step (one sequence, one GPU)
  *
- * Five launches per layer instead of thirteen (step_fused.cu):
- *   1. q | k | v projections  <- prologue: x += delta, RMSNorm, Q8_K;  epilogue: RoPE, KV-cache store
- *   2. attention over the cache, the split merge done by the last CTA of each kv head
- *   3. o projection            <- prologue: Q8_K of the attention row
- *   4. gate | up projection    <- prologue: x += o, RMSNorm, Q8_K;     epilogue: SwiGLU
- *   5. down projection         <- prologue: Q8_K of the SwiGLU row
- * and the LM head with the final norm in its prologue and the position increment at its end.  The residual row ping-pongs
- * between two buffers: every CTA of a launch reads the old row while the first CTA writes the new one. */
+ * step_persistent.cu: all layers and the LM head in one cooperative launch behind the embedding. */
 
-static int fused_fmt(const Tensor *t) { return t->fmt == FMT_Q4K ? SG_FMT_Q4K : (t->fmt == FMT_Q6K && t->planar ? SG_FMT_Q6K_PLANAR : -1); }
-
-static int fused_step_ok(const KqModel *m)
+static int ps_fmt(const Tensor *t)
 {
-    if (m->c.batch != 1 || m->c.tp_size != 1 || m->kv_eb != 4 || !ckb_tune_get("model_fused_step", 0)) return 0;
-    for (int l = 0; l < m->c.num_layers; ++l) {
-        static const int which[6] = { CKB_T_WQ, CKB_T_WK, CKB_T_WV, CKB_T_WO, CKB_T_W1, CKB_T_W2 };
-        for (int i = 0; i < 6; ++i)
-            if (fused_fmt(&m->layers[l].t[which[i]]) < 0) return 0;
-    }
-    if (fused_fmt(&m->lm_head) < 0) return 0;
-    return m->d % 2 == 0 && m->d / 2 <= 128 && m->Al % 2 == 0 && ckb_step_gemv_ctas_per_sm(m->Da / 256, SG_PRO_GLOBAL, 0) > 0 &&
-           ckb_step_gemv_ctas_per_sm(round256(m->Il) / 256, SG_PRO_GLOBAL, 0) > 0 && ckb_step_gemv_ctas_per_sm(m->Ala / 256, SG_PRO_GLOBAL, 0) > 0;
+    if (t->fmt == FMT_Q4K) return PS_FMT_Q4K;
+    if (!t->planar) return -1;
+    return t->fmt == FMT_Q6K ? PS_FMT_Q6K_PLANAR : (t->fmt == FMT_Q50 ? PS_FMT_Q50_PLANAR : -1);
 }
 
-static void seg_set(StepSeg *sg, const Tensor *t, float *out, int epi)
+static void ps_seg(PsSeg *s, const Tensor *t, int cta0, int ncta)
 {
-    sg->fmt = fused_fmt(t);
-    sg->W = (const uint8_t *)(sg->fmt == SG_FMT_Q6K_PLANAR ? t->planar : t->w);
-    sg->out = out;
-    sg->M = t->rows;
-    sg->epi = epi;
+    memset(s, 0, sizeof *s);
+    s->fmt = ps_fmt(t);
+    s->W = (const uint8_t *)(s->fmt == PS_FMT_Q4K ? t->w : t->planar);
+    s->M = t->rows;
+    s->nb = t->cols / (s->fmt == PS_FMT_Q50_PLANAR ? 32 : 256);
+    s->cta0 = cta0;
+    s->ncta = ncta;
+    ckb_step_persistent_plan(s);
 }
 
-/* Deals the CTAs of the grid to the segments and launches.  In the latency regime (few work items) a segment gets about one
- * CTA per SM of its share of the machine, each with as few busy warps as that allows, and long rows are split over the warps
- * of a CTA so that every warp has one load round; in the streaming regime the resident slots are shared out by bytes. */
-static int plan_and_launch(StepGemvParams *p, void *st)
+/* The table of layers that the kernel walks, and its arguments: once, the weights' places never change.  Whatever the kernel does not take (and what the
+ * other step refuses: mixed input formats of q, k and v, a down projection over 32-element blocks) stays with the launch-per-operation step. */
+static int ps_build(KqModel *m, cudaStream_t st)
 {
-    /* matrices of a few megabytes: the launch is a chain of latencies, and the rehearsing instantiation pays */
-    double launch_bytes = 0;
-    for (int i = 0; i < p->nseg; ++i) launch_bytes += (double)p->seg[i].M * p->nb * (p->seg[i].fmt == SG_FMT_Q6K_PLANAR ? 210 : 144);
-    p->dry_run = ckb_tune_get("step_dry_run", 1) && launch_bytes <= (double)ckb_tune_get("step_dry_run_max_mb", 24) * 1048576.0;
-    int occ = ckb_step_gemv_ctas_per_sm(p->nb, p->pro, p->dry_run);
-    if (occ <= 0) return ckb_fail(CKB_ERR_LIMIT, "fused step: rows of %d superblocks do not fit the kernel's shared memory", p->nb);
-    const int occ_cap = ckb_tune_get("step_occ_cap", 0);
-    if (occ_cap > 0 && occ_cap < occ) occ = occ_cap;
-    const int sms = ckb_sm_count(), cap = sms * occ;
-    int g4 = 2;
-    while (g4 < 32 && g4 < 2 * p->nb) g4 <<= 1;
-    const int g6 = g4 * 2 > 32 ? 32 : g4 * 2;
-    long want[3], total_want = 0;
-    double bytes[3], total_bytes = 0;
-    for (int i = 0; i < p->nseg; ++i) {
-        bytes[i] = (double)p->seg[i].M * p->nb * (p->seg[i].fmt == SG_FMT_Q6K_PLANAR ? 210 : 144);
-        total_bytes += bytes[i];
-    }
-    for (int i = 0; i < p->nseg; ++i) {
-        StepSeg *sg = &p->seg[i];
-        const int q6 = sg->fmt == SG_FMT_Q6K_PLANAR;
-        const int rpw = (32 / (q6 ? g6 : g4)) * 2;
-        const long items = (sg->M + rpw - 1) / rpw;
-        const int passes = ckb_step_gemv_passes(p->nb, sg->fmt);
-        long share = (long)((double)sms * bytes[i] / total_bytes + 0.5);       /* SMs of this segment at one CTA per SM */
-        if (share < 1) share = 1;
-        sg->split = passes > 1 && passes <= 8 && items * passes <= (long)cap * 8 && ckb_tune_get("step_split", 1);
-        if (sg->split) {
-            const int ipc = 8 / passes;
-            want[i] = (items + ipc - 1) / ipc;                                   /* one round per CTA */
-        } else {
-            long wpc = (items + share - 1) / share;                              /* busy warps per CTA */
-            if (wpc > 8) wpc = 8;
-            want[i] = (items + wpc - 1) / wpc;
+    const int L = m->c.num_layers, sms = ckb_sm_count();
+    if (m->c.batch != 1 || m->c.tp_size != 1 || (m->d != 64 && m->d != 128) || m->Hl / m->Hkvl > PS_MAX_GROUP || m->Hkvl > sms / 2 || L < 1 || sms < 3 || m->Il % 256) return 0;
+    size_t stage = 0;
+    PsLayer *table = (PsLayer *)calloc((size_t)L, sizeof *table);
+    if (!table) return ckb_fail(CKB_ERR_STATE, "model step: out of memory");
+    for (int l = 0; l <= L; ++l) {
+        const Tensor *t = l < L ? m->layers[l].t : NULL;
+        const Tensor *w[PS_SEGS] = { &m->lm_head, NULL, NULL, NULL, NULL, NULL };
+        if (t) {
+            static const int which[PS_SEGS] = { CKB_T_WQ, CKB_T_WK, CKB_T_WV, CKB_T_WO, CKB_T_W1, CKB_T_W2 };
+            for (int i = 0; i < PS_SEGS; ++i) w[i] = &t[which[i]];
         }
-        total_want += want[i];
-    }
-    int grid = 0;
-    for (int i = 0; i < p->nseg; ++i) {
-        long n = want[i];
-        if (total_want > cap) {
-            n = (long)((double)cap * bytes[i] / total_bytes);
-            if (n < 1) n = 1;
-            if (n > want[i]) n = want[i];
+        int ok = 1;
+        for (int i = 0; i < PS_SEGS && w[i]; ++i) ok &= ps_fmt(w[i]) >= 0;
+        if (t && (fmt_block32(w[PS_K]->fmt) != fmt_block32(w[PS_Q]->fmt) || fmt_block32(w[PS_V]->fmt) != fmt_block32(w[PS_Q]->fmt) || fmt_block32(w[PS_W2]->fmt))) ok = 0;
+        if (!ok) { free(table); return 0; }
+        if (t) {
+            /* q, k and v share the grid by their bytes */
+            double bytes[3], all = 0;
+            for (int i = 0; i < 3; ++i) { bytes[i] = (double)w[i]->bytes; all += bytes[i]; }
+            int nk = (int)(sms * bytes[PS_K] / all + 0.5), nv = (int)(sms * bytes[PS_V] / all + 0.5);
+            if (nk < 1) nk = 1;
+            if (nv < 1) nv = 1;
+            if (nk + nv > sms - 1) nk = nv = sms / 3;
+            const int at[4] = { 0, sms - nk - nv, sms - nv, sms };
+            for (int i = 0; i < 3; ++i) ps_seg(&table[l].seg[i], w[i], at[i], at[i + 1] - at[i]);
+            for (int i = PS_O; i < PS_SEGS; ++i) ps_seg(&table[l].seg[i], w[i], 0, sms);
+            table[l].ln1 = (const float *)t[CKB_T_LN1].w;
+            table[l].ln2 = (const float *)t[CKB_T_LN2].w;
+            table[l].kc = kv_at(m, l, 0);
+            table[l].vc = kv_at(m, l, 1);
+        } else ps_seg(&m->ps.head, w[0], 0, sms);
+        for (int i = 0; i < PS_SEGS && w[i]; ++i) {
+            const PsSeg *s = t ? &table[l].seg[i] : &m->ps.head;
+            const size_t b = ckb_step_persistent_stage_bytes(s->fmt, s->nb);
+            if (b > stage) stage = b;
         }
-        p->seg[i].cta0 = grid;
-        p->seg[i].ncta = (int)n;
-        grid += (int)n;
     }
-    const int rc = ckb_launch_step_gemv(p, grid, st);
-    return rc == -1 ? ckb_fail(CKB_ERR_SHAPE, "fused step: shape not handled") : rc;
-}
-
-/* The quantised input of a fused launch: built inside the launch when the row is short (every CTA repeats the work, which is
- * cheaper than a launch), else by the stand-alone kernel into `xq_buf`.  kind: SG_PRO_NORM (x row `cur` += delta, in place
- * when stand-alone, else into `nxt`) or SG_PRO_QUANT (fp32 row `src`).  Returns 1 when the residual row moved to `nxt`. */
-static int fused_input(KqModel *m, StepGemvParams *p, int kind, float *cur, float *nxt, const float *delta, const float *gamma, const float *src,
-                       uint8_t *xq_buf, void *st, int *rc)
-{
-    *rc = 0;
-    if (kind == SG_PRO_NORM) {
-        if (p->nb <= SG_NORM_MAX_NB && p->nb <= ckb_tune_get("step_norm_max_nb", SG_NORM_MAX_NB)) {
-            p->pro = SG_PRO_NORM;
-            p->x_in = cur;
-            p->delta = delta;
-            p->gamma = gamma;
-            p->x_out = delta ? nxt : NULL;
-            return delta != NULL;
-        }
-        *rc = ckb200_dev_add_rmsnorm_q8k(cur, delta, gamma, xq_buf, NULL, 1, m->D, m->Da, m->c.rms_eps, st);
-    } else {
-        if (p->nb <= ckb_tune_get("step_quant_max_nb", 8)) {       /* one block per warp: beyond that the blocks of a warp queue up */
-            p->pro = SG_PRO_QUANT;
-            p->src = src;
-            return 0;
-        }
-        *rc = ckb200_dev_quantize_q8_k(src, xq_buf, 1, p->nb * 256, st);
-    }
-    p->pro = SG_PRO_GLOBAL;
-    p->xq = xq_buf;
+    PsParams *p = &m->ps;
+    p->smem = ckb_step_persistent_smem(m->Da, stage, m->d, m->kv_eb == 2);
+    if (!p->smem) { free(table); return 0; }
+    const int rc = ckb_check_cuda((int)cudaMalloc(&m->ps_table, (size_t)L * sizeof *table), "cudaMalloc(step table)") ||
+                   ckb_check_cuda((int)cudaMalloc((void **)&m->ps_part, ckb_step_persistent_scratch_bytes(m->d)), "cudaMalloc(step scratch)") ||
+                   ckb_check_cuda((int)cudaMalloc((void **)&m->ps_sync, ckb_step_persistent_sync_bytes()), "cudaMalloc(step counters)") ||
+                   ckb_check_cuda((int)cudaMemcpyAsync(m->ps_table, table, (size_t)L * sizeof *table, cudaMemcpyHostToDevice, st), "step table") ||
+                   ckb_check_cuda((int)cudaMemsetAsync(m->ps_sync, 0, ckb_step_persistent_sync_bytes(), st), "step counters");
+    free(table);                                      /* a copy out of pageable memory has been staged when the call returns */
+    if (rc) return CKB_ERR_CUDA;
+    p->layers = (const PsLayer *)m->ps_table;
+    p->num_layers = L;
+    p->final_gamma = (const float *)m->final_gamma.w;
+    p->x = m->x; p->q = m->q; p->att = m->att; p->o = m->o; p->mf = m->mf; p->prev = m->prev; p->logits = m->logits;
+    p->part = m->ps_part; p->sync = m->ps_sync;
+    p->cos_cache = m->rope_cos; p->sin_cache = m->rope_sin; p->pos = m->pos_dev;
+    p->D = m->D; p->Da = m->Da; p->H = m->Hl; p->Hkv = m->Hkvl; p->head_dim = m->d; p->max_seq = m->c.max_seq_len; p->kv_f16 = m->kv_eb == 2;
+    p->eps = m->c.rms_eps;
+    m->ps_ready = 1;
     return 0;
 }
 
-static int issue_step_fused(KqModel *m, void *st)
+static int issue_step_persistent(KqModel *m, void *st)
 {
-    const CKB200ModelConfig *c = &m->c;
-    const int L = c->num_layers;
-    int rc;
-    rc = ckb200_dev_embedding_rows(m->tokens_dev, 1, c->vocab_size, m->emb.w, m->emb.fmt, m->emb.cols, m->x, m->Da, m->D, st);
-    if (rc) return rc;
-    float *cur = m->x, *nxt = m->x2;
-    const float *delta = NULL;
-    StepGemvParams base;
-    memset(&base, 0, sizeof base);
-    base.cos_cache = m->rope_cos;
-    base.sin_cache = m->rope_sin;
-    base.pos = m->pos_dev;
-    base.head_dim = m->d;
-    base.max_seq = c->max_seq_len;
-    base.d_model = m->D;
-    base.eps = c->rms_eps;
-    for (int l = 0; l < L; ++l) {
-        Tensor *t = m->layers[l].t;
-        float *kc = (float *)kv_at(m, l, 0), *vc = (float *)kv_at(m, l, 1);
-        StepGemvParams p = base;
-        /* 1: q | k | v */
-        p.nseg = 3;
-        p.nb = m->Da / 256;
-        int moved = fused_input(m, &p, SG_PRO_NORM, cur, nxt, delta, (const float *)t[CKB_T_LN1].w, NULL, m->hq, st, &rc);
-        if (rc) return rc;
-        seg_set(&p.seg[0], &t[CKB_T_WQ], m->q, SG_EPI_ROPE_Q);
-        seg_set(&p.seg[1], &t[CKB_T_WK], kc, SG_EPI_ROPE_K);
-        seg_set(&p.seg[2], &t[CKB_T_WV], vc, SG_EPI_STORE_V);
-        if ((rc = plan_and_launch(&p, st))) return rc;
-        if (moved) { float *tmp = cur; cur = nxt; nxt = tmp; }
-        /* 2: attention, merge inside */
-        ckb_attn_hint_early_rows(ckb_tune_get("model_attn_early_rows", 1));
-        if ((rc = ckb200_dev_attention_decode_fused(m->q, kc, vc, m->att, m->Ala, 1, m->kv_batch_stride, m->Hl, m->Hkvl, 1, c->max_seq_len, m->d, m->d,
-                                                    m->attn_splits, m->attn_scratch, m->attn_counters, m->pos_dev, NULL, 0, st))) return rc;
-        ckb_attn_hint_early_rows(0);
-        /* 3: o projection */
-        p = base;
-        p.nseg = 1;
-        p.nb = m->Ala / 256;
-        fused_input(m, &p, SG_PRO_QUANT, NULL, NULL, NULL, NULL, m->att, m->aq, st, &rc);
-        if (rc) return rc;
-        seg_set(&p.seg[0], &t[CKB_T_WO], m->o, SG_EPI_STORE);
-        if ((rc = plan_and_launch(&p, st))) return rc;
-        /* 4: gate | up with SwiGLU */
-        p = base;
-        p.nseg = 1;
-        p.nb = m->Da / 256;
-        moved = fused_input(m, &p, SG_PRO_NORM, cur, nxt, m->o, (const float *)t[CKB_T_LN2].w, NULL, m->hq, st, &rc);
-        if (rc) return rc;
-        seg_set(&p.seg[0], &t[CKB_T_W1], m->mf, SG_EPI_SWIGLU);
-        if ((rc = plan_and_launch(&p, st))) return rc;
-        if (moved) { float *tmp = cur; cur = nxt; nxt = tmp; }
-        /* 5: down projection */
-        p = base;
-        p.nseg = 1;
-        p.nb = round256(m->Il) / 256;
-        fused_input(m, &p, SG_PRO_QUANT, NULL, NULL, NULL, NULL, m->mf, m->mq, st, &rc);
-        if (rc) return rc;
-        seg_set(&p.seg[0], &t[CKB_T_W2], m->prev, SG_EPI_STORE);
-        if ((rc = plan_and_launch(&p, st))) return rc;
-        delta = m->prev;
-    }
-    StepGemvParams p = base;
-    p.nseg = 1;
-    p.nb = m->Da / 256;
-    fused_input(m, &p, SG_PRO_NORM, cur, nxt, delta, (const float *)m->final_gamma.w, NULL, m->hq, st, &rc);
-    if (rc) return rc;
-    p.x_out = NULL;
-    p.pos_advance = m->pos_dev;
-    seg_set(&p.seg[0], &m->lm_head, m->logits, SG_EPI_STORE);
-    return plan_and_launch(&p, st);
+    const int rc = ckb200_dev_embedding_rows(m->tokens_dev, 1, m->c.vocab_size, m->emb.w, m->emb.fmt, m->emb.cols, m->x, m->Da, m->D, st);
+    return rc ? rc : ckb_launch_step_persistent(&m->ps, st);
 }
 
 static int issue_step(KqModel *m, void *st)
 {
-    if (fused_step_ok(m)) return issue_step_fused(m, st);
+    if (m->ps_ready && ckb_tune_get("model_fused_step", 1)) return issue_step_persistent(m, st);
     const CKB200ModelConfig *c = &m->c;
     const int B = c->batch, L = c->num_layers;
     int rc;

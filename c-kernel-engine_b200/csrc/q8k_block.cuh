@@ -1,7 +1,6 @@
 // One warp quantises one 256-element block to Q8_K; lane l holds elements 8l..8l+7 in v[].
 // Bit-exact with the reference's quantize_row_q8_k (src/kernels/gemm_kernels_q4k_q8k.c:53-103):
-// the SIGNED value of the first element with the largest |x| sets the scale (the reduction compares
-// (|x|, index) so the lowest index wins ties), iscale = -127/max and d = 1/iscale are IEEE divisions,
+// the SIGNED value of the first element with the largest |x| sets the scale (ties: the lowest index), iscale = -127/max and d = 1/iscale are IEEE divisions,
 // and iscale*x is rounded to fp32 before the round-to-nearest-even conversion.
 #pragma once
 
@@ -13,23 +12,17 @@ namespace ckb {
 struct Q8kLane { int q[8], s; float d; };
 __device__ __forceinline__ Q8kLane quantize_lane_q8k(const float (&v)[8], int lane)
 {
-    float best = 0.0f;
-    int best_i = 8 * lane;
+    float best = 0.0f, mine = 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float ax = fabsf(v[j]);
-        if (ax > best) { best = ax; best_i = 8 * lane + j; }
+        if (ax > best) { best = ax; mine = v[j]; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-        if (ob > best || (ob == best && oi < best_i)) { best = ob; best_i = oi; }
-    }
-    float cand = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) if ((best_i & 7) == j) cand = v[j];
-    const float vmax = __shfl_sync(0xffffffffu, cand, best_i >> 3);
+    // non-negative floats order like their bits: one warp reduction instead of five rounds of (value, index) shuffles, a chain of 250 cycles; the lowest
+    // lane that has the maximum holds its first occurrence
+    const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(best));
+    const float vmax = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, __float_as_uint(best) == top)) - 1);
+    best = __uint_as_float(top);
 
     Q8kLane r;
     r.s = 0;
