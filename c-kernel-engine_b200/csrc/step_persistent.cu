@@ -399,6 +399,18 @@ struct PsRows {
     __device__ __forceinline__ const uint8_t *second(const uint8_t *r0, int n) const { return n + 1 < M ? r0 + pair : r0; }
 };
 
+// both sums over G adjacent lanes, in the first of them: the halves of the group take one each after the first exchange
+template <int G>
+__device__ __forceinline__ void ps_pair_sum(float &a0, float &a1, int lane)
+{
+    const bool up = (lane & (G / 2)) != 0;
+    float v = (up ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up ? a0 : a1, G / 2);
+#pragma unroll
+    for (int w = G / 4; w > 0; w >>= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
+    a1 = __shfl_xor_sync(0xffffffffu, v, G / 2);
+    a0 = v;
+}
+
 // G lanes per row, T::LPS of them per block.  SPLIT = false: a warp walks the passes of its rows, the next ones on their way.
 // SPLIT = true: the passes of a row pair go to different warps and meet in shared memory in a fixed order (one round of loads: the latency form).
 template <class T, int G, bool SPLIT, int HD, typename KVT>
@@ -423,12 +435,11 @@ __device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target)
 
     auto finish = [&](int it, float a0, float a1) {
         const int n0 = it * RPW + sub * PS_R;
-        const float s0 = group_sum<G>(a0), s1 = group_sum<G>(a1);
-        if (li == 0 && n0 < M) ps_epilogue<HD, KVT>(epi, w.out, M, n0, s0, s1);
+        ps_pair_sum<G>(a0, a1, lane);
+        if (li == 0 && n0 < M) ps_epilogue<HD, KVT>(epi, w.out, M, n0, a0, a1);
     };
     auto meet = [&](float a0, float a1) {                       // SPLIT: the passes of a pair
-        a0 = group_sum<G>(a0);
-        a1 = group_sum<G>(a1);
+        ps_pair_sum<G>(a0, a1, lane);
         if (li == 0) { sh.part[warp][2 * sub] = a0; sh.part[warp][2 * sub + 1] = a1; }
         __syncthreads();
         if (item < nitems && pass == 0 && li == 0) {
@@ -531,6 +542,12 @@ __device__ __forceinline__ void ps_widen(const uint4 &r, float (&v)[8])
         v[2 * i + 1] = f.y;
     }
 }
+__device__ __forceinline__ float ps_warp_max(float v)
+{
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, w));
+    return v;
+}
 template <int HD, typename KVT> struct PsRow;                  // a lane's HD / 32 elements of a value row
 template <> struct PsRow<128, float> { float4 r; __device__ void ld(const float *q) { r = __ldcg(reinterpret_cast<const float4 *>(q)); }
     __device__ void get(float (&v)[4]) const { v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w; } };
@@ -584,7 +601,7 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
     if (!ps_wait(target)) return false;
     PS_TRACE(target / gridDim.x, 2);
     if (!mine) return true;                                                  // uniform in the CTA
-    float *qs = reinterpret_cast<float *>(ps_stage()), *om = qs + PS_MAX_GROUP * HD, *ms = om + PS_NW / 2 * PS_MAX_GROUP * HD, *ls = ms + PS_NW * PS_MAX_GROUP;
+    float *qs = reinterpret_cast<float *>(ps_stage()), *om = qs + PS_MAX_GROUP * HD, *ms = om + PS_NW * PS_MAX_GROUP * HD, *ls = ms + PS_NW * PS_MAX_GROUP;
     const float scale = __fmul_rn(rsqrtf((float)HD), 1.4426950408889634f);
     for (int i = threadIdx.x; i < PS_MAX_GROUP * HD; i += PS_THREADS) qs[i] = i < group * HD ? __ldcg(p.q + (size_t)g * group * HD + i) * scale : 0.0f;
     if (!early && base < k1) { load_k(base); load_v(base); }
@@ -672,48 +689,27 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
         ms[lane * PS_NW + warp] = m;
         ls[lane * PS_NW + warp] = l;
     }
-    __syncthreads();
-    // warps of the CTA -> its run's result; the weights of the warps first, a warp per head
-    if (warp < group && lane < PS_NW) {
-        const float mk = ms[warp * PS_NW + lane];
-        float top = mk;
 #pragma unroll
-        for (int w = 8; w > 0; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffu, top, w));
-        const float f = mk == -INFINITY ? 0.0f : exp2f(mk - top);
-        float sum = f * ls[warp * PS_NW + lane];
+    for (int h = 0; h < PS_MAX_GROUP; ++h)
+        if (h < group) {
 #pragma unroll
-        for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffu, sum, w);
-        sh.part[warp][lane] = f;
-        if (lane == 0) { sh.part[warp][16] = top; sh.part[warp][17] = sum; }
-    }
-    __syncthreads();
-    // weighted outputs of the upper eight warps, those of the lower eight on top
-#pragma unroll
-    for (int half = 1; half >= 0; --half) {
-        if (warp / (PS_NW / 2) == half) {
-#pragma unroll
-            for (int h = 0; h < PS_MAX_GROUP; ++h)
-                if (h < group) {
-                    const float f = sh.part[h][warp];
-#pragma unroll
-                    for (int e = 0; e < E; ++e) {
-                        float *at = om + (warp % (PS_NW / 2) * PS_MAX_GROUP + h) * HD + lane * E + e;
-                        *at = half ? f * o[h][e] : fmaf(f, o[h][e], *at);
-                    }
-                }
+            for (int e = 0; e < E; ++e) om[(warp * PS_MAX_GROUP + h) * HD + lane * E + e] = o[h][e];
         }
-        __syncthreads();
-    }
+    __syncthreads();
+    // warps of the CTA -> its run's result.  A warp's 32 outputs are of one head: it weighs the partial results for itself, without another barrier.
     float *part = p.part + ((size_t)s * Hkv + g) * PS_MAX_GROUP * (HD + 2);          // [heads][HD], then [heads] of (maximum, sum)
+#pragma unroll 1
     for (int i = threadIdx.x; i < group * HD; i += PS_THREADS) {
         const int h = i / HD, e = i % HD;
+        const float mk = lane < PS_NW ? ms[h * PS_NW + lane] : -INFINITY, top = ps_warp_max(mk);
+        const float f = mk == -INFINITY ? 0.0f : exp2f(mk - top), sum = group_sum<32>(lane < PS_NW ? f * ls[h * PS_NW + lane] : 0.0f);
         float a = 0.0f;
 #pragma unroll
-        for (int k = 0; k < PS_NW / 2; ++k) a += om[(k * PS_MAX_GROUP + h) * HD + e];
-        if (used == 1) p.att[(size_t)g * group * HD + i] = __fdiv_rn(a, sh.part[h][17]);
+        for (int k = 0; k < PS_NW; ++k) a = fmaf(__shfl_sync(0xffffffffu, f, k), om[(k * PS_MAX_GROUP + h) * HD + e], a);
+        if (used == 1) p.att[(size_t)g * group * HD + i] = __fdiv_rn(a, sum);
         else {
             part[i] = a;
-            if (e == 0) *reinterpret_cast<float2 *>(part + PS_MAX_GROUP * HD + 2 * h) = make_float2(sh.part[h][16], sh.part[h][17]);
+            if (e == 0) *reinterpret_cast<float2 *>(part + PS_MAX_GROUP * HD + 2 * h) = make_float2(top, sum);
         }
     }
     if (used == 1) return true;
@@ -726,46 +722,30 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
     __syncthreads();
     PS_TRACE(target / gridDim.x, 7);
     if (!sh.last) return true;
-    // the last CTA of the kv head: a batch of runs at a time, their values on the way to registers while a warp per head makes their weights
+    // the last CTA of the kv head: a batch of runs at a time, their values on the way while the warp makes their weights, a lane per run
     const size_t stride = (size_t)Hkv * PS_MAX_GROUP * (HD + 2);
     const float *all = p.part + (size_t)g * PS_MAX_GROUP * (HD + 2);
-    constexpr int PER = (PS_MAX_GROUP * HD + PS_THREADS - 1) / PS_THREADS;
-    float acc[PER] = {}, top = -INFINITY, sum = 0.0f;          // top, sum: of head `warp`, in its warp
 #pragma unroll 1
-    for (int j = 0; j < used; j += PS_MERGE) {
-        const int n = min(PS_MERGE, used - j);
-        if (warp < group) {
-            const float2 ml = lane < n ? __ldcg(reinterpret_cast<const float2 *>(all + (size_t)(j + lane) * stride + PS_MAX_GROUP * HD + 2 * warp)) : make_float2(-INFINITY, 0.0f);
-            float now = ml.x;
-#pragma unroll
-            for (int w = 16; w > 0; w >>= 1) now = fmaxf(now, __shfl_xor_sync(0xffffffffu, now, w));
-            now = fmaxf(now, top);
-            const float f = top == now ? 1.0f : exp2f(top - now), e = lane < n ? exp2f(ml.x - now) : 0.0f;
-            sum = fmaf(sum, f, group_sum<32>(e * ml.y));
-            top = now;
-            sh.part[warp][lane] = e;
-            if (lane == 0) { ms[warp] = f; ls[warp] = sum; }
-        }
-#pragma unroll
-        for (int c = 0; c < PER; ++c) {
-            const int i = threadIdx.x + c * PS_THREADS, h = i / HD;
+    for (int i = threadIdx.x; i < group * HD; i += PS_THREADS) {
+        const int h = i / HD;
+        float a = 0.0f, top = -INFINITY, sum = 0.0f;
+#pragma unroll 1
+        for (int j = 0; j < used; j += PS_MERGE) {
+            const int n = min(PS_MERGE, used - j);
+            const float *at = all + (size_t)j * stride;
+            const float2 ml = lane < n ? __ldcg(reinterpret_cast<const float2 *>(at + lane * stride + PS_MAX_GROUP * HD + 2 * h)) : make_float2(-INFINITY, 0.0f);
             float v[PS_MERGE];
 #pragma unroll
-            for (int k = 0; k < PS_MERGE; ++k) v[k] = k < n && i < group * HD ? __ldcg(all + (size_t)(j + k) * stride + i) : 0.0f;
-            if (c == 0) __syncthreads();
-            if (i < group * HD) {
-                float a = acc[c] * ms[h];
+            for (int k = 0; k < PS_MERGE; ++k) v[k] = k < n ? __ldcg(at + k * stride + i) : 0.0f;
+            const float now = fmaxf(top, ps_warp_max(ml.x));
+            const float f = top == now ? 1.0f : exp2f(top - now), e = lane < n ? exp2f(ml.x - now) : 0.0f;
+            sum = fmaf(sum, f, group_sum<32>(e * ml.y));
+            a *= f;
 #pragma unroll
-                for (int k = 0; k < PS_MERGE; ++k) a = fmaf(sh.part[h][k], v[k], a);
-                acc[c] = a;
-            }
+            for (int k = 0; k < PS_MERGE; ++k) a = fmaf(__shfl_sync(0xffffffffu, e, k), v[k], a);
+            top = now;
         }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int c = 0; c < PER; ++c) {
-        const int i = threadIdx.x + c * PS_THREADS;
-        if (i < group * HD) p.att[(size_t)g * group * HD + i] = __fdiv_rn(acc[c], ls[i / HD]);
+        p.att[(size_t)g * group * HD + i] = __fdiv_rn(a, sum);
     }
     return true;
 }
@@ -888,7 +868,7 @@ extern "C" size_t ckb_step_persistent_stage_bytes(int fmt, int nb)
 
 extern "C" size_t ckb_step_persistent_smem(int Da, size_t stage, int head_dim, int kv_f16)
 {
-    const size_t attn = (size_t)(PS_MAX_GROUP * head_dim + PS_NW * PS_MAX_GROUP * (head_dim / 2 + 2)) * sizeof(float);
+    const size_t attn = (size_t)(PS_MAX_GROUP * head_dim + PS_NW * PS_MAX_GROUP * (head_dim + 2)) * sizeof(float);
     const size_t smem = (size_t)Da * 4 + (stage > attn ? stage : attn);
     int dev = 0, coop = 0;
     if (smem > PS_MAX_SMEM || ckb_sm_count() > PS_MAX_CTAS || cudaGetDevice(&dev) != cudaSuccess ||
