@@ -174,7 +174,7 @@ using namespace ckb;
 
 // q, out [H][T][ad]; k, v [Hkv][kv_stride_tokens][ad]; causal != 0: token i sees keys 0 .. i, else all T keys.
 extern "C" int ckb_launch_attn_prefill_mma(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim,
-                                           int aligned_head_dim, int kv_stride_tokens, int before, int causal, void *stream);
+                                           int aligned_head_dim, int kv_stride_tokens, int causal, void *stream);
 extern "C" int ckb200_dev_attention_prefill_window(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads,
                                                    int num_tokens, int head_dim, int aligned_head_dim, int kv_stride_tokens, int causal,
                                                    int sliding_window, void *stream)
@@ -191,7 +191,7 @@ extern "C" int ckb200_dev_attention_prefill_window(const float *q, const float *
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) return ckb_fail(CKB_ERR_ALIGN, "attention prefill: pointers must be 16-byte aligned");
     if (window == 0) {
         // without a sliding window: the tensor-core kernel of attention_prefill_mma.cu (-1: not for this call)
-        const int rc = ckb_launch_attn_prefill_mma(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, aligned_head_dim, kv_stride_tokens, 0, causal, stream);
+        const int rc = ckb_launch_attn_prefill_mma(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, aligned_head_dim, kv_stride_tokens, causal, stream);
         if (rc >= 0) return rc;
     }
     // 2 * BT * G threads per key set (a multiple of 32); two key sets when both fit 256 threads

@@ -86,14 +86,13 @@ __device__ __forceinline__ void pm_cp16(uint32_t dst, const void *src, uint32_t 
 __device__ __forceinline__ void pm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void pm_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// q, out: [H][T][AD]; kv16 as written by pm_split_kv_kernel for S keys; causal: query i sees keys 0 .. S - T + i (a later portion of a sequence has
-// S - T keys before its own).  grid (kv heads, query blocks), block = 32 * KH * (H / Hkv) threads:
+// q, out: [H][T][AD]; kv16 as written by pm_split_kv_kernel.  grid (kv heads, query blocks), block = 32 * KH * (H / Hkv) threads:
 // warp = key part * G + query head of the kv head.  With KH = 2 (up to four query heads per kv head) two warps share a head and
 // take 32 keys of each 64-key tile each, with their own running maximum; they are merged at the end.  The tiles of the next step
 // are copied (cp.async, rows padded to PITCH) while this step multiplies.
 template <int AD, int KH>
 __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__restrict__ q, const __half *__restrict__ kv16, float *__restrict__ out, int H, int Hkv,
-                                                               int T, int S, int hd, int causal, float scale)
+                                                               int T, int hd, int causal, float scale)
 {
     constexpr int KS = AD / 16, NTD = AD / 8, PITCH = (AD + 8) * 2;    // bytes per row of an fp16 tile
     constexpr int TILE = PM_BK * PITCH, STAGE = 4 * TILE;              // K hi, K lo, V hi, V lo
@@ -106,9 +105,9 @@ __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__re
     // block of every head, so the short blocks fill the gaps at the end (with the heads outermost the last heads' long blocks
     // started when most SMs were already idle: 40 % of the SM time was idle)
     const int qb = gridDim.y - 1 - blockIdx.y, q0 = qb * PM_BQ;
-    const int before = S - T, key_end = causal ? min(S, before + q0 + PM_BQ) : S;      // keys [0, key_end) matter to this block
+    const int key_end = causal ? min(T, q0 + PM_BQ) : T;                // keys [0, key_end) matter to this block
     const int ntiles = (key_end + PM_BK - 1) / PM_BK;
-    const size_t arr = (size_t)Hkv * S * AD;
+    const size_t arr = (size_t)Hkv * T * AD;
     pdl_trigger();
     pdl_wait();
 
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__re
         for (int c = tid; c < 4 * PM_BK * (AD / 8); c += nthreads) {
             const int a = c / (PM_BK * (AD / 8)), rem = c - a * (PM_BK * (AD / 8)), row = rem / (AD / 8), ch = rem - row * (AD / 8);
             const int key = key0 + row;
-            const __half *src = kv16 + (size_t)a * arr + ((size_t)kvh * S + min(key, S - 1)) * AD + ch * 8;
+            const __half *src = kv16 + (size_t)a * arr + ((size_t)kvh * T + min(key, T - 1)) * AD + ch * 8;
             pm_cp16(st + (uint32_t)(a * TILE + row * PITCH + ch * 16), src, key < key_end ? 16u : 0u);
         }
     };
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__re
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int key = key0 + koff + 8 * n + 2 * t + (e & 1), qrow = q0 + g + ((e & 2) ? 8 : 0);
-                    const bool valid = n < nt_lim && key < S && (!causal || key <= before + qrow);
+                    const bool valid = n < nt_lim && key < T && (!causal || key <= qrow);
                     s[n][e] = valid ? s[n][e] * (1.0f / PM_QSCALE) : -INFINITY;
                     mt[e >> 1] = fmaxf(mt[e >> 1], s[n][e]);
                 }
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__re
 }
 
 template <int AD, int KH>
-static int pm_launch(const float *q, const float *k, const float *v, float *out, int H, int Hkv, int T, int S, int hd, int kv_stride, int causal, float scale, cudaStream_t st)
+static int pm_launch(const float *q, const float *k, const float *v, float *out, int H, int Hkv, int T, int hd, int kv_stride, int causal, float scale, cudaStream_t st)
 {
     constexpr int smem = 2 * 4 * PM_BK * (AD + 8) * 2;
     static_assert(8 * (AD / 8 * 4 + 4) * 32 * 4 <= smem, "the merge buffer of up to 8 heads fits into the stages");
@@ -305,31 +304,31 @@ static int pm_launch(const float *q, const float *k, const float *v, float *out,
         if (ckb_check_cuda((int)cudaFuncSetAttribute(attn_prefill_mma_kernel<AD, KH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "attn_prefill_mma smem")) return CKB_ERR_CUDA;
         attr_set = true;
     }
-    const size_t arr = (size_t)Hkv * S * AD;
+    const size_t arr = (size_t)Hkv * T * AD;
     __half *kv16 = (__half *)ckb_scratch(CKB_SLOT_S, 4 * arr * sizeof(__half));
     if (!kv16) return CKB_ERR_CUDA;
     const size_t n4 = arr / 4;
     const unsigned blocks = (unsigned)((n4 + 255) / 256 < 8 * 148 ? (n4 + 255) / 256 : 8 * 148);
-    if (int rc = launch_pdl("attn_prefill_split_kv", pm_split_kv_kernel<AD>, dim3(blocks), dim3(256), 0, st, k, v, kv16, Hkv, S, hd, kv_stride)) return rc;
+    if (int rc = launch_pdl("attn_prefill_split_kv", pm_split_kv_kernel<AD>, dim3(blocks), dim3(256), 0, st, k, v, kv16, Hkv, T, hd, kv_stride)) return rc;
     return launch_pdl("attn_prefill_mma", attn_prefill_mma_kernel<AD, KH>, dim3(Hkv, (T + PM_BQ - 1) / PM_BQ), dim3(32 * KH * (H / Hkv)), (size_t)smem, st, q,
-                      (const __half *)kv16, out, H, Hkv, T, S, hd, causal, scale);
+                      (const __half *)kv16, out, H, Hkv, T, hd, causal, scale);
 }
 
 }  // namespace ckb
 
 using namespace ckb;
 
-// Arguments as ckb200_dev_attention_prefill (no sliding window), and `before` keys of earlier portions in front of the num_tokens own ones.  Returns -1 when this kernel does not take the call.
+// Arguments as ckb200_dev_attention_prefill (no sliding window).  Returns -1 when this kernel does not take the call.
 extern "C" int ckb_launch_attn_prefill_mma(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim,
-                                           int aligned_head_dim, int kv_stride_tokens, int before, int causal, void *stream)
+                                           int aligned_head_dim, int kv_stride_tokens, int causal, void *stream)
 {
     if (!ckb_tune_get("attn_prefill_mma", 1) || num_heads % num_kv_heads || num_heads / num_kv_heads > 8) return -1;
     if ((aligned_head_dim != 64 && aligned_head_dim != 128) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)) return -1;
     const float scale = 1.0f / sqrtf((float)head_dim);
     cudaStream_t st = ckb_stream(stream);
     if (num_heads / num_kv_heads <= 4)                     // two warps per query head, 32 keys of a tile each
-        return aligned_head_dim == 64 ? pm_launch<64, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, before + num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
-                                      : pm_launch<128, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, before + num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
-    return aligned_head_dim == 64 ? pm_launch<64, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, before + num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
-                                  : pm_launch<128, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, before + num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
+        return aligned_head_dim == 64 ? pm_launch<64, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
+                                      : pm_launch<128, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
+    return aligned_head_dim == 64 ? pm_launch<64, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
+                                  : pm_launch<128, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
 }

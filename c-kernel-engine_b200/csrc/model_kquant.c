@@ -70,7 +70,7 @@ typedef struct {
     Tensor t[CKB_T_PER_LAYER];
 } Layer;
 
-enum { PF_X, PF_DELTA, PF_O, PF_Q, PF_K, PF_V, PF_QH, PF_OH, PF_GU, PF_ROWS, PF_PART0, PF_PART1, PF_PART2, PF_IDS, PF_BUFFERS };
+enum { PF_X, PF_DELTA, PF_O, PF_Q, PF_K, PF_V, PF_QH, PF_OH, PF_GU, PF_ROWS, PF_PART0, PF_PART1, PF_PART2, PF_ATTN, PF_IDS, PF_BUFFERS };
 
 typedef struct {
     struct CKB200Model;     /* shared fields (model_internal.h) */
@@ -101,9 +101,10 @@ typedef struct {
     int ps_ready;
     int *attn_counters;     /* arrival counters of the attention kernel's in-launch split merge */
     /* batched prefill, grown on demand to the longest prompt seen: token-major rows, head-major attention tensors, quantised rows (Q8_K blocks, operand tiles of the
-     * tensor-core product, or row-planar Q8_0), partial sums of the three products that run side by side, prompt ids */
+     * tensor-core product, or row-planar Q8_0), partial sums of the three products that run side by side, parts of attention, prompt ids */
     float *pf_x, *pf_delta, *pf_o, *pf_q, *pf_k, *pf_v, *pf_qh, *pf_oh, *pf_gu;
     uint8_t *pf_rows, *pf_part[3];
+    float *pf_attn;
     int32_t *pf_ids;
     uint8_t *pf_arena;      /* all of them */
     size_t pf_cap[PF_BUFFERS];
@@ -771,7 +772,7 @@ static int issue_step(KqModel *m, void *st)
  * How a product is done depends on the format and on T:
  *   K-quants, T <= 64   Q8_K rows, integer-MMA kernels (48 x 4096 x 4096: 12 us; the tcgen05 kernel with 32-token tiles 17)
  *   K-quants, T > 64    the producer of the rows quantises them straight into operand tiles, tcgen05 kernel
- *   Q5_0, Q8_0          row-planar Q8_0 rows, gemm_q80_mma.cu
+ *   Q5_0                row-planar Q8_0 rows, gemm_q80_mma.cu
  * q, k and v run on three streams: one of them alone leaves SMs idle (512 x 1024 x 4096 is 32 tiles) or ends in a part of a wave. */
 
 int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens, void *stream);
@@ -786,8 +787,9 @@ int ckb_prefill_gather_tiles(const float *out_hm, void *tiles, int tile_nt, int 
 int ckb_prefill_gather_q80_planar(const float *out_hm, void *planar, int tokens, int num_heads, int head_dim, int cols, void *stream);
 int ckb_launch_gemm_q80_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream);   /* gemm_q80_mma.cu */
 int ckb_launch_gemm_q50_mma(const void *A_planar, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream);
-int ckb_launch_attn_prefill_mma(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, int aligned_head_dim,
-                                int kv_stride_tokens, int before, int causal, void *stream);                          /* attention_prefill_mma.cu */
+size_t ckb_attn_behind_part_bytes(int head_dim);                                                                      /* attention_behind.cu */
+int ckb_launch_attn_behind(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, int kv_stride_tokens,
+                                   int before, float *part, void *stream);
 
 #define PF_SMALL 64            /* most tokens of the integer-MMA kernels */
 
@@ -815,7 +817,6 @@ static int prefill_takes(const Tensor *w)
 static int prefill_ok(const KqModel *m, int T)
 {
     if (m->c.batch != 1 || m->c.tp_size != 1 || m->kv_eb != 4 || T < 16 || m->host_pos + T > m->c.max_seq_len || !ckb_tune_get("model_prefill", 1)) return 0;
-    if (m->host_pos && !ckb_tune_get("attn_prefill_mma", 1)) return 0;        /* the only prompt kernel that sees keys before its own */
     for (int l = 0; l < m->c.num_layers; ++l) {
         const Tensor *t = m->layers[l].t;
         static const int which[6] = { CKB_T_WQ, CKB_T_WK, CKB_T_WV, CKB_T_WO, CKB_T_W1, CKB_T_W2 };
@@ -833,6 +834,7 @@ static int prefill_buffers(KqModel *m, int T)
     const size_t t = (size_t)T, kvw = (size_t)m->Hkvl * m->d, widest = (size_t)(m->Da > m->Ala ? m->Da : m->Ala) > (size_t)m->Il ? (size_t)(m->Da > m->Ala ? m->Da : m->Ala) : (size_t)m->Il;
     size_t need[PF_BUFFERS] = { t * m->Da * 4, t * m->Da * 4, t * m->Da * 4, t * m->Al * 4, t * kvw * 4, t * kvw * 4, t * m->Al * 4, t * m->Al * 4, t * 2 * m->Il * 4 };
     need[PF_ROWS] = (t + 127) * (widest / 256) * 548;          /* operand tiles of any width up to 128: 548 bytes per token and superblock, more than the other forms */
+    need[PF_ATTN] = ckb_attn_behind_part_bytes(m->d);
     need[PF_IDS] = t * sizeof(int32_t);
     WidthMemo memo[CKB_T_PER_LAYER] = { { 0 } };
     if (T > PF_SMALL)
@@ -862,7 +864,7 @@ static int prefill_buffers(KqModel *m, int T)
     memset(m->pf_cap, 0, sizeof m->pf_cap);
     if (ckb_check_cuda((int)cudaMalloc((void **)&m->pf_arena, total), "cudaMalloc(prefill)")) return CKB_ERR_CUDA;
     void **ptrs[PF_BUFFERS] = { (void **)&m->pf_x, (void **)&m->pf_delta, (void **)&m->pf_o, (void **)&m->pf_q, (void **)&m->pf_k, (void **)&m->pf_v, (void **)&m->pf_qh,
-                                (void **)&m->pf_oh, (void **)&m->pf_gu, (void **)&m->pf_rows, (void **)&m->pf_part[0], (void **)&m->pf_part[1], (void **)&m->pf_part[2], (void **)&m->pf_ids };
+                                (void **)&m->pf_oh, (void **)&m->pf_gu, (void **)&m->pf_rows, (void **)&m->pf_part[0], (void **)&m->pf_part[1], (void **)&m->pf_part[2], (void **)&m->pf_attn, (void **)&m->pf_ids };
     size_t at = 0;
     for (int i = 0; i < PF_BUFFERS; ++i) {
         *ptrs[i] = m->pf_arena + at;
@@ -920,10 +922,20 @@ static int prefill_qkv(KqModel *m, const Tensor *t, int nt, int T, void *st)
     return 0;
 }
 
+/* Passes that stand in for decode steps (behind a filled cache, over Q5_0 projections) keep the steps' fp32 attention with its range and accuracy; a prompt of
+ * K-quants from an empty cache goes through the fp16 pieces of attention_prefill_mma.cu, as the reference's prefill calls do. */
+static int prefill_attention_fp32(const KqModel *m)
+{
+    int any = m->host_pos > 0;
+    for (int l = 0; l < m->c.num_layers && !any; ++l)
+        for (int i = 0; i < CKB_T_PER_LAYER; ++i) any |= m->layers[l].t[i].fmt == FMT_Q50;
+    return any;
+}
+
 static int issue_prefill(KqModel *m, int T, void *st)
 {
     const CKB200ModelConfig *c = &m->c;
-    const int L = c->num_layers, before = m->host_pos;
+    const int L = c->num_layers, before = m->host_pos, fp32 = prefill_attention_fp32(m);
     int rc;
     rc = ckb200_dev_embedding_rows(m->pf_ids, T, c->vocab_size, m->emb.w, m->emb.fmt, m->emb.cols, m->pf_x, m->Da, m->D, st);
     if (rc) return rc;
@@ -937,10 +949,8 @@ static int issue_prefill(KqModel *m, int T, void *st)
         if ((rc = prefill_norm(m, delta, &t[CKB_T_LN1], &t[CKB_T_WQ], nt_q, T, st))) return rc;
         if ((rc = prefill_qkv(m, t, nt_q, T, st))) return rc;
         if ((rc = ckb200_dev_prefill_rope_scatter(m->pf_q, m->pf_k, m->pf_v, m->pf_qh, kc, vc, m->rope_cos, m->rope_sin, T, m->Hl, m->Hkvl, m->d, c->max_seq_len, before, st))) return rc;
-        if (before) {
-            rc = ckb_launch_attn_prefill_mma(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, before, 1, st);
-            if (rc == -1) rc = ckb_fail(CKB_ERR_SHAPE, "prefill: attention over earlier keys not handled");
-        } else rc = ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st);
+        rc = fp32 ? ckb_launch_attn_behind(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, c->max_seq_len, before, m->pf_attn, st)
+                  : ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st);
         if (rc) return rc;
         if (fmt_block32(t[CKB_T_WO].fmt)) rc = ckb_prefill_gather_q80_planar(m->pf_oh, m->pf_rows, T, m->Hl, m->d, t[CKB_T_WO].cols, st);
         else if (nt_o) rc = ckb_prefill_gather_tiles(m->pf_oh, m->pf_rows, nt_o, T, m->Hl, m->d, m->Ala, st);

@@ -92,3 +92,50 @@ def test_q5_0_product_is_bit_identical(ck, orc, tile, m, n, k):
     got = c.cpu().numpy()
     assert np.array_equal(got[:, :n], want)
     assert np.isnan(got[:, n:]).all()
+
+
+@pytest.mark.parametrize("heads,kvh,d", [(4, 1, 128), (7, 1, 64), (8, 1, 128), (3, 3, 64), (10, 2, 128)])
+@pytest.mark.parametrize("before,T", [(0, 16), (1, 17), (63, 64), (64, 1), (1000, 16), (3000, 130), (129, 400)])
+@pytest.mark.parametrize("spread", ["ordinary", "small values", "huge values", "large queries"])
+def test_attention_behind_earlier_keys(ck, heads, kvh, d, before, T, spread):
+    """Attention of a portion against softmax in 64 bits, with scores of spread 1 so that every run of keys carries weight.  In fp32 a score is two chains of 16 products
+    per 32 dimensions, an output chains of 16 keys: some twenty roundings of 2^-24 at each that add like a random walk (four or five of them), the weight's own two
+    and those of the sum and the division: ten roundings of the output's norm.  Sixteen-bit pieces of fp32 numbers miss that, and fp16's range: values of 0.003 as well
+    as keys, values and queries beyond 65504."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(before + T)
+    S = before + T + 3
+    q, k, v = (torch.randn(n, d, device=dev, generator=g) for n in (heads * T, kvh * S, kvh * S))
+    q, k, v = q.view(heads, T, d), k.view(kvh, S, d), v.view(kvh, S, d)
+    if spread == "small values":
+        v *= 0.003
+    elif spread == "huge values":
+        v *= 1.0e6
+        k *= 1.0e5
+        q *= 1.0e-5
+    elif spread == "large queries":
+        q *= 1.0e4
+        k *= 1.0e-4
+    k[:, before + T:] = float("nan")                    # rows past the portion are nobody's
+    v[:, before + T:] = float("nan")
+    out = torch.full((heads, T, d), float("nan"), device=dev)
+    ck.ckb_attn_behind_part_bytes.restype = C.c_size_t
+    part = torch.empty(ck.ckb_attn_behind_part_bytes(d) // 4, device=dev)
+    torch.cuda.synchronize()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    assert ck.ckb_launch_attn_behind(p(q), p(k), p(v), p(out), heads, kvh, T, d, S, before, p(part), None) == 0, ck.ckb200_last_error_message()
+    assert ck.ckb200_synchronize() == 0
+    kk, vv = (t[:, :before + T].double().repeat_interleave(heads // kvh, 0) for t in (k, v))
+    s = q.double() @ kk.transpose(1, 2) / d ** 0.5
+    s = s.masked_fill(torch.arange(before + T, device=dev)[None, :] > torch.arange(before, before + T, device=dev)[:, None], -float("inf"))
+    want = torch.softmax(s, -1) @ vv
+    assert float((out.double() - want).norm() / want.norm()) <= 10 * 2.0 ** -24
+    # a value that a query may not see does not reach it, whatever it is
+    if T > 1:
+        v[:, before + T - 1] = float("inf")
+        torch.cuda.synchronize()
+        assert ck.ckb_launch_attn_behind(p(q), p(k), p(v), p(out), heads, kvh, T, d, S, before, p(part), None) == 0
+        assert ck.ckb200_synchronize() == 0
+        assert torch.isfinite(out[:, :T - 1]).all()
