@@ -828,7 +828,8 @@ static int prefill_ok(const KqModel *m, int T)
     return m->Il % 256 == 0 && m->d % 8 == 0 && (m->d == 64 || m->d == 128) && group <= 8 && m->Hl % m->Hkvl == 0;
 }
 
-/* Buffers of a prompt of T tokens.  Layers agree on nothing but their shapes, so the partial sums are sized over all of them. */
+/* Buffers of a prompt of T tokens.  Layers agree on nothing but their shapes, so the partial sums are sized over all of them.  -1: no room for them (on the device,
+ * or within tune model_prefill_max_mb), the prompt runs as decode steps, which need none. */
 static int prefill_buffers(KqModel *m, int T)
 {
     const size_t t = (size_t)T, kvw = (size_t)m->Hkvl * m->d, widest = (size_t)(m->Da > m->Ala ? m->Da : m->Ala) > (size_t)m->Il ? (size_t)(m->Da > m->Ala ? m->Da : m->Ala) : (size_t)m->Il;
@@ -856,13 +857,20 @@ static int prefill_buffers(KqModel *m, int T)
         else grow = 1;
         total += align_up(need[i] + 256, 256);
     }
+    const int max_mb = ckb_tune_get("model_prefill_max_mb", 0);
+    if (max_mb > 0 && total > (size_t)max_mb << 20) return -1;
     if (!grow) return 0;
     /* one allocation for all of them: each costs tens of microseconds, which a first prompt pays */
     cudaStreamSynchronize(ckb_stream(NULL));
     if (m->pf_arena) cudaFree(m->pf_arena);
     m->pf_arena = NULL;
     memset(m->pf_cap, 0, sizeof m->pf_cap);
-    if (ckb_check_cuda((int)cudaMalloc((void **)&m->pf_arena, total), "cudaMalloc(prefill)")) return CKB_ERR_CUDA;
+    const cudaError_t e = cudaMalloc((void **)&m->pf_arena, total);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        m->pf_arena = NULL;
+        return e == cudaErrorMemoryAllocation ? -1 : ckb_check_cuda((int)e, "cudaMalloc(prefill)");
+    }
     void **ptrs[PF_BUFFERS] = { (void **)&m->pf_x, (void **)&m->pf_delta, (void **)&m->pf_o, (void **)&m->pf_q, (void **)&m->pf_k, (void **)&m->pf_v, (void **)&m->pf_qh,
                                 (void **)&m->pf_oh, (void **)&m->pf_gu, (void **)&m->pf_rows, (void **)&m->pf_part[0], (void **)&m->pf_part[1], (void **)&m->pf_part[2], (void **)&m->pf_attn, (void **)&m->pf_ids };
     size_t at = 0;
@@ -976,9 +984,10 @@ static int kq_extend(CKB200Model *model, const int32_t *tokens, int count, const
     KqModel *m = (KqModel *)model;
     if (n_want > 1 || (n_want == 1 && want[0] != count - 1) || !prefill_ok(m, count)) return -1;
     cudaStream_t st = ckb_stream(NULL);
-    if (prefill_buffers(m, count)) return CKB_ERR_CUDA;
+    int rc = prefill_buffers(m, count);
+    if (rc) return rc;
     const int32_t end = m->host_pos + count;
-    int rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pf_ids, tokens, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, st), "prompt ids H2D");
+    rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pf_ids, tokens, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, st), "prompt ids H2D");
     if (!rc) rc = issue_prefill(m, count, st);
     if (!rc) rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pos_dev, &end, sizeof end, cudaMemcpyHostToDevice, st), "prefill pos");
     if (!rc && n_want) rc = ckb_check_cuda((int)cudaMemcpyAsync(logits_host, m->logits, (size_t)m->Vl * sizeof(float), cudaMemcpyDeviceToHost, st), "logits D2H");

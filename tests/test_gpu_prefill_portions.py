@@ -139,3 +139,34 @@ def test_attention_behind_earlier_keys(ck, heads, kvh, d, before, T, spread):
         assert ck.ckb_launch_attn_behind(p(q), p(k), p(v), p(out), heads, kvh, T, d, S, before, p(part), None) == 0
         assert ck.ckb200_synchronize() == 0
         assert torch.isfinite(out[:, :T - 1]).all()
+
+
+@pytest.mark.parametrize("before", [0, 40])
+def test_prompt_without_room_for_its_buffers_runs_as_steps(ck, before):
+    """A batched pass takes device memory that decode steps do without: where there is none, the prompt goes through as steps, with their results."""
+    so.bind_model_api(ck)
+    ids = np.random.default_rng(5).integers(0, QWEN["vocab_size"], size=before + 100).astype(np.int32)
+    ck.ckb200_launch_count.restype = C.c_longlong
+    results, launches = [], []
+    for max_mb, batched in ((1, 1), (0, 0), (64, 1)):
+        handle = ck.ckb200_model_create(C.byref(so.make_cfg(QWEN, batch=1)))
+        assert handle, ck.ckb200_last_error_message()
+        try:
+            assert ck.ckb200_model_fill_synthetic(handle, 9) == 0
+            ck.ckb200_tune_set(b"model_prefill", 0)
+            if before:
+                assert ck.ckb200_model_prefill(handle, cases.vptr(ids), before, None) == 0
+            ck.ckb200_tune_set(b"model_prefill", batched)
+            ck.ckb200_tune_set(b"model_prefill_max_mb", max_mb)
+            n0 = ck.ckb200_launch_count()
+            logits = np.full((1, QWEN["vocab_size"]), np.nan, np.float32)
+            assert ck.ckb200_model_prefill(handle, cases.vptr(ids[before:]), 100, cases.vptr(logits)) == 0, ck.ckb200_last_error_message()
+            launches.append(ck.ckb200_launch_count() - n0)
+            assert ck.ckb200_model_get_pos(handle) == before + 100
+            results.append(logits)
+        finally:
+            ck.ckb200_tune_set(b"model_prefill", 1)
+            ck.ckb200_tune_set(b"model_prefill_max_mb", 0)
+            ck.ckb200_model_free(handle)
+    assert launches[0] == launches[1] and launches[2] != launches[1], launches
+    assert np.array_equal(results[0], results[1])
