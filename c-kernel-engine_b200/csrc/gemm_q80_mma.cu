@@ -38,8 +38,9 @@ __host__ __device__ inline size_t qm_row5_bytes(int nb) { return ((size_t)nb * Q
 // four elements of a Q5_0 block as signed bytes: nib - 16 * (fifth bit clear); fifth: their four bits, lowest first
 __device__ __forceinline__ uint32_t q5_bytes(uint32_t nib, uint32_t fifth) { return nib | ((((~fifth & 15u) * 0x00204081u) & 0x01010101u) * 0xF0u); }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory"); }
+// rows past the end are filled with zeros, not fetched: copies of the last row in their place all went to one L2 slice (65 tokens x 4864 x 896: 44 us, with zeros 23)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory"); }
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src, bool in) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8 : 0) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -73,12 +74,12 @@ __global__ void __launch_bounds__(QM_THREADS) gemm_q80_mma_kernel(const uint8_t 
 #pragma unroll
         for (int i = 0; i < TILE * PIECES / QM_THREADS; ++i) {
             const int idx = tid + i * QM_THREADS, row = idx / PIECES, piece = idx % PIECES;
-            cp_async16(st + L::OFF_B + (uint32_t)(row * (Q5 ? QM_ROW5 : QM_ROW) + piece * 16), B + (size_t)min(n0 + row, N - 1) * rb + (size_t)kb * (Q5 ? 16 : 32) + piece * 16);
+            cp_async16(st + L::OFF_B + (uint32_t)(row * (Q5 ? QM_ROW5 : QM_ROW) + piece * 16), B + (size_t)min(n0 + row, N - 1) * rb + (size_t)kb * (Q5 ? 16 : 32) + piece * 16, n0 + row < N);
         }
         if (tid < TILE) {
             const uint8_t *src = B + (size_t)min(n0 + tid, N - 1) * rb;
-            if (Q5) cp_async16(st + L::OFF_FIFTH + (uint32_t)(tid * 16), src + (size_t)nb * 16 + (size_t)kb * 4);
-            cp_async8(st + L::OFF_DB + (uint32_t)(tid * 8), src + (size_t)nb * (Q5 ? 20 : 32) + (size_t)kb * 2);
+            if (Q5) cp_async16(st + L::OFF_FIFTH + (uint32_t)(tid * 16), src + (size_t)nb * 16 + (size_t)kb * 4, n0 + tid < N);
+            cp_async8(st + L::OFF_DB + (uint32_t)(tid * 8), src + (size_t)nb * (Q5 ? 20 : 32) + (size_t)kb * 2, n0 + tid < N);
         }
     };
     auto issue_a = [&](int chunk) {
@@ -87,11 +88,11 @@ __global__ void __launch_bounds__(QM_THREADS) gemm_q80_mma_kernel(const uint8_t 
 #pragma unroll
         for (int i = 0; i < TILE * 8 / QM_THREADS; ++i) {
             const int idx = tid + i * QM_THREADS, row = idx >> 3, piece = idx & 7;
-            cp_async16(st + (uint32_t)(row * QM_ROW + piece * 16), A + (size_t)min(m0 + row, M - 1) * ra + (size_t)kb * 32 + piece * 16);
+            cp_async16(st + (uint32_t)(row * QM_ROW + piece * 16), A + (size_t)min(m0 + row, M - 1) * ra + (size_t)kb * 32 + piece * 16, m0 + row < M);
         }
         if (tid >= QM_THREADS - TILE) {
             const int row = tid - (QM_THREADS - TILE);
-            cp_async8(st + L::OFF_DA + (uint32_t)(row * 8), A + (size_t)min(m0 + row, M - 1) * ra + (size_t)nb * 32 + (size_t)kb * 2);
+            cp_async8(st + L::OFF_DA + (uint32_t)(row * 8), A + (size_t)min(m0 + row, M - 1) * ra + (size_t)nb * 32 + (size_t)kb * 2, m0 + row < M);
         }
     };
 
