@@ -988,7 +988,11 @@ static int kq_extend(CKB200Model *model, const int32_t *tokens, int count, const
     if (rc) return rc;
     const int32_t end = m->host_pos + count;
     rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pf_ids, tokens, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, st), "prompt ids H2D");
-    if (!rc) rc = issue_prefill(m, count, st);
+    if (!rc && (rc = issue_prefill(m, count, st)) != 0) {
+        /* a launch that failed between fork and join leaves work on the side streams that nothing waits for: it reads the pass's buffers, which the next call may free */
+        for (int i = 0; i < 2; ++i) cudaStreamSynchronize(m->side[i]);
+        cudaStreamSynchronize(st);
+    }
     if (!rc) rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pos_dev, &end, sizeof end, cudaMemcpyHostToDevice, st), "prefill pos");
     if (!rc && n_want) rc = ckb_check_cuda((int)cudaMemcpyAsync(logits_host, m->logits, (size_t)m->Vl * sizeof(float), cudaMemcpyDeviceToHost, st), "logits D2H");
     if (!rc) rc = ckb_sync_check(st, "model_prefill");
