@@ -77,7 +77,7 @@ long long ckb200_launch_count(void) { return g.launches; }
 
 /* ------------------------------------------------------------------ tuning switches */
 
-#define CKB_MAX_TUNE 32
+#define CKB_MAX_TUNE 128
 static struct { char key[32]; int value; } g_tune[CKB_MAX_TUNE];
 static int g_ntune;
 
