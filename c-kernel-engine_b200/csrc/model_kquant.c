@@ -594,7 +594,7 @@ static int ensure_planar(KqModel *m, void *st)
 
 /* ------------------------------------------------------------------ the one-launch step (one sequence, one GPU)
  *
- * step_persistent.cu: all layers and the LM head in one cooperative launch behind the embedding. */
+ * step_persistent.cu: all layers and the LM head in one launch behind the embedding. */
 
 static int ps_fmt(const Tensor *t)
 {
@@ -674,6 +674,7 @@ static int ps_build(KqModel *m, cudaStream_t st)
     p->part = m->ps_part; p->sync = m->ps_sync;
     p->cos_cache = m->rope_cos; p->sin_cache = m->rope_sin; p->pos = m->pos_dev;
     p->D = m->D; p->Da = m->Da; p->H = m->Hl; p->Hkv = m->Hkvl; p->head_dim = m->d; p->max_seq = m->c.max_seq_len; p->kv_f16 = m->kv_eb == 2;
+    p->ctas = sms;
     p->eps = m->c.rms_eps;
     m->ps_ready = 1;
     return 0;

@@ -1,7 +1,7 @@
 // The unit of the Q4_K x Q8_K "pair" GEMV (gemv_q4k.cu) and what it needs from shared memory: two lanes per
 // superblock, lane p takes the nibble bytes of quarters p and p+2, i.e. sub-blocks 2p, 2p+1 (6-bit scales stored
-// directly) and 2p+4, 2p+5 (scales split over two bytes).  Kept in a header because the fused step kernels and the
-// integer-stage dump (subblock_sums.cu) run the very same functions.
+// directly) and 2p+4, 2p+5 (scales split over two bytes).  Kept in a header because the integer-stage dump (subblock_sums.cu) runs the
+// same functions, and the one-launch step (step_units.cuh) the same layouts.
 // Reference arithmetic: dot_q4_k_q8_k_ref, src/kernels/gemm_kernels_q4k_q8k.c:121-181.
 #pragma once
 
@@ -20,9 +20,6 @@ __host__ __device__ inline int q4p_smem_bytes(int nb) { return ((nb * (Q4P_SLOTS
 
 struct Q4pX { uint32_t q, d, lo, hi; };
 
-// LOCAL_SRC: the Q8_K vector was just built by this CTA in shared memory (a fused quantising prologue) and is read with plain
-// loads; otherwise it is global memory written by an earlier kernel and comes through L2.
-template <bool LOCAL_SRC = false>
 __device__ __forceinline__ Q4pX q4p_stage_x(const uint8_t *xg, int nb, uint8_t *smem)
 {
     uint32_t *xq = reinterpret_cast<uint32_t *>(smem);
@@ -38,8 +35,7 @@ __device__ __forceinline__ Q4pX q4p_stage_x(const uint8_t *xg, int nb, uint8_t *
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int i = base + u * blockDim.x + threadIdx.x;
-            if constexpr (LOCAL_SRC) v[u] = i < total ? src[i] : 0u;
-            else v[u] = i < total ? __ldcg(src + i) : 0u;  // through L2: the producer may overlap this kernel (programmatic launch)
+            v[u] = i < total ? __ldcg(src + i) : 0u;  // through L2: the producer may overlap this kernel (programmatic launch)
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {

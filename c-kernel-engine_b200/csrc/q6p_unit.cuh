@@ -1,6 +1,6 @@
 // The unit of the planar Q6_K x Q8_K GEMV (gemv_q6k_planar.cu): one quarter (n, h) of one superblock of one row, fetched with
-// aligned loads from the row-planar layout, multiplied in the exact-integer bit-plane form.  In a header because the fused
-// step kernels (step_persistent.cu) run the same functions.  Reference arithmetic: src/kernels/gemm_kernels_q6k_q8k.c:86-116.
+// aligned loads from the row-planar layout, multiplied in the exact-integer bit-plane form.  In a header because the one-launch
+// step (step_units.cuh) uses the same loads and plane sums.  Reference arithmetic: src/kernels/gemm_kernels_q6k_q8k.c:86-116.
 #pragma once
 
 #include "ring_x.cuh"

@@ -1,11 +1,10 @@
-// One decode step of one sequence as ONE cooperative launch: all layers and the LM head.
+// One decode step of one sequence as ONE launch: all layers and the LM head.
 //
 // The reference's generated decode function issues, per layer, residual add, RMSNorm, quantisation, q / k / v projections, RoPE, cache store, attention,
 // ... one call after another (version/v7/scripts/codegen_v7.py:569-931).  As a launch each, thirteen to a layer, the step was the chain of their latencies:
 // a token of the Qwen2-0.5B shape (1024 keys) reads 0.4 GB, 60 us at HBM speed, and took 829 us; of the Llama-3-8B shape (4096 keys) 6 GB, 0.9 ms, and took 2.28 ms.
-// In this form 603 us and 1.74 ms; Qwen2-0.5B with Q5_0 projections 1020 -> 639 us (2000 keys).  What is left is five barriers a layer (1 us each: release, poll) and the
-// pieces that wait for one another behind them; products run at 24 B a cycle and SM, which is both the integer-issue rate and the SM's share of HBM.  Here one CTA
-// per SM stays for the whole step and a layer is five phases with a grid-wide barrier behind each:
+//
+// Here one CTA per SM stays for the whole step and a layer is five phases with a grid-wide barrier behind each:
 //
 //   0  x += down, RMSNorm, quantise | q, k, v products | RoPE, query row and cache rows written
 //   1  attention: a CTA takes a run of keys of one kv head; the last CTA of a kv head to finish merges the runs
@@ -17,13 +16,22 @@
 // of a barrier and of a prologue is that weights do not depend on them: the first rows of the coming product are loaded into registers ahead of them.
 // The arithmetic of each piece is that of the stand-alone kernels (the same integer sums and rounding calls); sums over warps and keys are taken in another order.
 //
-// Every wait is bounded: a CTA that gives up sets the error word and leaves, the others follow; the last to leave zeroes the counters.
+// The two shapes above take 615 us and 1.79 ms in this form (603 and 1.74 as a cooperative launch that needs every SM), Qwen2-0.5B with Q5_0 projections 1020 -> 640 us (2000 keys).  What is left is five barriers a layer (1 us each: release, poll) and
+// the pieces that wait for one another behind them; products run at 24 B a cycle and SM, which is both the integer-issue rate and the SM's share of HBM.
+//
+// Barriers need every CTA that takes part to be on an SM, and the step does not ask for the whole GPU: CTAs enrol as they start, and those that have done so when all
+// are there, or a short while after the first, do the step between them (the deal of rows and keys is made for p.ctas CTAs, and a CTA takes several shares where there are
+// fewer: the same results, bit for bit).  One that comes later leaves at once.  So the step runs beside a kernel that holds SMs, and in a context that has fewer of
+// them.
+//
+// Every wait is bounded: a CTA that gives up sets the error word and leaves, the others follow; the last to leave zeroes the counters and, as every step does
+// whatever came of it, moves the position on.
 #include "add_rmsnorm_q8k.cuh"
 #include "launch.h"
-#include "q4p_unit.cuh"
-#include "q6p_unit.cuh"
+#include "pdl.cuh"
 #include "runtime.h"
 #include "step_persistent.h"
+#include "step_units.cuh"
 
 namespace ckb {
 
@@ -32,179 +40,20 @@ constexpr int PS_R = 2;                       // rows per lane group: the pair t
 constexpr int PS_KEYS = 4;                    // keys a warp scores at a time: 4 keys x 8 heads = one score per lane
 constexpr int PS_MIN_RUN = 32, PS_MERGE = 32; // attention: fewest keys of a CTA, runs of keys merged at a time
 constexpr int PS_MAX_CTAS = 256, PS_MAX_HALF = 64;
+constexpr int PS_JOIN_CYCLES = 40000;          // how long the first CTA waits for the others: they all start within 2 us on SMs that are free
+constexpr uint32_t PS_CLOSED = 0x80000000u;
+enum { PS_ARRIVALS = 0, PS_LEFT, PS_JOINED, PS_MEMBERS, PS_HEADS };      // words of p.sync; PS_HEADS + g: runs of keys of kv head g that are done
 constexpr int PS_MAX_SMEM = 219 * 1024;       // dynamic; the rest of the 227 KB holds PsShared
 enum { PS_EPI_ROPE_Q, PS_EPI_ROPE_K, PS_EPI_STORE_V, PS_EPI_SWIGLU, PS_EPI_STORE };
 
 #ifdef CKB_STEP_TRACE
 // Tuning aid (build with -DCKB_STEP_TRACE): cycle counts at the boundaries of every phase of every CTA; ckb200_step_trace copies them out.
 constexpr int PS_TRACE_PHASES = 512;
-static __device__ long long ps_trace[148 * PS_TRACE_PHASES * 8];
+static __device__ long long ps_trace[PS_MAX_CTAS * PS_TRACE_PHASES * 8];
 #define PS_TRACE(k, i) do { if (threadIdx.x == 0 && (k) < PS_TRACE_PHASES) ps_trace[((size_t)blockIdx.x * PS_TRACE_PHASES + (k)) * 8 + (i)] = clock64(); } while (0)
 #else
 #define PS_TRACE(k, i) do { } while (0)
 #endif
-
-// ---------------------------------------------------------------- weight formats: loading, multiplying a pair of rows, staging 256 elements of the input row
-
-__device__ __forceinline__ uint2 ps_pack8(const int (&q)[8])
-{
-    return make_uint2((q[0] & 255) | ((q[1] & 255) << 8) | ((q[2] & 255) << 16) | ((uint32_t)(q[3] & 255) << 24),
-                      (q[4] & 255) | ((q[5] & 255) << 8) | ((q[6] & 255) << 16) | ((uint32_t)(q[7] & 255) << 24));
-}
-
-// `pair`: both rows of a lane's pair against its part of a block, the activations read once, with plain loads that the compiler may place early.
-struct PsQ4 {                                 // two lanes per superblock
-    using W = Q4pW;
-    static constexpr int LPS = 2;
-    static constexpr bool DEEP = false;       // the next rows in registers of their own while a pair is multiplied (else in the same ones, behind it)
-    static __host__ __device__ __forceinline__ size_t row_bytes(int nb) { return (size_t)nb * Q4K_BYTES; }
-    static __device__ __forceinline__ void load(W &w, const uint8_t *row, int, int b, int u)
-    {
-        const uint8_t *pb = row + b * Q4K_BYTES;
-        w.hdr = __ldg(reinterpret_cast<const uint4 *>(pb));
-        w.a0 = __ldg(reinterpret_cast<const uint4 *>(pb + 16 + 32 * u));
-        w.a1 = __ldg(reinterpret_cast<const uint4 *>(pb + 32 + 32 * u));
-        w.b0 = __ldg(reinterpret_cast<const uint4 *>(pb + 80 + 32 * u));
-        w.b1 = __ldg(reinterpret_cast<const uint4 *>(pb + 96 + 32 * u));
-    }
-    static __device__ __forceinline__ void pair(const Q4pW &w0, const Q4pW &w1, const uint8_t *s, int nb, int b, int p, float &a0, float &a1)
-    {
-        const Q4pW *w[2] = {&w0, &w1};
-        int lo[2][2] = {}, hi[2][2] = {};
-        const uint8_t *xs = s + (b * Q4P_SLOTS + 4 * p) * 16, *d = s + nb * Q4P_SLOTS * 16, *sums = d + nb * 4 + 4 * (2 * b + p);
-        const uint32_t blo = *reinterpret_cast<const uint32_t *>(sums), bhi = *reinterpret_cast<const uint32_t *>(sums + nb * 8);
-        const float xd = *reinterpret_cast<const float *>(d + 4 * b);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const uint4 *x = reinterpret_cast<const uint4 *>(xs + 128 * q);
-            const uint4 l0 = x[0], l1 = x[1], h0 = x[2], h1 = x[3];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const uint4 c0 = q ? w[r]->b0 : w[r]->a0, c1 = q ? w[r]->b1 : w[r]->a1;
-                const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w},
-                               h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    lo[r][q] = dp4a_us(c[i] & 0x0F0F0F0Fu, l[i], lo[r][q]);
-                    hi[r][q] = dp4a_us(c[i] & 0xF0F0F0F0u, h[i], hi[r][q]);      // 16 x the high-nibble sum
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const uint4 hdr = w[r]->hdr;
-            const int t = 16 * p;
-            const uint32_t a = hdr.y >> t, bb = hdr.z >> t, c = hdr.w >> t;
-            const uint32_t scA = a & 0x3F3Fu, mA = bb & 0x3F3Fu, scB = (c & 0x0F0Fu) | ((a >> 2) & 0x3030u), mB = ((c >> 4) & 0x0F0Fu) | ((bb >> 2) & 0x3030u);
-            const int isum = (int)(scA & 255u) * lo[r][0] + (int)(scB & 255u) * lo[r][1] + (((int)(scA >> 8) * hi[r][0] + (int)(scB >> 8) * hi[r][1]) >> 4);
-            const uint32_t m4 = mA | (mB << 16);
-            const int imin = dp4a_us(m4, blo, 0) + 128 * dp4a_us(m4, bhi, 0);
-            const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
-            (r ? a1 : a0) += (dd.x * xd) * (float)isum - (dd.y * xd) * (float)imin;
-        }
-    }
-    // elements 256 b + 8 lane .. + 7, as q4p_stage_x lays them out
-    static __device__ __forceinline__ void put(const float (&v)[8], int b, int nb, int lane, uint8_t *s)
-    {
-        const Q8kLane r = quantize_lane_q8k(v, lane);
-        *reinterpret_cast<uint2 *>(s + (size_t)b * Q4P_SLOTS * 16 + 8 * lane) = ps_pack8(r.q);
-        int sum = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        uint8_t *d = s + (size_t)nb * Q4P_SLOTS * 16, *lo = d + nb * 4, *hi = lo + nb * 8;
-        if ((lane & 3) == 0) {
-            const int j = lane >> 2, at = (b * 2 + ((j >> 1) & 1)) * 4 + ((j & 1) | ((j >> 2) << 1));
-            lo[at] = (uint8_t)(sum & 127);
-            hi[at] = (uint8_t)(sum >> 7);
-        }
-        if (lane == 0) reinterpret_cast<float *>(d)[b] = r.d;
-    }
-};
-
-struct PsQ6 {                                 // four lanes per superblock
-    using W = Q6pW;
-    static constexpr int LPS = 4;
-    static constexpr bool DEEP = true;
-    static __host__ __device__ __forceinline__ size_t row_bytes(int nb) { return q6p_row_bytes(nb); }
-    static __device__ __forceinline__ void load(W &w, const uint8_t *row, int nb, int b, int u) { q6p_load(w, row, nb, b, u >> 1, u & 1); }
-    static __device__ __forceinline__ void pair(const W &w0, const W &w1, const uint8_t *s, int nb, int b, int u, float &a0, float &a1)
-    {
-        const uint8_t *d = s + nb * 320, *sums = d + nb * 4 + 4 * (b * 4 + u);
-        const uint4 *x = reinterpret_cast<const uint4 *>(s + b * 320 + (10 * (u >> 1) + (u & 1)) * 16);
-        const uint4 x0 = x[0], x1 = x[2], x2 = x[4], x3 = x[6];
-        const uint32_t lo4 = *reinterpret_cast<const uint32_t *>(sums), hi4 = *reinterpret_cast<const uint32_t *>(sums + nb * 16);
-        const float xd = *reinterpret_cast<const float *>(d + 4 * b);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const W &w = r ? w1 : w0;
-            int S1, S2, S3, S4;
-            q6k_plane_sums(w.qa, w.qb, w.qh, x0, x1, x2, x3, S1, S2, S3, S4);
-            const uint32_t sc4 = (u & 1) ? __byte_perm(w.sc.x, w.sc.y, 0x7531) : __byte_perm(w.sc.x, w.sc.y, 0x6420);      // scales of groups 8 n + h + {0, 2, 4, 6}
-            const int s0 = (int)(int8_t)(sc4 & 255u), s1 = (int)(int8_t)((sc4 >> 8) & 255u), s2 = (int)(int8_t)((sc4 >> 16) & 255u), s3 = (int)sc4 >> 24;
-            const int center = dp4a_ss(sc4, lo4, 0) + 128 * dp4a_ss(sc4, hi4, 0);
-            const int tot = s0 * S1 + s1 * S2 + s2 * S3 + s3 * S4 - 32 * center;
-            (r ? a1 : a0) += (half_bits_to_float(w.d) * xd) * (float)tot;
-        }
-    }
-    // as ring_stage_x lays them out
-    static __device__ __forceinline__ void put(const float (&v)[8], int b, int nb, int lane, uint8_t *s)
-    {
-        const Q8kLane r = quantize_lane_q8k(v, lane);
-        const int c = lane >> 1;
-        *reinterpret_cast<uint2 *>(s + (size_t)b * 320 + (c + 2 * (c >> 3)) * 16 + 8 * (lane & 1)) = ps_pack8(r.q);
-        const int sum = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
-        uint8_t *d = s + (size_t)nb * 320, *lo = d + nb * 4, *hi = lo + nb * 16;
-        if ((lane & 1) == 0) {
-            const int j = c >> 1, at = (b * 4 + (j >> 2) * 2 + (c & 1)) * 4 + (j & 3);
-            lo[at] = (uint8_t)(sum & 127);
-            hi[at] = (uint8_t)(sum >> 7);
-        }
-        if (lane == 0) reinterpret_cast<float *>(d)[b] = r.d;
-    }
-};
-
-struct PsQ5 {                                 // one lane per 32-element block; the input row in Q8_0
-    struct W { uint4 qs; uint32_t qh, d; };
-    static constexpr int LPS = 1;
-    static constexpr bool DEEP = true;
-    static __host__ __device__ __forceinline__ size_t row_bytes(int nb) { return ((size_t)nb * Q50_BYTES + 15) & ~(size_t)15; }
-    static __device__ __forceinline__ void load(W &w, const uint8_t *row, int nb, int b, int)
-    {
-        w.qs = __ldg(reinterpret_cast<const uint4 *>(row + (size_t)b * 16));
-        w.qh = __ldg(reinterpret_cast<const uint32_t *>(row + (size_t)nb * 16 + (size_t)b * 4));
-        w.d = ldg_nc_u16(row + (size_t)nb * 20 + (size_t)b * 2);
-    }
-    static __device__ __forceinline__ void pair(const W &w0, const W &w1, const uint8_t *s, int, int b, int, float &a0, float &a1)
-    {
-        a0 += q50_unit_presum(w0.d, w0.qh, w0.qs, smem_u32(s) + 48u * b);
-        a1 += q50_unit_presum(w1.d, w1.qh, w1.qs, smem_u32(s) + 48u * b);
-    }
-    // blocks 8 b .. 8 b + 7: four lanes each, 48-byte slots of quants, scale (rounded to fp16) and sum of the quants
-    static __device__ __forceinline__ void put(const float (&v)[8], int b, int nb, int lane, uint8_t *s)
-    {
-        float amax = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-        int q[8], sum = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            q[j] = __float2int_rn(__fmul_rn(v[j], id));
-            sum += (int)(int8_t)(q[j] & 255);
-        }
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const int blk = 8 * b + (lane >> 2);
-        if (blk >= nb) return;
-        uint8_t *slot = s + (size_t)blk * 48;
-        *reinterpret_cast<uint2 *>(slot + 8 * (lane & 3)) = ps_pack8(q);
-        if ((lane & 3) == 0) {
-            *reinterpret_cast<float *>(slot + 32) = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
-            *reinterpret_cast<int *>(slot + 36) = sum;
-        }
-    }
-};
 
 // ---------------------------------------------------------------- the CTA's state
 
@@ -218,7 +67,8 @@ struct PsShared {
     int *dev_err;
     float inv_d;
     int pos, dead, last;
-    int g, s, run, used;              // attention: this CTA's kv head and run of keys, keys of a run, runs of the context
+    int run, used;                    // attention: keys of a run, runs of the context
+    int rank, members;                // this CTA among those that do the step (-1: it came too late)
 };
 static_assert(sizeof(PsLayer) % 16 == 0, "copied by 16 bytes");
 __shared__ PsShared sh;
@@ -229,14 +79,14 @@ __device__ __forceinline__ uint8_t *ps_stage() { return ps_smem + (size_t)sh.p.D
 __device__ __forceinline__ void ps_arrive()
 {
     __syncthreads();                  // every thread's stores come before the release below
-    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sh.p.sync) : "memory");
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sh.p.sync + PS_ARRIVALS) : "memory");
 }
 // `target`: arrivals of all phases so far
 __device__ __forceinline__ bool ps_wait(uint32_t target)
 {
     asm volatile("cp.async.wait_all;" ::: "memory");      // next layer's entry
     if (threadIdx.x == 0) {
-        const unsigned *at = sh.p.sync;
+        const unsigned *at = sh.p.sync + PS_ARRIVALS;
         const long long t0 = clock64(), limit = sh.limit;
         for (;;) {
             uint32_t v;
@@ -251,6 +101,38 @@ __device__ __forceinline__ bool ps_wait(uint32_t target)
     }
     __syncthreads();
     return sh.dead == 0;
+}
+
+// One thread per CTA: its place among the CTAs that do this step, and how many those are.  Tickets are handed out until all are taken or the first CTA's patience
+// ends; whoever closes the list publishes its length.
+__device__ __forceinline__ void ps_enrol(unsigned *sync, int expected, long long limit, int *dev_err, int &rank, int &members)
+{
+    const uint32_t ticket = atomicAdd(sync + PS_JOINED, 1u);
+    rank = -1;
+    members = 0;
+    if (ticket >= (uint32_t)expected) return;                        // closed, or more CTAs than shares
+    const long long t0 = clock64();
+    uint32_t n = ticket + 1 == (uint32_t)expected ? (uint32_t)expected : 0;
+    if (n) {
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(sync + PS_MEMBERS), "r"(n) : "memory");
+    } else {
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(sync + PS_MEMBERS) : "memory");
+            if (n) break;
+            const long long waited = clock64() - t0;
+            if (ticket == 0 && waited > PS_JOIN_CYCLES) {
+                n = min(atomicOr(sync + PS_JOINED, PS_CLOSED), (uint32_t)expected);
+                asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(sync + PS_MEMBERS), "r"(n) : "memory");
+                break;
+            }
+            if (waited > PS_JOIN_CYCLES + limit) {
+                atomicExch(dev_err, DEV_ERR_FULL_WAIT);
+                return;
+            }
+        }
+    }
+    rank = n == (uint32_t)expected ? (int)blockIdx.x : (int)ticket;      // each its own share, where all are there
+    members = (int)n;
 }
 
 __device__ __forceinline__ void ps_copy16(void *dst, const void *src)
@@ -416,7 +298,7 @@ __device__ __forceinline__ void ps_pair_sum(float &a0, float &a1, int lane)
 // G lanes per row, T::LPS of them per block.  SPLIT = false: a warp walks the passes of its rows, the next ones on their way.
 // SPLIT = true: the passes of a row pair go to different warps and meet in shared memory in a fixed order (one round of loads: the latency form).
 template <class T, int G, bool SPLIT, int HD, typename KVT>
-__device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target)
+__device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target, int share, bool first)
 {
     constexpr int SPP = G / T::LPS, SUB = 32 / G, RPW = SUB * PS_R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -425,7 +307,7 @@ __device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target)
     const int nb = sg.nb, M = sg.M, epi = w.epi, ncta = sg.ncta, nitems = sg.items, npass = sg.passes;
     const PsRows<HD> rows(sg, epi);
     const int slot = SPLIT ? warp / npass : warp;               // items side by side in a CTA
-    int item = SPLIT && slot >= PS_NW / npass ? nitems : (int)blockIdx.x - sg.cta0 + ncta * slot, pass = SPLIT ? warp - slot * npass : 0;
+    int item = SPLIT && slot >= PS_NW / npass ? nitems : share - sg.cta0 + ncta * slot, pass = SPLIT ? warp - slot * npass : 0;
     const uint8_t *x = ps_stage();
 
     PsGamma gm = {};
@@ -460,11 +342,13 @@ __device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target)
         T::load(w0, r0, nb, b, u);
         T::load(w1, r1, nb, b, u);
     }
-    PS_TRACE(target / gridDim.x, 1);
-    if (!ps_wait(target)) return false;
-    PS_TRACE(target / gridDim.x, 2);
+    PS_TRACE(target / sh.members, 1);
+    if (first) {
+        if (!ps_wait(target)) return false;
+    } else __syncthreads();                                     // the share before this one has been multiplied
+    PS_TRACE(target / sh.members, 2);
     ps_input<T>(w, gm);
-    PS_TRACE(target / gridDim.x, 3);
+    PS_TRACE(target / sh.members, 3);
     if constexpr (SPLIT) {                                      // one round (ckb_step_persistent_plan)
         const int b = b0 + pass * SPP;
         if (item < nitems && b < nb) T::pair(w0, w1, x, nb, b, u, a0, a1);
@@ -508,11 +392,11 @@ __device__ __forceinline__ bool ps_run(const PsWork &w, uint32_t target)
 }
 
 template <int HD, typename KVT>
-__device__ __forceinline__ bool ps_product(const PsWork &w, uint32_t target)
+__device__ __forceinline__ bool ps_product(const PsWork &w, uint32_t target, int share, bool first)
 {
     const PsSeg &s = *w.seg;
     const int sel = s.fmt * 8 + (s.lanes >> 4) * 2 + s.split;             // lanes 8, 16, 32 -> 0, 1, 2
-#define PS_CASE(T, F, G, S) case (F) * 8 + ((G) >> 4) * 2 + (S): return ps_run<T, G, S, HD, KVT>(w, target);
+#define PS_CASE(T, F, G, S) case (F) * 8 + ((G) >> 4) * 2 + (S): return ps_run<T, G, S, HD, KVT>(w, target, share, first);
     switch (sel) {
         PS_CASE(PsQ4, PS_FMT_Q4K, 8, false)
         PS_CASE(PsQ4, PS_FMT_Q4K, 16, false)
@@ -576,13 +460,13 @@ __device__ __forceinline__ int ps_run_keys(int T, int per)
 // with the score of key kk and head h and takes its exponential; the probabilities go through shared memory to the lanes that hold the value rows, HD / 32
 // elements each.  (All 32 lanes to a key and the probabilities by shuffle took 61 shuffles a round: 1000 cycles of the SM's shuffle unit.)
 template <int HD, typename KVT>
-__device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
+__device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target, int share, bool first)
 {
     constexpr int E = HD / 32, VE = 16 / sizeof(KVT), NJ = HD / (8 * VE);
     const PsParams &p = sh.p;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kk = lane >> 3, ln = lane & 7;
     const int Hkv = p.Hkv, group = p.H / Hkv, T = sh.pos + 1;
-    const int g = sh.g, s = sh.s, run = sh.run, used = sh.used;
+    const int g = share % Hkv, s = share / Hkv, run = sh.run, used = sh.used;
     const bool mine = s < used;
     const int k0 = s * run, k1 = min(k0 + run, T);
     const KVT *kc = static_cast<const KVT *>(ly.kc) + (size_t)g * p.max_seq * HD, *vc = static_cast<const KVT *>(ly.vc) + (size_t)g * p.max_seq * HD;
@@ -600,16 +484,18 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
     };
     const bool early = mine && base < k1 && base + PS_KEYS <= sh.pos;        // rows of earlier steps
     if (early) { load_k(base); load_v(base); }
-    PS_TRACE(target / gridDim.x, 1);
-    if (!ps_wait(target)) return false;
-    PS_TRACE(target / gridDim.x, 2);
+    PS_TRACE(target / sh.members, 1);
+    if (first) {
+        if (!ps_wait(target)) return false;
+    } else __syncthreads();                                                  // the share before this one is done with the buffers
+    PS_TRACE(target / sh.members, 2);
     if (!mine) return true;                                                  // uniform in the CTA
     float *qs = reinterpret_cast<float *>(ps_stage()), *om = qs + PS_MAX_GROUP * HD, *ms = om + PS_NW * PS_MAX_GROUP * HD, *ls = ms + PS_NW * PS_MAX_GROUP;
     const float scale = __fmul_rn(rsqrtf((float)HD), 1.4426950408889634f);
     for (int i = threadIdx.x; i < PS_MAX_GROUP * HD; i += PS_THREADS) qs[i] = i < group * HD ? __ldcg(p.q + (size_t)g * group * HD + i) * scale : 0.0f;
     if (!early && base < k1) { load_k(base); load_v(base); }
     __syncthreads();
-    PS_TRACE(target / gridDim.x, 3);
+    PS_TRACE(target / sh.members, 3);
 
     float m = -INFINITY, l = 0.0f, o[PS_MAX_GROUP][E];
     float *prob = sh.prob[warp], *fix = prob + PS_KEYS * PS_MAX_GROUP;
@@ -685,7 +571,7 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
         __syncwarp();
         if (nbase < k1) load_v(nbase);
     }
-    PS_TRACE(target / gridDim.x, 5);
+    PS_TRACE(target / sh.members, 5);
     l += __shfl_xor_sync(0xffffffffu, l, 8);
     l += __shfl_xor_sync(0xffffffffu, l, 16);
     if (lane < PS_MAX_GROUP) {
@@ -719,11 +605,11 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned old;
-        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p.sync + 2 + g), "r"((unsigned)(used - 1)) : "memory");
+        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p.sync + PS_HEADS + g), "r"((unsigned)(used - 1)) : "memory");
         sh.last = old == (unsigned)(used - 1);
     }
     __syncthreads();
-    PS_TRACE(target / gridDim.x, 7);
+    PS_TRACE(target / sh.members, 7);
     if (!sh.last) return true;
     // the last CTA of the kv head: a batch of runs at a time, their values on the way while the warp makes their weights, a lane per run
     const size_t stride = (size_t)Hkv * PS_MAX_GROUP * (HD + 2);
@@ -755,6 +641,60 @@ __device__ __forceinline__ bool ps_attention(const PsLayer &ly, uint32_t target)
 
 // ---------------------------------------------------------------- the step
 
+// All phases of one CTA's shares: its own, or (MANY) every members-th from its own on.  An instantiation of each: with the loop over shares in the way the ordinary
+// case took 3 % longer (Qwen2-0.5B shape: 549 us for 533).
+template <int HD, typename KVT, bool MANY>
+__device__ __forceinline__ void ps_walk(const PsParams &p, int rank, int members)
+{
+    const int steps = 5 * p.num_layers;
+    bool alive = true;
+    auto qkv = [&](const PsLayer &ly, int share) { return share >= ly.seg[PS_V].cta0 ? PS_V : (share >= ly.seg[PS_K].cta0 ? PS_K : PS_Q); };
+    auto qkv_epi = [](int which) { return which == PS_Q ? PS_EPI_ROPE_Q : (which == PS_K ? PS_EPI_ROPE_K : PS_EPI_STORE_V); };
+    // one product in the code for all phases: five times the instructions would not stay in the caches
+#pragma unroll 1
+    for (int k = 0; k <= steps; ++k) {
+        PS_TRACE(k, 0);
+        const int l = k / 5, phase = k - 5 * l;
+        const PsLayer &ly = sh.layer[l & 1];
+        const uint32_t target = (uint32_t)k * members + (k ? p.extra_arrivals : 0);
+#pragma unroll 1
+        for (int share = rank; share < (MANY ? p.ctas : rank + 1) && alive; share += members) {
+            const bool first = !MANY || share == rank;
+            if (phase == 1 && k != steps) {
+                alive = ps_attention<HD, KVT>(ly, target, share, first);
+                continue;
+            }
+            PsWork w;
+            w.gamma = nullptr;
+            w.fetch = -1;
+            w.epi = PS_EPI_STORE;
+            // what is added to the residual row is added once
+            if (k == steps) {
+                w.seg = &p.head; w.out = p.logits; w.src = l && first ? p.prev : nullptr; w.gamma = p.final_gamma;
+            } else if (phase == 0) {
+                const int which = qkv(ly, share);
+                w.seg = &ly.seg[which]; w.src = l && first ? p.prev : nullptr; w.gamma = ly.ln1; w.fetch = first ? l + 1 : -1;
+                w.epi = qkv_epi(which);
+                w.out = which == PS_Q ? (void *)p.q : (which == PS_K ? ly.kc : ly.vc);
+            } else if (phase == 2) {
+                w.seg = &ly.seg[PS_O]; w.out = p.o; w.src = p.att;
+            } else if (phase == 3) {
+                w.seg = &ly.seg[PS_W1]; w.epi = PS_EPI_SWIGLU; w.out = p.mf; w.src = first ? p.o : nullptr; w.gamma = ly.ln2;
+            } else {
+                w.seg = &ly.seg[PS_W2]; w.out = p.prev; w.src = p.mf;
+            }
+            alive = ps_product<HD, KVT>(w, target, share, first);
+        }
+        PS_TRACE(k, 4);
+        if (!alive || k == steps) break;
+        ps_arrive();
+    }
+}
+
+// a function of its own, so that it takes no registers from the ordinary form
+template <int HD, typename KVT>
+__device__ __noinline__ void ps_walk_shares(const PsParams *p, int rank, int members) { ps_walk<HD, KVT, true>(*p, rank, members); }
+
 template <int HD, typename KVT>
 __global__ void __launch_bounds__(PS_THREADS, 1) step_persistent_kernel(const __grid_constant__ PsParams p, const long long limit, int *__restrict__ dev_err)
 {
@@ -766,10 +706,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) step_persistent_kernel(const __
         sh.inv_d = __fdiv_rn(1.0f, (float)p.D);
         sh.pos = pos;
         sh.dead = 0;
-        sh.g = (int)blockIdx.x % p.Hkv;
-        sh.s = (int)blockIdx.x / p.Hkv;
-        sh.run = ps_run_keys(pos + 1, (int)gridDim.x / p.Hkv);
+        sh.run = ps_run_keys(pos + 1, p.ctas / p.Hkv);
         sh.used = (pos + sh.run) / sh.run;
+        ps_enrol(p.sync, p.ctas, limit, dev_err, sh.rank, sh.members);
     }
     for (int i = threadIdx.x; i < p.Da; i += PS_THREADS) ps_x()[i] = __ldcg(p.x + i);
     for (int i = threadIdx.x; i < HD / 2; i += PS_THREADS) {
@@ -777,54 +716,22 @@ __global__ void __launch_bounds__(PS_THREADS, 1) step_persistent_kernel(const __
         sh.cs[1][i] = __ldg(p.sin_cache + (size_t)pos * (HD / 2) + i);
     }
     __syncthreads();
-    ps_fetch_layer(0);
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    const int steps = 5 * p.num_layers;
-    bool alive = true;
-    auto qkv = [&](const PsLayer &ly) { return (int)blockIdx.x >= ly.seg[PS_V].cta0 ? PS_V : ((int)blockIdx.x >= ly.seg[PS_K].cta0 ? PS_K : PS_Q); };
-    auto qkv_epi = [](int which) { return which == PS_Q ? PS_EPI_ROPE_Q : (which == PS_K ? PS_EPI_ROPE_K : PS_EPI_STORE_V); };
-    // one product in the code for all phases: five times the instructions would not stay in the caches
-#pragma unroll 1
-    for (int k = 0; k <= steps; ++k) {
-        PS_TRACE(k, 0);
-        const int l = k / 5, phase = k - 5 * l;
-        const PsLayer &ly = sh.layer[l & 1];
-        if (phase == 1) {
-            alive = ps_attention<HD, KVT>(ly, (uint32_t)k * gridDim.x);
-        } else {
-            PsWork w;
-            w.gamma = nullptr;
-            w.fetch = -1;
-            w.epi = PS_EPI_STORE;
-            if (k == steps) {
-                w.seg = &p.head; w.out = p.logits; w.src = l ? p.prev : nullptr; w.gamma = p.final_gamma;
-            } else if (phase == 0) {
-                const int which = qkv(ly);
-                w.seg = &ly.seg[which]; w.src = l ? p.prev : nullptr; w.gamma = ly.ln1; w.fetch = l + 1;
-                w.epi = qkv_epi(which);
-                w.out = which == PS_Q ? (void *)p.q : (which == PS_K ? ly.kc : ly.vc);
-            } else if (phase == 2) {
-                w.seg = &ly.seg[PS_O]; w.out = p.o; w.src = p.att;
-            } else if (phase == 3) {
-                w.seg = &ly.seg[PS_W1]; w.epi = PS_EPI_SWIGLU; w.out = p.mf; w.src = p.o; w.gamma = ly.ln2;
-            } else {
-                w.seg = &ly.seg[PS_W2]; w.out = p.prev; w.src = p.mf;
-            }
-            alive = ps_product<HD, KVT>(w, (uint32_t)k * gridDim.x);
-        }
-        PS_TRACE(k, 4);
-        if (!alive || k == steps) break;
-        ps_arrive();
+    const int rank = sh.rank, members = sh.members;
+    if (rank >= 0) {
+        ps_fetch_layer(0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (members == p.ctas) ps_walk<HD, KVT, false>(p, rank, members);
+        else ps_walk_shares<HD, KVT>(&p, rank, members);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (alive && blockIdx.x == 0) *p.pos = pos + 1;              // every CTA read it before the first barrier
         unsigned old;
-        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p.sync + 1), "r"(gridDim.x - 1) : "memory");
+        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p.sync + PS_LEFT), "r"(gridDim.x - 1) : "memory");
         if (old == gridDim.x - 1) {                                  // nobody waits any more
-            p.sync[0] = 0;
-            for (int g = 0; g < p.Hkv; ++g) p.sync[2 + g] = 0;       // zero already, unless a wait ran out
+            p.sync[PS_ARRIVALS] = p.sync[PS_JOINED] = p.sync[PS_MEMBERS] = 0;
+            for (int g = 0; g < p.Hkv; ++g) p.sync[PS_HEADS + g] = 0;      // zero already, unless a wait ran out
+            *p.pos = pos + 1;
         }
     }
 }
@@ -842,18 +749,13 @@ static int ps_prepare(size_t smem)
 template <int HD, typename KVT>
 static int ps_launch(const PsParams *p, cudaStream_t st)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ckb_sm_count());
-    cfg.blockDim = dim3(PS_THREADS);
-    cfg.dynamicSmemBytes = p->smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (ckb_check_cuda((int)cudaLaunchKernelEx(&cfg, step_persistent_kernel<HD, KVT>, *p, ckb_wait_limit_cycles(), ckb_device_error_word()), "step_persistent")) return CKB_ERR_CUDA;
-    return ckb_check_launch("step_persistent");
+    PsParams q = *p;
+    q.extra_arrivals = ckb_tune_get("step_extra_arrivals", 0);       // test aid: every barrier waits for arrivals that nobody makes
+    const int missing = ckb_tune_get("step_missing_ctas", 0);        // test aid: CTAs that the step counts on and that never start
+    if (int rc = launch_plain("step_persistent", step_persistent_kernel<HD, KVT>, dim3(missing > 0 && missing < p->ctas ? p->ctas - missing : p->ctas), dim3(PS_THREADS), p->smem, st, q,
+                              ckb_wait_limit_cycles(), ckb_device_error_word()))
+        return rc;
+    return 0;
 }
 
 }  // namespace ckb
@@ -861,7 +763,7 @@ static int ps_launch(const PsParams *p, cudaStream_t st)
 using namespace ckb;
 
 #ifdef CKB_STEP_TRACE
-extern "C" int ckb200_step_trace(long long *out) { return (int)cudaMemcpyFromSymbol(out, ps_trace, sizeof ps_trace); }      // 148 x 512 x 8
+extern "C" int ckb200_step_trace(long long *out) { return (int)cudaMemcpyFromSymbol(out, ps_trace, sizeof ps_trace); }      // 256 x 512 x 8
 #endif
 
 extern "C" size_t ckb_step_persistent_stage_bytes(int fmt, int nb)
@@ -873,16 +775,14 @@ extern "C" size_t ckb_step_persistent_smem(int Da, size_t stage, int head_dim, i
 {
     const size_t attn = (size_t)(PS_MAX_GROUP * head_dim + PS_NW * PS_MAX_GROUP * (head_dim + 2)) * sizeof(float);
     const size_t smem = (size_t)Da * 4 + (stage > attn ? stage : attn);
-    int dev = 0, coop = 0;
-    if (smem > PS_MAX_SMEM || ckb_sm_count() > PS_MAX_CTAS || cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return 0;
+    if (smem > PS_MAX_SMEM || ckb_sm_count() > PS_MAX_CTAS) return 0;
     const int fits = head_dim == 128 ? (kv_f16 ? ps_prepare<128, __half>(smem) : ps_prepare<128, float>(smem))
                                      : (head_dim == 64 ? (kv_f16 ? ps_prepare<64, __half>(smem) : ps_prepare<64, float>(smem)) : 0);
     return fits ? smem : 0;
 }
 
 extern "C" size_t ckb_step_persistent_scratch_bytes(int head_dim) { return (size_t)PS_MAX_CTAS * PS_MAX_GROUP * (head_dim + 2) * sizeof(float); }
-extern "C" size_t ckb_step_persistent_sync_bytes(void) { return (2 + PS_MAX_CTAS) * sizeof(unsigned); }
+extern "C" size_t ckb_step_persistent_sync_bytes(void) { return (PS_HEADS + PS_MAX_CTAS) * sizeof(unsigned); }
 
 // Lanes per row: as many as the row has units, 8 (Q4_K) or 16 (Q6_K) at least.  Rows of several passes are split over the warps of a CTA when all
 // pieces of the matrix fit its CTAs' warps at once: every warp then has one round of loads instead of a walk.

@@ -19,7 +19,7 @@ typedef struct {
     int lanes;              /* lanes that share a row */
     int split;              /* the passes of a row pair go to different warps of a CTA */
     int passes, items;      /* loads of a lane per row; row pairs (or groups of them) of the matrix */
-    int cta0, ncta;         /* the CTAs [cta0, cta0 + ncta) of the grid work on this matrix */
+    int cta0, ncta;         /* the shares [cta0, cta0 + ncta) of the deal work on this matrix */
     int pad[2];
 } PsSeg;
 
@@ -41,17 +41,19 @@ typedef struct {
     const float *x;         /* embedded token, Da values */
     float *q, *att, *o, *mf, *prev, *logits;       /* rows between the phases, widths rounded up to 256 with zero tails */
     float *part;            /* partial attention results: ckb_step_persistent_scratch_bytes() */
-    unsigned *sync;         /* zeroed once; [0] arrivals, [1] departures, [2 + g] arrivals of kv head g */
+    unsigned *sync;         /* zeroed once; ckb_step_persistent_sync_bytes() */
     const float *cos_cache, *sin_cache;
     int *pos;
     int D, Da, H, Hkv, head_dim, max_seq, kv_f16;
+    int ctas;               /* CTAs that rows and keys are dealt to */
+    int extra_arrivals;     /* 0 */
     float eps;
     size_t smem;            /* ckb_step_persistent_smem() */
 } PsParams;
 
 /* shared memory of a matrix's staged input row */
 size_t ckb_step_persistent_stage_bytes(int fmt, int nb);
-/* dynamic shared memory for rows of Da elements and staged inputs of at most `stage` bytes; 0: does not fit or cannot be launched on this device */
+/* dynamic shared memory for rows of Da elements and staged inputs of at most `stage` bytes; 0: does not fit */
 size_t ckb_step_persistent_smem(int Da, size_t stage, int head_dim, int kv_f16);
 size_t ckb_step_persistent_scratch_bytes(int head_dim);
 size_t ckb_step_persistent_sync_bytes(void);

@@ -9,16 +9,34 @@
 //
 //   Q4_K  variant 0: q4p_stage_x + q4p_isums      (pair kernel gemv_q4k.cu; the register-activation kernel runs the same dp4a chain)
 //         variant 1: load_x_q8k<1> + q4k_isums    (direct and ring kernels, gemv.cu)
+//         variant 2: PsQ4::put + PsQ4::isums    (one-launch decode step)
 //   Q6_K  variant 0: ring_stage_x<Q6_K> + q6k_plane_sums, minus 32 x the staged block sums   (planar kernel and ring kernel)
 //         variant 1: load_x_q8k<2> + q6k_isums    (direct kernel)
+//         variant 2: PsQ6::put + PsQ6::input + q6k_plane_sums    (one-launch decode step)
 //
+// The step quantises for itself: its variants put the quants of the given vector in as fp32 values, which come out as they are (iscale = +-1: with the other sign
+// where the first of the largest is positive, which the block's scale, +-1 too, undoes).
 // - on weights in the reference's own row layout.  One warp per row; not a fast path.
-#include "q4p_unit.cuh"
-#include "ring_x.cuh"
+#include "step_units.cuh"
 #include "launch.h"
 #include "runtime.h"
 
 namespace ckb {
+
+// the activation blocks of a Q8_K vector through the step's own quantiser and layout
+template <class T>
+__device__ __forceinline__ void put_q8k(const uint8_t *xg, int nb, uint8_t *smem)
+{
+    const int lane = threadIdx.x & 31;
+    for (int b = threadIdx.x >> 5; b < nb; b += blockDim.x >> 5) {
+        const int8_t *q = reinterpret_cast<const int8_t *>(xg + (size_t)b * Q8K_BYTES + 4) + 8 * lane;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (float)q[j];
+        T::put(v, b, nb, lane, smem);
+    }
+    __syncthreads();
+}
 
 // out[row][b][j], j = 0..7: sum over the 32 elements of sub-block j of (4-bit code) x q8
 template <int VARIANT>
@@ -46,6 +64,24 @@ __global__ void __launch_bounds__(256) subblock_sums_q4k_kernel(const uint8_t *_
                 o[2 * p + 1] = a_hi16 >> 4;          // the kernel leaves the high nibbles in place: 16 x the sum, exactly
                 o[2 * p + 4] = b_lo;
                 o[2 * p + 5] = b_hi16 >> 4;
+            }
+        }
+    } else if constexpr (VARIANT == 2) {
+        put_q8k<PsQ4>(xg, nb, smem);
+        for (int row = blockIdx.x * nw + warp; row < M; row += gridDim.x * nw) {
+            for (int i = lane; i < 2 * nb; i += 32) {
+                const int b = i >> 1, p = i & 1;
+                Q4pW w;
+                int lo[2][2], hi[2][2];
+                PsQ4::load(w, W + (size_t)row * nb * Q4K_BYTES, nb, b, p);
+                PsQ4::isums(w, w, smem, b, p, lo, hi);
+                const int sign = (int)reinterpret_cast<const float *>(smem + (size_t)nb * Q4P_SLOTS * 16)[b];
+                int32_t *o = out + ((size_t)row * nb + b) * 8;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    o[2 * p + 4 * q] = sign * lo[1][q];
+                    o[2 * p + 4 * q + 1] = sign * (hi[1][q] >> 4);
+                }
             }
         }
     } else {
@@ -76,6 +112,7 @@ __global__ void __launch_bounds__(256) subblock_sums_q6k_kernel(const uint8_t *_
     RingX rx = {};
     XQ8K kx = {};
     if constexpr (VARIANT == 0) rx = ring_stage_x<FMT_Q6K>(xg, nb, smem);
+    else if constexpr (VARIANT == 2) put_q8k<PsQ6>(xg, nb, smem);
     else kx = load_x_q8k<2>(xg, nb, smem);
     __syncthreads();
     for (int row = blockIdx.x * nw + warp; row < M; row += gridDim.x * nw) {
@@ -86,7 +123,12 @@ __global__ void __launch_bounds__(256) subblock_sums_q6k_kernel(const uint8_t *_
             const uint4 qb = ldg_u4_align2(p + 64 * n + 32 + 16 * h);
             const uint4 qh = ldg_u4_align2(p + 128 + 32 * n + 16 * h);
             int s[4];
-            if constexpr (VARIANT == 0) {
+            if constexpr (VARIANT == 2) {
+                const PsQ6::X x = PsQ6::input(smem, nb, b, u);
+                q6k_plane_sums(qa, qb, qh, x.q[0], x.q[1], x.q[2], x.q[3], s[0], s[1], s[2], s[3]);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) s[t] = (int)x.d * (s[t] - 32 * ((int)(int8_t)((x.lo4 >> (8 * t)) & 255u) + 128 * (int)(int8_t)((x.hi4 >> (8 * t)) & 255u)));
+            } else if constexpr (VARIANT == 0) {
                 const uint32_t xa = rx.q + (uint32_t)(b * 80 + (10 * n + h) * 4) * 4u;
                 const uint4 x0 = lds_u4(xa), x1 = lds_u4(xa + 32), x2 = lds_u4(xa + 64), x3 = lds_u4(xa + 96);
                 q6k_plane_sums(qa, qb, qh, x0, x1, x2, x3, s[0], s[1], s[2], s[3]);
@@ -132,6 +174,7 @@ extern "C" int ckb200_dev_subblock_sums_q4_k_q8_k(const void *W, const void *x_q
     cudaStream_t st = ckb_stream(stream);
     if (variant == 0) return launch_sums("subblock_sums_q4k", subblock_sums_q4k_kernel<0>, q4p_smem_bytes(nb), W, x_q8, out, M, nb, st);
     if (variant == 1) return launch_sums("subblock_sums_q4k", subblock_sums_q4k_kernel<1>, (xq8k_smem_bytes(nb, 1) + 127) & ~127, W, x_q8, out, M, nb, st);
+    if (variant == 2) return launch_sums("subblock_sums_q4k", subblock_sums_q4k_kernel<2>, q4p_smem_bytes(nb), W, x_q8, out, M, nb, st);
     return ckb_fail(CKB_ERR_STATE, "subblock_sums_q4_k_q8_k: unknown variant %d", variant);
 }
 
@@ -145,5 +188,6 @@ extern "C" int ckb200_dev_subblock_sums_q6_k_q8_k(const void *W, const void *x_q
     cudaStream_t st = ckb_stream(stream);
     if (variant == 0) return launch_sums("subblock_sums_q6k", subblock_sums_q6k_kernel<0>, ringx_smem_bytes(FMT_Q6K, nb), W, x_q8, out, M, nb, st);
     if (variant == 1) return launch_sums("subblock_sums_q6k", subblock_sums_q6k_kernel<1>, (xq8k_smem_bytes(nb, 2) + 127) & ~127, W, x_q8, out, M, nb, st);
+    if (variant == 2) return launch_sums("subblock_sums_q6k", subblock_sums_q6k_kernel<2>, ringx_smem_bytes(FMT_Q6K, nb), W, x_q8, out, M, nb, st);
     return ckb_fail(CKB_ERR_STATE, "subblock_sums_q6_k_q8_k: unknown variant %d", variant);
 }

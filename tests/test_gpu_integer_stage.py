@@ -79,3 +79,22 @@ def test_subblock_sums_recompose_the_gemv(ck, orc, fmt):
     y = cases.gemv(ck, "", fmt, w, xq, m, k)
     y_ref = cases.gemv(orc, "oracle_", fmt, w, xq, m, k)
     assert float(np.max(np.abs(y - y_ref))) <= 1e-5 * float(np.max(np.abs(y_ref)))
+
+
+@pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
+@pytest.mark.parametrize("m,k,seed", [(1, 256, 1), (7, 1024, 3), (130, 4864, 5), (5, 14336, 6)])
+def test_subblock_sums_of_the_one_launch_step(ck, orc, fmt, m, k, seed):
+    """The same for the functions of the one-launch decode step: its quantiser and layout of the input row, its products of row pairs."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    w = synth.make_weights(fmt, m, k, seed)
+    x = synth.make_x(k, seed)
+    x[:256] *= -1                                           # the largest of a block with either sign
+    xq = cases.quantize_act(orc, "oracle_", fmt, x)
+    tw, tx = torch.from_numpy(w).to(dev), torch.from_numpy(xq).to(dev)
+    out = torch.full((m, k // 256, 8 if fmt == "q4_k" else 16), -(2 ** 31), dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
+    assert getattr(ck, f"ckb200_dev_subblock_sums_{fmt}_q8_k")(C.c_void_p(tw.data_ptr()), C.c_void_p(tx.data_ptr()), m, k, C.c_void_p(out.data_ptr()), 2, None) == 0
+    assert ck.ckb200_synchronize() == 0
+    assert np.array_equal(out.cpu().numpy(), oracle_sums(orc, fmt, w, xq, m, k))
