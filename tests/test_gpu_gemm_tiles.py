@@ -101,3 +101,57 @@ def test_gemm_tiles_are_exact_over_the_scales(ck, orc, fmt, scales, width, m, n,
     bound = 2 * (k // 256 + 3) * 2.0 ** -24 * 8 * float(np.max(np.abs(want)))
     assert float(np.max(np.abs(outs[0].astype(np.float64) - want))) <= bound
     assert np.array_equal(outs[0], outs[1])
+
+
+def tiles_from_rows(rows, nt):
+    """What the operand tiles of `nt` tokens hold for Q8_K rows [tokens][superblocks][292]: halves of the quants [tile][superblock][32 chunks][token][8], the 16 sums as two more
+    chunks, the scales [tile][superblock][token]; tokens past the end are left out."""
+    T, nb, _ = rows.shape
+    q = rows[:, :, 4:260].view(np.int8).reshape(T, nb, 32, 8)[..., [0, 2, 1, 3, 4, 6, 5, 7]].astype(np.float16)
+    sums = rows[:, :, 260:292].copy().view(np.int16).reshape(T, nb, 2, 8).astype(np.float16)
+    return np.concatenate([q, sums], 2), rows[:, :, :4].copy().view(np.float32)[..., 0]
+
+
+def split_tiles(raw, nt, T, nb):
+    blobs = raw[:((T + nt - 1) // nt) * nb * nt * 548].reshape(-1, nb, nt * 548)
+    chunks = blobs[:, :, :nt * 544].copy().view(np.float16).reshape(-1, nb, 34, nt, 8)
+    scales = blobs[:, :, nt * 544:].copy().view(np.float32).reshape(-1, nb, nt)
+    return chunks.transpose(0, 3, 1, 2, 4).reshape(-1, nb, 34, 8)[:T], scales.transpose(0, 2, 1).reshape(-1, nb)[:T]
+
+
+@pytest.mark.parametrize("nt", [64, 96, 128])
+@pytest.mark.parametrize("T", [65, 96, 200])
+@pytest.mark.parametrize("producer", ["norm", "swiglu", "gather"])
+def test_producers_write_the_tiles_of_their_rows(ck, producer, nt, T):
+    """The kernels in front of a product write its operand tiles: the same quants, sums and scales as the rows that they write elsewhere, each in its place."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(T)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    nb = 3
+    rows = torch.zeros(T * nb * 292, dtype=torch.uint8, device=dev)
+    tiles = torch.zeros(((T + nt - 1) // nt) * nb * nt * 548, dtype=torch.uint8, device=dev)
+    if producer == "norm":
+        x, delta, gamma = torch.randn(T, 768, device=dev, generator=g), torch.randn(T, 768, device=dev, generator=g), torch.rand(768, device=dev, generator=g) + 0.5
+        x[:, 700:] = 0
+        delta[:, 700:] = 0
+        x2 = x.clone()
+        torch.cuda.synchronize()
+        assert ck.ckb200_dev_add_rmsnorm_q8k(p(x), p(delta), p(gamma), p(rows), None, T, 700, 768, C.c_float(1e-5), None) == 0
+        assert ck.ckb_add_rmsnorm_tiles(p(x2), p(delta), p(gamma), p(tiles), nt, T, 700, 768, C.c_float(1e-5), None) == 0
+    elif producer == "swiglu":
+        gu = torch.randn(T, 1536, device=dev, generator=g)
+        torch.cuda.synchronize()
+        assert ck.ckb200_dev_swiglu_q8k(p(gu), p(rows), T, 768, None) == 0
+        assert ck.ckb_swiglu_tiles(p(gu), p(tiles), nt, T, 768, None) == 0
+    else:
+        out = torch.randn(11, T, 64, device=dev, generator=g)          # 704 of 768 columns
+        torch.cuda.synchronize()
+        assert ck.ckb200_dev_prefill_gather_q8k(p(out), p(rows), T, 11, 64, 768, None) == 0
+        assert ck.ckb_prefill_gather_tiles(p(out), p(tiles), nt, T, 11, 64, 768, None) == 0
+    assert ck.ckb200_synchronize() == 0
+    want, scales = tiles_from_rows(rows.cpu().numpy().reshape(T, nb, 292), nt)
+    got, got_scales = split_tiles(tiles.cpu().numpy(), nt, T, nb)
+    assert np.array_equal(got, want)
+    assert np.array_equal(got_scales, scales)
