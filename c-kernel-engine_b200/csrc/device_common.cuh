@@ -128,16 +128,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     return false;
 }
 // Same contract, for pipelines whose barriers are usually complete already: polls without sleeping and gives up
-// after about a second of SM clock cycles.
+// after about a second of SM clock cycles.  Few instructions: it stands in loops of warps that share an instruction cache.
 __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
+    uint32_t t0, t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t0));
 #pragma unroll 1
-        for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (clock64() - t0 > (1ll << 31)) return false;
-    }
+    do {
+        if (mbar_try_wait(bar, parity)) return true;
+        asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    } while (t - t0 < (1u << 31));
+    return false;
 }
 // src and dst 16-byte aligned, bytes a multiple of 16.  No multicast: one CTA, its own shared memory.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t bar) {

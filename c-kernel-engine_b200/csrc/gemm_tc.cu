@@ -14,7 +14,7 @@
 // is no T2.  The product is an exact fp16 integer whenever |q6 - 32| * |sc| <= 2048, always for |sc| <= 64.  Above that fp16 holds the even integers
 // only: the operand is the nearest of them, and what it lacks (-1, 0 or 1) is an operand of its own, multiplied into the same accumulator.  Files made by a
 // quantiser that scales a superblock to its largest sub-scale have such scales in every superblock; whether there are rests is found per stage and 32 rows
-// (4096 x 14336 at 512 tokens: 110 us without, 125 with; 108 when the products stayed rounded, 1.3e-4 off).
+// (multiplying them costs about a seventh of the time).
 //
 // Two kernels:
 //  * gemm_x_tiles_kernel expands the Q8_K activations once into fp16 operand tiles in the exact shared-memory
@@ -22,11 +22,10 @@
 //    superblock), so the GEMM fetches them with plain 1-D bulk copies.
 //  * gemm_kq_tc_kernel<WF, NT>: one CTA owns 128 weight rows (the M = 128 operand, one TMEM lane each) and one tile of NT tokens
 //    (the N operand, TMEM columns; fewer tokens are zero-padded).  Warp-specialised:
-//        warp 0       loader of activations: bulk copies of 128-deep stages, of the bsum tile and of the block scales of each superblock
+//        warp 0       loader of activations: bulk copies of 128-deep stages (256-deep up to 64 tokens), of the bsum tile and of the block scales of each superblock
 //        warp 1       issuer: tcgen05.mma from one elected lane; tcgen05.commit frees stages and publishes accumulators
-//        warp 2       Q4_K: the 16-deep tile of mins and the (d, dmin) pairs of a superblock
 //        warp 3       loader of weights: the raw superblocks of all 128 rows, one tiled bulk copy each (Q6_K: one per plane)
-//        warps 4-11   two expander sets, thread = row: raw bytes -> fp16 operand, alternate 64-deep k-stages
+//        warps 4-11   two expander sets, thread = row: raw bytes -> fp16 operand in 64-deep k-stages; Q4_K: also the 16-deep tile of mins and the (d, dmin) pairs
 //        warps 12-    drain: tcgen05.ld of T and T2, fp32 sums in registers
 //    Every wait is bounded; a timeout sets the device error word, the CTA drains, frees TMEM and returns.
 //
@@ -37,10 +36,16 @@
 // fence needed between the two.  The raw weights come as 144-byte rows by tiled copies (coalesced, and conflict-free to read at that pitch).
 // A nibble becomes a half with one AND-OR (0x6400 | n = 1024 + n, or 1024 + 16 n for the upper one) and one fused multiply-add; the halves of a
 // register are then elements 0, 2 and 1, 3 of a 4-byte word, and the activation tiles are written in that order: k is a summation index.
-// The 512 TMEM columns at NT = 128: two T buffers (256), one T2 (128), four weight stages (128).
-// A superblock now takes about 1960 cycles: issuer, expanders and drain are each busy for 1500 of them and share four schedulers.
-// Measured (28672 x 4096 Q4_K at 512 / 2048 tokens): 142 / 512 us = 847 / 940 TFLOP/s, with the operand through shared memory 268 / 1055 us; 4096 x 14336 Q6_K
-// at 512 tokens 110 us (181 before); 333 tokens of 28672 x 4096: 126 us against 205 with activations quantised.
+// The 512 TMEM columns at NT = 128: two T buffers (256), one T2 (128), four weight stages (128); up to 96 tokens T2 has two buffers, up to 64 eight stages fit.
+//
+// No unit of the SM is full (counters at 32 tokens: issue slots 64 %, logic 48 %, fp16 and fp32 arithmetic 35 %, tensor 19 %; fp16 arithmetic and logic issue every
+// other cycle): what a superblock takes is instructions, and how far the warps' code lies apart, for eight kinds of work share one instruction cache.  So: the
+// mins are made by the threads that have the header in registers (a warp of its own took 800 cycles a superblock and held up the drain), expander sets take superblocks in turn,
+// waits are four instructions, the sums of a unit leave sixteen columns at a time (see there).  Before and after these, us, with activations made into tiles:
+//   28672 x 4096 Q4_K:  77 tokens 52.4 -> 45.9, 129: 80.6 -> 60.1, 333: 115 -> 105, 512: 140 -> 125 to 129 (935 TFLOP/s)
+//   4096 x 14336 Q6_K:  129 tokens 60.4 -> 47.5, 512: 111 -> 94 to 96
+//   57344 x 8192 Q4_K:  32 tokens 111 -> 76, 64: 222 -> 88;  8192 x 28672 Q6_K: 76 -> 62, 126 -> 72;  128256 x 8192 Q6_K at 32: 213 (4.05 TB/s of weights)
+// (with the operand through shared memory 28672 x 4096 at 512 tokens took 268).
 #include <cuda.h>
 
 #include "q8k_block.cuh"
@@ -54,8 +59,7 @@ namespace ckb {
 
 constexpr int TC_ROWS = 128;                          // rows of the weight operand per MMA
 constexpr int TC_AUX = TC_ROWS * 32;                  // 16-deep tile of the mins: 4 KB
-constexpr int TC_ASLOTS = 4, TC_BSLOTS = 4, TC_RSLOTS = 3, TC_XSLOTS = 4;   // rings: 64-deep weight stages in TMEM, 128-deep activation stages, raw
-                                                                          // superblocks, per-superblock extras (mins, bsums, scales)
+constexpr int TC_BSLOTS = 4, TC_XSLOTS = 4;           // rings: activation stages, per-superblock extras (mins, bsums, scales)
 enum { TC_W_Q4K = 0, TC_W_Q6K_PLANAR = 1 };           // weight operand formats
 
 // Activation blob of one (tile of NT tokens, superblock): four 64-deep k-stages, the 16-deep bsum tile, NT block scales.
@@ -68,42 +72,47 @@ struct TcTile {
     static_assert(XBLOB == q8k_tile_bytes(NT), "the layout that quantize_block_q8k_tile writes");
 };
 
-// Everything that depends on the width NT of the token tile and on the weight format.  NT = 32: the accumulators and the staging shrink so far that
-// two CTAs share an SM and each covers the other's latencies.
+// Everything that depends on the width NT of the token tile and on the weight format.
 template <int WF, int NT>
 struct TcCfg : TcTile<NT> {
     static constexpr bool Q4 = WF == TC_W_Q4K;
     // raw superblocks of 128 rows: 144-byte rows, or the planes ql | qh | scales (1024-byte aligned: they are written swizzled)
     static constexpr int RAW_QH = TC_ROWS * 128, RAW_SC = RAW_QH + TC_ROWS * 64, RAW = Q4 ? TC_ROWS * Q4K_BYTES : RAW_SC + TC_ROWS * 16;
+    static constexpr int RSLOTS = NT > 96 || NT == 64 ? 3 : (NT == 96 ? (Q4 ? 5 : 4) : (Q4 ? 7 : 5));        // ring of raw superblocks: what is left of shared memory
+    static constexpr int BDEEP = NT > 64 ? 2 : 4;                    // 64-deep stages in a slot of the activation ring: half a superblock or all of it
+    static constexpr int BSLOT = BDEEP * TcTile<NT>::STAGE;
+    static constexpr int ADEEP = NT > 64 ? 1 : 2, ASLOTS = 4;        // ring of weight stages in tensor memory, 64-deep or 128-deep: one superblock or two
+    // Q4_K: the expander sets take superblocks in turn; where they share the slots, each has barriers of its own for them.  Q6_K: a half of every superblock each.
+    static constexpr int AEMPTIES = Q4 && ADEEP == 1 ? 2 * ASLOTS : ASLOTS, TAKERS = Q4 ? 4 : 8;      // warps that read a raw superblock
     static constexpr int OFF_RAW = 0;
-    static constexpr int OFF_B = OFF_RAW + TC_RSLOTS * RAW;
-    static constexpr int OFF_A2 = OFF_B + TC_BSLOTS * 2 * TcTile<NT>::STAGE;
+    static constexpr int OFF_B = OFF_RAW + RSLOTS * RAW;
+    static constexpr int OFF_A2 = OFF_B + TC_BSLOTS * BSLOT;
     static constexpr int OFF_B2 = OFF_A2 + (Q4 ? TC_XSLOTS * TC_AUX : 0);
     static constexpr int OFF_DX = OFF_B2 + (Q4 ? TC_XSLOTS * TcTile<NT>::AUX : 0);
     static constexpr int OFF_DD = OFF_DX + TC_XSLOTS * NT * 4;                     // fp16 d | dmin of the rows
     static constexpr int OFF_BAR = OFF_DD + (Q4 ? TC_XSLOTS * TC_ROWS * 4 : 0);
-    static constexpr int A_FULL = 0, A_EMPTY = A_FULL + TC_ASLOTS, B_FULL = A_EMPTY + TC_ASLOTS, B_EMPTY = B_FULL + TC_BSLOTS, R_FULL = B_EMPTY + TC_BSLOTS,
-                         R_EMPTY = R_FULL + TC_RSLOTS, X_FULL = R_EMPTY + TC_RSLOTS, X_EMPTY = X_FULL + TC_XSLOTS, T_FULL = X_EMPTY + TC_XSLOTS, T_EMPTY = T_FULL + 2,
+    static constexpr int A_FULL = 0, A_EMPTY = A_FULL + ASLOTS, B_FULL = A_EMPTY + AEMPTIES, B_EMPTY = B_FULL + TC_BSLOTS, R_FULL = B_EMPTY + TC_BSLOTS,
+                         R_EMPTY = R_FULL + RSLOTS, X_FULL = R_EMPTY + RSLOTS, X_EMPTY = X_FULL + TC_XSLOTS, T_FULL = X_EMPTY + TC_XSLOTS, T_EMPTY = T_FULL + 2,
                          T2_EMPTY = T_EMPTY + 2, DONE = T2_EMPTY + 1, BARS = DONE + 1;
-    static constexpr int OFF_WIDE = OFF_BAR + BARS * 8 + 16;                       // Q6_K: a byte per (weight stage, lane quarter): there are rests
-    static constexpr int SMEM = OFF_WIDE + 4 * TC_ASLOTS;
+    // Q6_K, a byte per (weight stage, lane quarter): there are rests
+    static constexpr int OFF_WIDE = OFF_BAR + BARS * 8 + 16, SMEM = OFF_WIDE + 4 * ASLOTS * ADEEP;
     static constexpr int DRAIN_WARPS = NT > 32 ? 8 : 4;       // 4 TMEM lane quarters x column halves
     static constexpr int DRAIN_COLS = NT / (DRAIN_WARPS / 4); // token columns per drain thread
-    static constexpr int THREADS = (12 + DRAIN_WARPS) * 32, CTAS_PER_SM = NT > 32 ? 1 : 2;
+    static constexpr int THREADS = (12 + DRAIN_WARPS) * 32;
     // Register counts per role after setmaxnreg.  setmaxnreg.inc blocks until the CTA's own pool (threads x registers
     // at launch) can supply the registers, so 128 * CTL + 256 * EXP + 32 * DRAIN_WARPS * DRAIN must not exceed
     // THREADS * LAUNCH; the launcher checks the compiled register count against LAUNCH before the first launch.
-    static constexpr int REGS_LAUNCH = NT > 32 ? 96 : 64, REGS_CTL = 48, REGS_EXP = 72, REGS_DRAIN = NT > 32 ? 144 : 64;
+    static constexpr int REGS_LAUNCH = NT > 32 ? 96 : 128, REGS_CTL = NT > 32 ? 48 : 128, REGS_EXP = NT > 32 ? 72 : 128, REGS_DRAIN = NT > 32 ? 144 : 128;
     static_assert(128 * REGS_CTL + 256 * REGS_EXP + 32 * DRAIN_WARPS * REGS_DRAIN <= THREADS * REGS_LAUNCH, "setmaxnreg targets exceed the CTA's register pool");
-    static_assert(THREADS * REGS_LAUNCH * CTAS_PER_SM <= 65536, "register plan");
-    // T buffer u at column u * NT.  Q6_K has no T2; what its stages lack goes behind them, a slot per stage or (two CTAs on an SM) per expander set.
-    static constexpr uint32_t TM_T2 = 2 * NT, TM_A = (Q4 ? 3 : 2) * NT, TM_R = TM_A + 32 * TC_ASLOTS, TMEM_COLS = NT > 32 ? 512 : 256;
-    static constexpr uint32_t RESTS = Q4 ? 0 : (NT > 32 ? TC_ASLOTS : 2);
-    static_assert(TM_R + 32 * RESTS <= TMEM_COLS && CTAS_PER_SM * TMEM_COLS <= 512, "tensor memory plan");
+    static_assert(THREADS * REGS_LAUNCH <= 65536, "register plan");
+    // T buffer u at column u * NT; T2 has two buffers too where they fit.  Q6_K has no T2; what its stages lack goes behind them, a slot for each stage of a superblock.
+    static constexpr bool T2_TWICE = NT <= 96;
+    static constexpr uint32_t TM_T2 = 2 * NT, TM_A = Q4 ? (T2_TWICE ? 4 : 3) * NT : 2 * NT, TM_R = TM_A + 32 * ADEEP * ASLOTS, TMEM_COLS = 512;
+    static_assert(TM_R + (Q4 ? 0 : 32 * 4) <= TMEM_COLS, "tensor memory plan");
     // instruction descriptor: f16 x f16 -> f32, both operands K-major, M = 128, N = NT
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);
     static_assert(NT % 32 == 0 && NT <= 128 && RAW % (Q4 ? 16 : 1024) == 0 && OFF_BAR % 8 == 0 && OFF_B % 128 == 0, "layout");
-    static_assert(CTAS_PER_SM * (SMEM + 1024) <= 228 * 1024 && SMEM <= 227 * 1024, "shared memory plan");
+    static_assert(SMEM <= 227 * 1024, "shared memory plan");
 };
 
 // shared-memory matrix descriptor: K-major, no swizzle; LBO = distance between the two 8-element k-chunks of
@@ -146,8 +155,8 @@ __device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u));
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate));
 }
 // 32 columns of this warp's 32 lanes
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32])
@@ -181,14 +190,15 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 
-// The 64 weights of one row in k-stage s of a Q4_K superblock (sub-blocks 2s and 2s + 1: 32 nibble bytes) times their 6-bit scales:
+// 6-bit scales (or mins) of sub-blocks 4 n .. 4 n + 3 of a Q4_K superblock as bytes: their own word, and the four bits that lie with the other kind's
+__device__ __forceinline__ uint32_t q4k_scales4(uint32_t six, uint32_t four, int n) { return n ? (four & 0x0F0F0F0Fu) | ((six >> 2) & 0x30303030u) : six & 0x3F3F3F3Fu; }
+
+// The 64 weights of one row in a k-stage of a Q4_K superblock (two sub-blocks: 32 nibble bytes) times their scales (bytes 2 hi and 2 hi + 1 of sc):
 // (1024 + n) * sc - 1024 * sc and (1024 + 16 n) * sc / 16 - 64 * sc, exact: only the result (at most 945) is rounded
-__device__ __forceinline__ void q4k_expand(const uint4 &hdr, const uint4 &qa, const uint4 &qb, int s, uint32_t (&o)[32])
+__device__ __forceinline__ void q4k_expand(uint32_t sc, const uint4 &qa, const uint4 &qb, uint32_t (&o)[32])
 {
-    uint32_t sc2, m2;
-    q4k_scales(hdr.y, hdr.z, hdr.w, s, sc2, m2);
     const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f);
-    const __half2 s_lo = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4040)), k1024), s_hi = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4141)), k1024);
+    const __half2 s_lo = __hsub2(bits_h2(__byte_perm(sc, 0x64646464u, 0x4040)), k1024), s_hi = __hsub2(bits_h2(__byte_perm(sc, 0x64646464u, 0x4141)), k1024);
     const __half2 b_lo = __hmul2(s_lo, __floats2half2_rn(-1024.0f, -1024.0f)), b_hi = __hmul2(s_hi, __floats2half2_rn(-64.0f, -64.0f));
     const __half2 s_hi16 = __hmul2(s_hi, __floats2half2_rn(0.0625f, 0.0625f));
     const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
@@ -202,57 +212,67 @@ __device__ __forceinline__ void q4k_expand(const uint4 &hdr, const uint4 &qa, co
     }
 }
 
-// The same for Q6_K: k-stage 2 n + hi holds weights 128 n + 64 hi .. + 63: nibbles `hi` of the 64 ql bytes of half n, 2-bit planes 2 hi and
-// 2 hi + 1 of its 32 qh bytes, scales 8 n + 4 hi .. + 3.  raw: the row's planes as the swizzled copies left them.
-__device__ __forceinline__ void q6k_expand(const uint8_t *raw_ql, const uint8_t *raw_qh, uint32_t scw, int row, int n, int hi, uint32_t (&o)[32])
-{
-    const __half2 c66 = __floats2half2_rn(66.0f, 66.0f);
-    uint32_t qhw[8];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {            // 64-byte swizzle: 16-byte pieces permuted by bits 1-2 of the row
-        const uint4 v = *reinterpret_cast<const uint4 *>(raw_qh + row * 64 + (((2 * n + j) ^ ((row >> 1) & 3)) << 4));
-        qhw[4 * j] = v.x >> (4 * hi); qhw[4 * j + 1] = v.y >> (4 * hi); qhw[4 * j + 2] = v.z >> (4 * hi); qhw[4 * j + 3] = v.w >> (4 * hi);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {            // 128-byte swizzle: 16-byte pieces permuted by the row's low three bits
-        const uint4 v = *reinterpret_cast<const uint4 *>(raw_ql + row * 128 + (((4 * n + j) ^ (row & 7)) << 4));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        const float scf = 16.0f * (float)(int)(int8_t)((scw >> (8 * j)) & 255u);      // 16 weights per scale = one 16-byte piece
-        const __half2 sc2 = __floats2half2_rn(scf, scf);
+// The same for Q6_K: k-stage 2 n + hi holds weights 128 n + 64 hi .. + 63: nibbles hi of the 64 ql bytes of half n, 2-bit planes 2 hi and
+// 2 hi + 1 of its 32 qh bytes, scales 8 n + 4 hi .. + 3 (scw), one for each 16-byte piece of ql.  The row's planes lie as the swizzled copies left them.
+struct Q6kStage {
+    const uint8_t *ql, *qh;
+    uint32_t scw;
+    int n, row, shift, plane;         // right shift of ql; left rotation of qh that brings plane 2 hi to bits 4 and 5
+    __device__ __forceinline__ Q6kStage(const uint8_t *raw_ql, const uint8_t *raw_qh, uint32_t scales, int r, int half, int hi)
+        : ql(raw_ql + r * 128), qh(raw_qh + r * 64), scw(scales), n(half), row(r), shift(4 * hi), plane(4 - 4 * hi) {}
+    // 16-byte pieces are permuted by the row's low three bits (128-byte swizzle) and by its bits 1-2 (64-byte swizzle)
+    __device__ __forceinline__ uint4 low(int j) const { return *reinterpret_cast<const uint4 *>(ql + (((4 * n + j) ^ (row & 7)) << 4)); }
+    __device__ __forceinline__ uint4 high(int j) const { return *reinterpret_cast<const uint4 *>(qh + (((2 * n + j) ^ ((row >> 1) & 3)) << 4)); }
+    // four weights + 32 out of a word of each, piece J: bytes 0 .. 63
+    template <int J>
+    __device__ __forceinline__ uint32_t bytes(uint32_t l, uint32_t h) const { return ((l >> shift) & 0x0F0F0F0Fu) | (__funnelshift_l(h, h, J < 2 ? plane : plane - 2) & 0x30303030u); }
+    // scale of piece J, exact: 1152 + scale, less 1152
+    template <int J>
+    __device__ __forceinline__ __half2 scale() const { return __hsub2(bits_h2(__byte_perm(scw ^ 0x80808080u, 0x64646464u, 0x4040 + 0x0101 * J)), __floats2half2_rn(1152.0f, 1152.0f)); }
+    // weights of the bytes 0 2 (e = 0) or 1 3
+    static __device__ __forceinline__ __half2 weight(uint32_t q, int e) { return __hsub2(bits_h2(__byte_perm(q, 0x64646464u, e ? 0x4341 : 0x4240)), __floats2half2_rn(1056.0f, 1056.0f)); }
+
+    template <int J>
+    __device__ __forceinline__ void piece(const uint4 &l, const uint4 &h, uint32_t *o) const
+    {
+        const __half2 sc = scale<J>();
+        const uint32_t w[4] = {l.x, l.y, l.z, l.w}, g[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t nib = (w[i] >> (4 * hi)) & 0x0F0F0F0Fu, h = qhw[4 * (j & 1) + i];
-            const uint32_t q = nib | ((j < 2 ? h << 4 : h << 2) & 0x30303030u);
-            // 0x5400 | q is the fp16 bit pattern of 64 + q / 16: (q - 32) / 16 * 16 sc
-            o[8 * j + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(and_or(q, 0x00FF00FFu, 0x54005400u)), c66), sc2));
-            o[8 * j + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(and_or(q >> 8, 0x00FF00FFu, 0x54005400u)), c66), sc2));
+            const uint32_t q = bytes<J>(w[i], g[i]);
+            o[2 * i] = h2_bits(__hmul2(weight(q, 0), sc));
+            o[2 * i + 1] = h2_bits(__hmul2(weight(q, 1), sc));
         }
     }
-}
-// Half a stage (16-byte pieces 2 P and 2 P + 1) as the rounded products and what they lack, which one fused multiply-add gives exactly
-template <int P>
-__device__ __forceinline__ void q6k_expand_rests(const uint8_t *raw_ql, const uint8_t *raw_qh, uint32_t scw, int row, int n, int hi, uint32_t (&o)[16], uint32_t (&t)[16])
-{
-    const __half2 c66 = __floats2half2_rn(66.0f, 66.0f);
+    __device__ __forceinline__ void expand(uint32_t (&o)[32]) const
+    {
+        const uint4 h0 = high(0), h1 = high(1);
+        piece<0>(low(0), h0, o);
+        piece<1>(low(1), h1, o + 8);
+        piece<2>(low(2), h0, o + 16);
+        piece<3>(low(3), h1, o + 24);
+    }
+    // Pieces 2 h and 2 h + 1 as the rounded products and what they lack, which one fused multiply-add gives exactly.  Rarely run, so short rather than fast.
+    __device__ __forceinline__ void rests(int h, uint32_t (&o)[16], uint32_t (&t)[16]) const
+    {
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const uint4 g = *reinterpret_cast<const uint4 *>(raw_qh + row * 64 + (((2 * n + j) ^ ((row >> 1) & 3)) << 4));
-        const uint4 v = *reinterpret_cast<const uint4 *>(raw_ql + row * 128 + (((4 * n + 2 * P + j) ^ (row & 7)) << 4));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w}, qh[4] = {g.x, g.y, g.z, g.w};
-        const float scf = 16.0f * (float)(int)(int8_t)((scw >> (8 * (2 * P + j))) & 255u);
-        const __half2 sc2 = __floats2half2_rn(scf, scf);
+        for (int j = 0; j < 2; ++j) {
+            const uint4 l = low(2 * h + j), g4 = high(j);
+            const uint32_t w[4] = {l.x, l.y, l.z, l.w}, g[4] = {g4.x, g4.y, g4.z, g4.w};
+            const __half2 sc = __hsub2(bits_h2(__byte_perm(scw ^ 0x80808080u, 0x64646464u, 0x4040u + 0x0101u * (uint32_t)(2 * h + j))), __floats2half2_rn(1152.0f, 1152.0f));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t h = qh[i] >> (4 * hi), q = ((w[i] >> (4 * hi)) & 0x0F0F0F0Fu) | ((P == 0 ? h << 4 : h << 2) & 0x30303030u);
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t q = ((w[i] >> shift) & 0x0F0F0F0Fu) | (__funnelshift_l(g[i], g[i], plane - 2 * h) & 0x30303030u);
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const __half2 a = __hsub2(bits_h2(and_or(e ? q >> 8 : q, 0x00FF00FFu, 0x54005400u)), c66), p = __hmul2(a, sc2);
-                o[8 * j + 2 * i + e] = h2_bits(p);
-                t[8 * j + 2 * i + e] = h2_bits(__hfma2(a, sc2, __hneg2(p)));
+                for (int e = 0; e < 2; ++e) {
+                    const __half2 v = weight(q, e), p = __hmul2(v, sc);
+                    o[8 * j + 2 * i + e] = h2_bits(p);
+                    t[8 * j + 2 * i + e] = h2_bits(__hfma2(v, sc, __hneg2(p)));
+                }
             }
         }
     }
-}
+};
 // whether one of four scales is outside [-64, 63]
 __device__ __forceinline__ bool q6k_wide(uint32_t scw) { return ((((scw & 0x7F7F7F7Fu) + 0x40404040u) ^ scw) & 0x80808080u) != 0; }
 
@@ -307,31 +327,30 @@ __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__rest
 
 // ---------------------------------------------------------------- GEMM
 
-template <uint32_t V> struct TcConst { static constexpr uint32_t value = V; };
 struct TcMaps { CUtensorMap w[3]; };                  // Q4_K: rows; Q6_K: planes ql, qh, scales
 
-// Work of a launch: units of (K slice, row tile, token tile), token tiles innermost, dealt round-robin to persistent CTAs.  A slice z takes the superblocks
-// [z * nbz, z * nbz + nbz) and writes its partial sums to C + z * cz (the launcher adds the slices up in a fixed order); a single slice writes C
-// itself, bias included.  Only the loaders and the drain know where a unit ends; the other roles see one run of superblocks, so that the next unit's
+// Work of a product: units dealt round-robin to persistent CTAs, token tiles innermost; a launch does those from `begin` on.  First `whole` units, a tile of the first row tiles and all of K each,
+// which write C, bias included; then the last split_nt row tiles in K slices of nbz superblocks, which write partial sums (the launcher adds them up in a fixed
+// order).  Only the loaders and the drain know where a unit ends; the other roles see one run of superblocks, so that the next unit's
 // weights are expanded and multiplied while the last one's sums are stored (a CTA per unit spent 6 us of 23 starting and storing).
 struct TcWork {
-    int units, mtiles, ntiles, nb_row, nbz;
+    int begin, units, whole, mtiles, split_nt, nb_row, nbz;
     __device__ __forceinline__ int mt(int u) const { return u % mtiles; }
-    __device__ __forceinline__ int nt(int u) const { return u / mtiles % ntiles; }
-    __device__ __forceinline__ int z(int u) const { return u / mtiles / ntiles; }
+    __device__ __forceinline__ int nt(int u) const { return u < whole ? u / mtiles : whole / mtiles + (u - whole) / mtiles % split_nt; }
+    __device__ __forceinline__ int z(int u) const { return u < whole ? 0 : (u - whole) / mtiles / split_nt; }
     __device__ __forceinline__ int kb0(int u) const { return z(u) * nbz; }
-    __device__ __forceinline__ int nb(int u) const { return min(nbz, nb_row - kb0(u)); }
+    __device__ __forceinline__ int nb(int u) const { return u < whole ? nb_row : min(nbz, nb_row - kb0(u)); }
 };
 
 template <int WF, int NT>
-__global__ void __launch_bounds__(TcCfg<WF, NT>::THREADS, TcCfg<WF, NT>::CTAS_PER_SM)
+__global__ void __launch_bounds__(TcCfg<WF, NT>::THREADS, 1)
 gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const uint8_t *__restrict__ xt, const uint8_t *__restrict__ B, const float *__restrict__ bias,
-                  float *__restrict__ C, int ldc, size_t cz, int M, int N, int *__restrict__ dev_err)
+                  float *__restrict__ C, int ldc, float *__restrict__ part, int M, int N, int *__restrict__ dev_err)
 {
     using Cfg = TcCfg<WF, NT>;
     constexpr bool Q4 = Cfg::Q4;
     uint32_t total = 0;                               // superblocks of all this CTA's units
-    for (int u = blockIdx.x; u < work.units; u += gridDim.x) total += (uint32_t)work.nb(u);
+    for (int u = work.begin + blockIdx.x; u < work.units; u += gridDim.x) total += (uint32_t)work.nb(u);
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t s_base = smem_u32(smem), s_bar = s_base + Cfg::OFF_BAR;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Cfg::OFF_BAR + Cfg::BARS * 8);
@@ -340,11 +359,12 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     if (tid == 0) {
-        for (int i = 0; i < TC_ASLOTS; ++i) { mbar_init(BAR(Cfg::A_FULL + i), 4); mbar_init(BAR(Cfg::A_EMPTY + i), 1); }
+        for (int i = 0; i < Cfg::ASLOTS; ++i) { mbar_init(BAR(Cfg::A_FULL + i), 4); }
+        for (int i = 0; i < Cfg::AEMPTIES; ++i) mbar_init(BAR(Cfg::A_EMPTY + i), 1);
         for (int i = 0; i < TC_BSLOTS; ++i) { mbar_init(BAR(Cfg::B_FULL + i), 1); mbar_init(BAR(Cfg::B_EMPTY + i), 1); }
-        for (int i = 0; i < TC_RSLOTS; ++i) { mbar_init(BAR(Cfg::R_FULL + i), 1); mbar_init(BAR(Cfg::R_EMPTY + i), Q4 ? 9 : 8); }     // expander warps and warp 2
+        for (int i = 0; i < Cfg::RSLOTS; ++i) { mbar_init(BAR(Cfg::R_FULL + i), 1); mbar_init(BAR(Cfg::R_EMPTY + i), Cfg::TAKERS); }
         for (int i = 0; i < TC_XSLOTS; ++i) {
-            mbar_init(BAR(Cfg::X_FULL + i), Q4 ? 2 : 1);                            // loader (and its bytes), warp 2
+            mbar_init(BAR(Cfg::X_FULL + i), Q4 ? 5 : 1);                            // loader (and its bytes), the set that writes the mins
             mbar_init(BAR(Cfg::X_EMPTY + i), Cfg::DRAIN_WARPS + (Q4 ? 1 : 0));      // drain, T2's MMA
         }
         for (int i = 0; i < 2; ++i) { mbar_init(BAR(Cfg::T_FULL + i), 1); mbar_init(BAR(Cfg::T_EMPTY + i), Cfg::DRAIN_WARPS); }
@@ -363,29 +383,34 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
     pdl_trigger();
 
 #define TC_SETMAXNREG(op, n) asm volatile("setmaxnreg." op ".sync.aligned.u32 %0;" ::"n"(n))
+#define TC_REGISTERS(n)                                                          \
+    do {                                                                         \
+        if constexpr ((n) < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", n);           \
+        else if constexpr ((n) > Cfg::REGS_LAUNCH) TC_SETMAXNREG("inc", n);      \
+    } while (0)
 #define TC_WAIT(bar, parity, code)                                        \
     if (!mbar_wait_spin(bar, parity)) { atomicExch(dev_err, code); break; }
 
     if (warp < 4) {
-        TC_SETMAXNREG("dec", Cfg::REGS_CTL);
+        TC_REGISTERS(Cfg::REGS_CTL);
         if (warp == 0) {
             // ------------------------------------------------------------ activations
             pdl_wait();                                // the tiles are what the kernel before this one writes; weights are nobody's output
             uint32_t g = 0, issued = 0, extras = 0;
             bool go = true;
-            for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+            for (int u = work.begin + blockIdx.x; u < work.units && go; u += gridDim.x) {
                 const uint8_t *blob = xt + ((size_t)work.mt(u) * work.nb_row + work.kb0(u)) * Cfg::XBLOB;
                 for (int nb = work.nb(u); nb > 0 && go; --nb, ++g, blob += Cfg::XBLOB) {
                     const uint32_t x = g % TC_XSLOTS;
+                    constexpr uint32_t PARTS = 4 / Cfg::BDEEP;
 #pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) {
-                        const uint32_t i = 2 * (g & 1u) + h;
-                        if (!mbar_wait_spin(BAR(Cfg::B_EMPTY + i), ((g >> 1) & 1u) ^ 1u)) { go = false; break; }
+                    for (uint32_t h = 0; h < PARTS; ++h, ++issued) {
+                        const uint32_t i = issued % TC_BSLOTS;
+                        if (!mbar_wait_spin(BAR(Cfg::B_EMPTY + i), ((issued / TC_BSLOTS) & 1u) ^ 1u)) { go = false; break; }
                         if (tc_elect_one()) {
-                            mbar_arrive_expect_tx(BAR(Cfg::B_FULL + i), 2 * Cfg::STAGE);
-                            bulk_g2s(s_base + Cfg::OFF_B + i * 2 * Cfg::STAGE, blob + h * 2 * Cfg::STAGE, 2 * Cfg::STAGE, BAR(Cfg::B_FULL + i));
+                            mbar_arrive_expect_tx(BAR(Cfg::B_FULL + i), Cfg::BSLOT);
+                            bulk_g2s(s_base + Cfg::OFF_B + i * Cfg::BSLOT, blob + h * Cfg::BSLOT, Cfg::BSLOT, BAR(Cfg::B_FULL + i));
                         }
-                        ++issued;
                     }
                     if (!go || !mbar_wait_spin(BAR(Cfg::X_EMPTY + x), ((g / TC_XSLOTS) & 1u) ^ 1u)) { go = false; break; }
                     if (tc_elect_one()) {
@@ -402,96 +427,66 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             for (uint32_t b = extras > TC_XSLOTS ? extras - TC_XSLOTS : 0; b < extras; ++b) mbar_wait_spin(BAR(Cfg::X_FULL + b % TC_XSLOTS), (b / TC_XSLOTS) & 1u);
         } else if (warp == 1) {
             // ------------------------------------------------------------ issuer: the warp runs the loop and the waits uniformly, one lane issues.  This
-            // warp is a chain of short dependent steps, and the MMAs of a 64-deep stage take 256 cycles: two superblocks are unrolled so that
-            // slots, descriptors and most parities are constants (with them computed in a loop of stages the chain took 900 cycles a stage).
+            // warp is a chain of short dependent steps that the MMAs of a 64-deep stage (64 to 260 cycles) have to cover: the stages of a superblock are unrolled
+            // (in a loop they took a fifth longer); two superblocks unrolled as well were not faster and crowd the instruction cache.
             const uint64_t dB = tc_smem_desc(s_base + Cfg::OFF_B, Cfg::CHUNK), dA2 = tc_smem_desc(s_base + Cfg::OFF_A2, TC_ROWS * 16), dB2 = tc_smem_desc(s_base + Cfg::OFF_B2, Cfg::CHUNK);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             const bool leader = tc_elect_one();
-            auto superblock = [&](auto odd, uint32_t b) -> bool {
-                constexpr uint32_t u = decltype(odd)::value;
-                const uint32_t p = (b >> 1) & 1u, x [[maybe_unused]] = b % TC_XSLOTS;
-                if (!mbar_wait_spin(BAR(Cfg::T_EMPTY + u), p ^ 1u)) return false;
+            bool go = true;
+#pragma unroll 1
+            for (uint32_t b = 0; b < total && go; ++b) {
+                const uint32_t u = b & 1u, p = (b >> 1) & 1u, x [[maybe_unused]] = b % TC_XSLOTS;
+                const uint32_t a0 = Cfg::ADEEP == 2 ? 2 * u : 0, pa = Cfg::ADEEP == 2 ? p : u;
+                const uint32_t pb = Cfg::BDEEP == 4 ? (b >> 2) & 1u : p, b0 = Cfg::BDEEP == 4 ? b & 3u : 2 * u;
+                if (!mbar_wait_spin(BAR(Cfg::T_EMPTY + u), p ^ 1u)) { go = false; break; }
 #pragma unroll
                 for (uint32_t s = 0; s < 4; ++s) {
                     constexpr uint32_t half = Cfg::STAGE >> 4;
-                    const uint32_t i = 2 * u + (s >> 1);
-                    if (!(s & 1u) && !mbar_wait_spin(BAR(Cfg::B_FULL + i), p)) return false;
-                    if (!mbar_wait_spin(BAR(Cfg::A_FULL + s), u)) return false;
+                    const uint32_t i = b0 + s / Cfg::BDEEP, a = a0 + s / Cfg::ADEEP;
+                    if (s % Cfg::BDEEP == 0 && !mbar_wait_spin(BAR(Cfg::B_FULL + i), pb)) { go = false; break; }
+                    if (s % Cfg::ADEEP == 0 && !mbar_wait_spin(BAR(Cfg::A_FULL + a), pa)) { go = false; break; }
                     tc_fence_after();                  // the expanders' stores, and (s = 0) the drain's loads of this accumulator, come before these MMAs
                     if (leader) {
                         uint32_t wide = 0;
-                        if constexpr (!Q4) wide = *reinterpret_cast<const volatile uint32_t *>(smem + Cfg::OFF_WIDE + 4 * s);
+                        if constexpr (!Q4) wide = *reinterpret_cast<const volatile uint32_t *>(smem + Cfg::OFF_WIDE + 4 * (Cfg::ADEEP * a0 + s));
+                        const uint64_t d = dB + (uint64_t)(half * (Cfg::BDEEP * b0 + s));
 #pragma unroll
                         for (uint32_t k = 0; k < 4; ++k)
-                            tc_mma_ta(tm + NT * u, tm + Cfg::TM_A + 32 * s + 8 * k, dB + (uint64_t)(half * (2 * i + (s & 1u)) + k * (2 * Cfg::CHUNK >> 4)), Cfg::IDESC, (s | k) ? 1u : 0u);
+                            tc_mma_ta(tm + NT * u, tm + Cfg::TM_A + 32 * (Cfg::ADEEP * a0 + s) + 8 * k, d + (uint64_t)(k * (2 * Cfg::CHUNK >> 4)), Cfg::IDESC, (s | k) ? 1u : 0u);
                         if constexpr (!Q4) {
                             if (wide) {
-#pragma unroll
+#pragma unroll 1
                                 for (uint32_t k = 0; k < 4; ++k)
-                                    tc_mma_ta(tm + NT * u, tm + Cfg::TM_R + 32 * (s % Cfg::RESTS) + 8 * k, dB + (uint64_t)(half * (2 * i + (s & 1u)) + k * (2 * Cfg::CHUNK >> 4)), Cfg::IDESC, 1u);
+                                    tc_mma_ta(tm + NT * u, tm + Cfg::TM_R + 32 * s + 8 * k, d + (uint64_t)(k * (2 * Cfg::CHUNK >> 4)), Cfg::IDESC, 1u);
                             }
                         }
-                        tc_commit(BAR(Cfg::A_EMPTY + s));
-                        if (s & 1u) tc_commit(BAR(Cfg::B_EMPTY + i));
+                        if (s % Cfg::ADEEP == Cfg::ADEEP - 1) tc_commit(BAR(Cfg::A_EMPTY + (Cfg::AEMPTIES > 4 ? 4 * (u ^ 1u) : 0) + a));       // to the set that writes there next
+                        if (s % Cfg::BDEEP == Cfg::BDEEP - 1) tc_commit(BAR(Cfg::B_EMPTY + i));
                     }
                     __syncwarp();
                 }
+                if (!go) break;
                 if constexpr (Q4) {
-                    if (!mbar_wait_spin(BAR(Cfg::T2_EMPTY), u ^ 1u) || !mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) return false;
+                    if ((!Cfg::T2_TWICE && !mbar_wait_spin(BAR(Cfg::T2_EMPTY), u ^ 1u)) || !mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
                     tc_fence_after();
                 }
                 if (leader) {
                     if constexpr (Q4) {
-                        tc_mma(tm + Cfg::TM_T2, dA2 + (uint64_t)(x * (TC_AUX >> 4)), dB2 + (uint64_t)(x * (Cfg::AUX >> 4)), Cfg::IDESC, 0u);
+                        tc_mma(tm + Cfg::TM_T2 + (Cfg::T2_TWICE ? NT * u : 0), dA2 + (uint64_t)(x * (TC_AUX >> 4)), dB2 + (uint64_t)(x * (Cfg::AUX >> 4)), Cfg::IDESC, 0u);
                         tc_commit(BAR(Cfg::X_EMPTY + x));
                     }
                     tc_commit(BAR(Cfg::T_FULL + u));
                 }
                 __syncwarp();
-                return true;
-            };
-            for (uint32_t b = 0; b < total; b += 2)
-                if (!superblock(TcConst<0>(), b) || (b + 1 < total && !superblock(TcConst<1>(), b + 1))) {
-                    atomicExch(dev_err, DEV_ERR_MMA_WAIT);
-                    break;
-                }
+            }
+            if (!go) atomicExch(dev_err, DEV_ERR_MMA_WAIT);
             if (leader) tc_commit(BAR(Cfg::DONE));          // MMAs in flight finish before the tensor memory is freed
             mbar_wait_spin(BAR(Cfg::DONE), 0);
         } else if (warp == 2) {
-            // ------------------------------------------------------------ Q4_K: mins (each doubled: bsums come per 16 elements) and block scales
-            if constexpr (Q4) {
-                for (uint32_t b = 0; b < total; ++b) {
-                    const uint32_t r = b % TC_RSLOTS, x = b % TC_XSLOTS;
-                    TC_WAIT(BAR(Cfg::X_EMPTY + x), ((b / TC_XSLOTS) & 1u) ^ 1u, DEV_ERR_EMPTY_WAIT);
-                    TC_WAIT(BAR(Cfg::R_FULL + r), (b / TC_RSLOTS) & 1u, DEV_ERR_FULL_WAIT);
-#pragma unroll 1
-                    for (int row = lane; row < TC_ROWS; row += 32) {
-                        const uint4 hdr = *reinterpret_cast<const uint4 *>(smem + Cfg::OFF_RAW + r * Cfg::RAW + row * Q4K_BYTES);
-                        const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f);
-                        uint32_t o[8];
-#pragma unroll
-                        for (int s = 0; s < 4; ++s) {
-                            uint32_t sc2, m2;
-                            q4k_scales(hdr.y, hdr.z, hdr.w, s, sc2, m2);
-                            o[2 * s] = h2_bits(__hsub2(bits_h2(__byte_perm(m2, 0x64646464u, 0x4040)), k1024));
-                            o[2 * s + 1] = h2_bits(__hsub2(bits_h2(__byte_perm(m2, 0x64646464u, 0x4141)), k1024));
-                        }
-                        uint8_t *a2 = smem + Cfg::OFF_A2 + x * TC_AUX + (row >> 3) * 128 + (row & 7) * 16;
-                        *reinterpret_cast<uint4 *>(a2) = make_uint4(o[0], o[1], o[2], o[3]);
-                        *reinterpret_cast<uint4 *>(a2 + TC_ROWS * 16) = make_uint4(o[4], o[5], o[6], o[7]);
-                        *reinterpret_cast<uint32_t *>(smem + Cfg::OFF_DD + (x * TC_ROWS + row) * 4) = hdr.x;
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
-                    __threadfence_block();
-                    __syncwarp();
-                    if (lane == 0) { mbar_arrive(BAR(Cfg::X_FULL + x)); mbar_arrive(BAR(Cfg::R_EMPTY + r)); }
-                }
-            }
-        } else {
             // ------------------------------------------------------------ raw weights
             uint32_t issued = 0, r = 0, ph = 1;
             bool go = true;
-            for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+            for (int u = work.begin + blockIdx.x; u < work.units && go; u += gridDim.x) {
                 const int n0 = work.nt(u) * TC_ROWS, kb0 = work.kb0(u), end = kb0 + work.nb(u);
                 for (int kb = kb0; kb < end; ++kb) {
                     if (!mbar_wait_spin(BAR(Cfg::R_EMPTY + r), ph)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
@@ -507,74 +502,132 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                         }
                     }
                     ++issued;
-                    if (++r == TC_RSLOTS) { r = 0; ph ^= 1u; }
+                    if (++r == Cfg::RSLOTS) { r = 0; ph ^= 1u; }
                 }
             }
-            for (uint32_t b = issued > TC_RSLOTS ? issued - TC_RSLOTS : 0; b < issued; ++b) mbar_wait_spin(BAR(Cfg::R_FULL + b % TC_RSLOTS), (b / TC_RSLOTS) & 1u);
+            for (uint32_t b = issued > Cfg::RSLOTS ? issued - Cfg::RSLOTS : 0; b < issued; ++b) mbar_wait_spin(BAR(Cfg::R_FULL + b % Cfg::RSLOTS), (b / Cfg::RSLOTS) & 1u);
         }
     } else if (warp < 12) {
-        // ------------------------------------------------------------ weight expanders: thread = row = TMEM lane; set e takes the k-stages e and e + 2
-        if constexpr (Cfg::REGS_EXP < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", Cfg::REGS_EXP);
-        else TC_SETMAXNREG("inc", Cfg::REGS_EXP);
-        const int set = (warp - 4) >> 2, row = tid & 127;
-        const uint32_t ta = tmem + Cfg::TM_A + ((uint32_t)(row & 96) << 16);
+        // ------------------------------------------------------------ weight expanders: thread = row = TMEM lane.  A stage is stored while the next one is expanded: what
+        // is stored is waited for, and its barrier arrived at, behind that.
+        TC_REGISTERS(Cfg::REGS_EXP);
+        const uint32_t set = (uint32_t)(warp - 4) >> 2;
+        const int row = tid & 127;
         bool go = true;
-        uint32_t rests [[maybe_unused]] = 3;       // Q6_K, bit per stage of the set: not known to be zeros in this warp's rows
-        for (uint32_t b = 0; b < total && go; ++b) {
-            const uint32_t r = b % TC_RSLOTS;
-            const uint8_t *raw = smem + Cfg::OFF_RAW + r * Cfg::RAW;
-            TC_WAIT(BAR(Cfg::R_FULL + r), (b / TC_RSLOTS) & 1u, DEV_ERR_FULL_WAIT);
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int s = 2 * h + set;
-                if constexpr (Q4) {
+        auto publish = [&](uint32_t slot) {
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(Cfg::A_FULL + slot));
+        };
+        if constexpr (Q4) {
+            // The two sets take superblocks in turn: what a superblock costs beside its weights (waits, header, addresses, mins) is paid by four warps only
+            // (sets that made half of every superblock each executed 1.4 times the instructions and took 1.15 times as long at 32 tokens).
+            const uint32_t ta = tmem + Cfg::TM_A + ((uint32_t)(row & 96) << 16) + (Cfg::ADEEP == 2 ? 128 * set : 0);
+            const uint32_t full = Cfg::ADEEP == 2 ? 2 * set : 0, empty = BAR(Cfg::A_EMPTY + (Cfg::ADEEP == 2 ? 2 : 4) * set);
+            uint32_t r = set, rp = 0, pa = Cfg::ADEEP == 2 ? 1u : set ^ 1u;
+            // slot for stage s: what was stored before has been published, the slot is empty
+            auto acquire = [&](int s) -> bool {
+                if (s % Cfg::ADEEP) return true;
+                if (s) publish(full + (uint32_t)(s / Cfg::ADEEP - 1));
+                if (!mbar_wait_spin(empty + 8u * (uint32_t)(s / Cfg::ADEEP), pa)) return false;
+                tc_fence_after();
+                return true;
+            };
+            for (uint32_t b = set; b < total; b += 2, pa ^= 1u) {
+                const uint8_t *raw = smem + Cfg::OFF_RAW + r * Cfg::RAW;
+                TC_WAIT(BAR(Cfg::R_FULL + r), rp, DEV_ERR_FULL_WAIT);
+                const uint4 *p = reinterpret_cast<const uint4 *>(raw + row * Q4K_BYTES);
+                const uint4 hdr = p[0];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
                     uint32_t o[32];
-                    const uint8_t *p = raw + row * Q4K_BYTES;
-                    q4k_expand(*reinterpret_cast<const uint4 *>(p), *reinterpret_cast<const uint4 *>(p + 16 + 32 * s), *reinterpret_cast<const uint4 *>(p + 32 + 32 * s), s, o);
-                    if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + s), (b & 1u) ^ 1u)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
-                    tc_fence_after();
+                    q4k_expand(q4k_scales4(hdr.y, hdr.w, s >> 1) >> (16 * (s & 1)), p[1 + 2 * s], p[2 + 2 * s], o);
+                    if (!acquire(s)) { go = false; break; }
                     tc_st32(ta + 32 * s, o);
-                } else {
-                    const uint2 sc8 = *reinterpret_cast<const uint2 *>(raw + Cfg::RAW_SC + row * 16 + 8 * h);
-                    const uint32_t scw = set ? sc8.y : sc8.x;
-                    const bool wide = __any_sync(0xffffffffu, q6k_wide(scw));
-                    if (!wide && !rests) {
-                        uint32_t o[32];
-                        q6k_expand(raw, raw + Cfg::RAW_QH, scw, row, h, set, o);
-                        if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + s), (b & 1u) ^ 1u)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
-                        tc_fence_after();
-                        tc_st32(ta + 32 * s, o);
-                    } else {
-                        // The issuer multiplies a slot of rests when any warp of the set has some, so a warp without leaves zeros in its rows, once.
-                        // A slot per stage is free when the stage is; a slot per set when the set's stage before this one has been multiplied.
-                        const uint32_t tr = ta + Cfg::TM_R - Cfg::TM_A + 32 * (s % Cfg::RESTS);
-                        uint32_t o[16], t[16];
-                        q6k_expand_rests<0>(raw, raw + Cfg::RAW_QH, scw, row, h, set, o, t);
-                        if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + s), (b & 1u) ^ 1u) ||
-                            (Cfg::RESTS < TC_ASLOTS && !mbar_wait_spin(BAR(Cfg::A_EMPTY + (s ^ 2)), (b & 1u) ^ (h ? 0u : 1u)))) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
-                        tc_fence_after();
-                        tc_st16(ta + 32 * s, o);
-                        tc_st16(tr, t);
-                        q6k_expand_rests<1>(raw, raw + Cfg::RAW_QH, scw, row, h, set, o, t);
-                        tc_st16(ta + 32 * s + 16, o);
-                        tc_st16(tr + 16, t);
-                        rests = wide ? rests | (1u << h) : rests & ~(1u << h);
-                        if (lane == 0) *(volatile uint8_t *)(smem + Cfg::OFF_WIDE + 4 * s + (warp & 3)) = wide;
+                    if (s == 0) {
+                        // The row's mins (each doubled: bsums come per 16 elements) and its block scales, for the MMA of T2 and the drain.  What lay there four superblocks
+                        // ago has been read: the MMAs that emptied this slot were issued after the drain had taken the sums of that superblock.
+                        const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f);
+                        const uint32_t x = b % TC_XSLOTS;
+                        uint4 *a2 = reinterpret_cast<uint4 *>(smem + Cfg::OFF_A2 + x * TC_AUX + row * 16);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint32_t mins = q4k_scales4(hdr.z, hdr.w >> 4, h);
+                            uint32_t m[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) m[j] = h2_bits(__hsub2(bits_h2(__byte_perm(mins, 0x64646464u, 0x4040 + 0x0101 * j)), k1024));
+                            a2[h * TC_ROWS] = make_uint4(m[0], m[1], m[2], m[3]);
+                        }
+                        *reinterpret_cast<uint32_t *>(smem + Cfg::OFF_DD + (x * TC_ROWS + row) * 4) = hdr.x;
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
                     }
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
+                if (!go) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); break; }
+                // every lane's reads of the superblock have gone into what it stored
+                publish(full + (uint32_t)(4 / Cfg::ADEEP - 1));
                 if (lane == 0) {
-                    mbar_arrive(BAR(Cfg::A_FULL + s));
-                    if (h) mbar_arrive(BAR(Cfg::R_EMPTY + r));       // every lane's reads of the superblock have gone into what it stored
+                    mbar_arrive(BAR(Cfg::R_EMPTY + r));
+                    mbar_arrive(BAR(Cfg::X_FULL + b % TC_XSLOTS));
                 }
+                r += 2;
+                if (r >= Cfg::RSLOTS) { r -= Cfg::RSLOTS; rp ^= 1u; }
             }
+        } else {
+            // Set n makes stages 2 n and 2 n + 1 of every superblock.  (In turn, as above: every stage's code once more and both sets behind one ring, 1.3 times slower.)
+            const uint32_t ta = tmem + Cfg::TM_A + ((uint32_t)(row & 96) << 16);
+            uint32_t rests = 3, r = 0, rp = 0;        // rests, a bit per stage of the set: not known to be zeros in this warp's rows
+            int stored = -1;                          // slot whose stores have not been published
+            for (uint32_t b = 0; b < total; ++b) {
+                const uint8_t *raw = smem + Cfg::OFF_RAW + r * Cfg::RAW;
+                const uint32_t first = (Cfg::ADEEP == 2 ? 4 * (b & 1u) : 0) + 2 * set, pa = ((Cfg::ADEEP == 2 ? b >> 1 : b) & 1u) ^ 1u;      // 64-deep stage of the ring
+                TC_WAIT(BAR(Cfg::R_FULL + r), rp, DEV_ERR_FULL_WAIT);
+                const uint2 sc8 = *reinterpret_cast<const uint2 *>(raw + Cfg::RAW_SC + row * 16 + 8 * set);
+                auto acquire = [&](int hi) -> bool {
+                    if (hi % Cfg::ADEEP) return true;
+                    if (stored >= 0) publish((uint32_t)stored);
+                    stored = -1;
+                    if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + (first + (uint32_t)hi) / Cfg::ADEEP), pa)) return false;
+                    tc_fence_after();
+                    return true;
+                };
+#pragma unroll
+                for (int hi = 0; hi < 2; ++hi) {
+                    const uint32_t k = first + hi;
+                    const Q6kStage st(raw, raw + Cfg::RAW_QH, hi ? sc8.y : sc8.x, row, set, hi);
+                    const bool wide = __any_sync(0xffffffffu, q6k_wide(st.scw));
+                    if (!wide && !(rests & (1u << hi))) {
+                        uint32_t o[32];
+                        st.expand(o);
+                        if (!acquire(hi)) { go = false; break; }
+                        tc_st32(ta + 32 * k, o);
+                    } else {
+                        // The issuer multiplies a slot of rests when any warp of the set has some, so a warp without leaves zeros in its rows, once.
+                        // A slot of rests is free when the same stage of the superblock before this one has been multiplied.
+                        if (!acquire(hi) || (Cfg::ADEEP == 2 && b > 0 && !mbar_wait_spin(BAR(Cfg::A_EMPTY + ((k / 2) ^ 2u)), ((b - 1) >> 1) & 1u))) { go = false; break; }
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t o[16], f[16];
+                            st.rests(h, o, f);
+                            tc_st16(ta + 32 * k + 16 * h, o);
+                            tc_st16(ta + Cfg::TM_R - Cfg::TM_A + 32 * (2 * set + hi) + 16 * h, f);
+                        }
+                        rests = wide ? rests | (1u << hi) : rests & ~(1u << hi);
+                    }
+                    if (lane == 0) *(volatile uint8_t *)(smem + Cfg::OFF_WIDE + 4 * k + (warp & 3)) = wide;
+                    stored = (int)(k / Cfg::ADEEP);
+                }
+                if (!go) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); break; }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(Cfg::R_EMPTY + r));
+                if (++r == Cfg::RSLOTS) { r = 0; rp ^= 1u; }
+            }
+            if (stored >= 0) publish((uint32_t)stored);
         }
     } else {
         // ------------------------------------------------------------ accumulator drain: thread = TMEM lane (weight row), DRAIN_COLS token columns
-        if constexpr (Cfg::REGS_DRAIN < Cfg::REGS_LAUNCH) TC_SETMAXNREG("dec", Cfg::REGS_DRAIN);
-        else TC_SETMAXNREG("inc", Cfg::REGS_DRAIN);
+        TC_REGISTERS(Cfg::REGS_DRAIN);
         constexpr int COLS = Cfg::DRAIN_COLS;
         const int dw = warp - 12;
         const int q = dw & 3, ch = dw >> 2;           // warp % 4 is the TMEM lane quarter this warp may read (12 % 4 == 0)
@@ -582,7 +635,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
         const size_t rb6 = ((size_t)work.nb_row * Q6K_BYTES + 15) & ~(size_t)15;
         uint32_t b = 0;
         bool go = true;
-        for (int u = blockIdx.x; u < work.units && go; u += gridDim.x) {
+        for (int u = work.begin + blockIdx.x; u < work.units && go; u += gridDim.x) {
             const int n = work.nt(u) * TC_ROWS + row, m0 = work.mt(u) * NT, nb = work.nb(u);
             const uint8_t *d_plane = Q4 ? nullptr : B + (size_t)min(n, N - 1) * rb6 + (size_t)work.nb_row * 208 + (size_t)work.kb0(u) * 2;
             uint64_t acc[COLS / 2];
@@ -606,14 +659,14 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                 for (int c = 0; c < COLS / 16; ++c) {
                     uint32_t t1[16], t2[16];
                     tc_ld16(taddr + NT * buf + 16 * c, t1);
-                    if constexpr (Q4) tc_ld16(taddr + Cfg::TM_T2 + 16 * c, t2);
+                    if constexpr (Q4) tc_ld16(taddr + Cfg::TM_T2 + (Cfg::T2_TWICE ? NT * buf : 0) + 16 * c, t2);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (c == COLS / 16 - 1) {             // the accumulators are in registers: the next superblocks may overwrite them
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) {
                             mbar_arrive(BAR(Cfg::T_EMPTY + buf));
-                            if (Q4) mbar_arrive(BAR(Cfg::T2_EMPTY));
+                            if (Q4 && !Cfg::T2_TWICE) mbar_arrive(BAR(Cfg::T2_EMPTY));
                         }
                     }
 #pragma unroll
@@ -638,21 +691,33 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                 if (lane == 0) mbar_arrive(BAR(Cfg::X_EMPTY + x));
             }
             if (go && n < N) {
-                const float bv = bias && work.nbz == work.nb_row ? bias[n] : 0.0f;
-                float *Cz = C + (size_t)work.z(u) * cz;
+                const bool whole = u < work.whole;
+                const int m = m0 + COLS * ch, first = work.whole / work.mtiles * TC_ROWS;         // first row (column of C) of the split tiles
+                const float bv = whole && bias ? bias[n] : 0.0f;
+                const size_t ld = (size_t)(whole ? ldc : N - first);
+                float *Cz = whole ? C + (size_t)m * ld + n : part + (size_t)work.z(u) * M * ld + (size_t)m * ld + (n - first);
+                // This runs once per unit and comes from memory each time, 128 bytes of code at an L2 round trip each (a store per column, unrolled, took 17500 cycles a unit
+                // of 32 tokens): so sixteen columns at a time, the others moved down.
+#pragma unroll 1
+                for (int left = M - m; left > 0 && left > M - m - COLS; left -= 16) {
 #pragma unroll
-                for (int i = 0; i < COLS / 2; ++i) {
-                    const int m = m0 + COLS * ch + 2 * i;
-                    float lo, hi;
-                    unpack2(acc[i], lo, hi);
-                    if (m < M) Cz[(size_t)m * ldc + n] = lo + bv;
-                    if (m + 1 < M) Cz[(size_t)(m + 1) * ldc + n] = hi + bv;
+                    for (int i = 0; i < 8; ++i) {
+                        float lo, hi;
+                        unpack2(acc[i], lo, hi);
+                        if (2 * i < left) *Cz = lo + bv;
+                        Cz += ld;
+                        if (2 * i + 1 < left) *Cz = hi + bv;
+                        Cz += ld;
+                    }
+#pragma unroll
+                    for (int i = 0; i + 8 < COLS / 2; ++i) acc[i] = acc[i + 8];
                 }
             }
         }
         if (!go) atomicExch(dev_err, DEV_ERR_MMA_WAIT);
     }
 #undef TC_WAIT
+#undef TC_REGISTERS
 #undef TC_SETMAXNREG
     __syncwarp();
     tc_fence_before();
@@ -668,6 +733,8 @@ __global__ void __launch_bounds__(256) gemm_splitk_sum_kernel(const float *__res
                                                               int M, int N)
 {
     const size_t mn = (size_t)M * N;
+    pdl_wait();
+    pdl_trigger();
     if (VEC) {                                                 // N and ldc multiples of 4, C and bias 16-byte aligned: four outputs per thread
         for (size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4; i < mn; i += (size_t)gridDim.x * 1024) {
             const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
@@ -698,57 +765,67 @@ __global__ void __launch_bounds__(256) gemm_splitk_sum_kernel(const float *__res
 
 using namespace ckb;
 
-// How many K slices: enough CTAs to fill the resident slots (SMs x CTAs per SM) in whole waves.  Few tokens only (the
-// partial sums cost Z * M * N * 4 bytes of traffic), slices of at least 4 superblocks, at most 16.
-static int tc_pick_slices(int tiles, int nb, int slots)
+// How a product is cut: the first row tiles whole, the last split_nt of them in Z slices of nbz superblocks.
+struct TcPlan { int mtiles, ntiles, split_nt, Z, nbz; double us; };
+// us a superblock of a unit takes: units of 16 and 32 superblocks of one to five rounds, at 32, 64, 96 and 128 tokens
+static double tc_superblock_us(int wf, int width)
 {
-    int best = 1;
-    double best_eff = 0.0;
-    for (int z = 1; z <= 16 && nb / z >= 4; ++z) {
-        const long ctas = (long)tiles * z, waves = (ctas + slots - 1) / slots;
-        const double eff = (double)ctas / (double)(waves * slots);
-        if (eff > best_eff * 1.08) { best_eff = eff; best = z; }      // a larger Z must pay for its partial sums
-    }
-    return best;
+    static const double q4[4] = {0.74, 0.90, 1.07, 1.30}, q6[4] = {1.14, 1.49, 1.80, 1.85};
+    return (wf == TC_W_Q4K ? q4 : q6)[width / 32 - 1];
 }
-
-// How a product is cut: K slices of nbz superblocks, and row tiles that go to a second launch with K split.
-struct TcPlan { int mtiles, ntiles, Z, nbz, tail_nt, Zt, nbzt; double us; };
-static TcPlan tc_plan(int wf, int width, int M, int N, int nb, int ctas_per_sm, bool may_tail)
+static void tc_slice(TcPlan *p, int nb, int z)
 {
-    TcPlan p = {(M + width - 1) / width, (N + TC_ROWS - 1) / TC_ROWS, 1, nb, 0, 1, nb, 0.0};
-    const int slots = ckb_sm_count() * ctas_per_sm, tiles = p.ntiles * p.mtiles;
-    // K is split for a handful of tokens, and for any product whose tiles leave more than half of the SMs without a CTA (the k and
-    // v projections of a prompt: 8 x 4 tiles)
-    const int splitk = ckb_tune_get("gemm_tc_splitk", 1);
-    if (splitk && (M <= 128 || (splitk != 2 && 2 * tiles <= slots))) p.Z = tc_pick_slices(tiles, nb, slots);
-    const int forced = ckb_tune_get("gemm_tc_slices", 0);
-    if (forced > 0 && forced <= nb) p.Z = forced;
-    p.nbz = (nb + p.Z - 1) / p.Z;
-    p.Z = (nb + p.nbz - 1) / p.nbz;                    // no empty slice
+    p->nbz = (nb + z - 1) / z;
+    p->Z = (nb + p->nbz - 1) / p->nbz;                 // no empty slice
+}
+static TcPlan tc_plan(int wf, int width, int M, int N, int nb)
+{
+    TcPlan p = {(M + width - 1) / width, (N + TC_ROWS - 1) / TC_ROWS, 0, 1, nb, 0.0};
+    const int slots = ckb_sm_count(), tiles = p.ntiles * p.mtiles;
+    const double per_sb = tc_superblock_us(wf, width), store = 1.5 * width / 128;
+    p.us = (tiles + slots - 1) / slots * (nb * per_sb + store);
+    const int forced = ckb_tune_get("gemm_tc_slices", 0), splitk = ckb_tune_get("gemm_tc_splitk", 1);
+    if (forced > 0 && forced <= nb) {
+        p.split_nt = p.ntiles;
+        tc_slice(&p, nb, forced);
+        return p;
+    }
+    // K is split where that takes less time, with what the partial sums cost: a launch that adds them, 3 us behind the product, and their way to L2 and
+    // back at 3 TB/s.  Considered for up to 128 tokens and for any product whose tiles leave more than half of the SMs without a CTA (the k and
+    // v projections of a prompt: 8 x 4 tiles); slices of at least 4 superblocks, at most 16.
+    if (splitk && (M <= 128 || (splitk != 2 && 2 * tiles <= slots)))
+        for (int z = 2; z <= 16 && nb / z >= 4; ++z) {
+            TcPlan q = p;
+            q.split_nt = p.ntiles;
+            tc_slice(&q, nb, z);
+            q.us = (tiles * q.Z + slots - 1) / slots * (q.nbz * per_sb + store) + 3.0 + (double)q.Z * M * N * 8e-6 / 3.0;
+            if (q.us < p.us) p = q;
+        }
     // A grid of whole waves plus a few units pays a full wave for those few (28672 x 4096 at 512 tokens: 896 tiles = 6 waves of 148
-    // and 8 tiles).  The row tiles behind that remainder then go to a second launch with K split, which fills the SMs for a
-    // fraction of a wave; its partial sums are added as for any split.  The two extra launches cost about 10 us, so not where a unit takes
-    // less (9728 x 1024 at 129 tokens: 25.7 us with the second launch, 19 without).  Library workspace only (a caller's workspace is sized for one launch).
-    if (p.Z == 1 && may_tail && nb >= 8 && ckb_tune_get("gemm_tc_tail", 1)) {
-        const int rem = tiles % slots;
-        if (tiles > slots && rem > 0 && 4 * rem <= slots && rem % p.mtiles == 0 && rem / p.mtiles < p.ntiles && N % TC_ROWS == 0) {
-            p.Zt = tc_pick_slices(rem, nb, slots);
-            if (p.Zt > 1) p.tail_nt = rem / p.mtiles;
+    // and 8 tiles; 57344 rows at 32 tokens: 3 waves and 4).  The row tiles behind that remainder then go to a second launch with K split, which fills the SMs for a
+    // fraction of a wave; its partial sums are added as for any split.  The two extra launches cost about 8 us, so not where a unit takes
+    // less (9728 x 1024 at 129 tokens: 25.7 us with the second launch, 19 without).
+    const int rem = tiles % slots;
+    if (!p.split_nt && nb >= 8 && tiles > slots && rem > 0 && 4 * rem <= slots && rem % p.mtiles == 0 && rem / p.mtiles < p.ntiles && N % TC_ROWS == 0 && ckb_tune_get("gemm_tc_tail", 1)) {
+        int z = 1;
+        double best = 0.0;
+        for (int i = 1; i <= 16 && nb / i >= 4; ++i) {
+            const double us = (rem * i + slots - 1) / slots * ((nb + i - 1) / i * per_sb + store);
+            if (best == 0.0 || us < 0.93 * best) { best = us; z = i; }
+        }
+        if (z > 1) {
+            p.split_nt = rem / p.mtiles;
+            tc_slice(&p, nb, z);
+            p.us = tiles / slots * (nb * per_sb + store) + best + 8.0;
         }
     }
-    p.nbzt = (nb + p.Zt - 1) / p.Zt;
-    if (p.tail_nt) p.Zt = (nb + p.nbzt - 1) / p.nbzt;
-    // time: rounds of units, a superblock of a unit at the measured rate (us, by width and format), its stores, and the launches of a split
-    const double per_sb = wf == TC_W_Q4K ? (width == 128 ? 1.06 : (width == 96 ? 0.98 : 0.78)) : (width == 128 ? 1.32 : (width == 96 ? 1.26 : 1.13));
-    const int units = (p.ntiles - p.tail_nt) * p.mtiles * p.Z, rounds = (units + slots - 1) / slots;
-    p.us = rounds * (p.nbz * per_sb + 1.5 * width / 128) + (p.Z > 1 ? 4.0 : 0.0) + (p.tail_nt ? 10.0 + p.nbzt * per_sb : 0.0);
     return p;
 }
 
 static size_t tc_part_bytes(const TcPlan &p, int M, int N)
 {
-    return p.Z > 1 ? (size_t)p.Z * M * N * sizeof(float) : (p.tail_nt ? (size_t)p.Zt * M * p.tail_nt * TC_ROWS * sizeof(float) : 0);
+    const int rest = N - (p.ntiles - p.split_nt) * TC_ROWS;
+    return p.split_nt ? (size_t)p.Z * M * rest * sizeof(float) : 0;
 }
 
 typedef CUresult (*tc_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
@@ -796,7 +873,7 @@ static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float 
     if (!attr_set) {
         cudaFuncAttributes fa;
         if (ckb_check_cuda((int)cudaFuncGetAttributes(&fa, kernel), "func attributes")) return CKB_ERR_CUDA;
-        if (fa.numRegs != Cfg::REGS_LAUNCH)     // a different allocation at launch would make setmaxnreg.inc wait for registers that never come
+        if (Cfg::REGS_DRAIN != Cfg::REGS_LAUNCH && fa.numRegs != Cfg::REGS_LAUNCH)     // a different allocation at launch would make setmaxnreg.inc wait for registers that never come
             return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: kernel compiled with an unexpected register count");
         if (ckb_check_cuda((int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM), "smem attr")) return CKB_ERR_CUDA;
         attr_set = 1;
@@ -805,40 +882,23 @@ static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float 
     if (!tc_maps<WF>(&maps, (const uint8_t *)B, N, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", N, nb);
     if (tc_part_bytes(plan, M, N) > part_bytes)
         return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the workspace holds %zu bytes of partial sums, this call needs %zu", part_bytes, tc_part_bytes(plan, M, N));
-    const int slots = ckb_sm_count() * Cfg::CTAS_PER_SM;
-    const int mtiles = plan.mtiles, ntiles = plan.ntiles, Z = plan.Z, nbz = plan.nbz, tail_nt = plan.tail_nt, Zt = plan.Zt, nbzt = plan.nbzt;
-    const int Nt = tail_nt * TC_ROWS;                  // rows (output columns) of the tail launch
-    TcWork work = {(ntiles - tail_nt) * mtiles * Z, mtiles, ntiles - tail_nt, nb, nbz};
-    dim3 grid((unsigned)(work.units < slots ? work.units : slots));
-    if (Z == 1) {
-        if (int rc = launch_pdl("gemm_kq_tc", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, (const uint8_t *)B, bias, C, ldc, (size_t)0, M, N - Nt,
-                                ckb_device_error_word()))
+    const int slots = ckb_sm_count(), first = (plan.ntiles - plan.split_nt) * TC_ROWS, rest = N - first;
+    const int whole = (plan.ntiles - plan.split_nt) * plan.mtiles;
+    TcWork work = {0, whole, whole, plan.mtiles, plan.split_nt ? plan.split_nt : 1, nb, plan.nbz};
+    for (int i = 0; i < 2; ++i) {                      // whole tiles; slices
+        if (i) { work.begin = whole; work.units = whole + plan.split_nt * plan.mtiles * plan.Z; }
+        const int units = work.units - work.begin;
+        if (units == 0) continue;
+        if (int rc = launch_pdl(i ? "gemm_kq_tc slices" : "gemm_kq_tc", kernel, dim3((unsigned)(units < slots ? units : slots)), dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt,
+                                (const uint8_t *)B, bias, C, ldc, part, M, N, ckb_device_error_word()))
             return rc;
-        if (!tail_nt) return 0;
-        const int n0 = N - Nt;
-        const size_t rb = WF == TC_W_Q4K ? (size_t)nb * Q4K_BYTES : (((size_t)nb * Q6K_BYTES + 15) & ~(size_t)15);
-        const uint8_t *Bt = (const uint8_t *)B + (size_t)n0 * rb;
-        if (!tc_maps<WF>(&maps, Bt, Nt, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", Nt, nb);
-        work = {tail_nt * mtiles * Zt, mtiles, tail_nt, nb, nbzt};
-        grid = dim3((unsigned)(work.units < slots ? work.units : slots));
-        if (int rc = launch_pdl("gemm_kq_tc tail", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, Bt, nullptr, part, Nt, (size_t)M * Nt, M, Nt,
-                                ckb_device_error_word()))
-            return rc;
-        const size_t mnt = (size_t)M * Nt;
-        const unsigned tb = (unsigned)((mnt + 1023) / 1024 < 1184 ? (mnt + 1023) / 1024 : 1184);
-        const float *bt = bias ? bias + n0 : nullptr;
-        if (ldc % 4 == 0 && (((uintptr_t)(C + n0) | (uintptr_t)bt) & 15) == 0) gemm_splitk_sum_kernel<true><<<tb, 256, 0, st>>>(part, Zt, bt, C + n0, ldc, M, Nt);
-        else gemm_splitk_sum_kernel<false><<<tb, 256, 0, st>>>(part, Zt, bt, C + n0, ldc, M, Nt);
-        return ckb_check_launch("gemm_splitk_sum");
     }
-    if (int rc = launch_pdl("gemm_kq_tc", kernel, grid, dim3(Cfg::THREADS), (size_t)Cfg::SMEM, st, maps, work, xt, (const uint8_t *)B, nullptr, part, N, (size_t)M * N, M, N,
-                            ckb_device_error_word()))
-        return rc;
-    const size_t mn = (size_t)M * N;
+    if (!plan.split_nt) return 0;
+    const size_t mn = (size_t)M * rest;
     const unsigned blocks = (unsigned)((mn + 1023) / 1024 < 1184 ? (mn + 1023) / 1024 : 1184);
-    if (N % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)C | (uintptr_t)bias) & 15) == 0) gemm_splitk_sum_kernel<true><<<blocks, 256, 0, st>>>(part, Z, bias, C, ldc, M, N);
-    else gemm_splitk_sum_kernel<false><<<blocks, 256, 0, st>>>(part, Z, bias, C, ldc, M, N);
-    return ckb_check_launch("gemm_splitk_sum");
+    const float *b2 = bias ? bias + first : nullptr;
+    auto sum = rest % 4 == 0 && ldc % 4 == 0 && (((uintptr_t)(C + first) | (uintptr_t)b2 | (uintptr_t)part) & 15) == 0 ? gemm_splitk_sum_kernel<true> : gemm_splitk_sum_kernel<false>;
+    return launch_pdl("gemm_splitk_sum", sum, dim3(blocks), dim3(256), (size_t)0, st, (const float *)part, plan.Z, b2, C + first, ldc, M, rest);
 }
 
 static int tc_launch(int wf, int nt, const uint8_t *xt, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part,
@@ -856,31 +916,39 @@ static int tc_make_tiles(const void *A_q8, uint8_t *xt, int nt, int M, int nb, c
     return launch_pdl("gemm_x_tiles", kernel, dim3(nb, mtiles, xz), dim3(256), (size_t)0, st, (const uint8_t *)A_q8, xt, M, nb);
 }
 
-// Token tile: 32 for batched decode (up to 64 tokens: two CTAs per SM), else the width whose plan takes least.
-static int tc_width(int wf, int M, int N, int nb, bool may_tail)
+// Token tile: the width whose plan takes least, a wider one where two are alike.  Up to 32 tokens there is no choice.
+static int tc_width(int wf, int M, int N, int nb)
 {
-    if (M <= ckb_tune_get("gemm_tc_small_max", 64)) return 32;
     const int forced = ckb_tune_get("gemm_tc_nt", 0);
-    if (forced == 64 || forced == 96 || forced == 128) return forced;
-    const TcPlan wide = tc_plan(wf, 128, M, N, nb, 1, may_tail);
+    if (M > 32 && (forced == 64 || forced == 96 || forced == 128)) return forced;
+    if (M <= ckb_tune_get("gemm_tc_small_max", 32)) return 32;
+    const TcPlan wide = tc_plan(wf, 128, M, N, nb);
     double best = wide.us;
     int width = 128;
-    for (int w = 96; w >= 64 && !wide.tail_nt; w -= 32) {
-        const double us = tc_plan(wf, w, M, N, nb, 1, may_tail).us;
+    // one wave of the widest tiles and a few behind it: as it was, narrower ones not tried
+    const bool one_wave = wide.split_nt && wide.split_nt < wide.ntiles && (wide.ntiles - wide.split_nt) * wide.mtiles <= ckb_sm_count();
+    for (int w = 96; w >= 32 && !one_wave; w -= 32) {
+        const double us = tc_plan(wf, w, M, N, nb).us;
         if (us < 0.97 * best) { best = us; width = w; }
     }
     return width;
 }
+// Whether this kernel takes a product from Q8_K rows in less time than an integer-MMA kernel that needs other_us; 3 us for the launch that makes operand tiles.
+extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us)
+{
+    if (ckb_tune_get("gemm_tc", 1) == 0) return 0;
+    return tc_plan(wf, tc_width(wf, M, N, K / QK_K), M, N, K / QK_K).us + 3.0 < other_us;
+}
 
 // A caller that quantises rows straight into operand tiles (quantize_block_q8k_tile: one blob per tile of nt tokens and superblock) asks for the width
 // and the sizes first.  Products over the same rows share one width: the one that suits the largest of them.
-extern "C" int ckb_gemm_tc_width(int wf, int M, int N, int K) { return tc_width(wf, M, N, K / QK_K, true); }
+extern "C" int ckb_gemm_tc_width(int wf, int M, int N, int K) { return tc_width(wf, M, N, K / QK_K); }
 extern "C" size_t ckb_gemm_tc_tile_bytes(int nt, int M, int K) { return (size_t)((M + nt - 1) / nt) * (K / QK_K) * q8k_tile_bytes(nt); }
-extern "C" size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K) { return tc_part_bytes(tc_plan(wf, nt, M, N, K / QK_K, nt == 32 ? 2 : 1, true), M, N); }
+extern "C" size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K) { return tc_part_bytes(tc_plan(wf, nt, M, N, K / QK_K), M, N); }
 extern "C" int ckb_launch_gemm_tc_tiles(int wf, const void *tiles, int nt, const void *B, float *C, int ldc, int M, int N, int K, void *part, size_t part_bytes, void *stream)
 {
     if (K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)tiles & 15)) return -1;
-    return tc_launch(wf, nt, (const uint8_t *)tiles, B, nullptr, C, ldc, M, N, K / QK_K, tc_plan(wf, nt, M, N, K / QK_K, nt == 32 ? 2 : 1, true), (float *)part, part_bytes,
+    return tc_launch(wf, nt, (const uint8_t *)tiles, B, nullptr, C, ldc, M, N, K / QK_K, tc_plan(wf, nt, M, N, K / QK_K), (float *)part, part_bytes,
                      ckb_stream(stream));
 }
 
@@ -891,8 +959,8 @@ extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, co
                                      void *ws, size_t ws_bytes, void *stream)
 {
     if (M < min_tokens || K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3) || ((uintptr_t)ws & 255) || ckb_tune_get("gemm_tc", 1) == 0) return -1;
-    const int nb = K / QK_K, nt = tc_width(wf, M, N, nb, ws == nullptr);
-    const TcPlan plan = tc_plan(wf, nt, M, N, nb, nt == 32 ? 2 : 1, ws == nullptr);
+    const int nb = K / QK_K, nt = tc_width(wf, M, N, nb);
+    const TcPlan plan = tc_plan(wf, nt, M, N, nb);
     const size_t xt_bytes = (ckb_gemm_tc_tile_bytes(nt, M, K) + 255) & ~(size_t)255, part_bytes = tc_part_bytes(plan, M, N);
     // A caller that records the launch in a CUDA graph brings its own workspace: the library's pool may be freed and
     // regrown by any later call that needs more, which would leave a captured pointer dangling.

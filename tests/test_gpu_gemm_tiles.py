@@ -155,3 +155,55 @@ def test_producers_write_the_tiles_of_their_rows(ck, producer, nt, T):
     got, got_scales = split_tiles(tiles.cpu().numpy(), nt, T, nb)
     assert np.array_equal(got, want)
     assert np.array_equal(got_scales, scales)
+
+
+@pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
+@pytest.mark.parametrize("width,m,n,superblocks,launches", [
+    # every remainder of the expanders' turns, of the rings and of two accumulators, in whole units and in slices of four
+    (32, 20, 40, 1, 1), (32, 32, 129, 2, 1), (32, 17, 128, 3, 1), (32, 31, 200, 7, 1), (32, 32, 300, 9, 2), (64, 33, 129, 5, 1), (64, 64, 40, 10, 2), (96, 65, 130, 6, 1), (128, 97, 129, 11, 2),
+    # a wave and a few tiles: the whole ones and the slices of the last rows are launches of their own, with the sum of the slices three
+    (32, 19, 151 * 128, 8, 3), (64, 50, 150 * 128, 9, 3),
+    # several units a CTA, the last of them of fewer superblocks
+    (32, 25, 300 * 128 + 40, 2, 1), (64, 60, 299 * 128, 3, 1)])
+def test_gemm_tiles_at_the_edges_of_their_deal(ck, orc, fmt, width, m, n, superblocks, launches):
+    """The tcgen05 product over numbers of superblocks, tokens and row tiles at which its rings, its expander sets and its units have remainders.  Integer sums are the same on both
+    sides; per superblock three fp32 roundings on either, as above."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    k = 256 * superblocks
+    w = synth.make_weights(fmt, n, k, seed=superblocks)
+    aq = cases.quantize_act(orc, "oracle_", fmt, synth.make_x(k, seed=m, rows=m), rows=m)
+    rows = np.r_[0:min(n, 256), max(n - 300, 0):n] if n > 600 else np.arange(n)          # the oracle's share of tall matrices: first and last tiles
+    rows = np.unique(rows)
+    want = cases.gemm_nt(orc, "oracle_", fmt, aq, np.ascontiguousarray(w.reshape(n, -1)[rows]).reshape(-1), None, m, len(rows), k)
+    raw, taq = torch.from_numpy(w).to(dev), torch.from_numpy(aq).to(dev)
+    if fmt == "q6_k":
+        ck.ckb200_q6_k_planar_bytes.restype = C.c_size_t
+        wdev = torch.empty(ck.ckb200_q6_k_planar_bytes(n, k), dtype=torch.uint8, device=dev)
+        torch.cuda.synchronize()
+        assert ck.ckb200_dev_q6_k_to_planar(C.c_void_p(wdev.data_ptr()), C.c_void_p(raw.data_ptr()), n, k, None) == 0
+        fn = ck.ckb200_dev_gemm_nt_q6_k_planar_q8_k
+    else:
+        wdev, fn = raw, ck.ckb200_dev_gemm_nt_q4_k_q8_k
+    ck.ckb200_launch_count.restype = C.c_longlong
+    outs = []
+    try:
+        for key, value in ((b"gemm_tc_nt", width), (b"gemm_tc_slices", (superblocks + 3) // 4 if launches == 2 else 0), (b"gemm_q4k_mma", 0), (b"gemm_q6k_mma", 0)):
+            ck.ckb200_tune_set(key, value)
+        for _ in range(2):
+            c = torch.full((m, n), float("nan"), device=dev)
+            torch.cuda.synchronize()
+            n0 = ck.ckb200_launch_count()
+            assert fn(C.c_void_p(taq.data_ptr()), C.c_void_p(wdev.data_ptr()), None, C.c_void_p(c.data_ptr()), m, n, k, None) == 0
+            count = ck.ckb200_launch_count() - n0
+            assert ck.ckb200_synchronize() == 0
+            outs.append(c.cpu().numpy())
+    finally:
+        for key, value in ((b"gemm_tc_nt", 0), (b"gemm_tc_slices", 0), (b"gemm_q4k_mma", 1), (b"gemm_q6k_mma", 1)):
+            ck.ckb200_tune_set(key, value)
+    bound = 2 * (superblocks + 3) * 2.0 ** -24 * 8 * float(np.max(np.abs(want)))
+    assert float(np.max(np.abs(outs[0][:, rows].astype(np.float64) - want))) <= bound
+    assert np.array_equal(outs[0], outs[1]) and np.isfinite(outs[0]).all()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert count == 1 + launches, count          # and the launch that makes operand tiles
