@@ -16,7 +16,7 @@
 // scales, gemv_q50_planar.cu): word t of a block's 16 nibble bytes holds elements 4t .. 4t+3 and 16+4t .., exactly the two registers of lane t's fragment;
 // five instructions a register make them signed bytes.  The sums are the same int32 and the fp32 steps the same, so these are bit-identical too.
 //
-// Tiles: 128 tokens x 128 rows, or 64 x 64 where the wide ones leave half of the SMs without a CTA (the projections of a 896-wide model: 7 row tiles).
+// Tiles: 128 tokens x 128 rows, or 64 x 64 where the wide ones leave SMs idle, in their only round (the projections of a 896-wide model: 7 row tiles) or in their last.
 #include "device_common.cuh"
 #include "launch.h"
 #include "pdl.cuh"
@@ -198,9 +198,11 @@ template <bool Q5>
 static int qm_pick(const void *A, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int weights_ready, void *stream)
 {
     if (K % (32 * QM_KB) || M <= 0 || N <= 0 || (((uintptr_t)A | (uintptr_t)B) & 15)) return -1;
-    const long wide = (long)((N + 127) / 128) * ((M + 127) / 128);
+    // Rounds of wide tiles, one on an SM, against rounds of narrow ones, two on an SM, each of which takes 0.6 of a wide one's time (K of 4096: 61 against 103 us; of 896:
+    // 15 against 21).  9728 x 896 at 256 tokens is 152 wide tiles: two rounds, 43 us, narrow 33; at 130 tokens 38 and 26; 4096 x 4096 at 512 tokens 104 and 119.
+    const long sms = ckb_sm_count(), wide = (long)((N + 127) / 128) * ((M + 127) / 128), narrow = (long)((N + 63) / 64) * ((M + 63) / 64);
     int tile = ckb_tune_get("gemm_q80_tile", 0);
-    if (tile != 64 && tile != 128) tile = 2 * wide > ckb_sm_count() ? 128 : 64;
+    if (tile != 64 && tile != 128) tile = 10 * ((wide + sms - 1) / sms) < 6 * ((narrow + 2 * sms - 1) / (2 * sms)) ? 128 : 64;
     cudaStream_t st = ckb_stream(stream);
     return tile == 128 ? qm_launch<Q5, 128>(A, B, bias, C, ldc, M, N, K / 32, weights_ready, st) : qm_launch<Q5, 64>(A, B, bias, C, ldc, M, N, K / 32, weights_ready, st);
 }

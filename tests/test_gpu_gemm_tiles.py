@@ -207,3 +207,33 @@ def test_gemm_tiles_at_the_edges_of_their_deal(ck, orc, fmt, width, m, n, superb
     assert np.array_equal(outs[0], outs[1]) and np.isfinite(outs[0]).all()
     if torch.cuda.get_device_properties(0).multi_processor_count == 148:
         assert count == 1 + launches, count          # and the launch that makes operand tiles
+
+
+@pytest.mark.parametrize("m,n", [(130, 9600), (130, 9472), (129, 18944 + 40), (300, 4736)])
+def test_q8_0_product_is_the_same_in_either_tile(ck, orc, m, n):
+    """Wide tiles in whole rounds or a few behind them, narrow ones instead: the tile changes the deal, not a bit of the result."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    k = 256
+    g = torch.Generator(device=dev).manual_seed(n)
+    x, w = torch.randn(m, k, device=dev, generator=g), torch.randn(n, k, device=dev, generator=g)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    xq, wq = (torch.zeros(r * k // 32 * 34 + 64, dtype=torch.uint8, device=dev) for r in (m, n))
+    torch.cuda.synchronize()
+    assert ck.ckb200_dev_quantize_q8_0(p(x), p(xq), m, k, None) == 0 and ck.ckb200_dev_quantize_q8_0(p(w), p(wq), n, k, None) == 0
+    outs = []
+    try:
+        for tile in (0, 64, 128):
+            ck.ckb200_tune_set(b"gemm_q80_tile", tile)
+            y = torch.full((m, n), float("nan"), device=dev)
+            torch.cuda.synchronize()
+            assert ck.ckb200_dev_gemm_nt_q8_0_q8_0(p(xq), p(wq), None, p(y), m, n, k, None) == 0
+            assert ck.ckb200_synchronize() == 0
+            outs.append(y.cpu().numpy())
+    finally:
+        ck.ckb200_tune_set(b"gemm_q80_tile", 0)
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+    first = min(n, 200)
+    want = cases.gemm_nt(orc, "oracle_", "q8_0", xq.cpu().numpy()[:m * k // 32 * 34], np.ascontiguousarray(wq.cpu().numpy()[:first * k // 32 * 34]), None, m, first, k)
+    assert np.array_equal(outs[0][:, :first], want)
