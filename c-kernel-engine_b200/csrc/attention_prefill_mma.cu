@@ -14,6 +14,7 @@
 #include <cuda_fp16.h>
 
 #include "device_common.cuh"
+#include "fp16_pieces.cuh"
 #include "launch.h"
 #include "pdl.cuh"
 #include "runtime.h"
@@ -36,15 +37,6 @@ __device__ __forceinline__ void pm_mma(float (&c)[4], const uint32_t (&a)[4], ui
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void pm_split2(float a, float b, uint32_t &hi, uint32_t &lo)
-{
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 hf = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - hf.x, b - hf.y);
-    hi = *reinterpret_cast<const uint32_t *>(&h);
-    lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-
 // Keys and values as the four fp16 tiles want them, once per call: kv16 = K hi | K lo | V hi | V lo, each [Hkv][T][AD] (columns
 // past the head are zeros).  Every query block of a kv head reads the same keys, so the split is done here and not per block.
 template <int AD>
@@ -66,16 +58,9 @@ __global__ void __launch_bounds__(256) pm_split_kv_kernel(const float *__restric
             if (d + 2 >= hd) { kx.z = 0.f; vx.z = 0.f; }
             kx.w = 0.f; vx.w = 0.f;
         }
-        uint2 hi, lo;
         __half *dst = kv16 + row * AD + d;
-        pm_split2(kx.x, kx.y, hi.x, lo.x);
-        pm_split2(kx.z, kx.w, hi.y, lo.y);
-        *reinterpret_cast<uint2 *>(dst) = hi;
-        *reinterpret_cast<uint2 *>(dst + arr) = lo;
-        pm_split2(vx.x, vx.y, hi.x, lo.x);
-        pm_split2(vx.z, vx.w, hi.y, lo.y);
-        *reinterpret_cast<uint2 *>(dst + 2 * arr) = hi;
-        *reinterpret_cast<uint2 *>(dst + 3 * arr) = lo;
+        store_pieces4(dst, arr, kx);
+        store_pieces4(dst + 2 * arr, arr, vx);
     }
 }
 
@@ -294,8 +279,11 @@ __global__ void __launch_bounds__(256) attn_prefill_mma_kernel(const float *__re
     }
 }
 
+static __half *pm_pieces(int Hkv, int T, int ad) { return (__half *)ckb_scratch(CKB_SLOT_S, 4 * (size_t)Hkv * T * ad * sizeof(__half)); }
+
+// kv16: the pieces
 template <int AD, int KH>
-static int pm_launch(const float *q, const float *k, const float *v, float *out, int H, int Hkv, int T, int hd, int kv_stride, int causal, float scale, cudaStream_t st)
+static int pm_launch(const float *q, const __half *kv16, float *out, int H, int Hkv, int T, int hd, int causal, cudaStream_t st)
 {
     constexpr int smem = 2 * 4 * PM_BK * (AD + 8) * 2;
     static_assert(8 * (AD / 8 * 4 + 4) * 32 * 4 <= smem, "the merge buffer of up to 8 heads fits into the stages");
@@ -304,15 +292,26 @@ static int pm_launch(const float *q, const float *k, const float *v, float *out,
         if (ckb_check_cuda((int)cudaFuncSetAttribute(attn_prefill_mma_kernel<AD, KH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "attn_prefill_mma smem")) return CKB_ERR_CUDA;
         attr_set = true;
     }
-    const size_t arr = (size_t)Hkv * T * AD;
-    __half *kv16 = (__half *)ckb_scratch(CKB_SLOT_S, 4 * arr * sizeof(__half));
+    return launch_pdl("attn_prefill_mma", attn_prefill_mma_kernel<AD, KH>, dim3(Hkv, (T + PM_BQ - 1) / PM_BQ), dim3(32 * KH * (H / Hkv)), (size_t)smem, st, q, kv16, out, H, Hkv, T, hd,
+                      causal, 1.0f / sqrtf((float)hd));
+}
+template <int AD>
+static int pm_go(const float *q, const __half *kv16, float *out, int H, int Hkv, int T, int hd, int causal, cudaStream_t st)
+{
+    // two warps per query head, 32 keys of a tile each, while a kv head has at most four
+    return H / Hkv <= 4 ? pm_launch<AD, 2>(q, kv16, out, H, Hkv, T, hd, causal, st) : pm_launch<AD, 1>(q, kv16, out, H, Hkv, T, hd, causal, st);
+}
+template <int AD>
+static int pm_split_and_go(const float *q, const float *k, const float *v, float *out, int H, int Hkv, int T, int hd, int kv_stride, int causal, cudaStream_t st)
+{
+    __half *kv16 = pm_pieces(Hkv, T, AD);
     if (!kv16) return CKB_ERR_CUDA;
-    const size_t n4 = arr / 4;
+    const size_t n4 = (size_t)Hkv * T * AD / 4;
     const unsigned blocks = (unsigned)((n4 + 255) / 256 < 8 * 148 ? (n4 + 255) / 256 : 8 * 148);
     if (int rc = launch_pdl("attn_prefill_split_kv", pm_split_kv_kernel<AD>, dim3(blocks), dim3(256), 0, st, k, v, kv16, Hkv, T, hd, kv_stride)) return rc;
-    return launch_pdl("attn_prefill_mma", attn_prefill_mma_kernel<AD, KH>, dim3(Hkv, (T + PM_BQ - 1) / PM_BQ), dim3(32 * KH * (H / Hkv)), (size_t)smem, st, q,
-                      (const __half *)kv16, out, H, Hkv, T, hd, causal, scale);
+    return pm_go<AD>(q, kv16, out, H, Hkv, T, hd, causal, st);
 }
+static bool pm_takes(int H, int Hkv, int ad) { return ckb_tune_get("attn_prefill_mma", 1) && H % Hkv == 0 && H / Hkv <= 8 && (ad == 64 || ad == 128); }
 
 }  // namespace ckb
 
@@ -322,13 +321,21 @@ using namespace ckb;
 extern "C" int ckb_launch_attn_prefill_mma(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim,
                                            int aligned_head_dim, int kv_stride_tokens, int causal, void *stream)
 {
-    if (!ckb_tune_get("attn_prefill_mma", 1) || num_heads % num_kv_heads || num_heads / num_kv_heads > 8) return -1;
-    if ((aligned_head_dim != 64 && aligned_head_dim != 128) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)) return -1;
-    const float scale = 1.0f / sqrtf((float)head_dim);
+    if (!pm_takes(num_heads, num_kv_heads, aligned_head_dim) || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)) return -1;
     cudaStream_t st = ckb_stream(stream);
-    if (num_heads / num_kv_heads <= 4)                     // two warps per query head, 32 keys of a tile each
-        return aligned_head_dim == 64 ? pm_launch<64, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
-                                      : pm_launch<128, 2>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
-    return aligned_head_dim == 64 ? pm_launch<64, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st)
-                                  : pm_launch<128, 1>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, scale, st);
+    return aligned_head_dim == 64 ? pm_split_and_go<64>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, st)
+                                  : pm_split_and_go<128>(q, k, v, out, num_heads, num_kv_heads, num_tokens, head_dim, kv_stride_tokens, causal, st);
+}
+
+// For a caller whose kernel in front writes the pieces itself: where to (NULL: this kernel does not take such a call), and the causal attention over them.
+extern "C" void *ckb_attn_prefill_pieces(int num_heads, int num_kv_heads, int num_tokens, int head_dim)
+{
+    return pm_takes(num_heads, num_kv_heads, head_dim) ? pm_pieces(num_kv_heads, num_tokens, head_dim) : nullptr;
+}
+extern "C" int ckb_launch_attn_prefill_of_pieces(const float *q, const void *pieces, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, void *stream)
+{
+    if (((uintptr_t)q | (uintptr_t)out) & 15) return ckb_fail(CKB_ERR_ALIGN, "attention over pieces: q and out must be 16-byte aligned");
+    cudaStream_t st = ckb_stream(stream);
+    return head_dim == 64 ? pm_go<64>(q, (const __half *)pieces, out, num_heads, num_kv_heads, num_tokens, head_dim, 1, st)
+                          : pm_go<128>(q, (const __half *)pieces, out, num_heads, num_kv_heads, num_tokens, head_dim, 1, st);
 }

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) gemm_x_tiles_kernel(const uint8_t *__rest
 
 // ---------------------------------------------------------------- GEMM
 
-struct TcMaps { CUtensorMap w[3]; };                  // Q4_K: rows; Q6_K: planes ql, qh, scales
+struct TcMaps { CUtensorMap w[3]; };                  // Q4_K: rows of one matrix, or of two; Q6_K: planes ql, qh, scales
 
 // Work of a product: units dealt round-robin to persistent CTAs, token tiles innermost; a launch does those from `begin` on.  First `whole` units, a tile of the first row tiles and all of K each,
 // which write C, bias included; then the last split_nt row tiles in K slices of nbz superblocks, which write partial sums (the launcher adds them up in a fixed
@@ -335,6 +335,7 @@ struct TcMaps { CUtensorMap w[3]; };                  // Q4_K: rows; Q6_K: plane
 // weights are expanded and multiplied while the last one's sums are stored (a CTA per unit spent 6 us of 23 starting and storing).
 struct TcWork {
     int begin, units, whole, mtiles, split_nt, nb_row, nbz;
+    int rows0;                                         // rows of the first matrix, a multiple of TC_ROWS; a second one behind it, or INT_MAX
     __device__ __forceinline__ int mt(int u) const { return u % mtiles; }
     __device__ __forceinline__ int nt(int u) const { return u < whole ? u / mtiles : whole / mtiles + (u - whole) / mtiles % split_nt; }
     __device__ __forceinline__ int z(int u) const { return u < whole ? 0 : (u - whole) / mtiles / split_nt; }
@@ -494,7 +495,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                         const uint32_t dst = s_base + Cfg::OFF_RAW + r * Cfg::RAW;
                         mbar_arrive_expect_tx(BAR(Cfg::R_FULL + r), Cfg::RAW);
                         if constexpr (Q4) {
-                            tc_tma(dst, &maps.w[0], kb * Q4K_BYTES, n0, BAR(Cfg::R_FULL + r));
+                            tc_tma(dst, &maps.w[n0 < work.rows0 ? 0 : 1], kb * Q4K_BYTES, n0 < work.rows0 ? n0 : n0 - work.rows0, BAR(Cfg::R_FULL + r));
                         } else {
                             tc_tma(dst, &maps.w[0], kb * 128, n0, BAR(Cfg::R_FULL + r));
                             tc_tma(dst + Cfg::RAW_QH, &maps.w[1], kb * 64, n0, BAR(Cfg::R_FULL + r));
@@ -863,9 +864,11 @@ static bool tc_maps(TcMaps *maps, const uint8_t *B, int N, int nb)
            tc_make_map(&maps->w[2], B + (size_t)nb * 192, rb, (size_t)N, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
+struct TcSecond { const void *w; int rows0; };      // Q4_K: rows from rows0 on (a multiple of TC_ROWS) are those of a matrix of its own
 // The product over operand tiles: xt holds them (tiles of NT tokens), part the partial sums of a K split (part_bytes at hand).
 template <int WF, int NT>
-static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part, size_t part_bytes, cudaStream_t st)
+static int launch_tc(const uint8_t *xt, const void *B, TcSecond second, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part, size_t part_bytes,
+                     cudaStream_t st)
 {
     using Cfg = TcCfg<WF, NT>;
     auto kernel = gemm_kq_tc_kernel<WF, NT>;
@@ -879,12 +882,15 @@ static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float 
         attr_set = 1;
     }
     TcMaps maps;
-    if (!tc_maps<WF>(&maps, (const uint8_t *)B, N, nb)) return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", N, nb);
+    TcMaps more;
+    if (!tc_maps<WF>(&maps, (const uint8_t *)B, second.w ? second.rows0 : N, nb) || (second.w && !tc_maps<WF>(&more, (const uint8_t *)second.w, N - second.rows0, nb)))
+        return ckb_fail(CKB_ERR_SHAPE, "gemm_kq_tc: no tensor map for %d rows of %d superblocks", N, nb);
+    if (second.w) maps.w[1] = more.w[0];
     if (tc_part_bytes(plan, M, N) > part_bytes)
         return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the workspace holds %zu bytes of partial sums, this call needs %zu", part_bytes, tc_part_bytes(plan, M, N));
     const int slots = ckb_sm_count(), first = (plan.ntiles - plan.split_nt) * TC_ROWS, rest = N - first;
     const int whole = (plan.ntiles - plan.split_nt) * plan.mtiles;
-    TcWork work = {0, whole, whole, plan.mtiles, plan.split_nt ? plan.split_nt : 1, nb, plan.nbz};
+    TcWork work = {0, whole, whole, plan.mtiles, plan.split_nt ? plan.split_nt : 1, nb, plan.nbz, second.w ? second.rows0 : 0x7fffffff};
     for (int i = 0; i < 2; ++i) {                      // whole tiles; slices
         if (i) { work.begin = whole; work.units = whole + plan.split_nt * plan.mtiles * plan.Z; }
         const int units = work.units - work.begin;
@@ -901,10 +907,10 @@ static int launch_tc(const uint8_t *xt, const void *B, const float *bias, float 
     return launch_pdl("gemm_splitk_sum", sum, dim3(blocks), dim3(256), (size_t)0, st, (const float *)part, plan.Z, b2, C + first, ldc, M, rest);
 }
 
-static int tc_launch(int wf, int nt, const uint8_t *xt, const void *B, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part,
+static int tc_launch(int wf, int nt, const uint8_t *xt, const void *B, TcSecond second, const float *bias, float *C, int ldc, int M, int N, int nb, const TcPlan &plan, float *part,
                      size_t part_bytes, cudaStream_t st)
 {
-#define TC_GO(WF, NT) return launch_tc<WF, NT>(xt, B, bias, C, ldc, M, N, nb, plan, part, part_bytes, st)
+#define TC_GO(WF, NT) return launch_tc<WF, NT>(xt, B, second, bias, C, ldc, M, N, nb, plan, part, part_bytes, st)
     if (wf == TC_W_Q6K_PLANAR) switch (nt) { case 32: TC_GO(TC_W_Q6K_PLANAR, 32); case 64: TC_GO(TC_W_Q6K_PLANAR, 64); case 96: TC_GO(TC_W_Q6K_PLANAR, 96); default: TC_GO(TC_W_Q6K_PLANAR, 128); }
     switch (nt) { case 32: TC_GO(TC_W_Q4K, 32); case 64: TC_GO(TC_W_Q4K, 64); case 96: TC_GO(TC_W_Q4K, 96); default: TC_GO(TC_W_Q4K, 128); }
 #undef TC_GO
@@ -948,8 +954,21 @@ extern "C" size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K) { 
 extern "C" int ckb_launch_gemm_tc_tiles(int wf, const void *tiles, int nt, const void *B, float *C, int ldc, int M, int N, int K, void *part, size_t part_bytes, void *stream)
 {
     if (K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)tiles & 15)) return -1;
-    return tc_launch(wf, nt, (const uint8_t *)tiles, B, nullptr, C, ldc, M, N, K / QK_K, tc_plan(wf, nt, M, N, K / QK_K), (float *)part, part_bytes,
+    return tc_launch(wf, nt, (const uint8_t *)tiles, B, TcSecond{nullptr, 0}, nullptr, C, ldc, M, N, K / QK_K, tc_plan(wf, nt, M, N, K / QK_K), (float *)part, part_bytes,
                      ckb_stream(stream));
+}
+
+// Two Q4_K products over the same rows as one launch, the second's columns of C behind the first's: for products that are one round of whole tiles together (split along K,
+// or in several rounds, they run side by side faster).  -1: not such.
+extern "C" int ckb_gemm_tc_pairs(int nt, int M, int N, int N2, int K)
+{
+    const TcPlan p = tc_plan(TC_W_Q4K, nt, M, N + N2, K / QK_K), a = tc_plan(TC_W_Q4K, nt, M, N, K / QK_K), b = tc_plan(TC_W_Q4K, nt, M, N2, K / QK_K);
+    return N % TC_ROWS == 0 && !p.split_nt && !a.split_nt && !b.split_nt && p.mtiles * p.ntiles <= ckb_sm_count();
+}
+extern "C" int ckb_launch_gemm_tc_pair(const void *tiles, int nt, const void *B, int N, const void *B2, int N2, float *C, int ldc, int M, int K, void *stream)
+{
+    if (K % QK_K || (((uintptr_t)B | (uintptr_t)B2 | (uintptr_t)tiles) & 15) || !ckb_gemm_tc_pairs(nt, M, N, N2, K)) return -1;
+    return tc_launch(TC_W_Q4K, nt, (const uint8_t *)tiles, B, TcSecond{B2, N}, nullptr, C, ldc, M, N + N2, K / QK_K, tc_plan(TC_W_Q4K, nt, M, N + N2, K / QK_K), nullptr, 0, ckb_stream(stream));
 }
 
 // C[m * ldc + n] = A_q8[m] . W[n] (+ bias[n]).  wf: TC_W_Q4K (the reference's block_q4_K rows) or TC_W_Q6K_PLANAR.
@@ -970,7 +989,7 @@ extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, co
     if (!xt) return CKB_ERR_CUDA;
     cudaStream_t st = ckb_stream(stream);
     if (int rc = tc_make_tiles(A_q8, xt, nt, M, nb, st)) return rc;
-    return tc_launch(wf, nt, xt, B, bias, C, ldc, M, N, nb, plan, reinterpret_cast<float *>(xt + xt_bytes), part_bytes, st);
+    return tc_launch(wf, nt, xt, B, TcSecond{nullptr, 0}, bias, C, ldc, M, N, nb, plan, reinterpret_cast<float *>(xt + xt_bytes), part_bytes, st);
 }
 
 extern "C" int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,

@@ -779,6 +779,12 @@ static int issue_step(KqModel *m, void *st)
 int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens, void *stream);
 int ckb_gemm_tc_width(int wf, int M, int N, int K);                                                                    /* gemm_tc.cu */
 size_t ckb_gemm_tc_tile_bytes(int nt, int M, int K);
+int ckb_gemm_tc_pairs(int nt, int M, int N, int N2, int K);
+int ckb_launch_gemm_tc_pair(const void *tiles, int nt, const void *B, int N, const void *B2, int N2, float *C, int ldc, int M, int K, void *stream);
+void *ckb_attn_prefill_pieces(int num_heads, int num_kv_heads, int num_tokens, int head_dim);                          /* attention_prefill_mma.cu */
+int ckb_launch_attn_prefill_of_pieces(const float *q, const void *pieces, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, void *stream);
+int ckb_prefill_rope_rows(const float *q_tm, int ldq, const float *k_tm, int ldk, const float *v_tm, int ldv, float *q_hm, float *k_cache, float *v_cache, const float *cos_cache,
+                          const float *sin_cache, int tokens, int num_heads, int num_kv_heads, int head_dim, int max_seq_len, int pos0, void *pieces, void *stream);
 size_t ckb_gemm_tc_part_bytes(int wf, int nt, int M, int N, int K);
 int ckb_launch_gemm_tc_tiles(int wf, const void *tiles, int nt, const void *B, float *C, int ldc, int M, int N, int K, void *part, size_t part_bytes, void *stream);
 int ckb_add_rmsnorm_tiles(float *x, const float *delta, const float *gamma, void *tiles, int tile_nt, int tokens, int d_model, int aligned, float eps, void *stream);   /* step_kernels.cu */
@@ -834,7 +840,7 @@ static int prefill_ok(const KqModel *m, int T)
 static int prefill_buffers(KqModel *m, int T)
 {
     const size_t t = (size_t)T, kvw = (size_t)m->Hkvl * m->d, widest = (size_t)(m->Da > m->Ala ? m->Da : m->Ala) > (size_t)m->Il ? (size_t)(m->Da > m->Ala ? m->Da : m->Ala) : (size_t)m->Il;
-    size_t need[PF_BUFFERS] = { t * m->Da * 4, t * m->Da * 4, t * m->Da * 4, t * m->Al * 4, t * kvw * 4, t * kvw * 4, t * m->Al * 4, t * m->Al * 4, t * 2 * m->Il * 4 };
+    size_t need[PF_BUFFERS] = { t * m->Da * 4, t * m->Da * 4, t * m->Da * 4, t * (m->Al + kvw) * 4, t * kvw * 4, t * kvw * 4, t * m->Al * 4, t * m->Al * 4, t * 2 * m->Il * 4 };
     need[PF_ROWS] = (t + 127) * (widest / 256) * 548;          /* operand tiles of any width up to 128: 548 bytes per token and superblock, more than the other forms */
     need[PF_ATTN] = ckb_attn_behind_part_bytes(m->d);
     need[PF_IDS] = t * sizeof(int32_t);
@@ -909,20 +915,24 @@ static int prefill_norm(KqModel *m, const float *delta, const Tensor *gamma, con
     return ckb200_dev_add_rmsnorm_q8k(m->pf_x, delta, g, m->pf_rows, NULL, T, m->D, m->Da, m->c.rms_eps, st);
 }
 
-/* the three products over one set of rows, side by side; the 32-token form of the tcgen05 kernel shares the library's scratch and stays on one stream */
-static int prefill_qkv(KqModel *m, const Tensor *t, int nt, int T, void *st)
+/* The three products over one set of rows, side by side; the 32-token form of the tcgen05 kernel shares the library's scratch and stays on one stream.  q and k as one
+ * launch where they are one round of tiles: a short prompt of a small model waits for its launches to be issued.  out, ld: where the rows went. */
+static int prefill_qkv(KqModel *m, const Tensor *t, int nt, int T, float *out[3], int ld[3], void *st)
 {
     const Tensor *w[3] = { &t[CKB_T_WQ], &t[CKB_T_WK], &t[CKB_T_WV] };
-    float *out[3] = { m->pf_q, m->pf_k, m->pf_v };
-    const int ld[3] = { m->Al, m->Hkvl * m->d, m->Hkvl * m->d };
+    out[0] = m->pf_q; out[1] = m->pf_k; out[2] = m->pf_v;
+    ld[0] = m->Al; ld[1] = ld[2] = m->Hkvl * m->d;
+    const int pair = nt && w[0]->fmt == FMT_Q4K && w[1]->fmt == FMT_Q4K && w[0]->rows == m->Al && ckb_gemm_tc_pairs(nt, T, w[0]->rows, w[1]->rows, w[0]->cols);
+    if (pair) { ld[0] = ld[1] = m->Al + m->Hkvl * m->d; out[1] = m->pf_q + m->Al; }
     int apart = ckb_tune_get("model_qkv_streams", 1);
     for (int i = 0; i < 3 && apart && !nt && !fmt_block32(w[0]->fmt); ++i)
         apart = w[i]->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_takes(m->pf_rows, w[i]->w, T, w[i]->rows, w[i]->cols) : ckb_gemm_q6k_mma_takes(m->pf_rows, w[i]->planar, T, w[i]->rows, w[i]->cols);
     cudaStream_t main_st = (cudaStream_t)st;
     int rc;
     if (apart && ckb_check_cuda((int)cudaEventRecord(m->ev_fork, main_st), "fork")) return CKB_ERR_CUDA;
-    if ((rc = prefill_gemm(m, w[0], nt, out[0], ld[0], T, 0, st))) return rc;
-    for (int i = 1; i < 3; ++i) {
+    if ((rc = pair ? ckb_launch_gemm_tc_pair(m->pf_rows, nt, w[0]->w, w[0]->rows, w[1]->w, w[1]->rows, out[0], ld[0], T, w[0]->cols, st)
+                   : prefill_gemm(m, w[0], nt, out[0], ld[0], T, 0, st))) return rc == -1 ? ckb_fail(CKB_ERR_SHAPE, "prefill: q and k not handled as one product") : rc;
+    for (int i = pair ? 2 : 1; i < 3; ++i) {
         cudaStream_t s = apart ? m->side[i - 1] : main_st;
         if (apart && ckb_check_cuda((int)cudaStreamWaitEvent(s, m->ev_fork, 0), "fork wait")) return CKB_ERR_CUDA;
         if ((rc = prefill_gemm(m, w[i], nt, out[i], ld[i], T, i, s))) return rc;
@@ -956,10 +966,15 @@ static int issue_prefill(KqModel *m, int T, void *st)
         const int nt_q = tile_width(&t[CKB_T_WQ], T, &memo[0]), nt_o = tile_width(&t[CKB_T_WO], T, &memo[1]), nt_1 = tile_width(&t[CKB_T_W1], T, &memo[2]),
                   nt_2 = tile_width(&t[CKB_T_W2], T, &memo[3]);
         if ((rc = prefill_norm(m, delta, &t[CKB_T_LN1], &t[CKB_T_WQ], nt_q, T, st))) return rc;
-        if ((rc = prefill_qkv(m, t, nt_q, T, st))) return rc;
-        if ((rc = ckb200_dev_prefill_rope_scatter(m->pf_q, m->pf_k, m->pf_v, m->pf_qh, kc, vc, m->rope_cos, m->rope_sin, T, m->Hl, m->Hkvl, m->d, c->max_seq_len, before, st))) return rc;
+        float *qkv[3];
+        int ld[3];
+        if ((rc = prefill_qkv(m, t, nt_q, T, qkv, ld, st))) return rc;
+        void *pieces = fp32 ? NULL : ckb_attn_prefill_pieces(m->Hl, m->Hkvl, T, m->d);
+        rc = ckb_prefill_rope_rows(qkv[0], ld[0], qkv[1], ld[1], qkv[2], ld[2], m->pf_qh, kc, vc, m->rope_cos, m->rope_sin, T, m->Hl, m->Hkvl, m->d, c->max_seq_len, before, pieces, st);
+        if (rc) return rc == -1 ? ckb_fail(CKB_ERR_SHAPE, "prefill: rows of q, k and v not aligned") : rc;
         rc = fp32 ? ckb_launch_attn_behind(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, c->max_seq_len, before, m->pf_attn, st)
-                  : ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st);
+           : pieces ? ckb_launch_attn_prefill_of_pieces(m->pf_qh, pieces, m->pf_oh, m->Hl, m->Hkvl, T, m->d, st)
+                    : ckb200_dev_attention_prefill(m->pf_qh, kc, vc, m->pf_oh, m->Hl, m->Hkvl, T, m->d, m->d, c->max_seq_len, 1, st);
         if (rc) return rc;
         if (fmt_block32(t[CKB_T_WO].fmt)) rc = ckb_prefill_gather_q80_planar(m->pf_oh, m->pf_rows, T, m->Hl, m->d, t[CKB_T_WO].cols, st);
         else if (nt_o) rc = ckb_prefill_gather_tiles(m->pf_oh, m->pf_rows, nt_o, T, m->Hl, m->d, m->Ala, st);

@@ -8,6 +8,7 @@
 //                          q -> [H][T][d], k and v -> cache rows pos0 .. pos0 + T - 1 (kv_cache_store per token)
 //   prefill_gather_q8k     attention output [H][T][d] -> token rows, quantised to Q8_K for the o projection (quantize_row_q8_k)
 #include "add_rmsnorm_q8k.cuh"
+#include "fp16_pieces.cuh"
 #include "launch.h"
 #include "pdl.cuh"
 #include "q8k_block.cuh"
@@ -50,12 +51,15 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_kernel(const float *
     }
 }
 
-// The same with four rotation pairs per thread (16-byte accesses): d a multiple of 8, all pointers 16-byte aligned.
-__global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const float *__restrict__ q_tm, const float *__restrict__ k_tm, const float *__restrict__ v_tm,
-                                                                      float *__restrict__ q_hm, float *__restrict__ kc, float *__restrict__ vc,
+// The same with four rotation pairs per thread (16-byte accesses): d a multiple of 8, all pointers 16-byte aligned.  Rows of q, k and v are ldq, ldk and ldv floats apart.
+// pieces (not NULL): keys and values also as the fp16 pieces that prompt attention reads, K hi | K lo | V hi | V lo, each [Hkv][T][d] (a launch of its own for that
+// cost 3 us of the chain and its issue).
+__global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const float *__restrict__ q_tm, int ldq, const float *__restrict__ k_tm, int ldk, const float *__restrict__ v_tm,
+                                                                      int ldv, float *__restrict__ q_hm, float *__restrict__ kc, float *__restrict__ vc,
                                                                       const float *__restrict__ cos_cache, const float *__restrict__ sin_cache, int T, int H,
-                                                                      int Hkv, int d, int max_seq, int pos0)
+                                                                      int Hkv, int d, int max_seq, int pos0, __half *__restrict__ pieces)
 {
+    const size_t arr = (size_t)Hkv * T * d;
     pdl_wait();
     pdl_trigger();
     const int half = d / 2, q4 = half / 4;
@@ -66,20 +70,27 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const floa
         if (pos >= max_seq) continue;
         const float *src;
         float *dst;
+        __half *piece = nullptr;
         if (h < H) {
-            src = q_tm + ((size_t)t * H + h) * d;
+            src = q_tm + (size_t)t * ldq + h * d;
             dst = q_hm + ((size_t)h * T + t) * d;
         } else if (h < H + Hkv) {
-            src = k_tm + ((size_t)t * Hkv + (h - H)) * d;
+            src = k_tm + (size_t)t * ldk + (h - H) * d;
             dst = kc + ((size_t)(h - H) * max_seq + pos) * d;
+            if (pieces) piece = pieces + ((size_t)(h - H) * T + t) * d + j;
         } else {
-            src = v_tm + ((size_t)t * Hkv + (h - H - Hkv)) * d;
+            src = v_tm + (size_t)t * ldv + (h - H - Hkv) * d;
             dst = vc + ((size_t)(h - H - Hkv) * max_seq + pos) * d;
+            if (pieces) piece = pieces + 2 * arr + ((size_t)(h - H - Hkv) * T + t) * d + j;
         }
         const float4 a = __ldcg(reinterpret_cast<const float4 *>(src + j)), b = __ldcg(reinterpret_cast<const float4 *>(src + j + half));
         if (h >= H + Hkv) {
             *reinterpret_cast<float4 *>(dst + j) = a;
             *reinterpret_cast<float4 *>(dst + j + half) = b;
+            if (piece) {
+                store_pieces4(piece, arr, a);
+                store_pieces4(piece + half, arr, b);
+            }
             continue;
         }
         const float4 c = *reinterpret_cast<const float4 *>(cos_cache + (size_t)pos * half + j), sn = *reinterpret_cast<const float4 *>(sin_cache + (size_t)pos * half + j);
@@ -90,6 +101,10 @@ __global__ void __launch_bounds__(256) prefill_rope_scatter_v4_kernel(const floa
         lo.w = __fsub_rn(__fmul_rn(a.w, c.w), __fmul_rn(b.w, sn.w)); hi.w = __fadd_rn(__fmul_rn(a.w, sn.w), __fmul_rn(b.w, c.w));
         *reinterpret_cast<float4 *>(dst + j) = lo;
         *reinterpret_cast<float4 *>(dst + j + half) = hi;
+        if (piece) {
+            store_pieces4(piece, arr, lo);
+            store_pieces4(piece + half, arr, hi);
+        }
     }
 }
 
@@ -136,6 +151,19 @@ __global__ void __launch_bounds__(256) prefill_gather_q80_kernel(const float *__
 
 using namespace ckb;
 
+// -1: not in this form (head size, alignment)
+extern "C" int ckb_prefill_rope_rows(const float *q_tm, int ldq, const float *k_tm, int ldk, const float *v_tm, int ldv, float *q_hm, float *k_cache, float *v_cache,
+                                     const float *cos_cache, const float *sin_cache, int tokens, int num_heads, int num_kv_heads, int head_dim, int max_seq_len, int pos0, void *pieces,
+                                     void *stream)
+{
+    const uintptr_t all = (uintptr_t)q_tm | (uintptr_t)k_tm | (uintptr_t)v_tm | (uintptr_t)q_hm | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_cache |
+                          (uintptr_t)sin_cache | (uintptr_t)pieces;
+    if (head_dim % 8 || (all & 15) || ((ldq | ldk | ldv) & 3)) return -1;
+    const long long n4 = (long long)tokens * (num_heads + 2 * num_kv_heads) * (head_dim / 8);
+    const unsigned g4 = (unsigned)((n4 + 255) / 256 < 4736 ? (n4 + 255) / 256 : 4736);
+    return launch_pdl("prefill_rope_scatter", prefill_rope_scatter_v4_kernel, dim3(g4), dim3(256), (size_t)0, ckb_stream(stream), q_tm, ldq, k_tm, ldk, v_tm, ldv, q_hm, k_cache, v_cache,
+                      cos_cache, sin_cache, tokens, num_heads, num_kv_heads, head_dim, max_seq_len, pos0, (__half *)pieces);
+}
 extern "C" int ckb200_dev_prefill_rope_scatter(const float *q_tm, const float *k_tm, const float *v_tm, float *q_hm, float *k_cache, float *v_cache,
                                                const float *cos_cache, const float *sin_cache, int tokens, int num_heads, int num_kv_heads, int head_dim,
                                                int max_seq_len, int pos0, void *stream)
@@ -143,15 +171,10 @@ extern "C" int ckb200_dev_prefill_rope_scatter(const float *q_tm, const float *k
     if (!q_tm || !k_tm || !v_tm || !q_hm || !k_cache || !v_cache || !cos_cache || !sin_cache || tokens <= 0 || num_heads <= 0 || num_kv_heads <= 0) return 0;
     if (head_dim % 2 || pos0 < 0) return ckb_fail(CKB_ERR_SHAPE, "prefill_rope_scatter: head_dim %d, pos0 %d", head_dim, pos0);
     if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
+    const int rc = ckb_prefill_rope_rows(q_tm, num_heads * head_dim, k_tm, num_kv_heads * head_dim, v_tm, num_kv_heads * head_dim, q_hm, k_cache, v_cache, cos_cache, sin_cache, tokens,
+                                         num_heads, num_kv_heads, head_dim, max_seq_len, pos0, nullptr, stream);
+    if (rc != -1) return rc;
     const long long n = (long long)tokens * (num_heads + 2 * num_kv_heads) * (head_dim / 2);
-    const uintptr_t all = (uintptr_t)q_tm | (uintptr_t)k_tm | (uintptr_t)v_tm | (uintptr_t)q_hm | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_cache |
-                          (uintptr_t)sin_cache;
-    if (head_dim % 8 == 0 && (all & 15) == 0) {
-        const long long n4 = n / 4;
-        const unsigned g4 = (unsigned)((n4 + 255) / 256 < 4736 ? (n4 + 255) / 256 : 4736);
-        return launch_pdl("prefill_rope_scatter", prefill_rope_scatter_v4_kernel, dim3(g4), dim3(256), (size_t)0, ckb_stream(stream), q_tm, k_tm, v_tm, q_hm, k_cache, v_cache,
-                          cos_cache, sin_cache, tokens, num_heads, num_kv_heads, head_dim, max_seq_len, pos0);
-    }
     const unsigned grid = (unsigned)((n + 255) / 256 < 4736 ? (n + 255) / 256 : 4736);
     prefill_rope_scatter_kernel<<<grid, 256, 0, ckb_stream(stream)>>>(q_tm, k_tm, v_tm, q_hm, k_cache, v_cache, cos_cache, sin_cache, tokens, num_heads, num_kv_heads,
                                                                       head_dim, max_seq_len, pos0);

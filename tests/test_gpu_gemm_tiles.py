@@ -237,3 +237,60 @@ def test_q8_0_product_is_the_same_in_either_tile(ck, orc, m, n):
     first = min(n, 200)
     want = cases.gemm_nt(orc, "oracle_", "q8_0", xq.cpu().numpy()[:m * k // 32 * 34], np.ascontiguousarray(wq.cpu().numpy()[:first * k // 32 * 34]), None, m, first, k)
     assert np.array_equal(outs[0][:, :first], want)
+
+
+@pytest.mark.parametrize("nt,m,n,n2,nb", [(32, 17, 128, 1, 1), (32, 77, 896, 128, 4), (64, 65, 256, 300, 3), (96, 96, 1280, 129, 2), (128, 129, 896, 128, 5)])
+def test_two_products_over_the_same_rows_as_one_launch(ck, nt, m, n, n2, nb):
+    """Rows of two matrices in one deal: the bits of the two products on their own, side by side."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    k = 256 * nb
+    p = lambda t: C.c_void_p(t.data_ptr())
+    ws = [torch.from_numpy(synth.make_weights("q4_k", rows, k, seed=rows)).to(dev) for rows in (n, n2)]
+    g = torch.Generator(device=dev).manual_seed(m)
+    x, gamma = torch.randn(m, k, device=dev, generator=g), torch.ones(k, device=dev)
+    tiles = torch.zeros(((m + nt - 1) // nt) * nb * nt * 548, dtype=torch.uint8, device=dev)
+    both, apart = torch.full((m, n + n2), float("nan"), device=dev), [torch.full((m, rows), float("nan"), device=dev) for rows in (n, n2)]
+    torch.cuda.synchronize()
+    assert ck.ckb_add_rmsnorm_tiles(p(x), None, p(gamma), p(tiles), nt, m, k, k, C.c_float(1e-5), None) == 0
+    if not ck.ckb_gemm_tc_pairs(nt, m, n, n2, k):
+        assert ck.ckb_launch_gemm_tc_pair(p(tiles), nt, p(ws[0]), n, p(ws[1]), n2, p(both), n + n2, m, k, None) == -1
+        return
+    assert ck.ckb_launch_gemm_tc_pair(p(tiles), nt, p(ws[0]), n, p(ws[1]), n2, p(both), n + n2, m, k, None) == 0
+    for w, out in zip(ws, apart):
+        assert ck.ckb_launch_gemm_tc_tiles(0, p(tiles), nt, p(w), p(out), out.shape[1], m, out.shape[1], k, None, C.c_size_t(0), None) == 0
+    assert ck.ckb200_synchronize() == 0
+    assert torch.equal(both, torch.cat(apart, 1)) and torch.isfinite(both).all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,tokens", [(14, 2, 64, 77), (4, 4, 128, 17), (8, 1, 64, 129)])
+def test_rotation_writes_the_pieces_that_attention_splits(ck, heads, kv_heads, d, tokens):
+    """Attention over pieces from the rotation kernel gives the bits of attention that splits the cache itself; rows of q and k with gaps between them."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(tokens)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    at = lambda t, floats: C.c_void_p(t.data_ptr() + 4 * floats)
+    room, wq, wk = 160, heads * d, kv_heads * d
+    qk, v = torch.randn(tokens, wq + wk, device=dev, generator=g), torch.randn(tokens, wk, device=dev, generator=g)
+    angle = torch.rand(room, d // 2, device=dev, generator=g) * 6
+    cos, sin = angle.cos().contiguous(), angle.sin().contiguous()
+    q0, k0 = qk[:, :wq].contiguous(), qk[:, wq:].contiguous()
+    outs = []
+    ck.ckb_attn_prefill_pieces.restype = C.c_void_p
+    for own in (False, True):
+        qh, kc, vc, out = torch.zeros(heads, tokens, d, device=dev), torch.zeros(kv_heads, room, d, device=dev), torch.zeros(kv_heads, room, d, device=dev), torch.zeros(heads, tokens, d, device=dev)
+        torch.cuda.synchronize()
+        if own:
+            pieces = C.c_void_p(ck.ckb_attn_prefill_pieces(heads, kv_heads, tokens, d))
+            assert pieces.value
+            assert ck.ckb_prefill_rope_rows(p(qk), wq + wk, at(qk, wq), wq + wk, p(v), wk, p(qh), p(kc), p(vc), p(cos), p(sin), tokens, heads, kv_heads, d, room, 0, pieces, None) == 0
+            assert ck.ckb_launch_attn_prefill_of_pieces(p(qh), pieces, p(out), heads, kv_heads, tokens, d, None) == 0
+        else:
+            assert ck.ckb200_dev_prefill_rope_scatter(p(q0), p(k0), p(v), p(qh), p(kc), p(vc), p(cos), p(sin), tokens, heads, kv_heads, d, room, 0, None) == 0
+            assert ck.ckb200_dev_attention_prefill(p(qh), p(kc), p(vc), p(out), heads, kv_heads, tokens, d, d, room, 1, None) == 0
+        assert ck.ckb200_synchronize() == 0
+        outs.append((qh, kc, vc, out))
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and outs[0][3].abs().sum() > 0
