@@ -24,6 +24,8 @@ typedef struct CkbModelFamily {
     size_t (*step_weight_bytes)(const CKB200Model *m);        /* weight bytes one step streams */
 } CkbModelFamily;
 
+enum { CKB_OUT_CHUNKS = 16, CKB_OUT_MOST = 4 << 20 };
+
 struct CKB200Model {
     CKB200ModelConfig c;
     const CkbModelFamily *family;
@@ -35,11 +37,16 @@ struct CKB200Model {
     int graph_ready;
     cudaEvent_t ev_tokens;  /* the last copy out of tokens_pinned: the next call waits for it before it overwrites the buffer */
     int tokens_in_flight;
+    uint8_t *out_pinned;    /* logits on their way to pageable memory, [batch][vocab] up to CKB_OUT_MOST bytes; NULL: they go there directly */
+    cudaEvent_t ev_out[CKB_OUT_CHUNKS];
 };
 
 extern const CkbModelFamily ckb_family_kquant, ckb_family_stack;
 
 /* token and position staging and the logits rows of `m` (its config is set); 0 on success */
 int ckb_model_init_shared(struct CKB200Model *m);
+
+/* `bytes` of logits at `dev` (at most the model's own rows) to the caller's memory, and ckb_sync_check */
+int ckb_model_logits_out(struct CKB200Model *m, float *host, const float *dev, size_t bytes, cudaStream_t st, const char *what);
 
 #endif

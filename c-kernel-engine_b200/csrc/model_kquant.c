@@ -1010,8 +1010,7 @@ static int kq_extend(CKB200Model *model, const int32_t *tokens, int count, const
         cudaStreamSynchronize(st);
     }
     if (!rc) rc = ckb_check_cuda((int)cudaMemcpyAsync(m->pos_dev, &end, sizeof end, cudaMemcpyHostToDevice, st), "prefill pos");
-    if (!rc && n_want) rc = ckb_check_cuda((int)cudaMemcpyAsync(logits_host, m->logits, (size_t)m->Vl * sizeof(float), cudaMemcpyDeviceToHost, st), "logits D2H");
-    if (!rc) rc = ckb_sync_check(st, "model_prefill");
+    if (!rc) rc = n_want ? ckb_model_logits_out(model, logits_host, m->logits, (size_t)m->Vl * sizeof(float), st, "model_prefill") : ckb_sync_check(st, "model_prefill");
     if (!rc) m->host_pos = end;
     return rc;
 }

@@ -142,9 +142,17 @@ cudaStream_t ckb_stream(void *user) { return user ? (cudaStream_t)user : g.strea
 /* Synchronises `st` and folds in the device error word: kernels that gave up on a bounded wait (a peer that never wrote,
  * a copy that never landed) leave a code there and return, so without this check the caller would get rc 0 and a result
  * built from stale data.  The word travels in the same stream, just before the sync (4 bytes, pinned). */
+int ckb_fetch_error_word(cudaStream_t st)
+{
+    return ckb_check_cuda((int)cudaMemcpyAsync(g.err_pinned, g.dev_err, sizeof(int), cudaMemcpyDeviceToHost, st), "read error word") ? CKB_ERR_CUDA : 0;
+}
 int ckb_sync_check(cudaStream_t st, const char *what)
 {
-    if (ckb_check_cuda((int)cudaMemcpyAsync(g.err_pinned, g.dev_err, sizeof(int), cudaMemcpyDeviceToHost, st), "read error word")) return CKB_ERR_CUDA;
+    const int rc = ckb_fetch_error_word(st);
+    return rc ? rc : ckb_sync_fetched(st, what);
+}
+int ckb_sync_fetched(cudaStream_t st, const char *what)
+{
     if (ckb_check_cuda((int)cudaStreamSynchronize(st), what)) return CKB_ERR_CUDA;
     const int word = *g.err_pinned;
     if (word != 0) {

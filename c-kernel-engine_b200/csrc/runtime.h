@@ -18,6 +18,8 @@ cudaStream_t ckb_stream(void *user);       /* user stream, or the library stream
 int ckb_tune_get(const char *key, int dflt);
 int ckb_is_device_ptr(const void *p);      /* device or managed memory */
 int ckb_sync_check(cudaStream_t st, const char *what);   /* sync + device error word -> 0, CKB_ERR_CUDA or CKB_ERR_DEVICE_WAIT */
+int ckb_fetch_error_word(cudaStream_t st);               /* its two halves, for a caller that has something to do in between */
+int ckb_sync_fetched(cudaStream_t st, const char *what);
 long long ckb_wait_limit_cycles(void);     /* tune key wait_limit_ms in SM cycles */
 /* Row-planar copy (aligned 16-byte loads: gemv_q6k_planar.cu, gemv_q80_planar.cu, gemv_q50_planar.cu) of `rows` rows of a
  * REGISTERED weight range, built on first use and kept until the range is unregistered; NULL when dev_raw is not inside a

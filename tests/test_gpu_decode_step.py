@@ -184,3 +184,32 @@ def test_fused_step_matches_the_launch_per_op_step(ck, orc, cfg, pdl):
         scale = float(np.max(np.abs(want[i])))
         assert float(np.max(np.abs(got[1][i] - got[0][i]))) <= 2e-3 * scale, i
         assert cosine(got[1][i], got[0][i]) >= 0.99999, i
+
+
+@pytest.mark.parametrize("vocab,batch", [(300, 1), (32768, 1), (49153, 1), (151937, 1), (151937, 6), (140001, 8)])
+def test_logits_come_back_the_same_to_any_memory(ck, vocab, batch):
+    """To pageable memory in chunks over pinned memory (128 KB to 4 MB), else directly: the same bytes, at any offset, nothing beside them."""
+    import torch
+
+    so.bind_model_api(ck)
+    cfg = dict(embed_dim=256, num_heads=4, num_kv_heads=2, head_dim=64, intermediate_size=512, num_layers=1, vocab_size=vocab, max_seq_len=64, rms_eps=1e-5, rope_theta=1e4,
+               fmt_q=0, fmt_k=0, fmt_v=1, fmt_o=0, fmt_gate_up=0, fmt_down=1, fmt_lm_head=1)
+    model = so.CpuModel(cfg, seed=2)
+    st = so.make_cfg(cfg, batch=batch)
+    h = ck.ckb200_model_create(C.byref(st))
+    assert h, ck.ckb200_last_error_message()
+    try:
+        so.upload_whole_model(ck, h, model, batch)
+        ids = np.arange(batch, dtype=np.int32)
+        n = vocab * batch
+        outs = []
+        for kind in ("pageable", "odd", "pinned"):
+            room = torch.full((n + 8,), -7.0, pin_memory=kind == "pinned").numpy()
+            at = 3 if kind == "odd" else 4
+            assert ck.ckb200_model_set_pos(h, 5) == 0
+            assert ck.ckb200_model_decode(h, ids.ctypes.data_as(C.c_void_p), room[at:].ctypes.data_as(C.c_void_p)) == 0
+            assert (room[:at] == -7).all() and (room[at + n:] == -7).all()
+            outs.append(room[at:at + n].copy())
+        assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2]) and np.isfinite(outs[0]).all() and np.abs(outs[0]).max() > 0
+    finally:
+        ck.ckb200_model_free(h)
