@@ -28,7 +28,7 @@ static int gemm_nt_by_rows(gemv_fn fn, size_t a_row_bytes, const void *A_q8, con
     return bias ? ckb200_dev_add_bias_rows(C, bias, M, N, stream) : 0;
 }
 
-// Up to 64 tokens: the integer-MMA kernel that streams the weights through registers (gemm_q4k_mma.cu); above that the tcgen05 kernel.
+// Up to 16 tokens, and up to 64 where the product is small: the integer-MMA kernel that streams the weights through registers (gemm_q4k_mma.cu); above that the tcgen05 kernel.
 extern "C" int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);
 extern "C" int ckb200_dev_gemm_nt_q4_k_q8_k(const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)
 {

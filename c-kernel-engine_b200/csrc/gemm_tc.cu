@@ -84,6 +84,10 @@ struct TcCfg : TcTile<NT> {
     static constexpr int ADEEP = NT > 64 ? 1 : 2, ASLOTS = 4;        // ring of weight stages in tensor memory, 64-deep or 128-deep: one superblock or two
     // Q4_K: the expander sets take superblocks in turn; where they share the slots, each has barriers of its own for them.  Q6_K: a half of every superblock each.
     static constexpr int AEMPTIES = Q4 && ADEEP == 1 ? 2 * ASLOTS : ASLOTS, TAKERS = Q4 ? 4 : 8;      // warps that read a raw superblock
+    // A Q4_K set skips every other superblock, so it must not come to the wait for superblock b before b - RSLOTS has landed: to a waiter two phases ahead a phase parity
+    // reads as complete.  Where the sets share the weight slots b - 1 has to be multiplied first anyway; with slots of its own a set gets three superblocks ahead
+    // (its raw wait of b comes behind its stores of b - 2, which need b - 4 multiplied, while b - 3 may still be in flight).  A ring of three then needs b - 2 multiplied first.
+    static constexpr bool RAW_BEHIND_MMA = Q4 && ADEEP == 2 && RSLOTS <= 3;
     static constexpr int OFF_RAW = 0;
     static constexpr int OFF_B = OFF_RAW + RSLOTS * RAW;
     static constexpr int OFF_A2 = OFF_B + TC_BSLOTS * BSLOT;
@@ -537,6 +541,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             };
             for (uint32_t b = set; b < total; b += 2, pa ^= 1u) {
                 const uint8_t *raw = smem + Cfg::OFF_RAW + r * Cfg::RAW;
+                if constexpr (Cfg::RAW_BEHIND_MMA) TC_WAIT(empty, pa, DEV_ERR_EMPTY_WAIT);
                 TC_WAIT(BAR(Cfg::R_FULL + r), rp, DEV_ERR_FULL_WAIT);
                 const uint4 *p = reinterpret_cast<const uint4 *>(raw + row * Q4K_BYTES);
                 const uint4 hdr = p[0];

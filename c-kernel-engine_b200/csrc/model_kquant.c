@@ -491,8 +491,8 @@ static int matvec_standalone(const KqModel *m, const Tensor *w, const uint8_t *x
 /* y[b] = W . xq[b] for every sequence b; xq rows are `cols`-wide quantised vectors */
 static int matvec(KqModel *m, const Tensor *w, const uint8_t *xq, float *y, int y_stride, void *st)
 {
-    /* batched decode: the weights are streamed once for all sequences.  Q4_K from 4 sequences up on the integer-MMA kernel (no workspace),
-     * otherwise from 16 up on the tcgen05 kernel */
+    /* batched decode: the weights are streamed once for all sequences, by the integer-MMA kernels (no workspace) or, where those leave a product of 17 sequences
+     * and more to it, by the tcgen05 kernel */
     if (w->fmt == FMT_Q4K && m->c.batch > 1) {
         const int rc = ckb_launch_gemm_q4k_mma(xq, w->w, NULL, y, y_stride, m->c.batch, w->rows, w->cols, st);
         if (rc >= 0) return rc;
