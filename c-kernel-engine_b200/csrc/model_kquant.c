@@ -771,8 +771,10 @@ static int issue_step(KqModel *m, void *st)
  * fp32 caches; prompts shorter than 16 tokens and other cases fall back to T decode steps.
  *
  * How a product is done depends on the format and on T:
- *   K-quants, T <= 64   Q8_K rows, integer-MMA kernels (48 x 4096 x 4096: 12 us; the tcgen05 kernel with 32-token tiles 17)
- *   K-quants, T > 64    the producer of the rows quantises them straight into operand tiles, tcgen05 kernel
+ *   K-quants, T <= 16   Q8_K rows, integer-MMA kernels; up to 32 tokens so do products of less than 2 M weights, a few CTAs either way
+ *   K-quants, T > 16    the producer of the rows quantises them straight into operand tiles, tcgen05 kernel: no launch that makes tiles, and a chain of
+ *                       programmatic launches.  Whole prompts, us, with Q8_K rows up to 64 tokens / with tiles from 17 (everywhere / from 2 M or 8 M / from 12 M weights):
+ *                       896 wide, 24 layers, 32 tokens 1377 / 1363 / 1264 / 1320, 48 tokens 1603 / 1436;  4096 wide, 32 layers, 17 tokens 3700 / 3340, 48: 4160 / 3650
  *   Q5_0                row-planar Q8_0 rows, gemm_q80_mma.cu
  * q, k and v run on three streams: one of them alone leaves SMs idle (512 x 1024 x 4096 is 32 tiles) or ends in a part of a wave. */
 
@@ -798,7 +800,7 @@ size_t ckb_attn_behind_part_bytes(int head_dim);                                
 int ckb_launch_attn_behind(const float *q, const float *k, const float *v, float *out, int num_heads, int num_kv_heads, int num_tokens, int head_dim, int kv_stride_tokens,
                                    int before, float *part, void *stream);
 
-#define PF_SMALL 64            /* most tokens of the integer-MMA kernels */
+#define PF_SMALL 16            /* most tokens of which all products go to the integer-MMA kernels */
 
 static int tc_format(const Tensor *w) { return w->fmt == FMT_Q6K; }
 static const void *tc_weights(const Tensor *w) { return w->fmt == FMT_Q6K ? w->planar : w->w; }
@@ -808,6 +810,9 @@ typedef struct { int fmt, rows, cols, nt; } WidthMemo;
 static int tile_width(const Tensor *w, int T, WidthMemo *memo)
 {
     if (fmt_block32(w->fmt) || T <= PF_SMALL) return 0;
+    /* the rows will be aligned as weights are */
+    if (T <= 32 && (size_t)w->rows * w->cols < (size_t)2 << 20 &&
+        (w->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_takes(w->w, w->w, T, w->rows, w->cols) : ckb_gemm_q6k_mma_takes(w->planar, w->planar, T, w->rows, w->cols))) return 0;
     if (memo->fmt != w->fmt || memo->rows != w->rows || memo->cols != w->cols) {
         const WidthMemo now = { w->fmt, w->rows, w->cols, ckb_gemm_tc_width(tc_format(w), T, w->rows, w->cols) };
         *memo = now;

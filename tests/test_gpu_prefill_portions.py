@@ -64,6 +64,16 @@ def test_portion_matches_decode_steps(ck, cfg, before, T):
     assert cosine(got, want) >= 0.9999
 
 
+# products on both sides of 2 M weights, with a feed-forward width that the Q6_K integer kernel refuses
+WIDE = dict(LLAMA, intermediate_size=4352)
+
+
+@pytest.mark.parametrize("before,T", [(0, 17), (5, 32), (0, 33), (3, 64)])
+def test_portion_of_rows_and_tiles_matches_decode_steps(ck, before, T):
+    """From 17 tokens large products take operand tiles, up to 32 small ones rows: both in one pass, and k and v behind q."""
+    test_portion_matches_decode_steps(ck, WIDE, before, T)
+
+
 @pytest.mark.parametrize("tile", [64, 128])
 @pytest.mark.parametrize("m,n,k", [(16, 40, 128), (65, 130, 384), (200, 300, 896)])
 def test_q5_0_product_is_bit_identical(ck, orc, tile, m, n, k):
