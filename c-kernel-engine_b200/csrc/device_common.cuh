@@ -128,17 +128,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     return false;
 }
 // Same contract, for pipelines whose barriers are usually complete already: polls without sleeping and gives up
-// after about a second of SM clock cycles.  Few instructions: it stands in loops of warps that share an instruction cache.
+// after about a second of SM clock cycles.
 __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
-    uint32_t t0, t;
-    asm volatile("mov.u32 %0, %%clock;" : "=r"(t0));
+    const long long t0 = clock64();
+    for (;;) {
 #pragma unroll 1
-    do {
-        if (mbar_try_wait(bar, parity)) return true;
-        asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
-    } while (t - t0 < (1u << 31));
-    return false;
+        for (int i = 0; i < 256; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (clock64() - t0 > (1ll << 31)) return false;
+    }
 }
 // src and dst 16-byte aligned, bytes a multiple of 16.  No multicast: one CTA, its own shared memory.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t bar) {

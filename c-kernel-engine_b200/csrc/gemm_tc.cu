@@ -131,6 +131,19 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t chunk_b
     return d;
 }
 
+// mbar_wait_spin in fewer instructions: it stands in loops of warps that share an instruction cache.
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
+{
+    if (mbar_try_wait(bar, parity)) return true;
+    uint32_t t0, t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t0));
+#pragma unroll 1
+    do {
+        if (mbar_try_wait(bar, parity)) return true;
+        asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    } while (t - t0 < (1u << 31));
+    return false;
+}
 __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 // (a & mask) | bits in one instruction
@@ -394,7 +407,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
         else if constexpr ((n) > Cfg::REGS_LAUNCH) TC_SETMAXNREG("inc", n);      \
     } while (0)
 #define TC_WAIT(bar, parity, code)                                        \
-    if (!mbar_wait_spin(bar, parity)) { atomicExch(dev_err, code); break; }
+    if (!tc_wait(bar, parity)) { atomicExch(dev_err, code); break; }
 
     if (warp < 4) {
         TC_REGISTERS(Cfg::REGS_CTL);
@@ -411,13 +424,13 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
 #pragma unroll
                     for (uint32_t h = 0; h < PARTS; ++h, ++issued) {
                         const uint32_t i = issued % TC_BSLOTS;
-                        if (!mbar_wait_spin(BAR(Cfg::B_EMPTY + i), ((issued / TC_BSLOTS) & 1u) ^ 1u)) { go = false; break; }
+                        if (!tc_wait(BAR(Cfg::B_EMPTY + i), ((issued / TC_BSLOTS) & 1u) ^ 1u)) { go = false; break; }
                         if (tc_elect_one()) {
                             mbar_arrive_expect_tx(BAR(Cfg::B_FULL + i), Cfg::BSLOT);
                             bulk_g2s(s_base + Cfg::OFF_B + i * Cfg::BSLOT, blob + h * Cfg::BSLOT, Cfg::BSLOT, BAR(Cfg::B_FULL + i));
                         }
                     }
-                    if (!go || !mbar_wait_spin(BAR(Cfg::X_EMPTY + x), ((g / TC_XSLOTS) & 1u) ^ 1u)) { go = false; break; }
+                    if (!go || !tc_wait(BAR(Cfg::X_EMPTY + x), ((g / TC_XSLOTS) & 1u) ^ 1u)) { go = false; break; }
                     if (tc_elect_one()) {
                         mbar_arrive_expect_tx(BAR(Cfg::X_FULL + x), NT * 4 + (Q4 ? Cfg::AUX : 0));
                         bulk_g2s(s_base + Cfg::OFF_DX + x * NT * 4, blob + Cfg::XBLOB_DX, NT * 4, BAR(Cfg::X_FULL + x));
@@ -428,8 +441,8 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             }
             if (!go) atomicExch(dev_err, DEV_ERR_EMPTY_WAIT);
             // copies still in flight land before the CTA's shared memory goes away, whatever became of the roles that wait for them
-            for (uint32_t j = issued > TC_BSLOTS ? issued - TC_BSLOTS : 0; j < issued; ++j) mbar_wait_spin(BAR(Cfg::B_FULL + j % TC_BSLOTS), (j / TC_BSLOTS) & 1u);
-            for (uint32_t b = extras > TC_XSLOTS ? extras - TC_XSLOTS : 0; b < extras; ++b) mbar_wait_spin(BAR(Cfg::X_FULL + b % TC_XSLOTS), (b / TC_XSLOTS) & 1u);
+            for (uint32_t j = issued > TC_BSLOTS ? issued - TC_BSLOTS : 0; j < issued; ++j) tc_wait(BAR(Cfg::B_FULL + j % TC_BSLOTS), (j / TC_BSLOTS) & 1u);
+            for (uint32_t b = extras > TC_XSLOTS ? extras - TC_XSLOTS : 0; b < extras; ++b) tc_wait(BAR(Cfg::X_FULL + b % TC_XSLOTS), (b / TC_XSLOTS) & 1u);
         } else if (warp == 1) {
             // ------------------------------------------------------------ issuer: the warp runs the loop and the waits uniformly, one lane issues.  This
             // warp is a chain of short dependent steps that the MMAs of a 64-deep stage (64 to 260 cycles) have to cover: the stages of a superblock are unrolled
@@ -443,13 +456,13 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                 const uint32_t u = b & 1u, p = (b >> 1) & 1u, x [[maybe_unused]] = b % TC_XSLOTS;
                 const uint32_t a0 = Cfg::ADEEP == 2 ? 2 * u : 0, pa = Cfg::ADEEP == 2 ? p : u;
                 const uint32_t pb = Cfg::BDEEP == 4 ? (b >> 2) & 1u : p, b0 = Cfg::BDEEP == 4 ? b & 3u : 2 * u;
-                if (!mbar_wait_spin(BAR(Cfg::T_EMPTY + u), p ^ 1u)) { go = false; break; }
+                if (!tc_wait(BAR(Cfg::T_EMPTY + u), p ^ 1u)) { go = false; break; }
 #pragma unroll
                 for (uint32_t s = 0; s < 4; ++s) {
                     constexpr uint32_t half = Cfg::STAGE >> 4;
                     const uint32_t i = b0 + s / Cfg::BDEEP, a = a0 + s / Cfg::ADEEP;
-                    if (s % Cfg::BDEEP == 0 && !mbar_wait_spin(BAR(Cfg::B_FULL + i), pb)) { go = false; break; }
-                    if (s % Cfg::ADEEP == 0 && !mbar_wait_spin(BAR(Cfg::A_FULL + a), pa)) { go = false; break; }
+                    if (s % Cfg::BDEEP == 0 && !tc_wait(BAR(Cfg::B_FULL + i), pb)) { go = false; break; }
+                    if (s % Cfg::ADEEP == 0 && !tc_wait(BAR(Cfg::A_FULL + a), pa)) { go = false; break; }
                     tc_fence_after();                  // the expanders' stores, and (s = 0) the drain's loads of this accumulator, come before these MMAs
                     if (leader) {
                         uint32_t wide = 0;
@@ -472,7 +485,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                 }
                 if (!go) break;
                 if constexpr (Q4) {
-                    if ((!Cfg::T2_TWICE && !mbar_wait_spin(BAR(Cfg::T2_EMPTY), u ^ 1u)) || !mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
+                    if ((!Cfg::T2_TWICE && !tc_wait(BAR(Cfg::T2_EMPTY), u ^ 1u)) || !tc_wait(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
                     tc_fence_after();
                 }
                 if (leader) {
@@ -486,7 +499,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             }
             if (!go) atomicExch(dev_err, DEV_ERR_MMA_WAIT);
             if (leader) tc_commit(BAR(Cfg::DONE));          // MMAs in flight finish before the tensor memory is freed
-            mbar_wait_spin(BAR(Cfg::DONE), 0);
+            tc_wait(BAR(Cfg::DONE), 0);
         } else if (warp == 2) {
             // ------------------------------------------------------------ raw weights
             uint32_t issued = 0, r = 0, ph = 1;
@@ -494,7 +507,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             for (int u = work.begin + blockIdx.x; u < work.units && go; u += gridDim.x) {
                 const int n0 = work.nt(u) * TC_ROWS, kb0 = work.kb0(u), end = kb0 + work.nb(u);
                 for (int kb = kb0; kb < end; ++kb) {
-                    if (!mbar_wait_spin(BAR(Cfg::R_EMPTY + r), ph)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
+                    if (!tc_wait(BAR(Cfg::R_EMPTY + r), ph)) { atomicExch(dev_err, DEV_ERR_EMPTY_WAIT); go = false; break; }
                     if (tc_elect_one()) {
                         const uint32_t dst = s_base + Cfg::OFF_RAW + r * Cfg::RAW;
                         mbar_arrive_expect_tx(BAR(Cfg::R_FULL + r), Cfg::RAW);
@@ -510,7 +523,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                     if (++r == Cfg::RSLOTS) { r = 0; ph ^= 1u; }
                 }
             }
-            for (uint32_t b = issued > Cfg::RSLOTS ? issued - Cfg::RSLOTS : 0; b < issued; ++b) mbar_wait_spin(BAR(Cfg::R_FULL + b % Cfg::RSLOTS), (b / Cfg::RSLOTS) & 1u);
+            for (uint32_t b = issued > Cfg::RSLOTS ? issued - Cfg::RSLOTS : 0; b < issued; ++b) tc_wait(BAR(Cfg::R_FULL + b % Cfg::RSLOTS), (b / Cfg::RSLOTS) & 1u);
         }
     } else if (warp < 12) {
         // ------------------------------------------------------------ weight expanders: thread = row = TMEM lane.  A stage is stored while the next one is expanded: what
@@ -535,7 +548,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
             auto acquire = [&](int s) -> bool {
                 if (s % Cfg::ADEEP) return true;
                 if (s) publish(full + (uint32_t)(s / Cfg::ADEEP - 1));
-                if (!mbar_wait_spin(empty + 8u * (uint32_t)(s / Cfg::ADEEP), pa)) return false;
+                if (!tc_wait(empty + 8u * (uint32_t)(s / Cfg::ADEEP), pa)) return false;
                 tc_fence_after();
                 return true;
             };
@@ -593,7 +606,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                     if (hi % Cfg::ADEEP) return true;
                     if (stored >= 0) publish((uint32_t)stored);
                     stored = -1;
-                    if (!mbar_wait_spin(BAR(Cfg::A_EMPTY + (first + (uint32_t)hi) / Cfg::ADEEP), pa)) return false;
+                    if (!tc_wait(BAR(Cfg::A_EMPTY + (first + (uint32_t)hi) / Cfg::ADEEP), pa)) return false;
                     tc_fence_after();
                     return true;
                 };
@@ -610,7 +623,7 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                     } else {
                         // The issuer multiplies a slot of rests when any warp of the set has some, so a warp without leaves zeros in its rows, once.
                         // A slot of rests is free when the same stage of the superblock before this one has been multiplied.
-                        if (!acquire(hi) || (Cfg::ADEEP == 2 && b > 0 && !mbar_wait_spin(BAR(Cfg::A_EMPTY + ((k / 2) ^ 2u)), ((b - 1) >> 1) & 1u))) { go = false; break; }
+                        if (!acquire(hi) || (Cfg::ADEEP == 2 && b > 0 && !tc_wait(BAR(Cfg::A_EMPTY + ((k / 2) ^ 2u)), ((b - 1) >> 1) & 1u))) { go = false; break; }
                         tc_fence_after();
 #pragma unroll 1
                         for (int h = 0; h < 2; ++h) {
@@ -653,12 +666,12 @@ gemm_kq_tc_kernel(const __grid_constant__ TcMaps maps, const TcWork work, const 
                 const uint32_t buf = b & 1u, x = b % TC_XSLOTS;
                 uint32_t dd_bits = d_next;
                 if constexpr (!Q4) { if (kb + 1 < nb) d_next = ldg_nc_u16(d_plane + 2 * (size_t)(kb + 1)); }
-                if (!mbar_wait_spin(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
+                if (!tc_wait(BAR(Cfg::X_FULL + x), (b / TC_XSLOTS) & 1u)) { go = false; break; }
                 if constexpr (Q4) dd_bits = *reinterpret_cast<const uint32_t *>(smem + Cfg::OFF_DD + (x * TC_ROWS + row) * 4);
                 const float2 dd = __half22float2(bits_h2(dd_bits));
                 const uint64_t d2 = pack2f(dd.x, dd.x), m2 = pack2f(-dd.y, -dd.y);
                 const uint32_t dx = s_base + Cfg::OFF_DX + (x * NT + COLS * ch) * 4;
-                if (!mbar_wait_spin(BAR(Cfg::T_FULL + buf), (b >> 1) & 1u)) { go = false; break; }
+                if (!tc_wait(BAR(Cfg::T_FULL + buf), (b >> 1) & 1u)) { go = false; break; }
                 tc_fence_after();
                 const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(COLS * ch);
 #pragma unroll

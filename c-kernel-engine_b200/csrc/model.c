@@ -46,11 +46,13 @@ int ckb_model_init_shared(struct CKB200Model *m)
     return 0;
 }
 
-/* The driver copies to pageable memory through a buffer of its own, a memcpy behind the whole transfer (0.6 MB: 57 us).  Here the chunks of a pinned buffer are copied on as they
- * land (a token of a layer stack of 32768 words 473 -> 456 us).  Megabytes are bound by the memcpy either way (16 MB: 0.8 ms; four threads were no faster): the driver's way. */
+/* The driver copies to pageable memory through a buffer of its own, up to some hundred KB with the memcpy behind the whole transfer (608 KB: 57 us).  Here the chunks of a pinned
+ * buffer are copied on as they land: a step with 501 KB of logits 454 -> 448 us, with 608 KB 614 -> 605, with 131 KB 473 -> 456.  From 1 MB the driver does as much and is
+ * faster (1 MB 580 against 589, 4 MB 742 against 796): its way there. */
 int ckb_model_logits_out(struct CKB200Model *m, float *host, const float *dev, size_t bytes, cudaStream_t st, const char *what)
 {
-    enum { SMALLEST = 128 << 10, CHUNK = 192 << 10 };
+    enum { SMALLEST = 128 << 10 };
+    const size_t chunk = CKB_OUT_CHUNK;
     struct cudaPointerAttributes at;
     int pageable = 0;
     if (m->out_pinned && bytes >= SMALLEST && bytes <= (size_t)m->c.batch * m->c.vocab_size * sizeof(float)) {
@@ -61,8 +63,6 @@ int ckb_model_logits_out(struct CKB200Model *m, float *host, const float *dev, s
         if (ckb_check_cuda((int)cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st), "logits D2H")) return CKB_ERR_CUDA;
         return ckb_sync_check(st, what);
     }
-    size_t chunk = (bytes + CKB_OUT_CHUNKS - 1) / CKB_OUT_CHUNKS;
-    chunk = chunk < CHUNK ? CHUNK : (chunk + 4095) & ~(size_t)4095;
     for (size_t i = 0; i * chunk < bytes; ++i) {
         const size_t n = bytes - i * chunk < chunk ? bytes - i * chunk : chunk;
         if (ckb_check_cuda((int)cudaMemcpyAsync(m->out_pinned + i * chunk, (const uint8_t *)dev + i * chunk, n, cudaMemcpyDeviceToHost, st), "logits D2H") ||

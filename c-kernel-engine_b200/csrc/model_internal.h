@@ -24,7 +24,7 @@ typedef struct CkbModelFamily {
     size_t (*step_weight_bytes)(const CKB200Model *m);        /* weight bytes one step streams */
 } CkbModelFamily;
 
-enum { CKB_OUT_CHUNKS = 16, CKB_OUT_MOST = 4 << 20 };
+enum { CKB_OUT_CHUNKS = 4, CKB_OUT_CHUNK = 160 << 10, CKB_OUT_MOST = CKB_OUT_CHUNKS * CKB_OUT_CHUNK };
 
 struct CKB200Model {
     CKB200ModelConfig c;

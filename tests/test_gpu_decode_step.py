@@ -188,7 +188,7 @@ def test_fused_step_matches_the_launch_per_op_step(ck, orc, cfg, pdl):
 
 @pytest.mark.parametrize("vocab,batch", [(300, 1), (32768, 1), (49153, 1), (151937, 1), (151937, 6), (140001, 8)])
 def test_logits_come_back_the_same_to_any_memory(ck, vocab, batch):
-    """To pageable memory in chunks over pinned memory (128 KB to 4 MB), else directly: the same bytes, at any offset, nothing beside them."""
+    """To pageable memory in chunks over pinned memory (128 to 640 KB), else directly: the same bytes, at any offset, nothing beside them."""
     import torch
 
     so.bind_model_api(ck)
