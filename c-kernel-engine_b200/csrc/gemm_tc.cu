@@ -1047,7 +1047,7 @@ extern "C" int ckb200_dev_gemm_nt_q6_k_planar_q8_k(const void *A_q8, const void 
 {
     if (!A_q8 || !B_planar || !C || M <= 0 || N <= 0 || K <= 0) return 0;
     if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
-    int rc = ckb_launch_gemm_q6k_mma(A_q8, B_planar, bias, C, N, M, N, K, stream);        // 4 to 64 tokens: integer MMA over the planes (gemm_q6k_mma.cu)
+    int rc = ckb_launch_gemm_q6k_mma(A_q8, B_planar, bias, C, N, M, N, K, stream);        // up to 16 tokens, small products to 64: integer MMA over the planes (gemm_q6k_mma.cu)
     if (rc >= 0) return rc;
     rc = ckb_launch_gemm_tc(TC_W_Q6K_PLANAR, A_q8, B_planar, bias, C, N, M, N, K, ckb_tune_get("gemm_tc_min_tokens", 16), stream);
     if (rc >= 0) return rc;
