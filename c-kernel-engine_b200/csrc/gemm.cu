@@ -28,12 +28,20 @@ static int gemm_nt_by_rows(gemv_fn fn, size_t a_row_bytes, const void *A_q8, con
     return bias ? ckb200_dev_add_bias_rows(C, bias, M, N, stream) : 0;
 }
 
-// Up to 16 tokens, and up to 64 where the product is small: the integer-MMA kernel that streams the weights through registers (gemm_q4k_mma.cu); above that the tcgen05 kernel.
+// Up to 64 tokens: the integer-MMA kernel that streams the weights through registers (gemm_q4k_mma.cu); above that the tcgen05 kernel, and from 17 tokens up where
+// it is faster and the library has a workspace in order with the call (ckb_launch_gemm_tc_own).
+extern "C" int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, int N, int K);
+extern "C" int ckb_gemm_q4k_mma_best(const void *A_q8, const void *B, int M, int N, int K);
+extern "C" int ckb_launch_gemm_tc_own(int wf, const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream);
 extern "C" int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);
 extern "C" int ckb200_dev_gemm_nt_q4_k_q8_k(const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)
 {
     if (A_q8 && B && C && M > 0 && N > 0 && K > 0) {
-        int rc = ckb_launch_gemm_q4k_mma(A_q8, B, bias, C, N, M, N, K, stream);
+        int rc = -1;
+        if (ckb_gemm_q4k_mma_takes(A_q8, B, M, N, K)) {
+            if (!ckb_gemm_q4k_mma_best(A_q8, B, M, N, K)) rc = ckb_launch_gemm_tc_own(0, A_q8, B, bias, C, M, N, K, stream);
+            if (rc < 0) rc = ckb_launch_gemm_q4k_mma(A_q8, B, bias, C, N, M, N, K, stream);
+        }
         if (rc >= 0) return rc;
         rc = ckb_launch_gemm_q4k_tc(A_q8, B, bias, C, M, N, K, stream);
         if (rc >= 0) return rc;
@@ -42,7 +50,8 @@ extern "C" int ckb200_dev_gemm_nt_q4_k_q8_k(const void *A_q8, const void *B, con
 }
 // From 16 tokens up the reference's 210-byte rows are re-laid row-planar into the library's scratch (one pass over B, a few
 // microseconds against the product itself) and the tensor-core kernel runs over that copy; the scratch belongs to the library's
-// pool, so a caller that records its launches in a CUDA graph keeps its own planar copy and calls ckb200_dev_gemm_nt_q6_k_planar_q8_k.
+// pool, so a caller that records its launches in a CUDA graph keeps its own planar copy and calls ckb200_dev_gemm_nt_q6_k_planar_q8_k (up to 64 tokens: above
+// that its operand tiles are in that pool too).
 extern "C" size_t ckb200_q6_k_planar_bytes(int rows, int cols);
 extern "C" int ckb200_dev_q6_k_to_planar(void *dst, const void *src, int rows, int cols, void *stream);
 extern "C" int ckb200_dev_gemm_nt_q6_k_planar_q8_k(const void *A_q8, const void *B_planar, const float *bias, float *C, int M, int N, int K, void *stream);

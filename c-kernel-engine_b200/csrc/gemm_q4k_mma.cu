@@ -612,17 +612,20 @@ using namespace ckb;
 // Returns -1 when this kernel does not take the call (token count, alignment, switched off): the caller falls through to its other paths.
 // Whether the launcher below takes this product (a caller that wants to run several products side by side asks first: this
 // kernel needs no workspace, the tcgen05 kernel shares one).
-extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
 extern "C" int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, int N, int K)
 {
     if (!A_q8 || !B || N <= 0 || K <= 0 || K % QK_K) return 0;
     // from 2 tokens up one pass of this kernel beats a GEMV per token (measured: up to 8 tokens cost about 1.2 GEMVs on the 57344 x 8192 shape)
     if (M < ckb_tune_get("gemm_q4k_mma_min", 2) || M > ckb_tune_get("gemm_q4k_mma_max", 64) || M > 64 || !ckb_tune_get("gemm_q4k_mma", 1)) return 0;
-    if (((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3)) return 0;
-    // From 17 tokens up this kernel is bound by its integer instructions, 0.23 and (33 to 64 tokens) 0.39 us per million weights, and the tcgen05 kernel by the
-    // expansion of the weights, which does not grow with the tokens: large products go there (57344 x 8192: 109 against 82 us at 32 tokens, 185 against 110 at
-    // 64; 8192 x 8192 at 32: 18.6 against 21).
-    return M <= 16 || !ckb_gemm_tc_beats(0, M, N, K, 2.0 + (M <= 32 ? 2.32e-7 : 3.94e-7) * N * K);
+    return !(((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3));
+}
+// Whether it is also the faster one, for a caller that has a workspace for the tcgen05 kernel.  From 17 tokens up this kernel is bound by its integer
+// instructions, 0.23 and (33 to 64 tokens) 0.39 us per million weights, and the tcgen05 kernel by the expansion of the weights, which does not grow with the
+// tokens: large products go there (57344 x 8192: 109 against 82 us at 32 tokens, 185 against 110 at 64; 8192 x 8192 at 32: 18.6 against 21).
+extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
+extern "C" int ckb_gemm_q4k_mma_best(const void *A_q8, const void *B, int M, int N, int K)
+{
+    return ckb_gemm_q4k_mma_takes(A_q8, B, M, N, K) && (M <= 16 || !ckb_gemm_tc_beats(0, M, N, K, 2.0 + (M <= 32 ? 2.32e-7 : 3.94e-7) * N * K));
 }
 
 extern "C" int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, void *stream)

@@ -395,14 +395,18 @@ using namespace ckb;
 
 // B_planar: ckb200_q6_k_planar_bytes(N, K) of row-planar Q6_K weights.  Returns -1 when this kernel does not take the call.
 // Whether the launcher below takes this product (for a caller that runs several products side by side: no workspace here).
-extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
 extern "C" int ckb_gemm_q6k_mma_takes(const void *A_q8, const void *B_planar, int M, int N, int K)
 {
     if (!A_q8 || !B_planar || N <= 0 || K <= 0 || K % 1024) return 0;
     if (M < ckb_tune_get("gemm_q6k_mma_min", 2) || M > ckb_tune_get("gemm_q6k_mma_max", 64) || M > 64 || !ckb_tune_get("gemm_q6k_mma", 1)) return 0;
-    if (((uintptr_t)B_planar & 15) || ((uintptr_t)A_q8 & 15)) return 0;
-    // from 17 tokens up as for Q4_K: 0.36 and 0.68 us per million weights here (8192 x 28672: 84 against 62 us at 32 tokens, 159 against 90 at 64)
-    return M <= 16 || !ckb_gemm_tc_beats(1, M, N, K, 2.0 + (M <= 32 ? 3.58e-7 : 6.77e-7) * N * K);
+    return !(((uintptr_t)B_planar & 15) || ((uintptr_t)A_q8 & 15));
+}
+// Whether it is also the faster one, from 17 tokens up as for Q4_K: 0.36 and 0.68 us per million weights here (8192 x 28672: 84 against 62 us at 32 tokens, 159
+// against 90 at 64)
+extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
+extern "C" int ckb_gemm_q6k_mma_best(const void *A_q8, const void *B_planar, int M, int N, int K)
+{
+    return ckb_gemm_q6k_mma_takes(A_q8, B_planar, M, N, K) && (M <= 16 || !ckb_gemm_tc_beats(1, M, N, K, 2.0 + (M <= 32 ? 3.58e-7 : 6.77e-7) * N * K));
 }
 
 extern "C" int ckb_launch_gemm_q6k_mma(const void *A_q8, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, void *stream)

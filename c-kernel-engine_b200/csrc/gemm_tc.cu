@@ -47,6 +47,7 @@
 //   57344 x 8192 Q4_K:  32 tokens 111 -> 76, 64: 222 -> 88;  8192 x 28672 Q6_K: 76 -> 62, 126 -> 72;  128256 x 8192 Q6_K at 32: 213 (4.05 TB/s of weights)
 // (with the operand through shared memory 28672 x 4096 at 512 tokens took 268).
 #include <cuda.h>
+#include <pthread.h>
 
 #include "q8k_block.cuh"
 #include "quant_units.cuh"
@@ -989,25 +990,58 @@ extern "C" int ckb_launch_gemm_tc_pair(const void *tiles, int nt, const void *B,
     return tc_launch(TC_W_Q4K, nt, (const uint8_t *)tiles, B, TcSecond{B2, N}, nullptr, C, ldc, M, N + N2, K / QK_K, tc_plan(TC_W_Q4K, nt, M, N + N2, K / QK_K), nullptr, 0, ckb_stream(stream));
 }
 
+// What a product from Q8_K rows needs: the operand tiles, and behind them the partial sums.
+struct TcRows { int nt; TcPlan plan; size_t xt_bytes, part_bytes; };
+static TcRows tc_rows(int wf, int M, int N, int K)
+{
+    TcRows r;
+    r.nt = tc_width(wf, M, N, K / QK_K);
+    r.plan = tc_plan(wf, r.nt, M, N, K / QK_K);
+    r.xt_bytes = (ckb_gemm_tc_tile_bytes(r.nt, M, K) + 255) & ~(size_t)255;
+    r.part_bytes = tc_part_bytes(r.plan, M, N);
+    return r;
+}
+static int tc_launch_rows(int wf, const TcRows &r, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, uint8_t *ws, cudaStream_t st)
+{
+    if (int rc = tc_make_tiles(A_q8, ws, r.nt, M, K / QK_K, st)) return rc;
+    return tc_launch(wf, r.nt, ws, B, TcSecond{nullptr, 0}, bias, C, ldc, M, N, K / QK_K, r.plan, reinterpret_cast<float *>(ws + r.xt_bytes), r.part_bytes, st);
+}
+static bool tc_takes_rows(const void *A_q8, const void *B, int M, int K, int min_tokens)
+{
+    return !(M < min_tokens || K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3) || ckb_tune_get("gemm_tc", 1) == 0);
+}
+
 // C[m * ldc + n] = A_q8[m] . W[n] (+ bias[n]).  wf: TC_W_Q4K (the reference's block_q4_K rows) or TC_W_Q6K_PLANAR.
 // Returns -1 when the shape is not handled here (caller falls back to the per-token path).  min_tokens: smallest M
 // worth the tensor-core path (tokens past M are zeros).
 extern "C" int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,
                                      void *ws, size_t ws_bytes, void *stream)
 {
-    if (M < min_tokens || K % QK_K || ((uintptr_t)B & 15) || ((uintptr_t)A_q8 & 3) || ((uintptr_t)ws & 255) || ckb_tune_get("gemm_tc", 1) == 0) return -1;
-    const int nb = K / QK_K, nt = tc_width(wf, M, N, nb);
-    const TcPlan plan = tc_plan(wf, nt, M, N, nb);
-    const size_t xt_bytes = (ckb_gemm_tc_tile_bytes(nt, M, K) + 255) & ~(size_t)255, part_bytes = tc_part_bytes(plan, M, N);
+    if (!tc_takes_rows(A_q8, B, M, K, min_tokens) || ((uintptr_t)ws & 255)) return -1;
+    const TcRows r = tc_rows(wf, M, N, K);
     // A caller that records the launch in a CUDA graph brings its own workspace: the library's pool may be freed and
     // regrown by any later call that needs more, which would leave a captured pointer dangling.
-    if (ws && xt_bytes + part_bytes > ws_bytes)
-        return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the caller's workspace holds %zu bytes, this call needs %zu", ws_bytes, xt_bytes + part_bytes);
-    uint8_t *xt = ws ? (uint8_t *)ws : (uint8_t *)ckb_scratch(CKB_SLOT_G, xt_bytes + part_bytes);
+    if (ws && r.xt_bytes + r.part_bytes > ws_bytes)
+        return ckb_fail(CKB_ERR_LIMIT, "gemm_kq_tc: the caller's workspace holds %zu bytes, this call needs %zu", ws_bytes, r.xt_bytes + r.part_bytes);
+    uint8_t *xt = ws ? (uint8_t *)ws : (uint8_t *)ckb_scratch(CKB_SLOT_G, r.xt_bytes + r.part_bytes);
     if (!xt) return CKB_ERR_CUDA;
-    cudaStream_t st = ckb_stream(stream);
-    if (int rc = tc_make_tiles(A_q8, xt, nt, M, nb, st)) return rc;
-    return tc_launch(wf, nt, xt, B, TcSecond{nullptr, 0}, bias, C, ldc, M, N, nb, plan, reinterpret_cast<float *>(xt + xt_bytes), part_bytes, st);
+    return tc_launch_rows(wf, r, A_q8, B, bias, C, ldc, M, N, K, xt, ckb_stream(stream));
+}
+
+// The same for a product that needs no workspace elsewhere (the integer-MMA kernels take it), whose callers therefore use any stream and thread, record it in graphs
+// and call it on a full device.  It comes here where none of that matters: on the library's own stream, outside a capture, over a workspace that no call on another
+// stream touches, all launches of a call behind one another whichever thread makes them.  -1: elsewhere, or no room.
+extern "C" int ckb_launch_gemm_tc_own(int wf, const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)
+{
+    static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;
+    if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
+    if (!ckb_on_own_stream(stream) || !tc_takes_rows(A_q8, B, M, K, 0)) return -1;
+    const TcRows r = tc_rows(wf, M, N, K);
+    pthread_mutex_lock(&lock);
+    uint8_t *ws = (uint8_t *)ckb_scratch_if_room(CKB_SLOT_O, r.xt_bytes + r.part_bytes);
+    const int rc = ws ? tc_launch_rows(wf, r, A_q8, B, bias, C, N, M, N, K, ws, ckb_stream(stream)) : -1;
+    pthread_mutex_unlock(&lock);
+    return rc;
 }
 
 extern "C" int ckb_launch_gemm_tc(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens,
@@ -1043,11 +1077,17 @@ extern "C" int ckb_launch_gemm_q4k_tc(const void *A_q8, const void *B, const flo
 extern "C" int ckb200_dev_gemv_q6_k_planar_q8_k(float *, const void *, const void *, int, int, void *);
 extern "C" int ckb200_dev_add_bias_rows(float *, const float *, int, int, void *);
 extern "C" int ckb_launch_gemm_q6k_mma(const void *A_q8, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);
+extern "C" int ckb_gemm_q6k_mma_takes(const void *A_q8, const void *B_planar, int M, int N, int K);
+extern "C" int ckb_gemm_q6k_mma_best(const void *A_q8, const void *B_planar, int M, int N, int K);
 extern "C" int ckb200_dev_gemm_nt_q6_k_planar_q8_k(const void *A_q8, const void *B_planar, const float *bias, float *C, int M, int N, int K, void *stream)
 {
     if (!A_q8 || !B_planar || !C || M <= 0 || N <= 0 || K <= 0) return 0;
     if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
-    int rc = ckb_launch_gemm_q6k_mma(A_q8, B_planar, bias, C, N, M, N, K, stream);        // up to 16 tokens, small products to 64: integer MMA over the planes (gemm_q6k_mma.cu)
+    int rc = -1;
+    if (ckb_gemm_q6k_mma_takes(A_q8, B_planar, M, N, K)) {                                // up to 64 tokens: integer MMA over the planes (gemm_q6k_mma.cu), or as for Q4_K
+        if (!ckb_gemm_q6k_mma_best(A_q8, B_planar, M, N, K)) rc = ckb_launch_gemm_tc_own(TC_W_Q6K_PLANAR, A_q8, B_planar, bias, C, M, N, K, stream);
+        if (rc < 0) rc = ckb_launch_gemm_q6k_mma(A_q8, B_planar, bias, C, N, M, N, K, stream);
+    }
     if (rc >= 0) return rc;
     rc = ckb_launch_gemm_tc(TC_W_Q6K_PLANAR, A_q8, B_planar, bias, C, N, M, N, K, ckb_tune_get("gemm_tc_min_tokens", 16), stream);
     if (rc >= 0) return rc;

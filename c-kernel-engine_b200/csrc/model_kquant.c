@@ -47,6 +47,8 @@ size_t ckb_gemm_tc_workspace_bytes(int M, int N, int K);
 int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);
 int ckb_launch_gemm_q6k_mma(const void *A_q8, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);   /* gemm_q6k_mma.cu */
 int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, int N, int K);
+int ckb_gemm_q4k_mma_best(const void *A_q8, const void *B, int M, int N, int K);       /* and the tcgen05 kernel is not faster */
+int ckb_gemm_q6k_mma_best(const void *A_q8, const void *B_planar, int M, int N, int K);
 int ckb_gemm_q6k_mma_takes(const void *A_q8, const void *B_planar, int M, int N, int K);
 
 /* From this many sequences a projection runs as one batched product instead of a GEMV per sequence.  The tcgen05 kernel's time
@@ -483,8 +485,8 @@ static int matvec_standalone(const KqModel *m, const Tensor *w, const uint8_t *x
 {
     const int B = m->c.batch;
     if (B < MODEL_GEMM_MIN_BATCH) return 1;
-    if (w->fmt == FMT_Q4K) return ckb_gemm_q4k_mma_takes(xq, w->w, B, w->rows, w->cols);
-    if (w->fmt == FMT_Q6K && w->planar) return ckb_gemm_q6k_mma_takes(xq, w->planar, B, w->rows, w->cols);
+    if (w->fmt == FMT_Q4K) return ckb_gemm_q4k_mma_best(xq, w->w, B, w->rows, w->cols);
+    if (w->fmt == FMT_Q6K && w->planar) return ckb_gemm_q6k_mma_best(xq, w->planar, B, w->rows, w->cols);
     return 0;
 }
 
@@ -493,11 +495,11 @@ static int matvec(KqModel *m, const Tensor *w, const uint8_t *xq, float *y, int 
 {
     /* batched decode: the weights are streamed once for all sequences, by the integer-MMA kernels (no workspace) or, where those leave a product of 17 sequences
      * and more to it, by the tcgen05 kernel */
-    if (w->fmt == FMT_Q4K && m->c.batch > 1) {
+    if (w->fmt == FMT_Q4K && m->c.batch > 1 && ckb_gemm_q4k_mma_best(xq, w->w, m->c.batch, w->rows, w->cols)) {
         const int rc = ckb_launch_gemm_q4k_mma(xq, w->w, NULL, y, y_stride, m->c.batch, w->rows, w->cols, st);
         if (rc >= 0) return rc;
     }
-    if (w->fmt == FMT_Q6K && w->planar && m->c.batch > 1) {
+    if (w->fmt == FMT_Q6K && w->planar && m->c.batch > 1 && ckb_gemm_q6k_mma_best(xq, w->planar, m->c.batch, w->rows, w->cols)) {
         const int rc = ckb_launch_gemm_q6k_mma(xq, w->planar, NULL, y, y_stride, m->c.batch, w->rows, w->cols, st);
         if (rc >= 0) return rc;
     }
@@ -812,7 +814,7 @@ static int tile_width(const Tensor *w, int T, WidthMemo *memo)
     if (fmt_block32(w->fmt) || T <= PF_SMALL) return 0;
     /* the rows will be aligned as weights are */
     if (T <= 32 && (size_t)w->rows * w->cols < (size_t)2 << 20 &&
-        (w->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_takes(w->w, w->w, T, w->rows, w->cols) : ckb_gemm_q6k_mma_takes(w->planar, w->planar, T, w->rows, w->cols))) return 0;
+        (w->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_best(w->w, w->w, T, w->rows, w->cols) : ckb_gemm_q6k_mma_best(w->planar, w->planar, T, w->rows, w->cols))) return 0;
     if (memo->fmt != w->fmt || memo->rows != w->rows || memo->cols != w->cols) {
         const WidthMemo now = { w->fmt, w->rows, w->cols, ckb_gemm_tc_width(tc_format(w), T, w->rows, w->cols) };
         *memo = now;

@@ -138,6 +138,13 @@ int ckb_sm_count(void) { return g.sm_count > 0 ? g.sm_count : 148; }
 int *ckb_device_error_word(void) { return g.dev_err; }
 void *ckb200_stream(void) { return ckb_ensure_init() ? NULL : (void *)g.stream; }
 cudaStream_t ckb_stream(void *user) { return user ? (cudaStream_t)user : g.stream; }
+int ckb_on_own_stream(void *user)
+{
+    enum cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (ckb_stream(user) != g.stream) return 0;
+    if (cudaStreamIsCapturing(g.stream, &status) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return status == cudaStreamCaptureStatusNone;
+}
 
 /* Synchronises `st` and folds in the device error word: kernels that gave up on a bounded wait (a peer that never wrote,
  * a copy that never landed) leave a code there and return, so without this check the caller would get rc 0 and a result
@@ -349,7 +356,7 @@ void ckb200_host_free(void *p)
 
 static struct { uint8_t *p; size_t cap; } g_slot[CKB_NSLOTS];
 
-void *ckb_scratch(int slot, size_t bytes)
+static void *scratch(int slot, size_t bytes, int room_is_optional)
 {
     if (bytes <= g_slot[slot].cap) return g_slot[slot].p;
     if (g_slot[slot].p) {
@@ -359,9 +366,26 @@ void *ckb_scratch(int slot, size_t bytes)
         g_slot[slot].cap = 0;
     }
     size_t cap = (bytes + 256 + ((size_t)1 << 20) - 1) & ~(((size_t)1 << 20) - 1);
-    if (ckb_check_cuda((int)cudaMalloc((void **)&g_slot[slot].p, cap), "cudaMalloc(staging)")) return NULL;
+    const cudaError_t e = cudaMalloc((void **)&g_slot[slot].p, cap);
+    if (e != cudaSuccess) {
+        g_slot[slot].p = NULL;
+        if (room_is_optional && e == cudaErrorMemoryAllocation) cudaGetLastError();
+        else ckb_check_cuda((int)e, "cudaMalloc(staging)");
+        return NULL;
+    }
     g_slot[slot].cap = cap;
     return g_slot[slot].p;
+}
+void *ckb_scratch(int slot, size_t bytes) { return scratch(slot, bytes, 0); }
+/* Also beside a capture that another stream is under, which forbids allocations to every thread that has not said that it is no part of it. */
+void *ckb_scratch_if_room(int slot, size_t bytes)
+{
+    enum cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (bytes <= g_slot[slot].cap) return g_slot[slot].p;
+    if (ckb_check_cuda((int)cudaThreadExchangeStreamCaptureMode(&mode), "capture mode")) return NULL;
+    void *p = scratch(slot, bytes, 1);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return p;
 }
 
 int ckb_is_device_ptr(const void *p)

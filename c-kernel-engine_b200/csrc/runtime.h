@@ -9,12 +9,13 @@
 extern "C" {
 #endif
 
-enum { CKB_SLOT_W = 0, CKB_SLOT_X = 1, CKB_SLOT_Y = 2, CKB_SLOT_A = 3, CKB_SLOT_B = 4, CKB_SLOT_C = 5, CKB_SLOT_T = 6, CKB_SLOT_G = 7, CKB_SLOT_P = 8, CKB_SLOT_S = 9, CKB_NSLOTS = 10 };
+enum { CKB_SLOT_W = 0, CKB_SLOT_X = 1, CKB_SLOT_Y = 2, CKB_SLOT_A = 3, CKB_SLOT_B = 4, CKB_SLOT_C = 5, CKB_SLOT_T = 6, CKB_SLOT_G = 7, CKB_SLOT_P = 8, CKB_SLOT_S = 9, CKB_SLOT_O = 10, CKB_NSLOTS = 11 };
 
 int ckb_ensure_init(void);                 /* 0 or CKB_ERR_NO_DEVICE; initialises on first use */
 int ckb_sm_count(void);
 int *ckb_device_error_word(void);
 cudaStream_t ckb_stream(void *user);       /* user stream, or the library stream when NULL */
+int ckb_on_own_stream(void *user);         /* that is the library stream, and no capture is running on it */
 int ckb_tune_get(const char *key, int dflt);
 int ckb_is_device_ptr(const void *p);      /* device or managed memory */
 int ckb_sync_check(cudaStream_t st, const char *what);   /* sync + device error word -> 0, CKB_ERR_CUDA or CKB_ERR_DEVICE_WAIT */
@@ -28,6 +29,7 @@ const void *ckb_planar_shadow(int fmt, const void *dev_raw, int rows, int cols);
 
 /* Device scratch that grows on demand (never shrinks); one buffer per slot. */
 void *ckb_scratch(int slot, size_t bytes);
+void *ckb_scratch_if_room(int slot, size_t bytes);        /* NULL without an error when there is no room */
 /* Input staging: resident copy if registered (try_registry), the pointer itself if it is device
  * memory, else an async H2D copy into the slot.  NULL on failure. */
 const void *ckb_stage_in(const void *host, size_t bytes, int slot, int try_registry);
