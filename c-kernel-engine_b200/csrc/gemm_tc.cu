@@ -961,7 +961,7 @@ static int tc_width(int wf, int M, int N, int nb)
 // Whether this kernel takes a product from Q8_K rows in less time than an integer-MMA kernel that needs other_us; 3 us for the launch that makes operand tiles.
 extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us)
 {
-    if (ckb_tune_get("gemm_tc", 1) == 0) return 0;
+    if (ckb_tune_get("gemm_tc", 1) == 0 || M < ckb_tune_get("gemm_tc_min_tokens", 16)) return 0;
     return tc_plan(wf, tc_width(wf, M, N, K / QK_K), M, N, K / QK_K).us + 3.0 < other_us;
 }
 

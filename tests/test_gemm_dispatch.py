@@ -25,6 +25,19 @@ def test_integer_kernels_take_products_that_are_faster_elsewhere(pkg, fmt, m):
     assert takes(ALIGNED, ALIGNED, m, 512, 1024) == 1 and best(ALIGNED, ALIGNED, m, 512, 1024) == 1
 
 
+@pytest.mark.parametrize("fmt", ["q4k", "q6k"])
+def test_fewest_tokens_of_the_tcgen05_kernel(pkg, fmt):
+    """A product that tune gemm_tc_min_tokens keeps from the tcgen05 kernel stays with the integer kernel."""
+    lib = pkg.load_lib()
+    best = getattr(lib, f"ckb_gemm_{fmt}_mma_best")
+    try:
+        lib.ckb200_tune_set(b"gemm_tc_min_tokens", 33)
+        assert [best(ALIGNED, ALIGNED, m, N, K) for m in (17, 32, 33, 64)] == [1, 1, 0, 0]
+    finally:
+        lib.ckb200_tune_set(b"gemm_tc_min_tokens", 16)
+    assert best(ALIGNED, ALIGNED, 32, N, K) == 0
+
+
 class Product:
     """Resident weights, rows of activations, and the device entry over them."""
 
@@ -155,6 +168,25 @@ def test_product_in_a_graph(ck, orc, fmt, own):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(p.c, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
+def test_fewest_tokens_of_the_entry_points(ck, orc, fmt):
+    """With gemm_tc_min_tokens above the call's tokens: the integer kernel in one launch or two, not a GEMV per token."""
+    import torch
+
+    p = Product(ck, orc, fmt, 32)
+    try:
+        ck.ckb200_tune_set(b"gemm_tc", 0)
+        want = p.alone()
+        ck.ckb200_tune_set(b"gemm_tc", 1)
+        ck.ckb200_tune_set(b"gemm_tc_min_tokens", 65)
+        count, got = launches(ck, p.alone)
+    finally:
+        ck.ckb200_tune_set(b"gemm_tc", 1)
+        ck.ckb200_tune_set(b"gemm_tc_min_tokens", 16)
+    assert count <= 2 and torch.equal(got, want)
 
 
 @pytest.mark.gpu
