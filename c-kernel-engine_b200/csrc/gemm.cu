@@ -37,6 +37,7 @@ extern "C" int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const fl
 extern "C" int ckb200_dev_gemm_nt_q4_k_q8_k(const void *A_q8, const void *B, const float *bias, float *C, int M, int N, int K, void *stream)
 {
     if (A_q8 && B && C && M > 0 && N > 0 && K > 0) {
+        if (ckb_ensure_init()) return CKB_ERR_NO_DEVICE;
         int rc = -1;
         if (ckb_gemm_q4k_mma_takes(A_q8, B, M, N, K)) {
             if (!ckb_gemm_q4k_mma_best(A_q8, B, M, N, K)) rc = ckb_launch_gemm_tc_own(0, A_q8, B, bias, C, M, N, K, stream);

@@ -38,6 +38,21 @@ def test_fewest_tokens_of_the_tcgen05_kernel(pkg, fmt):
     assert best(ALIGNED, ALIGNED, 32, N, K) == 0
 
 
+@pytest.mark.parametrize("name", ["ckb200_dev_gemm_nt_q4_k_q8_k", "ckb200_dev_gemm_nt_q6_k_planar_q8_k"])
+@pytest.mark.parametrize("m", [16, 32, 64, 65, 200])
+def test_first_call_initialises(pkg, name, m):
+    """Whichever kernel takes it, a product comes behind the library's initialisation (its stream, the error word of the waits): without a device it ends there."""
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("needs a machine without a GPU")
+    lib = pkg.load_lib()
+    try:
+        assert getattr(lib, name)(ALIGNED, ALIGNED, None, ALIGNED, m, N, K, None) == 4          # CKB_ERR_NO_DEVICE
+    finally:
+        lib.ckb200_clear_error()
+
+
 class Product:
     """Resident weights, rows of activations, and the device entry over them."""
 
