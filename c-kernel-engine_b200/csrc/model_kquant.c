@@ -806,13 +806,21 @@ int ckb_launch_attn_behind(const float *q, const float *k, const float *v, float
 
 static int tc_format(const Tensor *w) { return w->fmt == FMT_Q6K; }
 static const void *tc_weights(const Tensor *w) { return w->fmt == FMT_Q6K ? w->planar : w->w; }
-/* Whether T tokens go through operand tiles for this consumer (0: no), and how wide those are.  Layers mostly repeat the same shapes: `memo` holds the
- * last answer for this kind of consumer during one pass. */
+/* whether the integer-MMA kernels take T rows for these n matrices (the rows will be aligned as weights are) */
+static int integer_takes(const Tensor *w, int n, int T)
+{
+    int all = 1;
+    for (int i = 0; i < n; ++i)
+        all &= w[i].fmt == FMT_Q4K ? ckb_gemm_q4k_mma_takes(w[i].w, w[i].w, T, w[i].rows, w[i].cols) : ckb_gemm_q6k_mma_takes(w[i].planar, w[i].planar, T, w[i].rows, w[i].cols);
+    return all;
+}
+/* Whether T tokens go through operand tiles for these consumers, n matrices of one set of rows (0: no), and how wide those are.  Layers mostly repeat the same shapes:
+ * `memo` holds the last answer for this kind of consumer during one pass. */
 typedef struct { int fmt, rows, cols, nt; } WidthMemo;
-static int tile_width(const Tensor *w, int T, WidthMemo *memo)
+static int tile_width(const Tensor *w, int n, int T, WidthMemo *memo)
 {
     if (fmt_block32(w->fmt) || T <= PF_SMALL) return 0;
-    /* the rows will be aligned as weights are */
+    if (!ckb_tune_get("gemm_tc", 1) && integer_takes(w, n, T)) return 0;
     if (T <= 32 && (size_t)w->rows * w->cols < (size_t)2 << 20 &&
         (w->fmt == FMT_Q4K ? ckb_gemm_q4k_mma_best(w->w, w->w, T, w->rows, w->cols) : ckb_gemm_q6k_mma_best(w->planar, w->planar, T, w->rows, w->cols))) return 0;
     if (memo->fmt != w->fmt || memo->rows != w->rows || memo->cols != w->cols) {
@@ -859,7 +867,7 @@ static int prefill_buffers(KqModel *m, int T)
                                              { CKB_T_WO, CKB_T_WO, PF_PART0 }, { CKB_T_W1, CKB_T_W1, PF_PART0 }, { CKB_T_W2, CKB_T_W2, PF_PART0 } };
             for (int i = 0; i < 6; ++i) {
                 const Tensor *p = &w[which[i][0]];
-                const int nt = tile_width(&w[which[i][1]], T, &memo[which[i][1]]);
+                const int nt = tile_width(&w[which[i][1]], which[i][1] == CKB_T_WQ ? 3 : 1, T, &memo[which[i][1]]);
                 const size_t b = nt ? ckb_gemm_tc_part_bytes(tc_format(p), nt, T, p->rows, p->cols) : 0;
                 if (b > need[which[i][2]]) need[which[i][2]] = b;
             }
@@ -970,8 +978,8 @@ static int issue_prefill(KqModel *m, int T, void *st)
     for (int l = 0; l < L; ++l) {
         Tensor *t = m->layers[l].t;
         float *kc = (float *)kv_at(m, l, 0), *vc = (float *)kv_at(m, l, 1);
-        const int nt_q = tile_width(&t[CKB_T_WQ], T, &memo[0]), nt_o = tile_width(&t[CKB_T_WO], T, &memo[1]), nt_1 = tile_width(&t[CKB_T_W1], T, &memo[2]),
-                  nt_2 = tile_width(&t[CKB_T_W2], T, &memo[3]);
+        const int nt_q = tile_width(&t[CKB_T_WQ], 3, T, &memo[0]), nt_o = tile_width(&t[CKB_T_WO], 1, T, &memo[1]), nt_1 = tile_width(&t[CKB_T_W1], 1, T, &memo[2]),
+                  nt_2 = tile_width(&t[CKB_T_W2], 1, T, &memo[3]);
         if ((rc = prefill_norm(m, delta, &t[CKB_T_LN1], &t[CKB_T_WQ], nt_q, T, st))) return rc;
         float *qkv[3];
         int ld[3];

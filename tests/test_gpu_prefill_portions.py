@@ -74,6 +74,33 @@ def test_portion_of_rows_and_tiles_matches_decode_steps(ck, before, T):
     test_portion_matches_decode_steps(ck, WIDE, before, T)
 
 
+@pytest.mark.parametrize("T", [17, 32, 33, 64])
+def test_prompt_without_the_tcgen05_kernel(ck, T):
+    """With tune gemm_tc 0 the integer kernels make all products of up to 64 tokens: how the other kernel would cut them changes no bit."""
+    cfg = dict(LLAMA, embed_dim=1024, intermediate_size=2048)
+    so.bind_model_api(ck)
+    model = so.CpuModel(cfg, seed=3)
+    ids = np.random.default_rng(T).integers(0, cfg["vocab_size"], size=T).astype(np.int32)
+    outs = []
+    handle = ck.ckb200_model_create(C.byref(so.make_cfg(cfg, batch=1)))
+    assert handle, ck.ckb200_last_error_message()
+    try:
+        so.upload_whole_model(ck, handle, model, 1)
+        for tc, slices in ((0, 0), (0, 2), (1, 0)):
+            ck.ckb200_tune_set(b"gemm_tc", tc)
+            ck.ckb200_tune_set(b"gemm_tc_slices", slices)
+            assert ck.ckb200_model_reset(handle) == 0
+            logits = np.full((1, cfg["vocab_size"]), np.nan, np.float32)
+            assert ck.ckb200_model_prefill(handle, cases.vptr(ids), T, cases.vptr(logits)) == 0, ck.ckb200_last_error_message()
+            outs.append(logits)
+    finally:
+        ck.ckb200_tune_set(b"gemm_tc", 1)
+        ck.ckb200_tune_set(b"gemm_tc_slices", 0)
+        ck.ckb200_model_free(handle)
+    assert np.array_equal(outs[0], outs[1])
+    assert cosine(outs[0], outs[2]) >= 0.9999
+
+
 @pytest.mark.parametrize("tile", [64, 128])
 @pytest.mark.parametrize("m,n,k", [(16, 40, 128), (65, 130, 384), (200, 300, 896)])
 def test_q5_0_product_is_bit_identical(ck, orc, tile, m, n, k):
