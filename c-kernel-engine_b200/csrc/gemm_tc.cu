@@ -950,8 +950,10 @@ static int tc_width(int wf, int M, int N, int nb)
     const TcPlan wide = tc_plan(wf, 128, M, N, nb);
     double best = wide.us;
     int width = 128;
-    // one wave of the widest tiles and a few behind it: as it was, narrower ones not tried
-    const bool one_wave = wide.split_nt && wide.split_nt < wide.ntiles && (wide.ntiles - wide.split_nt) * wide.mtiles <= ckb_sm_count();
+    // One wave of the widest tiles and a few behind it, more than 96 tokens: narrower tiles are not tried, the plan's times do not tell the two apart there (22016 x 2048
+    // Q4_K at 112 tokens: 29 us, with the 64-token tiles that the plan prefers 32; 9728 x 4096 at 150: 38 and 36).  Fewer tokens take the narrower tile that holds them
+    // (22016 x 4096 at 64: 35 against 28 us, at 77: 36 against 33; Q6_K 22016 x 2048 at 64: 31 against 26).
+    const bool one_wave = M > 96 && wide.split_nt && wide.split_nt < wide.ntiles && (wide.ntiles - wide.split_nt) * wide.mtiles <= ckb_sm_count();
     for (int w = 96; w >= 32 && !one_wave; w -= 32) {
         const double us = tc_plan(wf, w, M, N, nb).us;
         if (us < 0.97 * best) { best = us; width = w; }

@@ -38,6 +38,15 @@ def test_fewest_tokens_of_the_tcgen05_kernel(pkg, fmt):
     assert best(ALIGNED, ALIGNED, 32, N, K) == 0
 
 
+@pytest.mark.parametrize("wf,m,n,k,width", [
+    # one wave of 128-token tiles and a few behind it: no tokens computed for nothing where a narrower tile holds them all
+    (0, 40, 19072, 2048, 64), (0, 64, 22016, 4096, 64), (0, 77, 22016, 4096, 96), (0, 96, 23552, 2048, 96), (1, 64, 22016, 2048, 64), (1, 96, 22016, 4096, 96),
+    (0, 112, 22016, 2048, 128), (0, 128, 23552, 2048, 128), (1, 128, 23552, 8192, 128),
+    (0, 130, 9600, 2048, 128)])
+def test_width_of_token_tiles(pkg, wf, m, n, k, width):
+    assert pkg.load_lib().ckb_gemm_tc_width(wf, m, n, k) == width
+
+
 @pytest.mark.parametrize("name", ["ckb200_dev_gemm_nt_q4_k_q8_k", "ckb200_dev_gemm_nt_q6_k_planar_q8_k"])
 @pytest.mark.parametrize("m", [16, 32, 64, 65, 200])
 def test_first_call_initialises(pkg, name, m):
