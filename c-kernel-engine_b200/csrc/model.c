@@ -47,11 +47,13 @@ int ckb_model_init_shared(struct CKB200Model *m)
 }
 
 /* The driver copies to pageable memory through a buffer of its own, up to some hundred KB with the memcpy behind the whole transfer (608 KB: 57 us).  Here the chunks of a pinned
- * buffer are copied on as they land: a step with 501 KB of logits 454 -> 448 us, with 608 KB 614 -> 605, with 131 KB 473 -> 456.  From 1 MB the driver does as much and is
- * faster (1 MB 580 against 589, 4 MB 742 against 796): its way there. */
+ * buffer are copied on as they land.  Steps of a model of four small layers, us, the driver's way -> this, on two machines: 16 KB 118 -> 109, 64 KB 121 -> 114, 131 KB 128 -> 121,
+ * 262 KB 149 -> 142, 393 KB 170 -> 167; 513 to 655 KB level within 4 (whole models, timed in turn on three machines: 513 KB 1785 -> 1781, 608 KB 608 -> 602 a step; 32 tokens
+ * of a layer stack with 131 KB 15.1 -> 14.45 ms).  From 1 MB the driver does as much and is faster (1 MB 580 against 589, 4 MB 742 against 796): its way there.  Below the smallest size measured
+ * too. */
 int ckb_model_logits_out(struct CKB200Model *m, float *host, const float *dev, size_t bytes, cudaStream_t st, const char *what)
 {
-    enum { SMALLEST = 128 << 10 };
+    enum { SMALLEST = 16 << 10 };
     const size_t chunk = CKB_OUT_CHUNK;
     struct cudaPointerAttributes at;
     int pageable = 0;
