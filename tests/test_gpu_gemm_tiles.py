@@ -65,8 +65,7 @@ def wide_scales(w, n, k, mixed, seed):
 @pytest.mark.parametrize("width,m,n,k,slices", [(32, 17, 40, 256, 0), (32, 33, 300, 1792, 0), (32, 64, 1000, 4864, 0), (32, 64, 200, 2304, 3), (64, 65, 300, 1792, 0), (96, 97, 129, 768, 0),
                                                 (128, 129, 19200, 768, 0), (128, 200, 300, 4864, 3)])
 def test_gemm_tiles_are_exact_over_the_scales(ck, orc, fmt, scales, width, m, n, k, slices):
-    """Products of 6-bit weights and 8-bit scales beyond 2048 do not fit an fp16 operand: they are as exact as the others.  The 32-token form is what prompts and
-    batches of up to 64 tokens get where the integer-MMA kernels refuse (here they are switched off)."""
+    """Products of 6-bit weights and 8-bit scales beyond 2048 do not fit an fp16 operand: they are as exact as the others."""
     import torch
 
     dev = torch.device("cuda", 0)
@@ -86,7 +85,8 @@ def test_gemm_tiles_are_exact_over_the_scales(ck, orc, fmt, scales, width, m, n,
         wdev, fn = raw, ck.ckb200_dev_gemm_nt_q4_k_q8_k
     outs = []
     try:
-        for key, value in ((b"gemm_tc_nt", width if width > 32 else 0), (b"gemm_tc_slices", slices), (b"gemm_q4k_mma", 0), (b"gemm_q6k_mma", 0)):
+        for key, value in ((b"gemm_tc_nt", width if width > 32 else 0), (b"gemm_tc_small_max", 64 if width == 32 else 32), (b"gemm_tc_slices", slices), (b"gemm_q4k_mma", 0),
+                           (b"gemm_q6k_mma", 0)):
             ck.ckb200_tune_set(key, value)
         for _ in range(2):
             c = torch.full((m, n), float("nan"), device=dev)
@@ -95,7 +95,7 @@ def test_gemm_tiles_are_exact_over_the_scales(ck, orc, fmt, scales, width, m, n,
             assert ck.ckb200_synchronize() == 0
             outs.append(c.cpu().numpy())
     finally:
-        for key, value in ((b"gemm_tc_nt", 0), (b"gemm_tc_slices", 0), (b"gemm_q4k_mma", 1), (b"gemm_q6k_mma", 1)):
+        for key, value in ((b"gemm_tc_nt", 0), (b"gemm_tc_small_max", 32), (b"gemm_tc_slices", 0), (b"gemm_q4k_mma", 1), (b"gemm_q6k_mma", 1)):
             ck.ckb200_tune_set(key, value)
     # as above: integer sums are the same on both sides, K / 256 fp32 terms of three roundings each; with fp16-rounded products it would be about 1e-4
     bound = 2 * (k // 256 + 3) * 2.0 ** -24 * 8 * float(np.max(np.abs(want)))

@@ -209,20 +209,22 @@ def test_gemm_nt_matches_loop_of_gemv(ck, orc, fmt, m, n, k):
                                                (65, 129, 768, True), (300, 1000, 2048, False),
                                                (16, 128, 256, False), (32, 300, 4096, True), (40, 256, 2048, True), (33, 520, 8192, True)])
 def test_gemm_nt_q4_k_tensor_core(ck, orc, m, n, k, with_bias):
-    """M >= 16 takes the tcgen05 kernel (32-token tiles up to 64 tokens, 128-token tiles above): full tiles, ragged token
+    """The tcgen05 kernel from 16 tokens up (the integer-MMA kernel, which takes small products of up to 64, is switched off): full tiles, ragged token
     and row edges, one and many superblocks, K split over several CTAs where the grid would not fill the SMs."""
     w = synth.make_weights("q4_k", n, k, seed=m + n)
     a = synth.make_x(k, seed=m, rows=m)
     aq = cases.quantize_act(orc, "oracle_", "q4_k", a, rows=m)
     bias = np.random.default_rng(n).standard_normal(n).astype(np.float32) if with_bias else None
     want = cases.gemm_nt(orc, "oracle_", "q4_k", aq, w, bias, m, n, k)
-    got = cases.gemm_nt(ck, "", "q4_k", aq, w, bias, m, n, k)
-    assert_fp32_close(got, want, "q4_k tensor-core path")
     try:
+        ck.ckb200_tune_set(b"gemm_q4k_mma", 0)
+        got = cases.gemm_nt(ck, "", "q4_k", aq, w, bias, m, n, k)
         ck.ckb200_tune_set(b"gemm_tc", 0)
         by_rows = cases.gemm_nt(ck, "", "q4_k", aq, w, bias, m, n, k)
     finally:
+        ck.ckb200_tune_set(b"gemm_q4k_mma", 1)
         ck.ckb200_tune_set(b"gemm_tc", 1)
+    assert_fp32_close(got, want, "q4_k tensor-core path")
     assert_fp32_close(by_rows, want, "q4_k per-token path")
 
 
@@ -261,10 +263,10 @@ def test_gemm_nt_q4_k_integer_mma_small_batches(ck, orc, tma, shape, rw, m, n, k
 
 
 @pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
-@pytest.mark.parametrize("m,small_max,slices", [(24, 64, 3), (24, 0, 3), (70, 64, 4), (64, 64, 1), (64, 64, 10)])
-def test_gemm_tensor_core_split_k(ck, orc, fmt, m, small_max, slices):
-    """Both tile widths with a forced number of K slices (uneven last slice: 10 superblocks in 3 or 4 slices; one
-    superblock per slice), against the oracle; the slices are summed in a fixed order, so two runs agree bit for bit."""
+@pytest.mark.parametrize("m,width,slices", [(24, 32, 3), (40, 64, 3), (70, 96, 4), (70, 128, 4), (64, 64, 1), (64, 64, 10)])
+def test_gemm_tensor_core_split_k(ck, orc, fmt, m, width, slices):
+    """Every tile width with a forced number of K slices (uneven last slice: 10 superblocks in 3 or 4 slices; one
+    superblock per slice) and a bias, against the oracle; the slices are summed in a fixed order, so two runs agree bit for bit."""
     import torch
 
     dev = torch.device("cuda", 0)
@@ -285,9 +287,9 @@ def test_gemm_tensor_core_split_k(ck, orc, fmt, m, small_max, slices):
         wdev, fn = raw, ck.ckb200_dev_gemm_nt_q4_k_q8_k
     outs = []
     try:
-        ck.ckb200_tune_set(b"gemm_q4k_mma", 0)             # this test is about the tcgen05 kernel's K split
-        ck.ckb200_tune_set(b"gemm_tc_small_max", small_max)
-        ck.ckb200_tune_set(b"gemm_tc_slices", slices)
+        # this test is about the tcgen05 kernel's K split; up to 32 tokens its tile is 32 wide whatever gemm_tc_nt says
+        for key, value in ((b"gemm_q4k_mma", 0), (b"gemm_q6k_mma", 0), (b"gemm_tc_nt", width if width > 32 else 0), (b"gemm_tc_slices", slices)):
+            ck.ckb200_tune_set(key, value)
         for _ in range(2):
             c = torch.full((m, n), float("nan"), device=dev)
             torch.cuda.synchronize()
@@ -295,9 +297,8 @@ def test_gemm_tensor_core_split_k(ck, orc, fmt, m, small_max, slices):
             assert ck.ckb200_synchronize() == 0
             outs.append(c.cpu().numpy())
     finally:
-        ck.ckb200_tune_set(b"gemm_q4k_mma", 1)
-        ck.ckb200_tune_set(b"gemm_tc_small_max", 64)
-        ck.ckb200_tune_set(b"gemm_tc_slices", 0)
+        for key, value in ((b"gemm_q4k_mma", 1), (b"gemm_q6k_mma", 1), (b"gemm_tc_nt", 0), (b"gemm_tc_slices", 0)):
+            ck.ckb200_tune_set(key, value)
     assert_fp32_close(outs[0], want, f"{fmt} split-K gemm")
     assert np.array_equal(outs[0], outs[1])
 
@@ -367,16 +368,22 @@ def test_gemm_nt_tensor_core_tail_launch(ck, orc, fmt):
         assert with_tail == without + 2, (with_tail, without)
 
 
-@pytest.mark.parametrize("m", [64, 128])
+@pytest.mark.parametrize("m", [32, 64, 128])
 def test_gemm_nt_q4_k_tensor_core_extreme_values(ck, orc, m):
-    """Largest scales, nibbles and activations: the integer sums reach the top of the fp32-exact range (both tile widths)."""
+    """Largest scales, nibbles and activations, signs 1 to 2: integer sums of 1e7, two thirds of what an fp32 accumulator holds exactly, in tiles of 32, 64 and 128 tokens."""
     n, k = 128, 512
     w = synth.make_weights("q4_k", n, k, seed=9).reshape(n, k // 256, 144).copy()
     w[:, :, 4:16] = 0xFF          # every 6-bit scale and min = 63
     w[:, :, 16:] = 0xFF           # every nibble = 15
     a = np.where(np.arange(k) % 3 == 0, -1.0, 1.0).astype(np.float32)[None, :].repeat(m, 0) * np.linspace(0.5, 2.0, m, dtype=np.float32)[:, None]
     aq = cases.quantize_act(orc, "oracle_", "q4_k", a, rows=m)
-    got = cases.gemm_nt(ck, "", "q4_k", aq, w.reshape(-1), None, m, n, k)
+    try:
+        ck.ckb200_tune_set(b"gemm_q4k_mma", 0)
+        ck.ckb200_tune_set(b"gemm_tc_nt", m if m > 32 else 0)
+        got = cases.gemm_nt(ck, "", "q4_k", aq, w.reshape(-1), None, m, n, k)
+    finally:
+        ck.ckb200_tune_set(b"gemm_q4k_mma", 1)
+        ck.ckb200_tune_set(b"gemm_tc_nt", 0)
     want = cases.gemm_nt(orc, "oracle_", "q4_k", aq, w.reshape(-1), None, m, n, k)
     assert_fp32_close(got, want, "q4_k")
 
