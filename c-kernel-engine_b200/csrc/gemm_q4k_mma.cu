@@ -3,8 +3,8 @@
 //
 // With so few tokens the product is a weight-streaming problem: every weight byte should cross HBM once and be used for all tokens,
 // and the work per byte has to stay below what the stream allows.  The tcgen05 kernel of gemm_tc.cu expands the 4-bit weights into
-// fp16 operand tiles in shared memory, which costs the same per weight byte whether 32 or 512 tokens share it (about 1.1 TB/s of
-// weights at 32 tokens).  Here the weights are never expanded:
+// fp16 operands, which costs the same per weight byte whether 2 or 32 tokens share it (3.6 TB/s of weights).  Here the weights are never
+// expanded, up to 16 tokens the faster way (4.8 TB/s at 8; what decides from 17 on is beside ckb_gemm_q4k_mma_best):
 //
 //   * a warp owns 16 weight rows and walks its superblocks through a ring of its own in shared memory (plain 16-byte cp.async of
 //     the 144-byte blocks, two or three superblocks ahead; no other warp touches it); a lane reads the 8 nibble bytes (rows g and
@@ -609,9 +609,8 @@ static int qm4_pick(const void *A_q8, const void *B, const float *bias, float *C
 
 using namespace ckb;
 
-// Returns -1 when this kernel does not take the call (token count, alignment, switched off): the caller falls through to its other paths.
-// Whether the launcher below takes this product (a caller that wants to run several products side by side asks first: this
-// kernel needs no workspace, the tcgen05 kernel shares one).
+// Whether the launcher below takes this product (token count, alignment, not switched off); else it returns -1 and the caller goes on to its other paths.
+// A caller that runs several products side by side asks first: this kernel needs no workspace.
 extern "C" int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, int N, int K)
 {
     if (!A_q8 || !B || N <= 0 || K <= 0 || K % QK_K) return 0;
@@ -621,7 +620,8 @@ extern "C" int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, in
 }
 // Whether it is also the faster one, for a caller that has a workspace for the tcgen05 kernel.  From 17 tokens up this kernel is bound by its integer
 // instructions, 0.23 and (33 to 64 tokens) 0.39 us per million weights, and the tcgen05 kernel by the expansion of the weights, which does not grow with the
-// tokens: large products go there (57344 x 8192: 109 against 82 us at 32 tokens, 185 against 110 at 64; 8192 x 8192 at 32: 18.6 against 21).
+// tokens: large products go there (57344 x 8192: 108 against 74 us at 32 tokens, 189 against 88 at 64; 8192 x 8192: 19 against 20 at 32, 32 against 22 at 64).
+// Superblock sums of one sign beyond 2^24 are rounded there, to 3e-7 (Q6_K 7e-7) of the sum, where this kernel holds them in 32-bit integers and rounds once.
 extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
 extern "C" int ckb_gemm_q4k_mma_best(const void *A_q8, const void *B, int M, int N, int K)
 {

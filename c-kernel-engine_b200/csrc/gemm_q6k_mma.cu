@@ -393,16 +393,16 @@ static int qm6_pick(const void *A_q8, const void *B, const float *bias, float *C
 
 using namespace ckb;
 
-// B_planar: ckb200_q6_k_planar_bytes(N, K) of row-planar Q6_K weights.  Returns -1 when this kernel does not take the call.
-// Whether the launcher below takes this product (for a caller that runs several products side by side: no workspace here).
+// B_planar: ckb200_q6_k_planar_bytes(N, K) of row-planar Q6_K weights.  Whether the launcher below takes this product (else it returns -1), for a caller that
+// runs several side by side: no workspace here.
 extern "C" int ckb_gemm_q6k_mma_takes(const void *A_q8, const void *B_planar, int M, int N, int K)
 {
     if (!A_q8 || !B_planar || N <= 0 || K <= 0 || K % 1024) return 0;
     if (M < ckb_tune_get("gemm_q6k_mma_min", 2) || M > ckb_tune_get("gemm_q6k_mma_max", 64) || M > 64 || !ckb_tune_get("gemm_q6k_mma", 1)) return 0;
     return !(((uintptr_t)B_planar & 15) || ((uintptr_t)A_q8 & 15));
 }
-// Whether it is also the faster one, from 17 tokens up as for Q4_K: 0.36 and 0.68 us per million weights here (8192 x 28672: 84 against 62 us at 32 tokens, 159
-// against 90 at 64)
+// Whether it is also the faster one, from 17 tokens up as for Q4_K: 0.36 and 0.68 us per million weights here (8192 x 28672: 84 against 61 us at 32 tokens, 159
+// against 70 at 64)
 extern "C" int ckb_gemm_tc_beats(int wf, int M, int N, int K, double other_us);
 extern "C" int ckb_gemm_q6k_mma_best(const void *A_q8, const void *B_planar, int M, int N, int K)
 {

@@ -8,8 +8,11 @@
 // where S are int32 sub-block dots (gemm_kernels_q4k_q8k.c:144-173).  Here
 //     T [n,m] = sum_k (sc[n,k/32] * q4[n,k]) * q8[m,k]        256-deep f16 MMA, every operand an exact integer
 //     T2[n,m] = sum_i  mn[n,i/2]  * bsum16[m,i]               16-deep f16 MMA (one k-step)
-// are accumulated in fp32 in tensor memory (integers below 2^24 stay exact), read back with tcgen05.ld once per
+// are accumulated in fp32 in tensor memory, read back with tcgen05.ld once per
 // superblock and combined with the fp32 scales in registers: acc += d_x * (d * T - dmin * T2).
+// The accumulators hold every integer below 2^24, and no sum of a superblock is larger as long as its terms do not pile up on one side: the largest products all of one
+// sign make 3.1e7 (Q4_K) and 1.3e8 (Q6_K).  Beyond 2^24 each MMA cuts the running sum off at its last place: 3e-7 and 7e-7 from 64 bits on rows of one sign,
+// where the integer-MMA kernels, with 32-bit sums rounded once, are at 2e-7; on ordinary rows both are at 5e-8 (2-norm; 200 x 1280, 64 tokens).
 // Q6_K: A = (q6 - 32) * sc (src/kernels/gemm_kernels_q6k_q8k.c:86-116), the offset is inside the operand, so there
 // is no T2.  The product is an exact fp16 integer whenever |q6 - 32| * |sc| <= 2048, always for |sc| <= 64.  Above that fp16 holds the even integers
 // only: the operand is the nearest of them, and what it lacks (-1, 0 or 1) is an operand of its own, multiplied into the same accumulator.  Files made by a
@@ -24,7 +27,7 @@
 //    (the N operand, TMEM columns; fewer tokens are zero-padded).  Warp-specialised:
 //        warp 0       loader of activations: bulk copies of 128-deep stages (256-deep up to 64 tokens), of the bsum tile and of the block scales of each superblock
 //        warp 1       issuer: tcgen05.mma from one elected lane; tcgen05.commit frees stages and publishes accumulators
-//        warp 3       loader of weights: the raw superblocks of all 128 rows, one tiled bulk copy each (Q6_K: one per plane)
+//        warp 2       loader of weights: the raw superblocks of all 128 rows, one tiled bulk copy each (Q6_K: one per plane)
 //        warps 4-11   two expander sets, thread = row: raw bytes -> fp16 operand in 64-deep k-stages; Q4_K: also the 16-deep tile of mins and the (d, dmin) pairs
 //        warps 12-    drain: tcgen05.ld of T and T2, fp32 sums in registers
 //    Every wait is bounded; a timeout sets the device error word, the CTA drains, frees TMEM and returns.
@@ -38,13 +41,14 @@
 // register are then elements 0, 2 and 1, 3 of a 4-byte word, and the activation tiles are written in that order: k is a summation index.
 // The 512 TMEM columns at NT = 128: two T buffers (256), one T2 (128), four weight stages (128); up to 96 tokens T2 has two buffers, up to 64 eight stages fit.
 //
-// No unit of the SM is full (counters at 32 tokens: issue slots 64 %, logic 48 %, fp16 and fp32 arithmetic 35 %, tensor 19 %; fp16 arithmetic and logic issue every
-// other cycle): what a superblock takes is instructions, and how far the warps' code lies apart, for eight kinds of work share one instruction cache.  So: the
+// No unit of the SM is full (57344 x 8192 at 32 tokens / 28672 x 4096 at 333: issue slots 53 / 56 %, logic 40 / 33 %, fp16 27 / 16 %, fp32 21 / 26 %, tensor 23 / 55 %;
+// fp16 arithmetic and logic issue every other cycle): what a superblock takes is instructions, and how far the warps' code lies apart, for eight kinds of work share one instruction cache.  So: the
 // mins are made by the threads that have the header in registers (a warp of its own took 800 cycles a superblock and held up the drain), expander sets take superblocks in turn,
-// waits are four instructions, the sums of a unit leave sixteen columns at a time (see there).  Before and after these, us, with activations made into tiles:
-//   28672 x 4096 Q4_K:  77 tokens 52.4 -> 45.9, 129: 80.6 -> 60.1, 333: 115 -> 105, 512: 140 -> 125 to 129 (935 TFLOP/s)
-//   4096 x 14336 Q6_K:  129 tokens 60.4 -> 47.5, 512: 111 -> 94 to 96
-//   57344 x 8192 Q4_K:  32 tokens 111 -> 76, 64: 222 -> 88;  8192 x 28672 Q6_K: 76 -> 62, 126 -> 72;  128256 x 8192 Q6_K at 32: 213 (4.05 TB/s of weights)
+// waits are four instructions, the sums of a unit leave sixteen columns at a time (see there).  Before and after these, us, from Q8_K rows (the launch that makes tiles of
+// them included), 40 calls in a row on a cool GPU (the power cap makes long runs up to a sixth slower: 333 tokens 118 to 125, 512 tokens 153):
+//   28672 x 4096 Q4_K:  77 tokens 52.4 -> 45, 129: 80.6 -> 58, 333: 115 -> 108, 512: 140 -> 129 to 142
+//   4096 x 14336 Q6_K:  129 tokens 60.4 -> 48, 512: 111 -> 95
+//   57344 x 8192 Q4_K:  32 tokens 111 -> 74, 64: 222 -> 88;  8192 x 28672 Q6_K: 76 -> 61, 126 -> 70;  128256 x 8192 Q6_K at 32: 213 (4.05 TB/s of weights)
 // (with the operand through shared memory 28672 x 4096 at 512 tokens took 268).
 #include <cuda.h>
 #include <pthread.h>

@@ -43,7 +43,7 @@ void ckb_attn_hint_early_rows(int on);      /* attention.cu */
 int ckb_launch_gemm_tc_ws(int wf, const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, int min_tokens, void *ws,
                           size_t ws_bytes, void *stream);
 size_t ckb_gemm_tc_workspace_bytes(int M, int N, int K);
-/* integer-MMA kernel of gemm_q4k_mma.cu for up to 64 tokens (Q4_K rows, no workspace); -1 when it does not take the call */
+/* integer-MMA kernels for up to 64 tokens (Q4_K rows: gemm_q4k_mma.cu; row-planar Q6_K; no workspace); -1 when they do not take the call */
 int ckb_launch_gemm_q4k_mma(const void *A_q8, const void *B, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);
 int ckb_launch_gemm_q6k_mma(const void *A_q8, const void *B_planar, const float *bias, float *C, int ldc, int M, int N, int K, void *stream);   /* gemm_q6k_mma.cu */
 int ckb_gemm_q4k_mma_takes(const void *A_q8, const void *B, int M, int N, int K);

@@ -103,6 +103,66 @@ def test_gemm_tiles_are_exact_over_the_scales(ck, orc, fmt, scales, width, m, n,
     assert np.array_equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("fmt", ["q4_k", "q6_k"])
+@pytest.mark.parametrize("m,width", [(32, 32), (64, 64), (90, 96), (128, 128)])
+def test_sums_of_one_sign_beyond_the_exact_range(ck, orc, fmt, m, width):
+    """Sums of a superblock whose terms have one sign, beyond the 2^24 up to which an fp32 accumulator holds every integer: up to 3.0e7 (Q4_K) and 1.3e8 (Q6_K, with operands
+    that fp16 does not hold), against the same in 64 bits.  The bound: an MMA aligns its 16 products and the accumulator to the largest of them and cuts off what lies below
+    its last place (Fasi, Higham, Mikaitis, Pranesh, "Numerical behavior of NVIDIA tensor cores", 2021), so 17 addends and the result lose a unit of the running sum each at
+    most, and that is no larger than the last; 16 MMAs a superblock, 32 with those operands; then K / 256 terms of three fp32 roundings each.  Measured 3e-7 and 7e-7; the
+    integer kernels, which round such a sum once, 2e-7."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    n, nb = 200, 5
+    k = 256 * nb
+    rng = np.random.default_rng(m)
+    w = synth.make_weights(fmt, n, k, seed=9).reshape(n, nb, -1).copy()
+    if fmt == "q4_k":
+        w[:, :, 2:4] = 0                                                                # no mins: nothing cancels
+        w[:, :, 4:16] = 0xFF                                                            # scales of 63
+        w[:, :, 16:] = 0xF0 | rng.integers(13, 16, size=w[:, :, 16:].shape, dtype=np.uint8)
+        nibbles = w[:, :, 16:].reshape(n, nb, 4, 1, 32)
+        weights = 63 * np.concatenate([nibbles & 15, nibbles >> 4], 3).reshape(n, nb, 256).astype(np.int64)
+        d = w[:, :, 0:2].copy().view(np.float16)[..., 0].astype(np.float64)
+    else:
+        w[:, :, :192] = 0xFF                                                            # 63 - 32
+        w[:, :, 192:208] = rng.integers(121, 128, size=(n, nb, 16), dtype=np.uint8)     # odd products beyond 2048
+        weights = 31 * np.repeat(w[:, :, 192:208].astype(np.int64), 16, axis=2)
+        d = w[:, :, 208:210].copy().view(np.float16)[..., 0].astype(np.float64)
+    w[:, :, 1 if fmt == "q4_k" else 209] &= 0x7F                                        # d of one sign
+    d = np.abs(d)
+    x = rng.uniform(0.95, 1.0, size=(m, k)).astype(np.float32) * np.linspace(0.5, 2.0, m, dtype=np.float32)[:, None]
+    aq = cases.quantize_act(orc, "oracle_", fmt, x, rows=m)
+    rows = aq.reshape(m, nb, 292)
+    q, dx = rows[:, :, 4:260].copy().view(np.int8).astype(np.int64), rows[:, :, :4].copy().view(np.float32)[..., 0].astype(np.float64)
+    sums = np.einsum("mbk,nbk->mnb", q, weights)
+    assert np.abs(sums).max() > (1.7e7 if fmt == "q4_k" else 1.0e8)
+    want = np.einsum("mnb,nb,mb->mn", sums.astype(np.float64), d, dx)
+    raw, taq = torch.from_numpy(w.reshape(-1)).to(dev), torch.from_numpy(aq).to(dev)
+    if fmt == "q6_k":
+        ck.ckb200_q6_k_planar_bytes.restype = C.c_size_t
+        wdev = torch.empty(ck.ckb200_q6_k_planar_bytes(n, k), dtype=torch.uint8, device=dev)
+        torch.cuda.synchronize()
+        assert ck.ckb200_dev_q6_k_to_planar(C.c_void_p(wdev.data_ptr()), C.c_void_p(raw.data_ptr()), n, k, None) == 0
+        fn = ck.ckb200_dev_gemm_nt_q6_k_planar_q8_k
+    else:
+        wdev, fn = raw, ck.ckb200_dev_gemm_nt_q4_k_q8_k
+    c = torch.full((m, n), float("nan"), device=dev)
+    try:
+        for key, value in ((b"gemm_tc_nt", width if width > 32 else 0), (b"gemm_q4k_mma", 0), (b"gemm_q6k_mma", 0)):
+            ck.ckb200_tune_set(key, value)
+        torch.cuda.synchronize()
+        assert fn(C.c_void_p(taq.data_ptr()), C.c_void_p(wdev.data_ptr()), None, C.c_void_p(c.data_ptr()), m, n, k, None) == 0
+        assert ck.ckb200_synchronize() == 0
+    finally:
+        for key, value in ((b"gemm_tc_nt", 0), (b"gemm_q4k_mma", 1), (b"gemm_q6k_mma", 1)):
+            ck.ckb200_tune_set(key, value)
+    worst = float(np.max(np.abs(c.cpu().numpy().astype(np.float64) - want) / want))
+    print(f"{fmt} {m}: {worst:.3g}")
+    assert worst <= (16 if fmt == "q4_k" else 32) * 18 * 2.0 ** -23 + (nb + 3) * 2.0 ** -24
+
+
 def tiles_from_rows(rows, nt):
     """What the operand tiles of `nt` tokens hold for Q8_K rows [tokens][superblocks][292]: halves of the quants [tile][superblock][32 chunks][token][8], the 16 sums as two more
     chunks, the scales [tile][superblock][token]; tokens past the end are left out."""
